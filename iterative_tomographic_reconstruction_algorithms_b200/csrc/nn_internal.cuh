@@ -35,4 +35,10 @@ struct GemmArgs {
 
 int gemm_launch(const GemmArgs &g, cudaStream_t s);
 
+// Weight and bias gradients of a 3x3 (taps 9) or 1x1 (taps 1) convolution
+// (nn_wgrad.cu); work holds wgrad_workspace(...) bytes.
+size_t wgrad_workspace(int batch, int H, int W, int Cin, int Cout, int taps);
+int wgrad_launch(const __nv_bfloat16 *X, const __nv_bfloat16 *dY, int batch, int H, int W, int Cin, int Cout, int taps,
+                 float *dW, float *db, void *work, unsigned *status, int spins, cudaStream_t s);
+
 }  // namespace tomo_nn
