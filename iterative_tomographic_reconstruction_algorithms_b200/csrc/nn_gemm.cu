@@ -1,13 +1,8 @@
-// BF16 GEMM and 3x3 convolution on the 5th-generation tensor cores (sm_100a).
+// BF16 GEMM on the 5th-generation tensor cores (sm_100a).
 //
 //   C[M][N] = A[M][K] . B[N][K]^T  (+ bias[N], ReLU), FP32 accumulation
 //
-// A and B are K-major BF16.  A is either a dense row-major matrix or the
-// implicit im2col matrix of a 3x3, stride-1, zero-padded convolution over an
-// NHWC BF16 input (row = output pixel, k = (tap, channel) with the channel
-// fastest), so a convolution is one GEMM with M = pixels, N = output channels,
-// K = 9 * input channels, and its input gradient is the same GEMM over the
-// output gradient with the flipped, transposed weights.
+// A and B are dense, row-major (K-major) BF16 matrices.
 //
 // One CTA computes a 128 x BN tile with tcgen05.mma (cta_group::1, kind::f16,
 // M = 128, N = BN, K = 16 per instruction) into a TMEM accumulator of BN
@@ -22,9 +17,7 @@
 // up records an error in the status word, waits (with a long limit) for the
 // last committed MMAs, frees the TMEM and returns without storing.  The epilogue reads TMEM with tcgen05.ld
 // (warp w owns accumulator rows 32w..32w+31), applies bias and ReLU and
-// stores FP32 or BF16.  With ksplit > 1 the K range is split over gridDim.z
-// and each slice writes a partial FP32 tile, summed afterwards in a fixed
-// order (nn_ops.cu), so results stay deterministic.
+// stores FP32 or BF16.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -48,21 +41,8 @@ __device__ __forceinline__ void load_stage(const GemmArgs &g, int m0, int n0, in
   for (int idx = tid; idx < BM * 8; idx += kThreads) {
     const int row = idx >> 3, c = idx & 7, kc = kc0 + c;
     const int m = m0 + row;
-    const __nv_bfloat16 *src = g.A;
-    bool ok = false;
-    if (g.mode == GEMM_DENSE) {
-      ok = m < g.M && kc * 8 < g.K;
-      if (ok) src = g.A + (size_t)m * g.lda + kc * 8;
-    } else {  // implicit im2col of a 3x3, pad-1 convolution over X[batch][H][W][Cin]
-      const int cpt = g.Cin >> 3;  // chunks per tap
-      const int tap = kc / cpt, cb = kc - tap * cpt;
-      if (m < g.M && tap < 9) {
-        const int hw = g.H * g.W, b = m / hw, r = m - b * hw, y = r / g.W, x = r - y * g.W;
-        const int yy = y + tap / 3 - 1, xx = x + tap % 3 - 1;
-        ok = yy >= 0 && yy < g.H && xx >= 0 && xx < g.W;
-        if (ok) src = g.A + (((size_t)b * g.H + yy) * g.W + xx) * g.Cin + cb * 8;
-      }
-    }
+    const bool ok = m < g.M && kc * 8 < g.K;
+    const __nv_bfloat16 *src = ok ? g.A + (size_t)m * g.lda + kc * 8 : g.A;
     cp_async16(sa + c * (BM * 16) + row * 16, src, ok);
   }
   for (int idx = tid; idx < BN * 8; idx += kThreads) {
@@ -84,10 +64,7 @@ __global__ void __launch_bounds__(kThreads) gemm_tc_kernel(GemmArgs g) {
   uint32_t *tmem_slot = (uint32_t *)(bars + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  const int nkb_all = (g.K + BK - 1) / BK;
-  const int kb0 = (int)(((long long)nkb_all * blockIdx.z) / gridDim.z);
-  const int kb1 = (int)(((long long)nkb_all * (blockIdx.z + 1)) / gridDim.z);
-  const int nkb = kb1 - kb0;
+  const int nkb = (g.K + BK - 1) / BK;
 
   if (warp == 0) {  // TMEM accumulator: BN columns x 128 lanes of FP32
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)),
@@ -107,7 +84,7 @@ __global__ void __launch_bounds__(kThreads) gemm_tc_kernel(GemmArgs g) {
   bool ok = true;
   int last = -1;  // last K block whose MMAs were committed (block-uniform)
 
-  if (nkb > 0) load_stage<BN>(g, m0, n0, kb0, smem_u32(sA[0]), smem_u32(sB[0]));
+  if (nkb > 0) load_stage<BN>(g, m0, n0, 0, smem_u32(sA[0]), smem_u32(sB[0]));
   cp_async_commit();
   for (int it = 0; it < nkb; ++it) {
     const int s = it & 1;
@@ -118,7 +95,7 @@ __global__ void __launch_bounds__(kThreads) gemm_tc_kernel(GemmArgs g) {
         ok = __syncthreads_and(w) != 0;  // block-uniform
         if (!ok) break;
       }
-      load_stage<BN>(g, m0, n0, kb0 + it + 1, smem_u32(sA[s ^ 1]), smem_u32(sB[s ^ 1]));
+      load_stage<BN>(g, m0, n0, it + 1, smem_u32(sA[s ^ 1]), smem_u32(sB[s ^ 1]));
       cp_async_commit();
       cp_async_wait<1>();
     } else {
@@ -155,7 +132,6 @@ __global__ void __launch_bounds__(kThreads) gemm_tc_kernel(GemmArgs g) {
 
   if (ok) {
     const int m = m0 + warp * 32 + lane;
-    const size_t zoff = g.ksplit > 1 ? (size_t)blockIdx.z * g.M * g.ldc : 0;
 #pragma unroll 1
     for (int c0 = 0; c0 < BN; c0 += 16) {
       float v[16];
@@ -171,11 +147,9 @@ __global__ void __launch_bounds__(kThreads) gemm_tc_kernel(GemmArgs g) {
           const int n = n0 + c0 + i;
           if (n < g.N) {
             float o = v[i];
-            if (g.ksplit <= 1) {
-              if (g.bias) o += g.bias[n];
-              if (g.relu) o = fmaxf(o, 0.0f);
-            }
-            if (g.Cf) g.Cf[zoff + (size_t)m * g.ldc + n] = o;
+            if (g.bias) o += g.bias[n];
+            if (g.relu) o = fmaxf(o, 0.0f);
+            if (g.Cf) g.Cf[(size_t)m * g.ldc + n] = o;
             else g.Cb[(size_t)m * g.ldc + n] = __float2bfloat16_rn(o);
           }
         }
@@ -193,7 +167,7 @@ int launch_bn(const GemmArgs &g, cudaStream_t s) {
   if (cudaFuncSetAttribute(gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return NN_ECUDA;
-  dim3 grid((g.M + BM - 1) / BM, (g.N + BN - 1) / BN, g.ksplit > 1 ? g.ksplit : 1);
+  dim3 grid((g.M + BM - 1) / BM, (g.N + BN - 1) / BN);
   gemm_tc_kernel<BN><<<grid, kThreads, smem, s>>>(g);
   return cudaGetLastError() == cudaSuccess ? NN_OK : NN_ECUDA;
 }
@@ -202,10 +176,8 @@ int launch_bn(const GemmArgs &g, cudaStream_t s) {
 
 int gemm_launch(const GemmArgs &g, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0) return NN_EINVAL;
-  if (g.K % 8 || (g.mode == GEMM_DENSE && g.lda % 8) || g.ldb % 8) return NN_EINVAL;
-  if (g.mode == GEMM_CONV3X3 && (g.Cin % 8 || g.K != 9 * g.Cin || g.M % (g.H * g.W))) return NN_EINVAL;
+  if (g.K % 8 || g.lda % 8 || g.ldb % 8) return NN_EINVAL;
   if ((g.Cf == nullptr) == (g.Cb == nullptr)) return NN_EINVAL;
-  if (g.ksplit > 1 && !g.Cf) return NN_EINVAL;
   // 16-byte cp.async sources: base pointers must be 16-byte aligned
   if (((uintptr_t)g.A | (uintptr_t)g.B) & 15) return NN_EINVAL;
   if (g.N <= 32) return launch_bn<32>(g, s);

@@ -1,6 +1,7 @@
 // libtomo_nn: the C ABI of include/tomo_nn.h and the small kernels around the
-// tensor-core ones (nn_gemm.cu, nn_wgrad.cu): weight preparation, ReLU
+// tensor-core ones (nn_gemm.cu, nn_conv.cu, nn_wgrad.cu): weight preparation, ReLU
 // backward and Adam.
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -61,6 +62,38 @@ __global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g, 
 }
 
 }  // namespace
+
+int make_tensor_map(void *map, const void *base, int rank, const unsigned long long *dim,
+                    const unsigned long long *stride, const unsigned *box, int rb) {
+  using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                              const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess) fn = nullptr;
+    return (Encode)fn;
+  }();
+  if (!encode) return NN_ECUDA;
+  cuuint64_t d[5], s[4];
+  cuuint32_t bx[5], es[5];
+  for (int i = 0; i < rank; ++i) {
+    d[i] = dim[i];
+    bx[i] = box[i];
+    es[i] = 1;
+    if (i + 1 < rank) s[i] = stride[i];
+  }
+  const CUtensorMapSwizzle sw = rb == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                                : rb == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                : rb == 32 ? CU_TENSOR_MAP_SWIZZLE_32B
+                                           : CU_TENSOR_MAP_SWIZZLE_NONE;
+  return encode((CUtensorMap *)map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void *>(base), d, s, bx, es,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+             ? NN_OK
+             : NN_ECUDA;
+}
+
 }  // namespace tomo_nn
 
 using namespace tomo_nn;
@@ -70,7 +103,6 @@ extern "C" {
 int tomo_nn_gemm(const void *A, int lda, const void *B, int ldb, int M, int N, int K, float *Cf, void *Cb,
                  int ldc, const float *bias, int relu, void *stream) {
   GemmArgs g;
-  g.mode = GEMM_DENSE;
   g.A = (const __nv_bfloat16 *)A;
   g.lda = lda;
   g.B = (const __nv_bfloat16 *)B;
@@ -90,26 +122,8 @@ int tomo_nn_gemm(const void *A, int lda, const void *B, int ldb, int M, int N, i
 
 int tomo_nn_conv3x3(const void *X, int batch, int H, int W, int Cin, const void *Wt, int Cout, float *Yf,
                     void *Yb, const float *bias, int relu, void *stream) {
-  if (batch < 1 || H < 1 || W < 1) return NN_EINVAL;
-  GemmArgs g;
-  g.mode = GEMM_CONV3X3;
-  g.A = (const __nv_bfloat16 *)X;
-  g.B = (const __nv_bfloat16 *)Wt;
-  g.ldb = 9 * Cin;
-  g.M = batch * H * W;
-  g.N = Cout;
-  g.K = 9 * Cin;
-  g.H = H;
-  g.W = W;
-  g.Cin = Cin;
-  g.Cf = Yf;
-  g.Cb = (__nv_bfloat16 *)Yb;
-  g.ldc = Cout;
-  g.bias = bias;
-  g.relu = relu;
-  g.status = status_ptr();
-  g.spins = g_wait_spins.load();
-  return gemm_launch(g, (cudaStream_t)stream);
+  return conv_launch((const __nv_bfloat16 *)X, batch, H, W, Cin, (const __nv_bfloat16 *)Wt, Cout, Yf, (__nv_bfloat16 *)Yb,
+                     bias, relu, status_ptr(), g_wait_spins.load(), (cudaStream_t)stream);
 }
 
 size_t tomo_nn_wgrad_workspace(int batch, int H, int W, int Cin, int Cout, int taps) {

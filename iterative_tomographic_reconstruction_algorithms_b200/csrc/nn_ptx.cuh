@@ -2,6 +2,7 @@
 // cp.async, mbarriers with bounded waits, tcgen05 descriptors, MMA, TMEM loads.
 #pragma once
 
+#include <cuda.h>
 #include <stdint.h>
 
 #include "nn_internal.cuh"
@@ -69,6 +70,17 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
+// The same for rows of rb = 128, 64 or 32 bytes stored with the TMA swizzle of
+// that width, or of 16 bytes without one.  K-major: sbo is the stride between
+// 8-row groups; a K step within the row adds its bytes to the address.
+// MN-major: lbo is the stride between blocks of rb / 2 channels, sbo between
+// 8-row K groups (rb = 16: the reverse, as above).  The swizzle is a function
+// of the shared-memory address, so a descriptor may start at any row.
+__device__ __forceinline__ uint64_t smem_desc_rb(uint32_t addr, uint32_t lbo, uint32_t sbo, int rb) {
+  const uint64_t layout = rb == 128 ? 2 : rb == 64 ? 4 : rb == 32 ? 6 : 0;
+  return smem_desc(addr, lbo, sbo) | (layout << 61);
+}
+
 // Instruction descriptor: D F32, A and B BF16, both K-major, M = 128, N = n.
 __host__ __device__ constexpr uint32_t instr_desc(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -106,6 +118,116 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
+
+// KS consecutive K steps of one accumulator for a whole converged warp, issued
+// by one elected lane: descriptor a advances by sa, b by sb (bytes / 16) a
+// step; `more` accumulates onto what is there from the first step.  Issuing is
+// what bounds small MMAs, so the loop around it should be uniform (a warp index
+// the compiler can see is one: warp_index) and free of divisions; issued from a
+// branch on the lane, with a division per step, an MMA took 300 cycles, here 60.
+template <int KS>
+__device__ __forceinline__ void mma_warp(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t more, uint32_t sa = 2,
+                                         uint32_t sb = 2) {
+  if constexpr (KS == 4)
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 a1, a2, a3, b1, b2, b3, s, t;\n\t"
+        "cvt.u64.u32 s, %5;\n\tcvt.u64.u32 t, %6;\n\t"
+        "add.s64 a1, %1, s;\n\tadd.s64 a2, a1, s;\n\tadd.s64 a3, a2, s;\n\t"
+        "add.s64 b1, %2, t;\n\tadd.s64 b2, b1, t;\n\tadd.s64 b3, b2, t;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, 1;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, 1;\n\t}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(more), "r"(sa), "r"(sb)
+        : "memory");
+  else if constexpr (KS == 2)
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 a1, b1, s, t;\n\t"
+        "cvt.u64.u32 s, %5;\n\tcvt.u64.u32 t, %6;\n\t"
+        "add.s64 a1, %1, s;\n\tadd.s64 b1, %2, t;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, 1;\n\t}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(more), "r"(sa), "r"(sb)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(more)
+        : "memory");
+}
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
+__device__ __forceinline__ void mma_commit_warp(uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar)
+      : "memory");
+}
+
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tma_load3(uint32_t dst, const CUtensorMap *m, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(dst),
+      "l"(m), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load4(uint32_t dst, const CUtensorMap *m, int x, int y, int z, int w, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(dst),
+      "l"(m), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
+      : "memory");
+}
+
+// A role's wait: like mbar_wait, and false too once another role gave up.
+__device__ __forceinline__ bool role_wait(const uint64_t *bar, uint32_t parity, int spins, const volatile int *gave_up) {
+  const uint32_t b = smem_u32(bar);
+  for (int i = 0; i < spins; ++i) {
+    if (mbar_try_wait(b, parity)) return true;
+    if ((i & 255) == 255 && *gave_up) return false;
+  }
+  return false;
+}
+
+// The same for a converged warp: one answer for all its lanes.
+__device__ __forceinline__ bool warp_wait(const uint64_t *bar, uint32_t parity, int spins, const volatile int *gave_up) {
+  return __all_sync(0xffffffffu, role_wait(bar, parity, spins, gave_up));
+}
+
+// x / d for 0 <= x < 2^31 as umulhi(x, m) >> s (m = ceil(2^(31 + l) / d), 2^l >= d).
+struct FastDiv {
+  unsigned m;
+  int s, d;
+};
+__device__ __forceinline__ int fast_div(int x, const FastDiv &f) {
+  return f.d == 1 ? x : (int)(__umulhi((unsigned)x, f.m) >> f.s);
+}
+inline FastDiv make_div(int d) {
+  int l = 0;
+  while ((1ll << l) < d) ++l;
+  return {(unsigned)(((1ull << (31 + l)) + d - 1) / d), l - 1, d};
+}
+
+// Place in a ring of n stages and the parity of its current round.  (A
+// division of the running count by n costs the issuing warp more than an MMA.)
+struct Ring {
+  int s = 0;
+  uint32_t ph = 0;
+  __device__ __forceinline__ void next(int n) {
+    if (++s == n) {
+      s = 0;
+      ph ^= 1u;
+    }
+  }
+};
 
 }  // namespace
 }  // namespace tomo_nn

@@ -48,15 +48,6 @@ constexpr int kSms = 148;
 constexpr int kSmemMax = 224 * 1024;
 constexpr int kDrainSpins = 1 << 22;
 
-// x / d for 0 <= x < 2^31 as umulhi(x, m) >> s (m = ceil(2^(31 + l) / d), 2^l >= d).
-struct FastDiv {
-  unsigned m;
-  int s, d;
-};
-__device__ __forceinline__ int fast_div(int x, const FastDiv &f) {
-  return f.d == 1 ? x : (int)(__umulhi((unsigned)x, f.m) >> f.s);
-}
-
 struct WgradArgs {
   const __nv_bfloat16 *X, *dY;
   float *part;  // [S][Cout][taps][Cin]
@@ -318,12 +309,6 @@ __global__ void __launch_bounds__(128) colsum_final_kernel(const double *__restr
 }
 
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
-
-FastDiv make_div(int d) {
-  int l = 0;
-  while ((1ll << l) < d) ++l;
-  return {(unsigned)(((1ull << (31 + l)) + d - 1) / d), l - 1, d};
-}
 
 // Ranges of 64-pixel blocks whose partial sums are added afterwards: a
 // function of the layer's shape (128 x 256 tiles of its weight matrix), at
