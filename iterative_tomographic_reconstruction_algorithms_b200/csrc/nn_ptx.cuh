@@ -1,5 +1,5 @@
-// PTX wrappers shared by the tensor-core kernels (nn_gemm.cu, nn_wgrad.cu):
-// cp.async, mbarriers with bounded waits, tcgen05 descriptors, MMA, TMEM loads.
+// PTX wrappers shared by the tensor-core kernels (nn_gemm.cu, nn_conv.cu, nn_wgrad.cu):
+// cp.async, TMA, mbarriers with bounded waits, tcgen05 descriptors, MMA, TMEM loads.
 #pragma once
 
 #include <cuda.h>

@@ -5,30 +5,35 @@
 // one GEMM per tap with M = output channels, N = input channels and K =
 // pixels, read straight from the NHWC tensors.
 //
-// Both operands are MN-major: a 16-byte unit holds 8 channels of one pixel,
-// which is how NHWC memory lies, so no transposed copy is made.  A stage holds
-// 64 pixels (in image order) of the output gradient as [8-channel chunk][pixel]
-// [16 bytes] and what their taps need of the input.  Where W is a multiple of
-// 8 that is, per input row of the taps, a strip of 8 groups of 10 pixels (8
-// and one on each side): a tap is then an offset of (row, dx) into the strip
-// and the two K groups of an MMA lie 10 pixels apart, so one staged strip
-// serves the three taps of its row.  Otherwise (W not a multiple of 8: a
-// group would run over the end of a row; 1x1) the stage holds the shifted 64
-// pixels of every tap.  Each tap accumulates in TMEM columns of its own.
+// Both operands are MN-major: a pixel's channels are a row, which is how NHWC
+// memory lies, so no transposed copy is made.  A stage holds 64 pixels (in
+// image order) of the output gradient and what their taps need of the input.
 //
-// Bound: the copies from L2 (with 32 channels 3.75 x the input and 3 x the
-// gradient instead of 9 x the input).  Eight producer warps issue zero-filled
-// 16-byte cp.async copies several stages ahead of one MMA thread.  The kernel
-// this one replaces wrote the im2col matrix (9 copies of X, transposed) to
-// memory and read it back: at 4 x 192^2, 128 -> 128 channels the whole
-// gradient took 1.28 ms, now 0.17 ms; at 4 x 768^2, 32 -> 32, 6.19, now 0.69.
+// wgrad_tma_kernel (1x1, and 3x3 where W is a multiple of 8): TMA boxes of
+// 128-byte (64, 32, 16) swizzled rows; of the input, per tap row dy and block
+// of 64 (32, 16, 8) channels, strips of 64 (16, 8) pixels and one on each side,
+// whose fill is the zero padding.  The taps dx = 0, 1, 2 of a row are one pixel
+// apart, so ONE MMA takes all three: its N blocks, a descriptor's block stride
+// apart, are the same block of channels one row of memory further on.  That
+// matters with few channels, where an MMA takes its minimum of 50 cycles: at
+// 32 -> 32 channels 64 pixels take 12 MMAs of N = 96, not 36 of N = 32.
 //
-// Work split: a CTA owns up to 128 output channels, a block of input channels
-// and a group of taps (TMEM holds 512 FP32 columns = taps x channels), and one
-// of S contiguous ranges of 64-pixel blocks; it writes its partial sums once
-// and wgrad_reduce_kernel adds the S partials in order.  S depends on the
-// layer's shape alone, and pixels are added 16 at a time in image order, so
-// the result depends neither on the grouping of the taps nor on scheduling.
+// wgrad_gather_kernel (3x3, W not a multiple of 8: the pixels of a group would
+// run over the end of a row): eight producer warps stage the shifted 64 pixels
+// of every tap by zero-filled 16-byte cp.async.  TMA moves 50-60 bytes per
+// clock and SM in 128-byte rows, those copies 15.
+//
+// Measured at 4 x 192^2, 128 -> 128 channels: 1.28 ms when the im2col matrix
+// was written out, 0.17 with 16-byte copies, now 0.097; 4 x 768^2, 32 -> 32:
+// 6.19, 0.69, 0.42; 4 x 192^2, 384 -> 128: 3.42, 0.86, 0.20.
+//
+// Work split: a CTA owns up to 128 output channels, some of the (tap row,
+// channel block) units that fit its 512 TMEM columns, and one of S contiguous
+// ranges of 64-pixel blocks; it writes its partial sums once and
+// wgrad_reduce_kernel adds the S partials in order.  S depends on the layer's
+// shape alone, and pixels are added 16 at a time in image order, so the result
+// depends neither on the units' grouping nor on scheduling.
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -45,7 +50,7 @@ constexpr int kProd = 256;         // producer threads (warps 0-7); warps 0-3 al
 constexpr int kWgThreads = kProd + 32;
 constexpr int kMaxStages = 8;
 constexpr int kSms = 148;
-constexpr int kSmemMax = 224 * 1024;
+constexpr int kSmemMax = 225 * 1024;
 constexpr int kDrainSpins = 1 << 22;
 
 struct WgradArgs {
@@ -56,19 +61,172 @@ struct WgradArgs {
   int H, W, Cin, Cout, ldY, taps;  // ldY: channels per pixel of dY in memory (Cout rounded up to 8)
   int P, nkb;                      // pixels, 64-pixel blocks
   FastDiv fhw, fw;
-  int S, G, ntap, NB, Nb, Mb;  // splits; tap groups and taps per group; input-channel blocks and their width; output rows staged
-  int mrows;                   // rows of an MMA: 64 up to 64 output channels, else 128
-  int strip, sxc, syc, stage_bytes, tail_bytes, nst, cols;
+  int S, mrows;                    // splits; rows of an MMA: 64 up to 64 output channels, else 128
+  int stage_bytes, tail_bytes, nst, cols;
+  // wgrad_tma_kernel
+  int U, G, upg;                   // units, groups of them, units of a group
+  int rb, chb, nblk, ndx, nmma;    // bytes of X's rows, their channels, channel blocks; taps of an MMA and its N
+  int gw, strip_bytes, unit_bytes; // pixels of a strip, bytes of a strip and of a unit's strips
+  int rby, chby, nby, yblk;        // the same of dY: rows, channels, blocks of a CTA's output channels, bytes of one
+  // wgrad_gather_kernel
+  int ntap, NB, Nb, Mb, sxc, syc;  // taps per group; input-channel blocks and their width; output rows staged
 };
 
+// The partial sums of 16 accumulator columns: row co, `n` of them from column
+// element e of part's [taps][Cin].
+__device__ __forceinline__ void store_part(const WgradArgs &g, int co, size_t e, const float (&v)[16], int n) {
+  if (co >= g.Cout) return;
+  float4 *o = (float4 *)(g.part + ((size_t)blockIdx.y * g.Cout + co) * g.taps * g.Cin + e);
+  o[0] = make_float4(v[0], v[1], v[2], v[3]);
+  o[1] = make_float4(v[4], v[5], v[6], v[7]);
+  if (n > 8) {
+    o[2] = make_float4(v[8], v[9], v[10], v[11]);
+    o[3] = make_float4(v[12], v[13], v[14], v[15]);
+  }
+}
+
+__global__ void __launch_bounds__(192) wgrad_tma_kernel(WgradArgs g, const __grid_constant__ CUtensorMap mx,
+                                                        const __grid_constant__ CUtensorMap my) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ uint64_t full[kMaxStages], empty[kMaxStages], done;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int gave_up;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
+  const int tg = blockIdx.x % g.G, m0 = (blockIdx.x / g.G) * 128;
+  const int u0 = tg * g.upg, nu = min(g.upg, g.U - u0);
+  const int t0 = (int)((long long)g.nkb * blockIdx.y / g.S), t1 = (int)((long long)g.nkb * (blockIdx.y + 1) / g.S);
+  const int nby = min(g.nby, (g.ldY - m0 + g.chby - 1) / g.chby);
+  const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u;  // swizzle period
+
+  if (warp == 5) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
+                 "r"(g.cols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+  }
+  if (tid == 0) {
+    for (int s = 0; s < g.nst; ++s) {
+      mbar_init(smem_u32(&full[s]), 1);
+      mbar_init(smem_u32(&empty[s]), 1);
+    }
+    mbar_init(smem_u32(&done), 1);
+    gave_up = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  const uint32_t y_off = g.upg * g.unit_bytes;
+  bool ok = true;
+
+  if (warp == 4) {  // loads
+    if (lane == 0) {
+      const int halo = g.ndx >> 1, hw = g.H * g.W, nstrip = kKP / g.gw;
+      const uint32_t bytes = nu * nstrip * (g.gw + 2 * halo) * g.rb + nby * kKP * g.rby;
+      Ring r;
+      int it = 0;
+      for (int t = t0; t < t1; ++t, ++it, r.next(g.nst)) {
+        if (it >= g.nst) ok = role_wait(&empty[r.s], r.ph ^ 1u, g.spins, &gave_up);
+        if (!ok) break;
+        const uint32_t bar = smem_u32(&full[r.s]), st = base + r.s * g.stage_bytes;
+        mbar_expect(bar, bytes);
+        for (int q = 0; q < nstrip; ++q) {
+          const int p = t * kKP + q * g.gw;
+          int b = 0, y = 0, x = p;
+          if (halo) {  // pixels from P on lie in images that do not exist: zero
+            b = fast_div(p, g.fhw);
+            const int rem = p - b * hw;
+            y = fast_div(rem, g.fw);
+            x = rem - y * g.W;
+          }
+          int dy = u0 / g.nblk, c = u0 - dy * g.nblk;
+          for (int u = 0; u < nu; ++u) {
+            tma_load4(st + u * g.unit_bytes + q * g.strip_bytes, &mx, c * g.chb, x - halo, y + dy - halo, b, bar);
+            if (++c == g.nblk) c = 0, ++dy;
+          }
+        }
+        for (int c = 0; c < nby; ++c) tma_load3(st + y_off + c * g.yblk, &my, m0 + c * g.chby, t * kKP, 0, bar);
+      }
+      // copies still in flight (after a wait that gave up nobody else waits for them)
+      for (int k = max(0, it - g.nst); k < it; ++k)
+        if (!mbar_wait(smem_u32(&full[k % g.nst]), (k / g.nst) & 1, kDrainSpins)) ok = false;
+    }
+  } else if (warp == 5) {  // MMAs
+    const uint32_t idesc = instr_desc_mn(g.nmma, g.mrows);
+    // K groups of 8 pixels follow one another, or, in strips of 8, lie a strip
+    // apart; N blocks (taps) one pixel apart
+    const uint32_t kg = g.gw == 8 ? g.strip_bytes : 8 * g.rb;
+    const uint64_t dx0 = g.rb == 16 ? smem_desc_rb(0, kg, 16, 16) : smem_desc_rb(0, g.rb, kg, g.rb);
+    const uint64_t dy0 = g.rby == 16 ? smem_desc_rb(0, 128, g.yblk, 16) : smem_desc_rb(0, g.yblk, 8 * g.rby, g.rby);
+    const uint32_t sa = g.rby, sb = g.gw == 64 ? g.rb : g.gw == 16 ? g.strip_bytes >> 4 : g.strip_bytes >> 3;  // 16 pixels on
+    Ring r;
+    bool issued = false;
+    uint32_t more = 0;
+    for (int t = t0; t < t1; ++t, r.next(g.nst)) {
+      ok = warp_wait(&full[r.s], r.ph, g.spins, &gave_up);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t st = base + r.s * g.stage_bytes;
+      const uint64_t da = dy0 + ((st + y_off) >> 4);
+      uint64_t db = dx0 + (st >> 4);
+      uint32_t d = tmem;
+      for (int u = 0; u < nu; ++u) {
+        mma_warp<4>(d, da, db, idesc, more, sa, sb);
+        d += g.nmma;
+        db += g.unit_bytes >> 4;
+      }
+      mma_commit_warp(smem_u32(&empty[r.s]));
+      issued = true;
+      more = 1;
+    }
+    // every MMA issued so far, also on the way out of a wait that gave up
+    if (issued) {
+      mma_commit_warp(smem_u32(&done));
+      if (!mbar_wait(smem_u32(&done), 0, kDrainSpins)) ok = false;
+    }
+  }
+  if (!ok) atomicOr(&gave_up, 1);
+  __syncwarp();
+  __syncthreads();
+  tc_fence_after();
+  if (gave_up && tid == 0 && g.status) atomicOr(g.status, 1);
+  if (!gave_up && warp < 4) {
+    // 64-row accumulators lie in lanes 0-15 of each warp's 32
+    const int co = g.mrows == 64 ? (lane < 16 ? m0 + warp * 16 + lane : g.Cout) : m0 + warp * 32 + lane;
+    for (int u = 0; u < nu; ++u) {
+      const int dy = (u0 + u) / g.nblk, c = (u0 + u) % g.nblk;
+      for (int k = 0; k < g.ndx * g.chb; k += 16) {  // columns: dx, channel of the block
+        float v[16];
+        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(u * g.nmma + k), v);
+        if (t1 <= t0)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = 0.0f;
+        if (g.chb >= 16) {
+          store_part(g, co, (size_t)(dy * 3 + k / g.chb) * g.Cin + c * g.chb + k % g.chb, v, 16);
+        } else {  // 8 channels: two taps
+          float w[16];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) w[i] = v[i + 8];
+          store_part(g, co, (size_t)(dy * 3 + k / 8) * g.Cin + c * 8, v, 8);
+          if (k + 8 < g.ndx * 8) store_part(g, co, (size_t)(dy * 3 + k / 8 + 1) * g.Cin + c * 8, w, 8);
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 5)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(g.cols));
+}
+
 // LAG: copy groups a producer keeps in flight behind the one it just issued.
-template <int LAG, bool STRIP>
-__global__ void __launch_bounds__(kWgThreads) wgrad_tc_kernel(WgradArgs g) {
+template <int LAG>
+__global__ void __launch_bounds__(kWgThreads) wgrad_gather_kernel(WgradArgs g) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint64_t full[kMaxStages], empty[kMaxStages], done;
   __shared__ uint32_t tmem_slot;
   __shared__ int gave_up;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   // unit: (output-channel block, input-channel block, tap group)
   int u = blockIdx.x;
   const int tg = u % g.G;
@@ -78,7 +236,6 @@ __global__ void __launch_bounds__(kWgThreads) wgrad_tc_kernel(WgradArgs g) {
   const int t0 = (int)((long long)g.nkb * blockIdx.y / g.S), t1 = (int)((long long)g.nkb * (blockIdx.y + 1) / g.S);
   const int ncx = min(g.Nb, g.Cin - n0) >> 3;                 // 8-channel chunks of X staged
   const int ncy = (min(128, g.Cout - m0) + 7) >> 3;           // and of dY
-  const int r0 = tap0 / 3, nrow = (tap0 + ntap - 1) / 3 - r0 + 1;  // STRIP: input rows of the taps
 
   if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
@@ -99,54 +256,33 @@ __global__ void __launch_bounds__(kWgThreads) wgrad_tc_kernel(WgradArgs g) {
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   const uint32_t base = smem_u32(smem);
+  bool ok = true;
 
-  if (warp < 8) {  // producers
-    // Warp w stages pixels 8w .. 8w+7 of the block: of X, per input row (STRIP)
-    // their strip of 10, else per tap the 8 shifted pixels; consecutive lanes
-    // take consecutive chunks.
-    constexpr int kGrp = STRIP ? 10 : 8;
-    const int nx = (STRIP ? nrow : ntap) * kGrp * ncx, ny = 8 * ncy;
+  if (warp < 8) {  // producers: warp w stages pixels 8w .. 8w+7 of the block, consecutive lanes consecutive chunks
+    const int nx = ntap * 8 * ncx, ny = 8 * ncy;
     // a lane's copies are 32 apart: (position, chunk) advances by (q, r)
     const int qx = 32 / ncx, rx = 32 % ncx, px0 = lane / ncx, cx0 = lane % ncx;
     const int qy = 32 / ncy, ry = 32 % ncy, py0 = lane / ncy, cy0 = lane % ncy;
     const int hw = g.H * g.W;
+    Ring r, a;        // the stage being filled, the oldest not yet announced
     int pending = 0;  // stages issued and not yet announced
-    bool ok = true;
-    for (int t = t0; t < t1 && ok; ++t) {
-      const int it = t - t0, s = it % g.nst;
-      if (it >= g.nst) ok = mbar_wait(smem_u32(&empty[s]), ((it / g.nst) - 1) & 1, g.spins);
+    for (int t = t0; t < t1; ++t, r.next(g.nst)) {
+      if (t - t0 >= g.nst) ok = role_wait(&empty[r.s], r.ph ^ 1u, g.spins, &gave_up);
       if (!ok) break;
-      const uint32_t sx = base + s * g.stage_bytes + warp * kGrp * 16;
-      const uint32_t sy = base + s * g.stage_bytes + (g.Nb >> 3) * g.sxc + warp * 128;
+      const uint32_t sx = base + r.s * g.stage_bytes + warp * 128;
+      const uint32_t sy = sx + (g.Nb >> 3) * g.sxc;
       const int p = t * kKP + warp * 8;
-      if (STRIP) {  // the 8 pixels lie in one image row
-        const int b = fast_div(p, g.fhw), q = p - b * hw, yc = fast_div(q, g.fw), xc = q - yc * g.W - 1;
-        const int ya = yc + r0 - 1;
-        const bool live = p < g.P;
-        // strip position 0 of row ya (may lie outside the image: never read then)
-        const __nv_bfloat16 *Xb = g.X + ((long long)b * hw + (long long)ya * g.W + xc) * g.Cin + n0;
-#pragma unroll 4
-        for (int i = lane, pos = px0, c = cx0; i < nx; i += 32) {
-          const int r = pos / 10, o = pos - 10 * r;
-          const bool in = live && (unsigned)(ya + r) < (unsigned)g.H && (unsigned)(xc + o) < (unsigned)g.W;
-          cp_async16(sx + c * g.sxc + (r * 80 + o) * 16, in ? Xb + (r * g.W + o) * g.Cin + c * 8 : g.X, in);
-          pos += qx;
-          c += rx;
-          if (c >= ncx) c -= ncx, ++pos;
-        }
-      } else {
 #pragma unroll 2
-        for (int i = lane, pos = px0, c = cx0; i < nx; i += 32) {
-          const int j = pos >> 3, o = pos & 7, tap = g.taps == 9 ? tap0 + j : 4;
-          const int b = fast_div(p + o, g.fhw), q = p + o - b * hw, yc = fast_div(q, g.fw);
-          const int y = yc + tap / 3 - 1, x = q - yc * g.W + tap % 3 - 1;
-          const bool in = p + o < g.P && (unsigned)y < (unsigned)g.H && (unsigned)x < (unsigned)g.W;
-          const __nv_bfloat16 *src = in ? g.X + (size_t)(b * hw + y * g.W + x) * g.Cin + n0 + c * 8 : g.X;
-          cp_async16(sx + c * g.sxc + (j * kKP + o) * 16, src, in);
-          pos += qx;
-          c += rx;
-          if (c >= ncx) c -= ncx, ++pos;
-        }
+      for (int i = lane, pos = px0, c = cx0; i < nx; i += 32) {
+        const int j = pos >> 3, o = pos & 7, tap = tap0 + j;
+        const int b = fast_div(p + o, g.fhw), q = p + o - b * hw, yc = fast_div(q, g.fw);
+        const int y = yc + tap / 3 - 1, x = q - yc * g.W + tap % 3 - 1;
+        const bool in = p + o < g.P && (unsigned)y < (unsigned)g.H && (unsigned)x < (unsigned)g.W;
+        const __nv_bfloat16 *src = in ? g.X + (size_t)(b * hw + y * g.W + x) * g.Cin + n0 + c * 8 : g.X;
+        cp_async16(sx + c * g.sxc + (j * kKP + o) * 16, src, in);
+        pos += qx;
+        c += rx;
+        if (c >= ncx) c -= ncx, ++pos;
       }
       const __nv_bfloat16 *Yb = g.dY + (size_t)p * g.ldY + m0;
 #pragma unroll 2
@@ -161,58 +297,43 @@ __global__ void __launch_bounds__(kWgThreads) wgrad_tc_kernel(WgradArgs g) {
       if (++pending > LAG) {  // the oldest pending stage has landed
         cp_async_wait<LAG>();
         fence_proxy_async();
-        mbar_arrive(smem_u32(&full[(it - LAG) % g.nst]));
+        mbar_arrive(smem_u32(&full[a.s]));
+        a.next(g.nst);
         --pending;
       }
     }
     cp_async_wait<0>();
     fence_proxy_async();
-    if (ok)
-      for (int it = t1 - t0 - pending; it < t1 - t0; ++it) mbar_arrive(smem_u32(&full[it % g.nst]));
-    else
-      atomicOr(&gave_up, 1);
-  } else if (lane == 0) {  // the MMA thread
+    for (; ok && pending > 0; --pending, a.next(g.nst)) mbar_arrive(smem_u32(&full[a.s]));
+  } else {  // MMAs
     const uint32_t idesc = instr_desc_mn(g.Nb, g.mrows);
-    constexpr uint32_t kgroup = STRIP ? 160 : 128;  // bytes between groups of 8 pixels
     // descriptors of stage 0; an address advances by its bytes / 16
-    const uint64_t da0 = smem_desc(base + (g.Nb >> 3) * g.sxc, 128, g.syc), db0 = smem_desc(base, kgroup, g.sxc);
-    bool ok = true;
-    int last = -1;
-    for (int t = t0; t < t1; ++t) {
-      const int it = t - t0, s = it % g.nst;
-      ok = mbar_wait(smem_u32(&full[s]), (it / g.nst) & 1, g.spins);
+    const uint64_t da0 = smem_desc(base + (g.Nb >> 3) * g.sxc, 128, g.syc), db0 = smem_desc(base, 128, g.sxc);
+    Ring r;
+    bool issued = false;
+    for (int t = t0; t < t1; ++t, r.next(g.nst)) {
+      ok = warp_wait(&full[r.s], r.ph, g.spins, &gave_up);
       if (!ok) break;
       tc_fence_after();
-      const uint64_t da = da0 + (uint32_t)(s * g.stage_bytes >> 4), db = db0 + (uint32_t)(s * g.stage_bytes >> 4);
-      const uint32_t more = it > 0;
-      int r = 0, dx = tap0 - 3 * r0;
-      for (int j = 0; j < ntap; ++j) {
-        const uint64_t dbj = db + (uint32_t)(STRIP ? r * 80 + dx : j * kKP);
-        const uint32_t d = tmem + j * g.Nb;
-        mma_bf16(d, da, dbj, idesc, more);
-#pragma unroll
-        for (int k = 1; k < kKP / 16; ++k) mma_bf16(d, da + k * 16, dbj + k * (2 * kgroup / 16), idesc, 1u);
-        if (++dx == 3) dx = 0, ++r;
-      }
-      mma_commit(smem_u32(&empty[s]));
-      last = it;
+      const uint32_t st = (uint32_t)(r.s * g.stage_bytes) >> 4;
+      for (int j = 0; j < ntap; ++j)
+        mma_warp<4>(tmem + j * g.Nb, da0 + st, db0 + (st + j * kKP), idesc, t > t0, 16, 16);
+      mma_commit_warp(smem_u32(&empty[r.s]));
+      issued = true;
     }
-    if (!ok) atomicOr(&gave_up, 1);
     // every MMA issued so far, also on the way out of a wait that gave up
-    if (last >= 0) {
-      mma_commit(smem_u32(&done));
-      if (!mbar_wait(smem_u32(&done), 0, kDrainSpins)) atomicOr(&gave_up, 1);
+    if (issued) {
+      mma_commit_warp(smem_u32(&done));
+      if (!mbar_wait(smem_u32(&done), 0, kDrainSpins)) ok = false;
     }
   }
+  if (!ok) atomicOr(&gave_up, 1);
   __syncwarp();
   __syncthreads();
   tc_fence_after();
-  const bool ok = gave_up == 0;
-  if (!ok && tid == 0 && g.status) atomicOr(g.status, 1);
-  if (ok && warp < 4) {
-    // 64-row accumulators lie in lanes 0-15 of each warp's 32
+  if (gave_up && tid == 0 && g.status) atomicOr(g.status, 1);
+  if (!gave_up && warp < 4) {
     const int co = g.mrows == 64 ? (lane < 16 ? m0 + warp * 16 + lane : g.Cout) : m0 + warp * 32 + lane;
-    float *dst = g.part + ((size_t)blockIdx.y * g.Cout + (co < g.Cout ? co : 0)) * g.taps * g.Cin;
     for (int j = 0; j < ntap; ++j)
 #pragma unroll 1
       for (int c0 = 0; c0 < (ncx << 3); c0 += 16) {
@@ -221,15 +342,7 @@ __global__ void __launch_bounds__(kWgThreads) wgrad_tc_kernel(WgradArgs g) {
         if (t1 <= t0)
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] = 0.0f;
-        if (co < g.Cout) {
-          float4 *o = (float4 *)(dst + (size_t)(tap0 + j) * g.Cin + n0 + c0);
-          o[0] = make_float4(v[0], v[1], v[2], v[3]);
-          o[1] = make_float4(v[4], v[5], v[6], v[7]);
-          if (c0 + 8 < (ncx << 3)) {
-            o[2] = make_float4(v[8], v[9], v[10], v[11]);
-            o[3] = make_float4(v[12], v[13], v[14], v[15]);
-          }
-        }
+        store_part(g, co, (size_t)(tap0 + j) * g.Cin + n0 + c0, v, (ncx << 3) - c0);
       }
   }
   tc_fence_before();
@@ -321,11 +434,14 @@ int wgrad_split(long long P, int M, int N) {
   return (int)std::min(s, 64LL);
 }
 
-// How a gradient is cut: TMEM's 512 columns hold ntap x Nb accumulators, so
-// wide layers split their taps into groups (each stages its pixels again) and,
-// above 256 input channels, the channels too.  Fewer groups stage less; more
-// give more CTAs: the smallest count that fits TMEM and gives at least 90
-// CTAs (192^2, 128 -> 128: 0.17 ms with 96 CTAs; with 160, a second wave).
+int row_bytes(int c) { return c % 64 == 0 ? 128 : c % 32 == 0 ? 64 : c % 16 == 0 ? 32 : 16; }
+
+// What a CTA of either kernel accumulates is limited by TMEM's 512 columns;
+// fewer units (taps) to a CTA stage less per MMA but give more CTAs: the most
+// that fit, or as many fewer as it takes to have 90 CTAs (4 x 192^2, 128 ->
+// 128: 96 CTAs in one wave took 0.17 ms with the gather kernel, 160 in two 0.21).
+constexpr int kMinCtas = 90;
+
 WgradArgs wgrad_plan(int batch, int H, int W, int Cin, int Cout, int taps) {
   WgradArgs g{};
   g.H = H;
@@ -339,30 +455,60 @@ WgradArgs wgrad_plan(int batch, int H, int W, int Cin, int Cout, int taps) {
   g.fhw = make_div(H * W);
   g.fw = make_div(W);
   g.S = wgrad_split(g.P, taps * Cin, Cout);
-  g.NB = (Cin + 255) / 256;
-  g.Nb = ((Cin + g.NB - 1) / g.NB + 15) / 16 * 16;
-  g.NB = (Cin + g.Nb - 1) / g.Nb;
-  const int MB = (Cout + 127) / 128;
-  g.Mb = std::min(Cout, 128);
   g.mrows = Cout <= 64 ? 64 : 128;
-  g.strip = taps == 9 && W % 8 == 0;
-  for (g.G = 1; g.G <= taps; ++g.G) {
-    g.ntap = (taps + g.G - 1) / g.G;
-    if (g.G > 1 && (taps + g.ntap - 1) / g.ntap != g.G) continue;  // a smaller count gives the same groups
-    if (g.ntap * g.Nb <= 512 && (MB * g.NB * g.G * g.S >= 90 || g.G == taps)) break;
-  }
+  const int MB = (Cout + 127) / 128;
   g.cols = 32;
-  while (g.cols < g.ntap * g.Nb) g.cols *= 2;
-  int rows = 0;  // most input rows of a group's taps
-  for (int t = 0; t < taps; t += g.ntap) rows = std::max(rows, (std::min(t + g.ntap, taps) - 1) / 3 - t / 3 + 1);
-  // one 16-byte unit of padding per chunk spreads the copies over the banks
-  g.sxc = (g.strip ? rows * 80 : g.ntap * kKP) * 16 + 16;
-  g.syc = kKP * 16 + 16;
-  g.stage_bytes = (g.Nb / 8) * g.sxc + ((g.Mb + 7) / 8) * g.syc;
-  g.tail_bytes = (g.mrows / 8 - (g.Mb + 7) / 8) * g.syc;
+  if (taps == 1 || W % 8 == 0) {
+    g.rb = row_bytes(Cin);
+    g.chb = g.rb / 2;
+    g.nblk = Cin / g.chb;
+    g.ndx = taps == 9 ? 3 : 1;
+    g.nmma = (g.ndx * g.chb + 15) / 16 * 16;
+    g.U = g.ndx * g.nblk;
+    g.upg = std::min(g.U, 512 / g.nmma);
+    while (g.upg > 1 && MB * ((g.U + g.upg - 1) / g.upg) * g.S < kMinCtas) --g.upg;
+    g.rby = row_bytes(g.ldY);
+    g.chby = g.rby / 2;
+    g.nby = (std::min(g.ldY, 128) + g.chby - 1) / g.chby;
+    g.yblk = kKP * g.rby;
+    const int halo = g.ndx >> 1;
+    g.gw = taps == 1 || W % 64 == 0 ? 64 : W % 16 == 0 ? 16 : 8;
+    g.strip_bytes = ((g.gw + 2 * halo) * g.rb + 1023) / 1024 * 1024;
+    g.unit_bytes = kKP / g.gw * g.strip_bytes;
+    for (;; --g.upg) {  // two stages at least
+      g.stage_bytes = g.upg * g.unit_bytes + g.nby * g.yblk;
+      // an MMA reads mrows rows of dY whatever Cout: blocks behind the staged
+      // ones are other bytes of the allocation, and feed accumulator rows that
+      // nothing reads
+      g.tail_bytes = std::max(0, g.mrows / g.chby - g.nby) * g.yblk;
+      if (2 * g.stage_bytes + g.tail_bytes <= kSmemMax || g.upg == 1) break;
+    }
+    g.G = (g.U + g.upg - 1) / g.upg;
+    while (g.cols < g.upg * g.nmma) g.cols *= 2;
+  } else {
+    g.NB = (Cin + 255) / 256;
+    g.Nb = ((Cin + g.NB - 1) / g.NB + 15) / 16 * 16;
+    g.NB = (Cin + g.Nb - 1) / g.Nb;
+    g.Mb = std::min(Cout, 128);
+    g.ntap = std::min(taps, 512 / g.Nb);
+    while (g.ntap > 1 && MB * g.NB * ((taps + g.ntap - 1) / g.ntap) * g.S < kMinCtas) --g.ntap;
+    g.G = (taps + g.ntap - 1) / g.ntap;
+    g.ntap = (taps + g.G - 1) / g.G;
+    // one 16-byte unit of padding per chunk spreads the copies over the banks
+    g.syc = kKP * 16 + 16;
+    for (;; --g.ntap) {
+      g.sxc = g.ntap * kKP * 16 + 16;
+      g.stage_bytes = (g.Nb / 8) * g.sxc + ((g.Mb + 7) / 8) * g.syc;
+      g.tail_bytes = (g.mrows / 8 - (g.Mb + 7) / 8) * g.syc;
+      if (2 * g.stage_bytes + g.tail_bytes <= kSmemMax || g.ntap == 1) break;
+    }
+    g.G = (taps + g.ntap - 1) / g.ntap;
+    while (g.cols < g.ntap * g.Nb) g.cols *= 2;
+  }
+  const int ctas = MB * (g.NB ? g.NB : 1) * g.G * g.S;
   // two CTAs to an SM when there are more than one for each
-  int budget = MB * g.NB * g.G * g.S > kSms && 2 * g.cols <= 512 ? kSmemMax / 2 : kSmemMax;
-  if (2 * g.stage_bytes + g.tail_bytes > budget) budget = kSmemMax;
+  int budget = ctas > kSms && 2 * g.cols <= 512 ? kSmemMax / 2 - 1024 : kSmemMax;
+  if (3 * g.stage_bytes + g.tail_bytes > budget) budget = kSmemMax;
   g.nst = std::min(kMaxStages, (budget - g.tail_bytes) / g.stage_bytes);
   return g;
 }
@@ -419,22 +565,30 @@ int wgrad_launch(const __nv_bfloat16 *X, const __nv_bfloat16 *dY, int batch, int
   g.part = (float *)work;
   g.status = status;
   g.spins = spins;
-  // an MMA reads mrows rows of A and Nb of B whatever the channel counts: rows
-  // behind the staged ones are other bytes of the allocation, and only feed
-  // accumulators that nothing reads
-  const size_t smem = (size_t)g.nst * g.stage_bytes + g.tail_bytes;
-  const int lag = g.nst >= 7 ? 5 : g.nst >= 5 ? 3 : g.nst >= 3 ? 2 : 1;
-  auto fn = g.strip ? (lag == 5   ? wgrad_tc_kernel<5, true>
-                       : lag == 3 ? wgrad_tc_kernel<3, true>
-                       : lag == 2 ? wgrad_tc_kernel<2, true>
-                                  : wgrad_tc_kernel<1, true>)
-                    : (lag == 5   ? wgrad_tc_kernel<5, false>
-                       : lag == 3 ? wgrad_tc_kernel<3, false>
-                       : lag == 2 ? wgrad_tc_kernel<2, false>
-                                  : wgrad_tc_kernel<1, false>);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return NN_ECUDA;
-  const int units = (Cout + 127) / 128 * g.NB * g.G;
-  fn<<<dim3(units, g.S), kWgThreads, smem, s>>>(g);
+  const int smem = 1024 + g.nst * g.stage_bytes + g.tail_bytes, MB = (Cout + 127) / 128;
+  if (g.rb) {
+    CUtensorMap mx, my;
+    const unsigned long long uc = Cin, up = P, ul = g.ldY;
+    const unsigned long long dx[4] = {uc, taps == 9 ? (unsigned long long)W : up, taps == 9 ? (unsigned long long)H : 1ull,
+                                      taps == 9 ? (unsigned long long)batch : 1ull};
+    const unsigned long long sx[3] = {2 * uc, 2 * uc * dx[1], 2 * uc * dx[1] * dx[2]};
+    const unsigned bx[4] = {(unsigned)g.chb, (unsigned)(g.gw + g.ndx - 1), 1, 1};
+    if (int rc = make_tensor_map(&mx, X, 4, dx, sx, bx, g.rb)) return rc;
+    const unsigned long long dy[3] = {ul, up, 1}, sy[2] = {2 * ul, 2 * ul * up};
+    const unsigned by[3] = {(unsigned)g.chby, kKP, 1};
+    if (int rc = make_tensor_map(&my, dY, 3, dy, sy, by, g.rby)) return rc;
+    if (cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      return NN_ECUDA;
+    wgrad_tma_kernel<<<dim3(MB * g.G, g.S), 192, smem, s>>>(g, mx, my);
+  } else {
+    const int lag = g.nst >= 7 ? 5 : g.nst >= 5 ? 3 : g.nst >= 3 ? 2 : 1;
+    auto fn = lag == 5   ? wgrad_gather_kernel<5>
+              : lag == 3 ? wgrad_gather_kernel<3>
+              : lag == 2 ? wgrad_gather_kernel<2>
+                         : wgrad_gather_kernel<1>;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return NN_ECUDA;
+    fn<<<dim3(MB * g.NB * g.G, g.S), kWgThreads, smem, s>>>(g);
+  }
   const size_t nout = (size_t)taps * Cin * Cout;
   wgrad_reduce_kernel<<<(unsigned)((nout + 255) / 256), 256, 0, s>>>(g.part, g.S, nout, dW);
   if (db) {
