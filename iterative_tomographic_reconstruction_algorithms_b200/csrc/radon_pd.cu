@@ -14,14 +14,12 @@
 // x86-64 code), reproduced exactly: t = |fma(-c, y, x*s)|, the sign test uses
 // (x*s) * (1/c), and the first weight is |(t + ceil(T)) - nh|.
 //
-// Forward = per (angle, block of bins) a pass over the band of pixels whose
-// sub-samples land in the bins, summed in fixed point; adjoint =
-// gather per pixel over angles.  The duplicate sub-samples are evaluated once
-// with weight 2 * 1/4.
+// Forward = gather per bin over image lines; adjoint = gather per pixel over
+// angles.  The duplicate sub-samples are evaluated once with weight 2 * 1/4.
 #include <algorithm>
 #include <cmath>
 
-#include "fixed_sum.cuh"
+#include "f32x2.cuh"
 #include "tomo_internal.cuh"
 
 namespace tomo {
@@ -31,138 +29,290 @@ constexpr double kPi = 3.141592653589793;
 constexpr float kPdMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr int kPdMagicBits = 0x4B400000;  // its bit pattern
 
-struct PdEval {
-  float wl, wu;  // weights of bins l = floor(T), u = ceil(T)
-  int l, u;      // -1 when the reference's bound test (0 < bin < n) fails
+// T = nh - t with t = fma(c', y, RN(x s')), (s', c') = (sigma sin, -sigma cos),
+// sigma = -1 for cos >= 0, else +1: for every angle the sign rule (y > x s / c)
+// picks t = sigma (x s - y c), and rounding is symmetric.  (Where the test and
+// the product round differently, |t| is below the rounding of T.)
+__device__ __forceinline__ float2 pd_line(const PdAngle &g) {
+  const float sg = g.c >= 0.0f ? -1.0f : 1.0f;
+  return make_float2(sg * g.s, -(sg * g.c));
+}
+
+// Framed copies of the image for the forward: rows[i][P + j] and
+// cols[j][P + i] hold pixel (loop row i, column j), with P = kPdFrame zeros on
+// either side of a line.
+constexpr int kPdFrame = 4;
+
+__global__ void __launch_bounds__(256) pd_frame_kernel(const float *__restrict__ img, float *__restrict__ rows,
+                                                       float *__restrict__ cols, int n) {
+  __shared__ float tile[32][33];
+  const size_t z = blockIdx.z;
+  const int w = n + 2 * kPdFrame;
+  const float *src = img + z * (size_t)n * n;
+  float *R = rows + z * (size_t)n * w, *C = cols + z * (size_t)n * w;
+  const int j0 = blockIdx.x * 32 - kPdFrame, i0 = blockIdx.y * 32 - kPdFrame;  // tiles cover the frame too
+  for (int dy = threadIdx.y; dy < 32; dy += 8) {
+    const int i = i0 + dy, j = j0 + threadIdx.x;
+    const float v = i >= 0 && i < n && j >= 0 && j < n ? __ldg(src + (size_t)(n - 1 - i) * n + j) : 0.0f;
+    tile[dy][threadIdx.x] = v;
+    if (i >= 0 && i < n && j < n + kPdFrame) R[(size_t)i * w + kPdFrame + j] = v;
+  }
+  __syncthreads();
+  for (int dy = threadIdx.y; dy < 32; dy += 8) {
+    const int j = j0 + dy, i = i0 + threadIdx.x;
+    if (j >= 0 && j < n && i < n + kPdFrame) C[(size_t)j * w + kPdFrame + i] = tile[threadIdx.x][dy];
+  }
+}
+
+// Forward: a lane owns a bin b of an angle and walks the lines (ROWS: image
+// rows, when T moves faster along x; else columns).  On a line and for a
+// sub-sample, T rises by sigma = max(|s|, |c|) in [0.707, 1] per pixel in
+// direction DIR, so the pixels with T in (b - 1, b + 1) are among three
+// consecutive ones, found from the line's crossing of b - 1 (0.05 early, far
+// above its rounding: a fourth pixel would lie past b - 1.05 + 3 sigma > b + 1).
+// Each is evaluated with the reference's arithmetic: the first lies below b
+// (floor(T) = b - 1, weight T - floor(T)), the third above (floor(T) = b,
+// weight (t + ceil(T)) - nh), the second on either side; an integral T puts
+// nothing into either bin.  Six products of a line are added in float, lines
+// in double, rounded once: deterministic, and as close to the exact sum as the
+// 64-bit fixed-point sums in shared memory that this replaces.  Those took two
+// 32-bit atomics per product, and bounded the forward: 1.57 ms at 768^2 x 720,
+// now 0.97 (2048^2 x 1800: 25.2, now 14.8).  Bound now by instruction issue (52
+// per bin and line).
+template <bool ROWS, int DIR>
+__device__ __forceinline__ double pd_fwd_bin(const float *__restrict__ L, int w, float s, float c, int b, int n, int nh,
+                                             int i0, int i1) {
+  const float fnh = (float)nh, fb = (float)b, bm = fb - 1.0f, bp = fb + 1.0f;
+  const float k = ROWS ? s : c, o = ROWS ? c : s;  // t along the line, across lines
+  const float inv = 1.0f / k, slope = -o * inv;
+  // position (pixel index) at which T = b - 1: base + slope * (line coordinate)
+  float base[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) base[e] = (fnh - bm) * inv + fnh - 0.5f - (e ? 0.25f : -0.25f) - DIR * 0.05f;
+  const float lo = DIR > 0 ? -4.0f : -2.0f, hi = DIR > 0 ? (float)(n + 1) : (float)(n + 3);
+  const float *line = L + (size_t)i0 * w + kPdFrame - kPdMagicBits;
+  float lc = (float)i0 - fnh + 0.5f;  // the line's own coordinate
+  double acc = 0.0;
+  // both sub-samples at once, as pairs; nt = -t
+  const F2 base2 = f2(base[0], base[1]), slope2 = f2(slope), magic = f2(kPdMagic), nmagic = f2(-kPdMagic);
+  const F2 off = f2(0.25f - fnh, 0.75f - fnh), dir = f2((float)DIR), d2 = f2(-0.25f, 0.25f), nh2 = f2(fnh);
+  const F2 ns = f2(-s), nc = f2(-c), nbm = f2(-bm), nbp = f2(-bp);
+#pragma unroll 2
+  for (int i = i0; i < i1; ++i, line += w, lc += 1.0f) {
+    const F2 l = add2(f2(lc), d2);
+    const float2 ps = unpack(fma2(slope2, l, base2));
+    const F2 pos = f2(fminf(fmaxf(ps.x, lo), hi), fminf(fmaxf(ps.y, lo), hi));
+    const F2 fm = DIR > 0 ? add2_ru(pos, magic) : add2_rd(pos, magic);  // next pixels in DIR
+    const float2 fs = unpack(fm);
+    const float *va = line + __float_as_int(fs.x), *vb = line + __float_as_int(fs.y);
+    const F2 u0 = add2(add2(fm, nmagic), off);  // their coordinates along the line, exactly
+    const F2 u1 = add2(u0, dir), u2 = add2(u1, dir);
+    F2 t0, t1, t2;
+    if (ROWS) {
+      t0 = fma2(nc, l, mul2(u0, ns));
+      t1 = fma2(nc, l, mul2(u1, ns));
+      t2 = fma2(nc, l, mul2(u2, ns));
+    } else {
+      const F2 xs = mul2(l, ns);
+      t0 = fma2(nc, u0, xs);
+      t1 = fma2(nc, u1, xs);
+      t2 = fma2(nc, u2, xs);
+    }
+    const float2 w0 = unpack(add2(add2(nh2, t0), nbm));
+    const F2 T1 = add2(nh2, t1);
+    const float2 Ts = unpack(T1), wa = unpack(add2(T1, nbm)), wb = unpack(add2(add2(t1, nbp), nh2));  // wb: -weight
+    const float2 w2 = unpack(add2(add2(t2, nbp), nh2));                                               // -weight
+    // below b the first of wa, -wb is the smaller one, above the second
+    const float w1x = fminf(wa.x, -wb.x), w1y = fminf(wa.y, -wb.y);
+    float p = 0.0f;
+    const float a0 = __ldg(va), a1 = __ldg(va + DIR), a2 = __ldg(va + 2 * DIR);
+    const float b0 = __ldg(vb), b1 = __ldg(vb + DIR), b2 = __ldg(vb + 2 * DIR);
+    if (w0.x > 0.0f) p = w0.x * a0;
+    if (Ts.x != fb) p = fmaf(w1x, a1, p);
+    if (w2.x < 0.0f) p = fmaf(-w2.x, a2, p);
+    if (w0.y > 0.0f) p = fmaf(w0.y, b0, p);
+    if (Ts.y != fb) p = fmaf(w1y, b1, p);
+    if (w2.y < 0.0f) p = fmaf(-w2.y, b2, p);
+    acc += (double)p;
+  }
+  return acc;
+}
+
+// SPLIT = 1: a block takes 32 bins of kPdAng angles, whose warps read the same
+// pixels.  SPLIT > 1, for small images, whose bins alone are too few warps to
+// hide a line's latency: one angle, its lines shared by SPLIT warps, whose sums
+// are added in order.  The split depends on n alone (pd_fwd_split), so a plan
+// for some of the angles or several slices gives the same bits.
+constexpr int kPdAng = 4;
+
+template <int SPLIT>
+__global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : kPdAng)) pd_forward_kernel(
+    const float *__restrict__ rows, const float *__restrict__ cols, float *__restrict__ sino, const PdAngle *__restrict__ tab,
+    int n, int nh, int na, FwdEpi ep) {
+  __shared__ double part[SPLIT > 1 ? SPLIT : 1][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, v = SPLIT > 1 ? blockIdx.y : blockIdx.y * kPdAng + warp;
+  const int B0 = blockIdx.x * 32, b = B0 + lane, w = n + 2 * kPdFrame;
+  const size_t z = blockIdx.z;
+  const bool live = v < na && b < n;
+  double acc = 0.0;
+  if (v < na) {  // warp-uniform
+    const float2 g = pd_line(tab[v]);
+    const float s = g.x, c = g.y, fnh = (float)nh;
+    const bool by_rows = fabsf(s) >= fabsf(c);
+    // lines whose T range, nh - o l +- |k| (nh + 2), meets (B0 - 1, B0 + 32)
+    const float k = fabsf(by_rows ? s : c), o = by_rows ? c : s, half = k * (fnh + 2.0f);
+    int i0 = 0, i1 = n;
+    if (fabsf(o) > 1e-4f) {
+      const float l0 = (fnh - half - (float)(B0 + 33)) / o, l1 = (fnh + half - (float)(B0 - 2)) / o;
+      i0 = max(0, (int)floorf(fminf(fmaxf(fminf(l0, l1) + fnh - 2.0f, 0.0f), (float)n)));
+      i1 = min(n, (int)ceilf(fminf(fmaxf(fmaxf(l0, l1) + fnh + 2.0f, 0.0f), (float)n)));
+    }
+    if (SPLIT > 1) {
+      const int len = max(0, i1 - i0);
+      i1 = i0 + len * (warp + 1) / SPLIT;
+      i0 += len * warp / SPLIT;
+    }
+    const float *L = (by_rows ? rows : cols) + z * (size_t)n * w;
+    if (by_rows)
+      acc = s < 0.0f ? pd_fwd_bin<true, 1>(L, w, s, c, b, n, nh, i0, i1) : pd_fwd_bin<true, -1>(L, w, s, c, b, n, nh, i0, i1);
+    else
+      acc = c < 0.0f ? pd_fwd_bin<false, 1>(L, w, s, c, b, n, nh, i0, i1) : pd_fwd_bin<false, -1>(L, w, s, c, b, n, nh, i0, i1);
+  }
+  if (SPLIT > 1) {
+    part[warp][lane] = acc;
+    __syncthreads();
+    if (warp > 0) return;
+    for (int q = 1; q < SPLIT; ++q) acc += part[q][lane];
+  }
+  // bin 0 never receives; 0.5: two coinciding quarter-weight sub-samples
+  const float out = b >= 1 ? (float)(0.5 * acc) : 0.0f;
+  double r2 = 0.0;
+  const size_t e = z * (size_t)na * n + (size_t)v * n + b;
+  if (live) sino[e] = fwd_apply(ep, out, e, r2);
+  const size_t block = ((size_t)z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  fwd_resid_commit(ep, r2, SPLIT > 1 ? block : block * kPdAng + warp);
+}
+
+int pd_fwd_split(int n) { return n > 448 ? 1 : n > 320 ? 4 : 8; }
+
+// Sinogram rows as pairs, entry e = l + pads of angle v: {S_l, S_l+1}, the two
+// bins a sub-sample with floor(T) = l is split between; bin 0 and the bins
+// outside [0, n) never receive and are 0 here, so the adjoint's loop tests no
+// bounds.
+__global__ void __launch_bounds__(256) pd_expand_kernel(const float *__restrict__ sino, float2 *__restrict__ out, int n,
+                                                        int pads, int w2) {
+  const size_t row = blockIdx.x;  // z * na + v
+  const float *src = sino + row * n;
+  float2 *dst = out + row * w2;
+  for (int e = threadIdx.x; e < w2; e += blockDim.x) {
+    const int l = e - pads;
+    dst[e] = make_float2(l >= 1 && l < n ? __ldg(src + l) : 0.0f, l + 1 >= 1 && l + 1 < n ? __ldg(src + l + 1) : 0.0f);
+  }
+}
+
+// Adjoint: a lane holds 4 x 4 pixels of a 32 x 16 tile; the Q warps of a block
+// sum Q contiguous shares of the angles, added in order through shared memory
+// (Q depends on n alone, so the result does not depend on the device).
+//
+// Per sub-sample: t and T as the reference rounds them, the pair at floor(T)
+// in one 8-byte read, and its two weights.  An integral T puts nothing into
+// either bin: its weights are the rounding of t, and are skipped.
+//
+// Bound by L1 (70 % of its rate) and FP32 (65 %): 9 operations and 2 FMAs per
+// sub-sample, whose table pairs hit L1.  The two sub-samples go as f32x2 pairs,
+// which halves the instructions (scalar ones: 0.57 ms against 0.51).  A thread
+// per pixel with four reads, bounds tests and the sign rule per sub-sample took
+// 1.52 ms at 768^2 x 720 and 25.5 at 2048^2 x 1800; this one 0.51 and 7.8.
+template <int Q>
+__global__ void __launch_bounds__(32 * Q) pd_adjoint_kernel(const float2 *__restrict__ pairs, float *__restrict__ img,
+                                                            const PdAngle *__restrict__ tab, int n, int nh, int na, int pads,
+                                                            int w2, AdjEpi ep) {
+  __shared__ float part[(Q - 1) * 16][32];
+  const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+  const int b0 = blockIdx.x * 32 + 4 * (lane & 7), a0 = blockIdx.y * 16 + 4 * (lane >> 3);
+  const size_t z = blockIdx.z;
+  const float fnh = (float)nh;
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+  const int u0 = (int)((long long)na * q / Q), u1 = (int)((long long)na * (q + 1) / Q);
+  if (a0 < n && b0 < n) {
+    const float x0 = (float)b0 - fnh + 0.5f, y0 = (float)(n - 1 - a0) - fnh + 0.5f;  // rows go up in y
+    const F2 nh2 = f2(fnh), magic = f2(kPdMagic), nmagic = f2(-kPdMagic), magic1 = f2(kPdMagic - 1.0f);
+    // row base minus the bits of the magic floor
+    const float2 *row = pairs + (z * na + u0) * (size_t)w2 + pads - kPdMagicBits;
+#pragma unroll 1
+    for (int u = u0; u < u1; ++u, row += w2) {
+      const float2 g = pd_line(tab[u]);
+      const float s = g.x, c = g.y;
+      // both sub-samples as a pair; nt = -t
+      const F2 ns = f2(-s), nc = f2(-c);
+      F2 xs[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) xs[j] = mul2(f2(x0 + (float)j - 0.25f, x0 + (float)j + 0.25f), ns);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const F2 y = f2(y0 - (float)i - 0.25f, y0 - (float)i + 0.25f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const F2 nt = fma2(nc, y, xs[j]);
+          const F2 T = add2(nh2, nt);
+          // floor(T) without the conversion pipe: T + 1.5 * 2^23 rounded down
+          // lies where floats are the integers (|T| < 2^22), and its bits give
+          // the integer
+          const F2 fd = add2_rd(T, magic);
+          const float2 fs = unpack(fd);
+          const float2 Sa = __ldg(row + __float_as_int(fs.x)), Sb = __ldg(row + __float_as_int(fs.y));
+          const float2 wu = unpack(rsub2(add2(fd, nmagic), T));
+          const float2 wl = unpack(add2(add2(nt, rsub2(fd, magic1)), nh2));  // -(t + (floor(T) + 1) - nh)
+          if (wu.x != 0.0f) acc[i][j] = __fmaf_rn(-wl.x, Sa.x, __fmaf_rn(wu.x, Sa.y, acc[i][j]));
+          if (wu.y != 0.0f) acc[i][j] = __fmaf_rn(-wl.y, Sb.x, __fmaf_rn(wu.y, Sb.y, acc[i][j]));
+        }
+      }
+    }
+  }
+  if (q > 0)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) part[(q - 1) * 16 + 4 * i + j][lane] = acc[i][j];
+  __syncthreads();
+  if (q > 0) return;
+#pragma unroll
+  for (int r = 0; r < Q - 1; ++r)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] += part[r * 16 + 4 * i + j][lane];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int R = a0 + i, C = b0 + j;
+      const bool live = R < n && C < n;
+      // 0.5: the two coinciding quarter-weight sub-samples
+      adj_store(ep, 0.5f * acc[i][j], live, z * (size_t)n * n + (live ? (size_t)R * n + C : 0), img);
+    }
+}
+
+// What the pair owns beside the angle table.
+struct PdState {
+  float *rows = nullptr, *cols = nullptr;  // [nz][n][n + 2 kPdFrame]
+  float2 *pairs = nullptr;    // [nz][na][w2]
+  int pads = 0, w2 = 0;
 };
 
-__device__ __forceinline__ PdEval pd_eval(float x, float y, const PdAngle &g, float fnh, int n) {
-  const float xs = __fmul_rn(x, g.s);
-  const float t = fabsf(__fmaf_rn(-g.c, y, xs));
-  const float r = __fmul_rn(xs, g.rc);
-  const bool keep = ((g.flags & 1) && y > r) || ((g.flags & 2) && y > r) || ((g.flags & 4) && y > 0.0f);
-  const float ts = keep ? t : -t;
-  const float T = __fsub_rn(fnh, ts);
-  // floor and ceil of T without the conversion pipe: T + 1.5 * 2^23 rounded
-  // down / up lies where floats are the integers (|T| < 2^22), so it is
-  // 1.5 * 2^23 + floor(T) / ceil(T) exactly, and its bits give the integer
-  const float fd = __fadd_rd(T, kPdMagic), fu = __fadd_ru(T, kPdMagic);
-  const float lf = __fsub_rn(fd, kPdMagic), uf = __fsub_rn(fu, kPdMagic);
-  PdEval e;
-  e.wl = fabsf(__fsub_rn(__fadd_rn(ts, uf), fnh));
-  e.wu = fabsf(__fsub_rn(T, lf));
-  e.l = (lf >= 1.0f && lf < (float)n) ? __float_as_int(fd) - kPdMagicBits : -1;
-  e.u = (uf >= 1.0f && uf < (float)n) ? __float_as_int(fu) - kPdMagicBits : -1;
-  return e;
+void pd_state_free(void *q) {
+  auto *st = (PdState *)q;
+  cudaFree(st->pairs);
+  delete st;
 }
 
-// Forward: a block owns kPdBins consecutive bins of one angle and slice; its
-// warps walk the band of pixels whose sub-samples can land in (B0 - 1, Bend)
-// (a line per warp, each pixel once, along the axis on which T moves fastest)
-// and add 0.5 w value for every sub-sample and bin into shared-memory bins
-// summed in fixed point (fixed_sum.cuh): deterministic, each bin the sum of
-// its float products to within the fixed-point unit, rounded once.  Per line and sub-sample at
-// most 3 pixels reach a bin (T moves by at least 1/sqrt(2) per pixel), so a
-// bin is bounded by 2 (sub-samples) x 3 n x 0.5 x max|finite image value|;
-// inf and NaN products flag their bins instead (fixed_sum.cuh).
-constexpr int kPdBins = 128, kPdThreads = 256;
-
-__global__ void __launch_bounds__(kPdThreads) pd_forward_kernel(
-    const float *__restrict__ img, float *__restrict__ sino, const PdAngle *__restrict__ tab,
-    int n, int nh, int na, const unsigned *__restrict__ vmax, FwdEpi ep) {
-  __shared__ unsigned long long acc[kPdBins];
-  __shared__ unsigned flg[kPdBins];  // non-finite products per bin (fixed_sum.cuh)
-  const int B0 = blockIdx.x * kPdBins, v = blockIdx.y;
-  const size_t z = blockIdx.z;
-  for (int i = threadIdx.x; i < kPdBins; i += blockDim.x) {
-    acc[i] = 0ull;
-    flg[i] = 0u;
-  }
-  const FixedScale fs = fixed_scale(3.0 * n * (double)__uint_as_float(vmax[z]));
-  __syncthreads();
-  const PdAngle g = tab[v];
-  const float *I = img + z * (size_t)n * n;
-  const float fnh = (float)nh;
-  const int Bend = min(B0 + kPdBins, n);
-  // T ~ nh - sigma*((y0+d) c - (x0+d) s), sigma = sign(c)
-  const float sg = g.c >= 0.0f ? 1.0f : -1.0f;
-  const bool by_rows = fabsf(g.s) >= fabsf(g.c);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int line = warp; line < n; line += kPdThreads / 32) {
-    const float o0 = (float)line - fnh + 0.5f;  // y0 (rows) or x0 (columns)
-    float lo = 1e30f, hi = -1e30f;
-    for (int e = 0; e < 2; ++e) {
-      const float d = e ? 0.25f : -0.25f;
-      for (int f = 0; f < 2; ++f) {
-        const float T = (float)(f ? Bend : B0 - 1);
-        float w;  // the other pixel-centre coordinate giving this T
-        if (by_rows) w = (T - fnh + sg * ((o0 + d) * g.c)) / (sg * g.s) - d;
-        else w = (fnh - T + sg * ((o0 + d) * g.s)) / (sg * g.c) - d;
-        lo = fminf(lo, w);
-        hi = fmaxf(hi, w);
-      }
-    }
-    int j0 = (int)floorf(lo + fnh - 0.5f) - 1, j1 = (int)ceilf(hi + fnh - 0.5f) + 1;
-    j0 = max(j0, 0);
-    j1 = min(j1, n - 1);
-    for (int j = j0 + lane; j <= j1; j += 32) {
-      const int ii = by_rows ? line : j, jj = by_rows ? j : line;
-      const float val = __ldg(I + (size_t)(n - 1 - ii) * n + jj);
-      if (val == 0.0f) continue;  // adds exactly nothing
-      const float x0 = (float)jj - fnh + 0.5f, y0 = (float)ii - fnh + 0.5f;
-      for (int e = 0; e < 2; ++e) {
-        const float d = e ? 0.25f : -0.25f;
-        const PdEval q = pd_eval(__fadd_rn(x0, d), __fadd_rn(y0, d), g, fnh, n);
-        if (q.l >= B0 && q.l < Bend) fixed_add_product(acc + (q.l - B0), flg + (q.l - B0), __fmul_rn(0.5f * q.wl, val), fs);
-        if (q.u >= B0 && q.u < Bend) fixed_add_product(acc + (q.u - B0), flg + (q.u - B0), __fmul_rn(0.5f * q.wu, val), fs);
-      }
-    }
-  }
-  __syncthreads();
-  const int b = B0 + (int)threadIdx.x;
-  const bool live = threadIdx.x < kPdBins && b < n;
-  float out = 0.0f;
-  if (live) out = flg[threadIdx.x] ? nonfinite_value(flg[threadIdx.x]) : fixed_to_float(acc[threadIdx.x], fs);
-  fwd_store(ep, out, live, z * (size_t)na * n + (size_t)v * n + (live ? b : 0), sino);
-}
-
-constexpr int kPdChunk = 1024;
-
-// Adjoint: thread per output pixel (memory row R, column j); the reference's
-// loop row is i = n-1-R.
-__global__ void __launch_bounds__(256) pd_adjoint_kernel(
-    const float *__restrict__ sino, float *__restrict__ img, const PdAngle *__restrict__ tab,
-    int n, int nh, int na, AdjEpi ep) {
-  __shared__ PdAngle stab[kPdChunk];
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int R = blockIdx.y * blockDim.y + threadIdx.y;
-  const size_t z = blockIdx.z;
-  const bool live = R < n && j < n;
-  const float *S = sino + z * (size_t)na * n;
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = blockDim.x * blockDim.y;
-  const float fnh = (float)nh;
-  const int i = n - 1 - R;
-  const float x0 = (float)j - fnh + 0.5f, y0 = (float)i - fnh + 0.5f;
-  float acc = 0.0f;
-  for (int v0 = 0; v0 < na; v0 += kPdChunk) {
-    const int cnt = min(kPdChunk, na - v0);
-    __syncthreads();
-    for (int t = tid; t < cnt; t += nthr) stab[t] = tab[v0 + t];
-    __syncthreads();
-    if (!live) continue;
-    for (int u = 0; u < cnt; ++u) {
-      const PdAngle g = stab[u];
-      const float *row = S + (size_t)(v0 + u) * n;
-      for (int e = 0; e < 2; ++e) {
-        const float d = e ? 0.25f : -0.25f;
-        const PdEval q = pd_eval(__fadd_rn(x0, d), __fadd_rn(y0, d), g, fnh, n);
-        if (q.l >= 0) acc = fmaf(0.5f * q.wl, __ldg(row + q.l), acc);
-        if (q.u >= 0) acc = fmaf(0.5f * q.wu, __ldg(row + q.u), acc);
-      }
-    }
-  }
-  adj_store(ep, acc, live, z * (size_t)n * n + (size_t)(live ? R : 0) * n + (live ? j : 0), img);
-}
+// Warps of an adjoint tile: more shares of the angles where the tiles alone
+// leave the SMs short of warps (148 x 32 of them hide the reads' latency).
+int pd_adj_warps(int n) { return n > 640 ? 4 : n > 384 ? 8 : 16; }
 
 }  // namespace
 
@@ -183,30 +333,45 @@ int pd_setup(Plan &p) {
   }
   TOMO_CUDA(cudaMalloc(&p.d_angles, sizeof(PdAngle) * (size_t)na));
   TOMO_CUDA(cudaMemcpy(p.d_angles, tab.data(), sizeof(PdAngle) * (size_t)na, cudaMemcpyHostToDevice));
-  // per-slice max |finite image value| of the forward's fixed-point sums
-  TOMO_CUDA(cudaMalloc(&p.ext, sizeof(unsigned) * (size_t)std::max(1, p.g.nz)));
-  p.ext_free = [](void *q) { cudaFree(q); };
+  auto *st = new PdState();
+  p.ext = st;
+  p.ext_free = pd_state_free;
+  // |t| stays below sqrt(2) (nh + 1), also for the pixels of a tile that lie
+  // up to 3 outside the image
+  st->pads = (int)std::ceil((p.nh + 1) * 0.41422) + 12;
+  st->w2 = p.g.n + 2 * st->pads;
+  // one workspace: the adjoint's pairs, then the forward's framed copies
+  const size_t pairs = (size_t)p.g.nz * na * st->w2, framed = (size_t)p.g.nz * p.g.n * (p.g.n + 2 * kPdFrame);
+  TOMO_CUDA(cudaMalloc(&st->pairs, sizeof(float2) * pairs + 2 * sizeof(float) * framed));
+  st->rows = (float *)(st->pairs + pairs);
+  st->cols = st->rows + framed;
   // residual partials of the fused solvers: one per warp of the forward launch
-  p.fwd_warps = (size_t)((p.g.n + kPdBins - 1) / kPdBins) * (kPdThreads / 32) * na * p.g.nz;
+  p.fwd_warps = (size_t)((p.g.n + 31) / 32) * p.g.nz *
+                (pd_fwd_split(p.g.n) > 1 ? na : (na + kPdAng - 1) / kPdAng * kPdAng);
   return TOMO_OK;
 }
 
 int pd_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const FwdEpi &ep) {
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
-  unsigned *vmax = (unsigned *)p.ext;
-  const size_t per = (size_t)n * n;
-  TOMO_CUDA(cudaMemsetAsync(vmax, 0, sizeof(unsigned) * nz, s));
-  fixed_finite_absmax_kernel<<<dim3((unsigned)std::min<size_t>((per + 255) / 256, 1184), nz), 256, 0, s>>>(d_img, per, vmax);
-  dim3 fg((n + kPdBins - 1) / kPdBins, na, nz);
-  pd_forward_kernel<<<fg, kPdThreads, 0, s>>>(d_img, d_sino, (const PdAngle *)p.d_angles, n, p.nh, na, vmax, ep);
+  PdState &st = *(PdState *)p.ext;
+  const int tiles = (n + 2 * kPdFrame + 31) / 32;
+  pd_frame_kernel<<<dim3(tiles, tiles, nz), dim3(32, 8), 0, s>>>(d_img, st.rows, st.cols, n);
+  const int split = pd_fwd_split(n), warps = split > 1 ? split : kPdAng;
+  auto fn = split == 8 ? pd_forward_kernel<8> : split == 4 ? pd_forward_kernel<4> : pd_forward_kernel<1>;
+  fn<<<dim3((n + 31) / 32, split > 1 ? na : (na + kPdAng - 1) / kPdAng, nz), 32 * warps, 0, s>>>(
+      st.rows, st.cols, d_sino, (const PdAngle *)p.d_angles, n, p.nh, na, ep);
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
 }
 
 int pd_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const AdjEpi &ep) {
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
-  dim3 ab(32, 8), ag((n + 31) / 32, (n + 7) / 8, nz);
-  pd_adjoint_kernel<<<ag, ab, 0, s>>>(d_sino, d_img, (const PdAngle *)p.d_angles, n, p.nh, na, ep);
+  PdState &st = *(PdState *)p.ext;
+  pd_expand_kernel<<<na * nz, 256, 0, s>>>(d_sino, st.pairs, n, st.pads, st.w2);
+  const int Q = pd_adj_warps(n);
+  auto fn = Q == 4 ? pd_adjoint_kernel<4> : Q == 8 ? pd_adjoint_kernel<8> : pd_adjoint_kernel<16>;
+  fn<<<dim3((n + 31) / 32, (n + 15) / 16, nz), 32 * Q, 0, s>>>(st.pairs, d_img, (const PdAngle *)p.d_angles, n, p.nh, na,
+                                                               st.pads, st.w2, ep);
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
 }
