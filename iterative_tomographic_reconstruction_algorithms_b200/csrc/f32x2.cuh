@@ -1,6 +1,10 @@
 // Packed pairs of floats (sm_100a): one instruction, two results, each rounded
 // as the scalar one.  The pipe takes as long as for two scalar instructions,
 // so pairs pay where a loop is bound by instruction issue, not by FP32 itself.
+// A product that goes into an add2 is contracted into one fma (ptxas 12.9,
+// explicit rounding notwithstanding, also through a multiplication by 1): where
+// the product has to be rounded, unpack it and go on with scalar operations.
+// As the addend of an fma2 it is safe.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -21,7 +21,7 @@
 #include <algorithm>
 #include <cmath>
 
-#include "fixed_sum.cuh"
+#include "f32x2.cuh"
 #include "tomo_internal.cuh"
 
 namespace tomo {
@@ -29,157 +29,243 @@ namespace {
 
 constexpr double kS45 = 0.70710678118654757;
 
-__global__ void ss_transpose_kernel(const float *__restrict__ in, float *__restrict__ out, int n) {
+constexpr float kSsMagic = 12582912.0f;  // 1.5 * 2^23
+constexpr int kSsMagicBits = 0x4B400000;  // its bit pattern
+constexpr int kSsFrame = 4;
+
+// Framed copies of the image: rows[y][P + x] and cols[x][P + y], with P =
+// kSsFrame zeros on either side of a line.
+__global__ void __launch_bounds__(256) ss_frame_kernel(const float *__restrict__ img, float *__restrict__ rows,
+                                                       float *__restrict__ cols, int n) {
   __shared__ float tile[32][33];
-  const size_t stride = (size_t)n * n;
-  const float *src = in + (size_t)blockIdx.z * stride;
-  float *dst = out + (size_t)blockIdx.z * stride;
-  int x = blockIdx.x * 32 + threadIdx.x;
-  int y0 = blockIdx.y * 32;
-  for (int dy = threadIdx.y; dy < 32; dy += blockDim.y) {
-    int y = y0 + dy;
-    if (x < n && y < n) tile[dy][threadIdx.x] = src[(size_t)y * n + x];
+  const size_t z = blockIdx.z;
+  const int w = n + 2 * kSsFrame;
+  const float *src = img + z * (size_t)n * n;
+  float *R = rows + z * (size_t)n * w, *C = cols + z * (size_t)n * w;
+  const int x0 = blockIdx.x * 32 - kSsFrame, y0 = blockIdx.y * 32 - kSsFrame;  // tiles cover the frame too
+  for (int dy = threadIdx.y; dy < 32; dy += 8) {
+    const int y = y0 + dy, x = x0 + threadIdx.x;
+    const float v = y >= 0 && y < n && x >= 0 && x < n ? __ldg(src + (size_t)y * n + x) : 0.0f;
+    tile[dy][threadIdx.x] = v;
+    if (y >= 0 && y < n && x < n + kSsFrame) R[(size_t)y * w + kSsFrame + x] = v;
   }
   __syncthreads();
-  int ox = blockIdx.y * 32 + threadIdx.x;
-  for (int dy = threadIdx.y; dy < 32; dy += blockDim.y) {
-    int oy = blockIdx.x * 32 + dy;
-    if (ox < n && oy < n) dst[(size_t)oy * n + ox] = tile[threadIdx.x][dy];
+  for (int dy = threadIdx.y; dy < 32; dy += 8) {
+    const int x = x0 + dy, y = y0 + threadIdx.x;
+    if (x >= 0 && x < n && y < n + kSsFrame) C[(size_t)x * w + kSsFrame + y] = tile[threadIdx.x][dy];
   }
 }
 
-// Forward: one thread per (t, angle, slice).  For the steep branch the minor
-// axis is x (row mm, columns q, q+1 of the image); otherwise the minor axis is
-// y (rows q, q+1 of column mm), read from the transposed image so that
-// neighbouring threads read neighbouring words.
-__global__ void __launch_bounds__(128) ss_forward_kernel(
-    const float *__restrict__ img, const float *__restrict__ imgT, float *__restrict__ sino,
-    const SsAngle *__restrict__ tab, const int2 *__restrict__ lim, int n, int nh, int na, FwdEpi ep) {
-  const int kt = blockIdx.x * blockDim.x + threadIdx.x;  // t + nh
+// Forward: a lane owns a ray (t, angle, slice) and steps along its major axis;
+// a step interpolates across the minor one (steep rays: in an image row, else
+// in a column, i.e. a row of the transposed copy, so that neighbouring lanes
+// read neighbouring words).  The frame stands in for bounds tests, the angle's
+// factor wt is applied once.  SPLIT warps share a ray's steps and are added in
+// order: small images have too few rays to hide a step's latency (256^2 x 200:
+// 61 us unsplit, now 18; 768^2 x 720: 0.58 ms unsplit, 0.38 by two); the split
+// depends on n alone (ss_fwd_split).
+// 4 x 641^2 x 600: 1.28 ms with bounds tests and weights per step, now 0.78;
+// 2048^2 x 1800: 9.6, now 6.3.
+template <int SPLIT>
+__global__ void __launch_bounds__(128) ss_forward_kernel(const float *__restrict__ rows, const float *__restrict__ cols,
+                                                         float *__restrict__ sino, const SsAngle *__restrict__ tab,
+                                                         const int2 *__restrict__ lim, int n, int nh, int na, FwdEpi ep) {
+  __shared__ float part[SPLIT][128 / SPLIT];
+  constexpr int kRays = 128 / SPLIT;
+  const int lane = threadIdx.x % kRays, q = threadIdx.x / kRays;  // kRays is a multiple of 32: q is warp-uniform
+  const int kt = blockIdx.x * kRays + lane;  // t + nh
   const int v = blockIdx.y;
   const size_t z = blockIdx.z;
   const bool live = kt < n;  // kt == 2nh (odd n) is never reached by a ray: stays 0
   const SsAngle g = tab[v];
   const int2 L = kt < 2 * nh ? lim[(size_t)v * (2 * nh) + kt] : make_int2(0, 0);
-  const float ft = (float)(kt - nh);
-  const float *M = (g.steep ? img : imgT) + z * (size_t)n * n;
-  float acc = 0.0f;
-  for (int m = L.x; m < L.y; ++m) {
-    const int mm = m + nh;
-    if (mm < 0 || mm > n - 1) continue;
-    const float f = __fmul_rn(__fmaf_rn(-(float)m, g.a, ft), g.rb);
-    float fl;
-    const int q = floor_i(f, fl) + nh;
-    const float w = __fsub_rn(f, fl), w1 = __fsub_rn(__fadd_rn(fl, 1.0f), f);
-    const float *row = M + (size_t)mm * n;
-    if (q >= 0 && q <= n - 1) acc = fmaf(g.wt * w1, __ldg(row + q), acc);
-    if (q + 1 >= 0 && q + 1 <= n - 1) acc = fmaf(g.wt * w, __ldg(row + q + 1), acc);
+  int m0 = max(L.x, -nh), m1 = min(L.y, n - nh);  // rays that miss the square may leave it
+  if (SPLIT > 1) {
+    const int len = max(0, m1 - m0), s0 = m0;
+    m0 = s0 + len * q / SPLIT;
+    m1 = s0 + len * (q + 1) / SPLIT;
   }
-  fwd_store(ep, acc, live, z * (size_t)na * n + (size_t)g.out_row * n + (live ? kt : 0), sino);
+  const int w = n + 2 * kSsFrame;
+  const float ft = (float)(kt - nh), lo = (float)(-nh) - 2.0f, hi = (float)(n - nh) + 1.0f;
+  const float *row = (g.steep ? rows : cols) + z * (size_t)n * w + (ptrdiff_t)(m0 + nh) * w + kSsFrame + nh - kSsMagicBits;
+  float nm = (float)(-m0), acc = 0.0f;
+#pragma unroll 4
+  for (int m = m0; m < m1; ++m, nm -= 1.0f, row += w) {
+    const float f = fminf(fmaxf(__fmul_rn(__fmaf_rn(nm, g.a, ft), g.rb), lo), hi);
+    const float fd = __fadd_rd(f, kSsMagic);  // floor(f), as a float among the integers and in its bits
+    const float wq = __fsub_rn(f, __fsub_rn(fd, kSsMagic));
+    const float *p = row + __float_as_int(fd);
+    acc = fmaf(__fsub_rn(1.0f, wq), __ldg(p), acc);  // 1 - w is exactly (floor(f) + 1) - f
+    acc = fmaf(wq, __ldg(p + 1), acc);
+  }
+  if (SPLIT > 1) {
+    part[q][lane] = acc;
+    __syncthreads();
+    if (q > 0) return;  // warp-uniform
+    for (int k = 1; k < SPLIT; ++k) acc += part[k][lane];
+  }
+  acc *= g.wt;
+  double r2 = 0.0;
+  const size_t e = z * (size_t)na * n + (size_t)g.out_row * n + kt;
+  if (live) sino[e] = fwd_apply(ep, acc, e, r2);
+  const size_t block = ((size_t)z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  fwd_resid_commit(ep, r2, block * (kRays / 32) + lane / 32);
 }
 
-// Adjoint: a thread holds 4 x 4 output pixels (rows R0..R0+3, columns
-// C0..C0+3), all angles in order.  For an angle the pixels fall into 4
-// groups of 4 along the minor axis (a row of the block for steep angles, a
-// column otherwise); the rays that touch a pixel are those whose minor
-// coordinate lands in [minor - 1, minor + 1) at the pixel's major coordinate,
-// so a group's candidate rays are the integers t of one short interval (at
-// most 7: |rb| >= 1), each checked once with the forward arithmetic and
-// credited to the one or two pixels of the group it reaches.  Each pixel gets
-// the credits of its rays in the order t ascending, angle after angle, as a
-// thread per pixel would give them.
-constexpr int kSsChunk = 512;
-constexpr int kSsPix = 4;  // pixels per thread along each axis
+int ss_fwd_split(int n) { return n > 448 ? 2 : 4; }
 
-// The credits of angle g to the group of pixels with major coordinate m and
-// minor indices minor0 .. minor0 + 3 (a0 .. a3 the pixels at minor0 + 0 .. 3).
-__device__ __forceinline__ void ss_adj_group(const SsAngle &g, float cb, int m, int minor0, int nh,
-                                             const float *__restrict__ row, const int2 *__restrict__ lrow,
-                                             float &a0, float &a1, float &a2, float &a3) {
-  // f(t) = fma(-m, a, t) * rb ~ (t - m a) rb must land in [minor0 - nh - 1,
-  // minor0 + 3 - nh + 1): t in [ta, tb] up to rounding (below 1e-3 here), so
-  // the integers in [ta - 0.01, tb + 0.01] are the candidates
-  const float ma = (float)m * g.a;
-  const float lo = (float)(minor0 - nh - 1), hi = (float)(minor0 + kSsPix - nh);
-  float ta = fmaf(lo, cb, ma), tb = fmaf(hi, cb, ma);
-  if (ta > tb) {
-    const float x = ta;
-    ta = tb;
-    tb = x;
-  }
-  float fl0, fl1;
-  const int t0 = max(floor_i(ta - 0.01f, fl0) + 1, -nh), t1 = min(floor_i(tb + 0.01f, fl1), nh - 1);
-  for (int t = t0; t <= t1; ++t) {
-    const int2 L = __ldg(lrow + t + nh);
-    if (m < L.x || m >= L.y) continue;
-    const float f = __fmul_rn(__fmaf_rn(-(float)m, g.a, (float)t), g.rb);
-    float fl;
-    const int d = floor_i(f, fl) + nh - minor0;  // the ray's left pixel, relative to minor0
-    if (d < -1 || d >= kSsPix) continue;
-    const float y = __ldg(row + t + nh);
-    const float c1 = __fmul_rn(g.wt, __fsub_rn(__fadd_rn(fl, 1.0f), f));  // to pixel d
-    const float c0 = __fmul_rn(g.wt, __fsub_rn(f, fl));                     // to pixel d + 1
-    if (d == 0) a0 = fmaf(c1, y, a0);
-    if (d == -1) a0 = fmaf(c0, y, a0);
-    if (d == 1) a1 = fmaf(c1, y, a1);
-    if (d == 0) a1 = fmaf(c0, y, a1);
-    if (d == 2) a2 = fmaf(c1, y, a2);
-    if (d == 1) a2 = fmaf(c0, y, a2);
-    if (d == 3) a3 = fmaf(c1, y, a3);
-    if (d == 2) a3 = fmaf(c0, y, a3);
+// Sinogram rows as pairs in the order of the angles, entry e = t + nh + pads of
+// angle v: wt {S_t, S_t+1}, 0 outside the rays.
+__global__ void __launch_bounds__(256) ss_expand_kernel(const float *__restrict__ sino, float2 *__restrict__ out,
+                                                        const SsAngle *__restrict__ tab, int n, int nh, int na, int pads,
+                                                        int w2) {
+  const int v = blockIdx.x;
+  const size_t z = blockIdx.y;
+  const SsAngle g = tab[v];
+  const float *src = sino + (z * na + g.out_row) * (size_t)n;
+  float2 *dst = out + (z * na + v) * (size_t)w2;
+  for (int e = threadIdx.x; e < w2; e += blockDim.x) {
+    const int t = e - pads;
+    dst[e] = make_float2(t >= 0 && t < 2 * nh ? g.wt * __ldg(src + t) : 0.0f,
+                         t + 1 >= 0 && t + 1 < 2 * nh ? g.wt * __ldg(src + t + 1) : 0.0f);
   }
 }
 
-__global__ void __launch_bounds__(256) ss_adjoint_kernel(
-    const float *__restrict__ sino, float *__restrict__ img, const SsAngle *__restrict__ tab,
-    const int2 *__restrict__ lim, int n, int nh, int na, AdjEpi ep) {
-  __shared__ SsAngle stab[kSsChunk];
-  __shared__ float cbs[kSsChunk];  // 1 / rb (cos or sin)
-  const int C0 = (blockIdx.x * blockDim.x + threadIdx.x) * kSsPix;
-  const int R0 = (blockIdx.y * blockDim.y + threadIdx.y) * kSsPix;
-  const size_t z = blockIdx.z;
-  const float *S = sino + z * (size_t)na * n;
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = blockDim.x * blockDim.y;
-  const int nt = 2 * nh;
-  float acc[kSsPix][kSsPix];
+// Adjoint: a lane holds 4 x 4 pixels of a 32 x 16 tile; warp q of a block's Q
+// sums every Q-th angle from q on (the costlier angles near an axis go to all),
+// and the sums are added in order.  Q depends on n alone.
+//
+// At a pixel's major coordinate m the rays' minor coordinates f(t) = fma(-m, a,
+// t) * rb lie |rb| = 1 / |cb| >= 1 apart, so a ray within 1 of the pixel's minor
+// coordinate c is within |cb| <= 1 of the crossing t* of c: it is floor(t*) or
+// the next.  Each has weight wt (1 - |f - c|), exactly the forward's (f - floor
+// f or floor f + 1 - f).  A rounding of t* across an integer loses nothing while
+// |cb| < 1 by more than that rounding (below n 2^-22 in all); the few angles
+// nearer to an axis (NEAR) look at the rays before and behind too.  The two
+// rays come as one pair, evaluated as packed operations.
+//
+// The ray's own limits (EDGE) matter only next to the border: at a pixel 4 or
+// more inside the square both rays are inside it.
+//
+// Bound by FP32 and issue.  Candidate rays checked one by one against their
+// limits, each credited to 4 pixels by 8 tests, took 3.53 ms at 4 x 641^2 x
+// 600 and 18.1 at 2048^2 x 1800; this takes 1.22 and 6.5.
+// Whether ray t passes major coordinate m (without branches: the loads of a
+// block's rays overlap).
+__device__ __forceinline__ bool ss_in_limits(const int2 *__restrict__ lrow, int t, int m, int nh) {
+  const int2 l = __ldg(lrow + min(max(t, -nh), nh - 1) + nh);
+  return (t >= -nh) & (t < nh) & (m >= l.x) & (m < l.y);
+}
+
+template <bool STEEP, bool EDGE, bool NEAR>
+__device__ __forceinline__ void ss_adj_angle(const SsAngle &g, const float2 *__restrict__ row, const int2 *__restrict__ lrow,
+                                             int a0, int b0, int nh, float (&acc)[4][4]) {
+  const int M0 = (STEEP ? a0 : b0) - nh, C0 = (STEEP ? b0 : a0) - nh;  // major and minor coordinates of the block
+  const float cb = 1.0f / g.rb;
+  const F2 rb = f2(g.rb), a = f2(g.a), step = f2(0.0f, 1.0f);
 #pragma unroll
-  for (int i = 0; i < kSsPix; ++i)
+  for (int i = 0; i < 4; ++i) {  // along the major axis
+    const float m = (float)(M0 + i), ma = m * g.a;
+    const F2 nm = f2(-m);
 #pragma unroll
-    for (int j = 0; j < kSsPix; ++j) acc[i][j] = 0.0f;
-  for (int v0 = 0; v0 < na; v0 += kSsChunk) {
-    const int cnt = min(kSsChunk, na - v0);
-    __syncthreads();
-    for (int t = tid; t < cnt; t += nthr) {
-      stab[t] = tab[v0 + t];
-      cbs[t] = 1.0f / tab[v0 + t].rb;
-    }
-    __syncthreads();
-    if (R0 >= n || C0 >= n) continue;
-    for (int u = 0; u < cnt; ++u) {
-      const SsAngle g = stab[u];
-      const float cb = cbs[u];
-      const int v = v0 + u;
-      const float *row = S + (size_t)g.out_row * n;
-      const int2 *lrow = lim + (size_t)v * nt;
-      if (g.steep) {  // major axis y: row R is m = R - nh, minor = column
-#pragma unroll
-        for (int i = 0; i < kSsPix; ++i)
-          ss_adj_group(g, cb, R0 + i - nh, C0, nh, row, lrow, acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-      } else {  // major axis x: column C is m = C - nh, minor = row
-#pragma unroll
-        for (int j = 0; j < kSsPix; ++j)
-          ss_adj_group(g, cb, C0 + j - nh, R0, nh, row, lrow, acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
+    for (int j = 0; j < 4; ++j) {  // along the minor axis
+      const float c = (float)(C0 + j);
+      const float fm = __fadd_rd(fmaf(c, cb, ma), kSsMagic);  // first ray
+      const float2 S = __ldg(row + __float_as_int(fm));
+      const F2 t = add2(f2(__fsub_rn(fm, kSsMagic)), step);
+      const float2 f = unpack(mul2(fma2(nm, a, t), rb));  // scalar from here: see f32x2.cuh
+      const float h0 = 1.0f - fabsf(__fsub_rn(f.x, c)), h1 = 1.0f - fabsf(__fsub_rn(f.y, c));
+      const int ti = __float_as_int(fm) - kSsMagicBits;
+      float &o = STEEP ? acc[i][j] : acc[j][i];
+      if (NEAR) {
+        const float h = 1.0f - fabsf(__fsub_rn(__fmul_rn(__fmaf_rn(-m, g.a, __fsub_rn(fm, kSsMagic) - 1.0f), g.rb), c));
+        if (h > 0.0f && (!EDGE || ss_in_limits(lrow, ti - 1, M0 + i, nh))) o = fmaf(h, __ldg(row + __float_as_int(fm) - 1).x, o);
+      }
+      const bool in0 = EDGE ? ss_in_limits(lrow, ti, M0 + i, nh) : true, in1 = EDGE ? ss_in_limits(lrow, ti + 1, M0 + i, nh) : true;
+      if ((h0 > 0.0f) & in0) o = fmaf(h0, S.x, o);
+      if ((h1 > 0.0f) & in1) o = fmaf(h1, S.y, o);
+      if (NEAR) {
+        const float h = 1.0f - fabsf(__fsub_rn(__fmul_rn(__fmaf_rn(-m, g.a, __fsub_rn(fm, kSsMagic) + 2.0f), g.rb), c));
+        if (h > 0.0f && (!EDGE || ss_in_limits(lrow, ti + 2, M0 + i, nh))) o = fmaf(h, __ldg(row + __float_as_int(fm) + 1).y, o);
       }
     }
   }
+}
+
+template <int Q>
+__global__ void __launch_bounds__(32 * Q) ss_adjoint_kernel(const float2 *__restrict__ pairs, float *__restrict__ img,
+                                                            const SsAngle *__restrict__ tab, const int2 *__restrict__ lim,
+                                                            int n, int nh, int na, int pads, int w2, AdjEpi ep) {
+  __shared__ float part[(Q - 1) * 16][32];
+  const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+  // the tiles of the border take longest: both border rows of tiles first
+  const int by = blockIdx.y == 0 ? 0 : blockIdx.y == 1 ? gridDim.y - 1 : blockIdx.y - 1;
+  const int b0 = blockIdx.x * 32 + 4 * (lane & 7), a0 = by * 16 + 4 * (lane >> 3);
+  const size_t z = blockIdx.z;
+  float acc[4][4];
 #pragma unroll
-  for (int i = 0; i < kSsPix; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < kSsPix; ++j) {
-      const int R = R0 + i, C = C0 + j;
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+  // the tile's pixels are all 4 or more inside the square [0, 2 nh - 1]
+  const bool edge = blockIdx.x * 32 < 4 || by * 16 < 4 || blockIdx.x * 32 + 36 > 2 * nh || by * 16 + 20 > 2 * nh;
+  if (a0 < n && b0 < n) {
+    const float near = 1.0f - (float)n * 0x1p-22f;
+    const float2 *row = pairs + (z * na + q) * (size_t)w2 + pads + nh - kSsMagicBits;
+    const int2 *lrow = lim + (size_t)q * 2 * nh;
+#pragma unroll 1
+    for (int u = q; u < na; u += Q, row += (size_t)Q * w2, lrow += (size_t)Q * 2 * nh) {
+      const SsAngle g = tab[u];
+      const bool nr = fabsf(g.rb) * near < 1.0f;
+      if (nr) {
+        if (g.steep) ss_adj_angle<true, true, true>(g, row, lrow, a0, b0, nh, acc);
+        else ss_adj_angle<false, true, true>(g, row, lrow, a0, b0, nh, acc);
+      } else if (edge) {
+        if (g.steep) ss_adj_angle<true, true, false>(g, row, lrow, a0, b0, nh, acc);
+        else ss_adj_angle<false, true, false>(g, row, lrow, a0, b0, nh, acc);
+      } else {
+        if (g.steep) ss_adj_angle<true, false, false>(g, row, lrow, a0, b0, nh, acc);
+        else ss_adj_angle<false, false, false>(g, row, lrow, a0, b0, nh, acc);
+      }
+    }
+  }
+  if (q > 0)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) part[(q - 1) * 16 + 4 * i + j][lane] = acc[i][j];
+  __syncthreads();
+  if (q > 0) return;
+#pragma unroll
+  for (int r = 0; r < Q - 1; ++r)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] += part[r * 16 + 4 * i + j][lane];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int R = a0 + i, C = b0 + j;
       const bool live = R < n && C < n;
       adj_store(ep, acc[i][j], live, z * (size_t)n * n + (live ? (size_t)R * n + C : 0), img);
     }
+}
+
+// Warps of an adjoint tile: more shares of the angles where the tiles alone
+// leave the SMs short of warps.
+int ss_adj_warps(int n) { return n > 640 ? 4 : n > 384 ? 8 : 16; }
+
+struct SsState {
+  float2 *pairs = nullptr;                 // [nz][na][w2]
+  float *rows = nullptr, *cols = nullptr;  // [nz][n][n + 2 kSsFrame]
+  int pads = 0, w2 = 0;
+};
+
+void ss_state_free(void *q) {
+  auto *st = (SsState *)q;
+  cudaFree(st->pairs);
+  delete st;
 }
 
 static void sort4(float *a) {
@@ -228,27 +314,46 @@ int ss_setup(Plan &p) {
   TOMO_CUDA(cudaMemcpy(p.d_angles, tab.data(), sizeof(SsAngle) * (size_t)na, cudaMemcpyHostToDevice));
   TOMO_CUDA(cudaMalloc(&p.d_aux, sizeof(int2) * lim.size()));
   TOMO_CUDA(cudaMemcpy(p.d_aux, lim.data(), sizeof(int2) * lim.size(), cudaMemcpyHostToDevice));
-  p.scratch_bytes = sizeof(float) * image_elems(p);
-  TOMO_CUDA(cudaMalloc(&p.d_scratch, p.scratch_bytes));
+  auto *st = new SsState();
+  p.ext = st;
+  p.ext_free = ss_state_free;
+  // |t| at a pixel stays below sqrt(2) (nh + 1) + 2, also for the pixels of a
+  // tile that lie up to 3 outside the image
+  st->pads = (int)std::ceil((nh + 1) * 0.41422) + 14;
+  st->w2 = 2 * nh + 2 * st->pads;
+  // one workspace: the adjoint's pairs, then the forward's framed copies
+  const int n = p.g.n;
+  const size_t pairs = (size_t)p.g.nz * na * st->w2, framed = (size_t)p.g.nz * n * (n + 2 * kSsFrame);
+  TOMO_CUDA(cudaMalloc(&st->pairs, sizeof(float2) * pairs + 2 * sizeof(float) * framed));
+  st->rows = (float *)(st->pairs + pairs);
+  st->cols = st->rows + framed;
+  // residual partials of the fused solvers: one per 32 rays
+  const int rays = 128 / ss_fwd_split(n);
+  p.fwd_warps = (size_t)((n + rays - 1) / rays) * (rays / 32) * na * p.g.nz;
   return TOMO_OK;
 }
 
 int ss_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const FwdEpi &ep) {
   const int n = p.g.n, na = p.g.na, nz = p.g.nz, nh = p.nh;
-  dim3 tb(32, 8), tg((n + 31) / 32, (n + 31) / 32, nz);
-  ss_transpose_kernel<<<tg, tb, 0, s>>>(d_img, p.d_scratch, n);
-  dim3 fb(128), fg((n + 127) / 128, na, nz);
-  ss_forward_kernel<<<fg, fb, 0, s>>>(d_img, p.d_scratch, d_sino, (const SsAngle *)p.d_angles,
-                                      (const int2 *)p.d_aux, n, nh, na, ep);
+  SsState &st = *(SsState *)p.ext;
+  const int tiles = (n + 2 * kSsFrame + 31) / 32;
+  ss_frame_kernel<<<dim3(tiles, tiles, nz), dim3(32, 8), 0, s>>>(d_img, st.rows, st.cols, n);
+  const int split = ss_fwd_split(n), rays = 128 / split;
+  auto fn = split == 4 ? ss_forward_kernel<4> : ss_forward_kernel<2>;
+  fn<<<dim3((n + rays - 1) / rays, na, nz), 128, 0, s>>>(st.rows, st.cols, d_sino, (const SsAngle *)p.d_angles,
+                                                         (const int2 *)p.d_aux, n, nh, na, ep);
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
 }
 
 int ss_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const AdjEpi &ep) {
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
-  dim3 ab(32, 8), ag((n + 32 * kSsPix - 1) / (32 * kSsPix), (n + 8 * kSsPix - 1) / (8 * kSsPix), nz);
-  ss_adjoint_kernel<<<ag, ab, 0, s>>>(d_sino, d_img, (const SsAngle *)p.d_angles,
-                                      (const int2 *)p.d_aux, n, p.nh, na, ep);
+  SsState &st = *(SsState *)p.ext;
+  ss_expand_kernel<<<dim3(na, nz), 256, 0, s>>>(d_sino, st.pairs, (const SsAngle *)p.d_angles, n, p.nh, na, st.pads, st.w2);
+  const int Q = ss_adj_warps(n);
+  auto fn = Q == 4 ? ss_adjoint_kernel<4> : Q == 8 ? ss_adjoint_kernel<8> : ss_adjoint_kernel<16>;
+  fn<<<dim3((n + 31) / 32, (n + 15) / 16, nz), 32 * Q, 0, s>>>(st.pairs, d_img, (const SsAngle *)p.d_angles,
+                                                               (const int2 *)p.d_aux, n, p.nh, na, st.pads, st.w2, ep);
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
 }
