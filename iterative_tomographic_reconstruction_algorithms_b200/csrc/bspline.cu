@@ -11,10 +11,11 @@
 // lut[angle][li].  ds = (int)(support/2 + 0.5), lut_step = (lut_size/2) /
 // (support/2).  The table itself is built on the host (bspline_functions.py).
 //
-// Forward = per (angle, block of bins) a pass over the band of pixels whose
-// taps can reach the bins, summed in fixed point; adjoint = gather
-// per pixel over angles and taps.  Output rows follow the angle order (no
-// reversal).
+// Forward = gather per bin over image lines, adjoint = gather per pixel over
+// angles, for tables of support 4 and power-of-two length; otherwise forward =
+// per (angle, block of bins) a pass over the band of pixels whose taps can reach
+// the bins, summed in fixed point, and adjoint = gather per pixel over angles
+// and taps.  Output rows follow the angle order (no reversal).
 #include <algorithm>
 #include <cmath>
 
@@ -204,6 +205,364 @@ __global__ void __launch_bounds__(256) bs_adjoint_kernel(
   adj_store(ep, acc, live, z * (size_t)n * n + (size_t)(live ? kyi : 0) * n + (live ? kxi : 0), img);
 }
 
+// ---------------------------------------------------------------------------
+// Tables with support 4 and a power-of-two length (the class's default: 2048)
+// ---------------------------------------------------------------------------
+// The step of the table index is then a power of two, so (y - ps) * step is
+// exact, and the index is a function of the exact distance d = y - ps.  fl(s +
+// ps) is exact too unless |ps| < 4 or s carries |ps| across a power of two: a
+// tap's bin is otherwise floor(s + ps) + n/2, every bin within reach gets one
+// tap, and the index alone decides whether it counts.  What is left (pixels
+// close to an integer there, and bin 0, onto which the truncation folds bin -1)
+// goes through the reference's rule tap by tap (bs_bin).  Other tables and
+// images above 4096^2 take the general kernels above.
+constexpr float kBsMagic = 12582912.0f;   // 1.5 * 2^23
+constexpr int kBsMagicBits = 0x4B400000;  // its bit pattern
+constexpr int kBsFrame = 8;
+
+// Framed copies of the image: rows[ky_i][P + kx_i] and cols[kx_i][P + ky_i],
+// P = kBsFrame zeros on either side.
+__global__ void __launch_bounds__(256) bs_frame_kernel(const float *__restrict__ img, float *__restrict__ rows,
+                                                       float *__restrict__ cols, int n) {
+  __shared__ float tile[32][33];
+  const size_t z = blockIdx.z;
+  const int w = n + 2 * kBsFrame;
+  const float *src = img + z * (size_t)n * n;
+  float *R = rows + z * (size_t)n * w, *C = cols + z * (size_t)n * w;
+  const int x0 = blockIdx.x * 32 - kBsFrame, y0 = blockIdx.y * 32 - kBsFrame;  // tiles cover the frame too
+  for (int dy = threadIdx.y; dy < 32; dy += 8) {
+    const int y = y0 + dy, x = x0 + threadIdx.x;
+    const float v = y >= 0 && y < n && x >= 0 && x < n ? __ldg(src + (size_t)y * n + x) : 0.0f;
+    tile[dy][threadIdx.x] = v;
+    if (y >= 0 && y < n && x < n + kBsFrame) R[(size_t)y * w + kBsFrame + x] = v;
+  }
+  __syncthreads();
+  for (int dy = threadIdx.y; dy < 32; dy += 8) {
+    const int x = x0 + dy, y = y0 + threadIdx.x;
+    if (x >= 0 && x < n && y < n + kBsFrame) C[(size_t)x * w + kBsFrame + y] = tile[threadIdx.x][dy];
+  }
+}
+
+// Whether bin y (from the centre) is reached by pixels whose taps' bins may not
+// be floor(s + ps): |ps| < 4, or |ps| within 2 below a power of two.
+__device__ __forceinline__ bool bs_special(float y) {
+  const float a = fabsf(y);
+  if (a < 8.0f) return true;
+  const float p = __int_as_float(__float_as_int(a) & 0x7f800000);  // 2^e <= a
+  return a - p < 4.0f || 2.0f * p - a < 6.0f;
+}
+
+// Above the rounding of fl(s + ps), |ps| <= n/sqrt(2) + 2.
+__device__ __forceinline__ float bs_near(int n) { return (float)(n + 8) * 0x1p-24f; }
+
+// The six pixels of a line and bin b, each with the number of taps that the
+// reference puts into the bin (0, 1 or 2).
+template <bool ROWS, int DIR>
+__device__ __noinline__ float bs_fwd_taps(const float *v, const float *tab, int entries, unsigned org, float u0, float l, float C,
+                                          float S, int b, const BsConst &k) {
+  float p = 0.0f;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    const float u = u0 + (float)(q * DIR);
+    const float ps = ROWS ? __fmaf_rn(u, C, l) : __fmaf_rn(l, C, __fmul_rn(S, -u));
+    const float d = __fsub_rn((float)b - k.fmid, ps);
+    const unsigned fl = __float_as_uint(__fmaf_rd(d, k.lut_step, kBsMagic)), ce = __float_as_uint(__fmaf_ru(d, k.lut_step, kBsMagic));
+    const float wt = tab[min(fl + ce + org, (unsigned)entries)];
+    const float s0 = rintf(d);  // a tap on the bin is within 1 of the distance
+    int m = 0;
+#pragma unroll
+    for (int s = -1; s <= 1; ++s) {
+      const float t = s0 + (float)s;
+      m += (fabsf(t) <= 2.0f) & (bs_bin((int)t, ps, k.mid) == b);
+    }
+    if (wt == wt && m) p = fmaf(wt * (float)m, __ldg(v + q * DIR), p);
+  }
+  return p;
+}
+
+// Forward: a lane owns a bin and walks the lines (ROWS: image rows, when ps
+// moves faster along x; else columns).  Per line the pixels with |y - ps| < 2
+// (+ 1 table step) are among six consecutive ones, sigma = max(|C|, |S|) in
+// [0.707, 1] apart (a seventh would lie 6 x 0.707 > 4.03 behind the first).
+// The angle's table is in shared memory by half steps of the distance, with the
+// index's truncation toward zero applied: entry floor(a) + ceil(a), a = d *
+// step, needs no conversion.  MODE 1: some of the warp's bins are special, 2:
+// it holds bin 0, whose pixels count twice (the reference's truncation folds
+// the tap on bin -1 onto it).  Six products of a line are added in float, lines
+// in double, rounded once.
+//
+// Bound by shared memory: six reads at the lanes' own phases, about 3.5 bank
+// conflicts each.  Adding every tap to 64-bit fixed-point sums by two
+// shared-memory atomics took 2.15 ms at 768^2 x 720 and 31.7 at 2048^2 x 1800;
+// this takes 1.46 and 22.2.
+template <bool ROWS, int DIR, int MODE>
+__device__ __forceinline__ double bs_fwd_bin(const float *__restrict__ L, const float *tab, int entries, int w, float C, float S,
+                                             int b, const BsConst &k, int i0, int i1) {
+  const float fmid = k.fmid, y = (float)b - fmid, step = k.lut_step;
+  const float inv = 1.0f / (ROWS ? C : -S);  // 1 / (ps per pixel)
+  // pixel at which ps = y - 2 - 1/64
+  const float base = (y - 2.015625f) * inv + fmid, slope = -(ROWS ? S : C) * inv;
+  const float lo = DIR > 0 ? -8.0f : -3.0f, hi = DIR > 0 ? (float)(k.n + 2) : (float)(k.n + 7);
+  const float *line = L + (size_t)i0 * w + kBsFrame - kBsMagicBits;
+  const unsigned org = (unsigned)entries / 2u - 2u * (unsigned)kBsMagicBits;  // entry of distance 0
+  float lc = ROWS ? fmid - (float)i0 : (float)i0 - fmid;
+  const float thr = bs_special(y) ? bs_near(k.n) : -1.0f;
+  const bool twice = b == 0;  // a tap on bin -1 folds onto bin 0, where the next tap lies
+  double acc = 0.0;
+#pragma unroll 1
+  for (int i = i0; i < i1; ++i, line += w, lc += ROWS ? -1.0f : 1.0f) {
+    const float pos = fminf(fmaxf(fmaf(slope, lc, base), lo), hi);
+    const float fm = DIR > 0 ? __fadd_ru(pos, kBsMagic) : __fadd_rd(pos, kBsMagic);  // the first of the six
+    const float *v = line + __float_as_int(fm);
+    const float u0 = __fsub_rn(__fsub_rn(fm, kBsMagic), fmid);
+    const float so = ROWS ? __fmul_rn(S, lc) : 0.0f;
+    float p = 0.0f, near = 1.0f;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      const float u = u0 + (float)(q * DIR);
+      const float ps = ROWS ? __fmaf_rn(u, C, so) : __fmaf_rn(lc, C, __fmul_rn(S, -u));
+      const float d = __fsub_rn(y, ps);
+      const unsigned fl = __float_as_uint(__fmaf_rd(d, step, kBsMagic)), ce = __float_as_uint(__fmaf_ru(d, step, kBsMagic));
+      const float wt = tab[min(fl + ce + org, (unsigned)entries)];  // outside: the NaN behind the table
+      const float x = __ldg(v + q * DIR);
+      if (wt == wt) p = fmaf(wt, x, p);
+      if (MODE > 0) {
+        const float r = fabsf(__fsub_rn(d, __fsub_rn(__fadd_rn(d, kBsMagic), kBsMagic)));
+        near = fminf(near, r);
+        if (MODE > 1 && twice && wt == wt && d > -2.0f && r > 0.0f) p = fmaf(wt, x, p);
+      }
+    }
+    if (MODE > 0 && near < thr) p = bs_fwd_taps<ROWS, DIR>(v, tab, entries, org, u0, ROWS ? so : lc, C, S, b, k);
+    acc += (double)p;
+  }
+  return acc;
+}
+
+// A block takes 128 / SPLIT bins of an angle, SPLIT warps sharing each bin's
+// lines (added in order): lines of very unequal number per bin then balance
+// better (513^2 x 400: 0.75 ms unsplit, 0.43 by four; 2048^2 x 1800 the same by
+// two).  The split is a function of n alone (bs_fwd_split).
+template <int SPLIT>
+__global__ void __launch_bounds__(128) bs_forward_pow2_kernel(const float *__restrict__ rows, const float *__restrict__ cols,
+                                                              float *__restrict__ sino, const float2 *__restrict__ cs,
+                                                              const float *__restrict__ lut, int entries, BsConst k, FwdEpi ep) {
+  extern __shared__ float tab[];  // [entries] by half steps, distances within 2 (+ 2 steps); NaN where no tap counts
+  __shared__ double part[SPLIT][128 / SPLIT];
+  constexpr int kBins = 128 / SPLIT;
+  const int lane = threadIdx.x % kBins, q = threadIdx.x / kBins;
+  const int b = blockIdx.x * kBins + lane, v = blockIdx.y, n = k.n, w = n + 2 * kBsFrame;
+  const size_t z = blockIdx.z;
+  const float *Lv = lut + (size_t)v * k.lut_size;
+  const int org = entries / 2;
+  for (int e = threadIdx.x; e <= entries; e += 128) {
+    const int i2 = e - org;                    // floor(a) + ceil(a)
+    const int li = (i2 >= 0 ? i2 >> 1 : -(-i2 >> 1)) + k.lut_half;  // toward zero
+    tab[e] = e < entries && li >= 0 && li < k.lut_max ? __ldg(Lv + li) : __int_as_float(0x7fffffff);
+  }
+  __syncthreads();
+  const float C = cs[v].x, S = cs[v].y;
+  const bool by_rows = fabsf(C) >= fabsf(S);
+  const int W0 = blockIdx.x * kBins + (lane & ~31);  // the warp's first bin
+  // lines whose ps range, o l +- |K| (n/2 + 1), meets the warp's bins
+  const float K = fabsf(by_rows ? C : S), o = by_rows ? S : C, half = K * (k.fmid + 2.0f);
+  int i0 = 0, i1 = n;
+  if (fabsf(o) > 1e-4f) {
+    const float y0 = (float)W0 - k.fmid - 3.0f - half, y1 = (float)(W0 + 31) - k.fmid + 3.0f + half;
+    const float l0 = fminf(y0 / o, y1 / o), l1 = fmaxf(y0 / o, y1 / o);
+    const float j0 = by_rows ? k.fmid - l1 : l0 + k.fmid, j1 = by_rows ? k.fmid - l0 : l1 + k.fmid;
+    i0 = (int)floorf(fminf(fmaxf(j0 - 2.0f, 0.0f), (float)n));
+    i1 = (int)ceilf(fminf(fmaxf(j1 + 2.0f, 0.0f), (float)n));
+  }
+  if (SPLIT > 1) {
+    const int len = max(0, i1 - i0);
+    i1 = i0 + len * (q + 1) / SPLIT;
+    i0 += len * q / SPLIT;
+  }
+  const float *L = (by_rows ? rows : cols) + z * (size_t)n * w;
+  const bool spec = __any_sync(0xffffffffu, bs_special((float)b - k.fmid)), first = __any_sync(0xffffffffu, b == 0);
+  double acc;
+#define BS_BIN(R, D) (first  ? bs_fwd_bin<R, D, 2>(L, tab, entries, w, C, S, b, k, i0, i1) \
+                      : spec ? bs_fwd_bin<R, D, 1>(L, tab, entries, w, C, S, b, k, i0, i1) \
+                             : bs_fwd_bin<R, D, 0>(L, tab, entries, w, C, S, b, k, i0, i1))
+  if (by_rows) acc = C > 0.0f ? BS_BIN(true, 1) : BS_BIN(true, -1);
+  else acc = S < 0.0f ? BS_BIN(false, 1) : BS_BIN(false, -1);
+#undef BS_BIN
+  if (SPLIT > 1) {
+    part[q][lane] = acc;
+    __syncthreads();
+    if (q > 0) return;  // warp-uniform
+    for (int r = 1; r < SPLIT; ++r) acc += part[r][lane];
+  }
+  double r2 = 0.0;
+  const size_t e = z * (size_t)k.na * n + (size_t)v * n + b;
+  if (b < n) sino[e] = fwd_apply(ep, (float)acc, e, r2);
+  const size_t block = ((size_t)z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  fwd_resid_commit(ep, r2, block * (kBins / 32) + lane / 32);
+}
+
+int bs_fwd_split(int n) { return n > 1024 ? 2 : 4; }
+
+// The adjoint's table of an angle, by half steps of the fraction of ps: entry
+// floor(f) + ceil(f), f = (ps - floor ps) step in (0, step), holds the four taps'
+// weights, distances k - f / step for k = -1 .. 2.
+__global__ void bs_lut4_kernel(const float *__restrict__ lut, float4 *__restrict__ out, BsConst k) {
+  const float *L = lut + (size_t)blockIdx.x * k.lut_size;
+  const int step = (int)k.lut_step;
+  for (int i = threadIdx.x; i < 2 * step; i += blockDim.x) {
+    const int fl = i >> 1, ce = (i + 1) >> 1;
+    const int li[4] = {step - fl, 2 * step - fl, 3 * step - ce, 4 * step - ce};
+    float v[4];
+    for (int t = 0; t < 4; ++t) v[t] = li[t] >= 0 && li[t] < k.lut_max ? L[li[t]] : 0.0f;
+    out[(size_t)blockIdx.x * 2 * step + i] = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
+// Sinogram rows as groups, entry e = m + pads: {S_m-1, S_m, S_m+1, S_m+2}, 0
+// outside [0, n); bin 0 twice, for the tap on bin -1 that folds onto it with
+// the same weight.
+__global__ void __launch_bounds__(256) bs_expand_kernel(const float *__restrict__ sino, float4 *__restrict__ out, int n, int pads,
+                                                        int w2) {
+  const float *src = sino + (size_t)blockIdx.x * n;
+  float4 *dst = out + (size_t)blockIdx.x * w2;
+  for (int e = threadIdx.x; e < w2; e += blockDim.x) {
+    float v[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const int m = e - pads - 1 + t;
+      v[t] = m >= 0 && m < n ? __ldg(src + m) : 0.0f;
+      if (m == 0) v[t] *= 2.0f;
+    }
+    dst[e] = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
+// One angle's taps of a pixel by the reference's rule.
+__device__ __noinline__ float bs_adj_taps(float ps, const float *__restrict__ row, const float *__restrict__ L, const BsConst &k,
+                                          float acc) {
+  for (int s = -2; s <= 2; ++s) {
+    const int yi = bs_bin(s, ps, k.mid);
+    if (yi >= k.n || yi < 0) continue;
+    const int li = bs_lut(yi, ps, k);
+    if (li >= k.lut_max || li < 0) continue;
+    acc = fmaf(__ldg(row + yi), __ldg(L + li), acc);
+  }
+  return acc;
+}
+
+__device__ __forceinline__ bool bs_near_step(float f) { return fabsf(f - rintf(f)) < 0x1p-12f; }
+
+// Adjoint: a block holds a 64 x 32 pixel tile, 4 rows per lane, and goes
+// through its share of the angles with the angle's table of four weights (16
+// KB) in shared memory, the next one on its way in registers.  A pixel and
+// angle: floor of ps, one 16-byte read of four bins, one of four weights.
+// Q shares of the angles for small images, whose tiles alone
+// do not fill the SMs, added in order by bs_adj_sum_kernel (Q depends on n).
+//
+// Bound by L1 / shared memory: the weight reads are at the lanes' own phases
+// (about 11 wavefronts), the bins' about 5.  A thread per pixel with five table
+// reads from L1, each at its own line, took 3.04 ms at 768^2 x 720 and 46.3 at
+// 2048^2 x 1800; this 1.28 and 22.0.
+constexpr int kBsTW = 64, kBsTH = 32, kBsThreads4 = 512;
+
+template <bool ODD>
+__global__ void __launch_bounds__(kBsThreads4) bs_adjoint_pow2_kernel(const float *__restrict__ sino, const float4 *__restrict__ S4,
+                                                                      const float4 *__restrict__ lut4,
+                                                                      const float *__restrict__ lut, float *__restrict__ img,
+                                                                      const float2 *__restrict__ cs, BsConst k, int pads, int w2,
+                                                                      int Q, float *__restrict__ partial, AdjEpi ep) {
+  extern __shared__ float4 tab4[];
+  const int n = k.n, nh = n / 2, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const size_t z = blockIdx.z;
+  const int q = blockIdx.x % Q;
+  const int b0 = blockIdx.x / Q * kBsTW + 32 * (warp & 1) + lane, a0 = blockIdx.y * kBsTH + 4 * (warp >> 1);
+  const int u0 = (int)((long long)k.na * q / Q), u1 = (int)((long long)k.na * (q + 1) / Q);
+  const int entries = 2 * (int)k.lut_step;
+  const float step = k.lut_step, x0 = (float)b0 - k.fmid, y0 = k.fmid - (float)a0;
+  const float edge = 1.0f / step;
+  float acc[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc[i] = 0.0f;
+  const float near = bs_near(n);
+  const bool inside = a0 < n && b0 < n;
+  constexpr int kPer = 2;  // entries of a thread: tables of up to 1024 entries
+  float4 next[kPer];
+  auto fetch = [&](int u) {
+#pragma unroll
+    for (int r = 0; r < kPer; ++r)
+      if (tid + r * kBsThreads4 < entries) next[r] = __ldg(lut4 + (size_t)u * entries + tid + r * kBsThreads4);
+  };
+  if (u0 < u1) fetch(u0);
+#pragma unroll 1
+  for (int u = u0; u < u1; ++u) {
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kPer; ++r)
+      if (tid + r * kBsThreads4 < entries) tab4[tid + r * kBsThreads4] = next[r];
+    __syncthreads();
+    if (u + 1 < u1) fetch(u + 1);
+    if (!inside) continue;
+    const float2 g = __ldg(cs + u);
+    const float L0 = __ldg(lut + (size_t)u * k.lut_size);
+    const float *srow = sino + (z * k.na + u) * (size_t)n;
+    const float4 *row = S4 + (z * k.na + u) * (size_t)w2 + pads + nh - kBsMagicBits;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float ps = __fmaf_rn(x0, g.x, __fmul_rn(g.y, y0 - (float)i));
+      const float fd = __fadd_rd(ODD ? __fadd_rn(ps, 0.5f) : ps, kBsMagic);
+      const float frac = __fsub_rn(ps, __fsub_rn(__fsub_rn(fd, kBsMagic), ODD ? 0.5f : 0.0f));
+      const unsigned e = __float_as_uint(__fmaf_rd(frac, step, kBsMagic)) + __float_as_uint(__fmaf_ru(frac, step, kBsMagic)) -
+                         2u * (unsigned)kBsMagicBits;
+      const float4 *sp = row + __float_as_int(fd);
+      const float4 s = __ldg(sp), w = tab4[min(e, (unsigned)entries - 1u)];
+      float o = acc[i];
+      if (frac < edge) {  // the tap at distance -2 counts too (on bin 0 once)
+        const int m = __float_as_int(fd) - kBsMagicBits + nh - 2;
+        if (m >= 0 && m < n) o = fmaf(__ldg(srow + m), L0, o);
+      }
+      o = fmaf(s.x, w.x, o);
+      o = fmaf(s.y, w.y, o);
+      o = fmaf(s.z, w.z, o);
+      if (frac > edge) o = fmaf(s.w, w.w, o);  // else the table has ended
+      // |ps| < 4, where y - ps rounds, next to a table step; next to an integer
+      // where fl(s + ps) may round across it; an integral ps next to bin 0, onto
+      // which nothing folds then
+      if ((fabsf(ps) < 4.0f && bs_near_step(frac * step)) ||
+          (fabsf(frac - 0.5f) > 0.5f - near && (bs_special(ps) || ps < 4.0f - k.fmid)))
+        o = bs_adj_taps(ps, srow, lut + (size_t)u * k.lut_size, k, acc[i]);
+      acc[i] = o;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int R = a0 + i;
+    const bool live = R < n && b0 < n;
+    const size_t p = z * (size_t)n * n + (live ? (size_t)R * n + b0 : 0);
+    if (Q > 1) {
+      if (live) partial[(size_t)q * gridDim.z * n * n + p] = acc[i];
+    } else {
+      adj_store(ep, acc[i], live, p, img);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) bs_adj_sum_kernel(const float *__restrict__ partial, int Q, size_t total, float *__restrict__ img,
+                                                         AdjEpi ep) {
+  const size_t p = (size_t)blockIdx.x * 256 + threadIdx.x;
+  const bool live = p < total;
+  float acc = 0.0f;
+  if (live)
+    for (int q = 0; q < Q; ++q) acc += partial[(size_t)q * total + p];
+  adj_store(ep, acc, live, live ? p : 0, img);
+}
+
+// Shares of the angles: blocks enough for four rounds of two to an SM, since
+// those at the rim finish early (768^2 x 720: 1.90 ms with 288 blocks, 1.28 with
+// 1152), at most 16.
+int bs_adj_shares(int n) {
+  const int tiles = ((n + kBsTW - 1) / kBsTW) * ((n + kBsTH - 1) / kBsTH);
+  return std::max(1, std::min(16, 1184 / tiles));
+}
+
 BsConst make_const(const Plan &p) {
   BsConst k{};
   k.n = p.g.n;
@@ -220,12 +579,18 @@ BsConst make_const(const Plan &p) {
 
 struct BsState {
   float lutmax = 0.0f;        // max |lut|
-  unsigned *vmax = nullptr;   // per slice: max |image| as float bits
+  unsigned *vmax = nullptr;   // per slice: max |image| as float bits (general kernels)
+  bool pow2 = false;          // support 4, power-of-two table
+  void *work = nullptr;       // one workspace for what follows
+  float4 *lut4 = nullptr, *S4 = nullptr;
+  float *rows = nullptr, *cols = nullptr, *partial = nullptr;
+  int pads = 0, w2 = 0, Q = 1, entries = 0;
 };
 
 void bs_state_free(void *q) {
   auto *st = (BsState *)q;
   cudaFree(st->vmax);
+  cudaFree(st->work);
   delete st;
 }
 
@@ -254,13 +619,36 @@ int bs_setup(Plan &p) {
   auto *st = new BsState();
   p.ext = st;
   p.ext_free = bs_state_free;
-  for (size_t i = 0; i < (size_t)na * p.g.lut_size; ++i) st->lutmax = std::max(st->lutmax, std::fabs(p.g.lut[i]));
-  TOMO_CUDA(cudaMalloc(&st->vmax, sizeof(unsigned) * (size_t)std::max(1, p.g.nz)));
-  if (sizeof(float) * (size_t)p.g.lut_size > 48 * 1024)
-    TOMO_CUDA(cudaFuncSetAttribute(bs_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(sizeof(float) * (size_t)p.g.lut_size)));
-  // residual partials of the fused solvers: one per warp of the forward launch
-  p.fwd_warps = (size_t)((p.g.n + kBsBins - 1) / kBsBins) * (kBsThreads / 32) * na * p.g.nz;
+  const BsConst k = make_const(p);
+  const int n = p.g.n, L = p.g.lut_size;
+  st->pow2 = p.g.support == 4.0f && (L & (L - 1)) == 0 && L >= 64 && L <= 2048 && n >= 4 && n <= 4096;
+  if (st->pow2) {
+    // |ps| stays below sqrt(2) (n/2 + 1) + 4, also for a tile's pixels outside the image
+    st->pads = (int)std::ceil((p.nh + 1) * 0.41422) + 64;
+    st->w2 = n + 2 * st->pads;
+    st->Q = bs_adj_shares(n);
+    st->entries = 8 * (int)k.lut_step + 8;
+    const size_t nz = p.g.nz, lut4 = (size_t)na * 2 * (size_t)k.lut_step, s4 = nz * na * st->w2;
+    const size_t framed = nz * n * (n + 2 * kBsFrame), part = st->Q > 1 ? st->Q * nz * n * n : 0;
+    TOMO_CUDA(cudaMalloc(&st->work, sizeof(float4) * (lut4 + s4) + sizeof(float) * (2 * framed + part)));
+    st->lut4 = (float4 *)st->work;
+    st->S4 = st->lut4 + lut4;
+    st->rows = (float *)(st->S4 + s4);
+    st->cols = st->rows + framed;
+    st->partial = st->cols + framed;
+    bs_lut4_kernel<<<na, 256>>>((const float *)p.d_aux, st->lut4, k);
+    TOMO_CUDA(cudaGetLastError());
+    TOMO_CUDA(cudaStreamSynchronize(0));  // later calls may come on streams that do not wait for this one
+    const int bins = 128 / bs_fwd_split(n);
+    p.fwd_warps = (size_t)((n + bins - 1) / bins) * (bins / 32) * na * p.g.nz;
+  } else {
+    for (size_t i = 0; i < (size_t)na * L; ++i) st->lutmax = std::max(st->lutmax, std::fabs(p.g.lut[i]));
+    TOMO_CUDA(cudaMalloc(&st->vmax, sizeof(unsigned) * (size_t)std::max(1, p.g.nz)));
+    if (sizeof(float) * (size_t)L > 48 * 1024)
+      TOMO_CUDA(cudaFuncSetAttribute(bs_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * L)));
+    // residual partials of the fused solvers: one per warp of the forward launch
+    p.fwd_warps = (size_t)((n + kBsBins - 1) / kBsBins) * (kBsThreads / 32) * na * p.g.nz;
+  }
   p.g.lut = nullptr;
   return TOMO_OK;
 }
@@ -268,6 +656,15 @@ int bs_setup(Plan &p) {
 int bs_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const FwdEpi &ep) {
   const BsConst k = make_const(p);
   BsState &st = *(BsState *)p.ext;
+  if (st.pow2) {
+    const int n = k.n, tiles = (n + 2 * kBsFrame + 31) / 32, split = bs_fwd_split(n), bins = 128 / split;
+    bs_frame_kernel<<<dim3(tiles, tiles, p.g.nz), dim3(32, 8), 0, s>>>(d_img, st.rows, st.cols, n);
+    auto fn = split == 4 ? bs_forward_pow2_kernel<4> : bs_forward_pow2_kernel<2>;
+    fn<<<dim3((n + bins - 1) / bins, k.na, p.g.nz), 128, sizeof(float) * (st.entries + 1), s>>>(
+        st.rows, st.cols, d_sino, (const float2 *)p.d_angles, (const float *)p.d_aux, st.entries, k, ep);
+    TOMO_CUDA(cudaGetLastError());
+    return TOMO_OK;
+  }
   const size_t per = (size_t)k.n * k.n;
   TOMO_CUDA(cudaMemsetAsync(st.vmax, 0, sizeof(unsigned) * p.g.nz, s));
   fixed_finite_absmax_kernel<<<dim3((unsigned)std::min<size_t>((per + 255) / 256, 1184), p.g.nz), 256, 0, s>>>(d_img, per,
@@ -281,6 +678,22 @@ int bs_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
 
 int bs_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const AdjEpi &ep) {
   const BsConst k = make_const(p);
+  BsState &st = *(BsState *)p.ext;
+  if (st.pow2) {
+    const int n = k.n, nz = p.g.nz;
+    bs_expand_kernel<<<k.na * nz, 256, 0, s>>>(d_sino, st.S4, n, st.pads, st.w2);
+    const dim3 grid((n + kBsTW - 1) / kBsTW * st.Q, (n + kBsTH - 1) / kBsTH, nz);
+    const size_t smem = sizeof(float4) * 2 * (size_t)k.lut_step;
+    auto fn = (n & 1) ? bs_adjoint_pow2_kernel<true> : bs_adjoint_pow2_kernel<false>;
+    fn<<<grid, kBsThreads4, smem, s>>>(d_sino, st.S4, st.lut4, (const float *)p.d_aux, d_img, (const float2 *)p.d_angles, k,
+                                       st.pads, st.w2, st.Q, st.partial, ep);
+    if (st.Q > 1) {
+      const size_t total = (size_t)nz * n * n;
+      bs_adj_sum_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(st.partial, st.Q, total, d_img, ep);
+    }
+    TOMO_CUDA(cudaGetLastError());
+    return TOMO_OK;
+  }
   dim3 ab(32, 8), ag((k.n + 31) / 32, (k.n + 7) / 8, p.g.nz);
   bs_adjoint_kernel<<<ag, ab, 0, s>>>(d_sino, d_img, (const float2 *)p.d_angles,
                                       (const float *)p.d_aux, k, ep);
