@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(256) bs_adjoint_kernel(
 // tap's bin is otherwise floor(s + ps) + n/2, every bin within reach gets one
 // tap, and the index alone decides whether it counts.  What is left (pixels
 // close to an integer there, and bin 0, onto which the truncation folds bin -1)
-// goes through the reference's rule tap by tap (bs_bin).  Other tables and
-// images above 4096^2 take the general kernels above.
+// goes through the reference's rule tap by tap (bs_bin).  Other tables, images above
+// 4096^2 and the solvers (epilogue.cuh) take the general kernels above.
 constexpr float kBsMagic = 12582912.0f;   // 1.5 * 2^23
 constexpr int kBsMagicBits = 0x4B400000;  // its bit pattern
 constexpr int kBsFrame = 8;
@@ -345,7 +345,7 @@ __device__ __forceinline__ double bs_fwd_bin(const float *__restrict__ L, const 
 template <int SPLIT>
 __global__ void __launch_bounds__(128) bs_forward_pow2_kernel(const float *__restrict__ rows, const float *__restrict__ cols,
                                                               float *__restrict__ sino, const float2 *__restrict__ cs,
-                                                              const float *__restrict__ lut, int entries, BsConst k, FwdEpi ep) {
+                                                              const float *__restrict__ lut, int entries, BsConst k) {
   extern __shared__ float tab[];  // [entries] by half steps, distances within 2 (+ 2 steps); NaN where no tap counts
   __shared__ double part[SPLIT][128 / SPLIT];
   constexpr int kBins = 128 / SPLIT;
@@ -393,11 +393,7 @@ __global__ void __launch_bounds__(128) bs_forward_pow2_kernel(const float *__res
     if (q > 0) return;  // warp-uniform
     for (int r = 1; r < SPLIT; ++r) acc += part[r][lane];
   }
-  double r2 = 0.0;
-  const size_t e = z * (size_t)k.na * n + (size_t)v * n + b;
-  if (b < n) sino[e] = fwd_apply(ep, (float)acc, e, r2);
-  const size_t block = ((size_t)z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  fwd_resid_commit(ep, r2, block * (kBins / 32) + lane / 32);
+  if (b < n) sino[z * (size_t)k.na * n + (size_t)v * n + b] = (float)acc;
 }
 
 int bs_fwd_split(int n) { return n > 1024 ? 2 : 4; }
@@ -469,7 +465,7 @@ __global__ void __launch_bounds__(kBsThreads4) bs_adjoint_pow2_kernel(const floa
                                                                       const float4 *__restrict__ lut4,
                                                                       const float *__restrict__ lut, float *__restrict__ img,
                                                                       const float2 *__restrict__ cs, BsConst k, int pads, int w2,
-                                                                      int Q, float *__restrict__ partial, AdjEpi ep) {
+                                                                      int Q, float *__restrict__ partial) {
   extern __shared__ float4 tab4[];
   const int n = k.n, nh = n / 2, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const size_t z = blockIdx.z;
@@ -537,22 +533,16 @@ __global__ void __launch_bounds__(kBsThreads4) bs_adjoint_pow2_kernel(const floa
     const int R = a0 + i;
     const bool live = R < n && b0 < n;
     const size_t p = z * (size_t)n * n + (live ? (size_t)R * n + b0 : 0);
-    if (Q > 1) {
-      if (live) partial[(size_t)q * gridDim.z * n * n + p] = acc[i];
-    } else {
-      adj_store(ep, acc[i], live, p, img);
-    }
+    if (live) (Q > 1 ? partial + (size_t)q * gridDim.z * n * n : img)[p] = acc[i];
   }
 }
 
-__global__ void __launch_bounds__(256) bs_adj_sum_kernel(const float *__restrict__ partial, int Q, size_t total, float *__restrict__ img,
-                                                         AdjEpi ep) {
+__global__ void __launch_bounds__(256) bs_adj_sum_kernel(const float *__restrict__ partial, int Q, size_t total, float *__restrict__ img) {
   const size_t p = (size_t)blockIdx.x * 256 + threadIdx.x;
-  const bool live = p < total;
+  if (p >= total) return;
   float acc = 0.0f;
-  if (live)
-    for (int q = 0; q < Q; ++q) acc += partial[(size_t)q * total + p];
-  adj_store(ep, acc, live, live ? p : 0, img);
+  for (int q = 0; q < Q; ++q) acc += partial[(size_t)q * total + p];
+  img[p] = acc;
 }
 
 // Shares of the angles: blocks enough for four rounds of two to an SM, since
@@ -639,16 +629,13 @@ int bs_setup(Plan &p) {
     bs_lut4_kernel<<<na, 256>>>((const float *)p.d_aux, st->lut4, k);
     TOMO_CUDA(cudaGetLastError());
     TOMO_CUDA(cudaStreamSynchronize(0));  // later calls may come on streams that do not wait for this one
-    const int bins = 128 / bs_fwd_split(n);
-    p.fwd_warps = (size_t)((n + bins - 1) / bins) * (bins / 32) * na * p.g.nz;
-  } else {
-    for (size_t i = 0; i < (size_t)na * L; ++i) st->lutmax = std::max(st->lutmax, std::fabs(p.g.lut[i]));
-    TOMO_CUDA(cudaMalloc(&st->vmax, sizeof(unsigned) * (size_t)std::max(1, p.g.nz)));
-    if (sizeof(float) * (size_t)L > 48 * 1024)
-      TOMO_CUDA(cudaFuncSetAttribute(bs_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * L)));
-    // residual partials of the fused solvers: one per warp of the forward launch
-    p.fwd_warps = (size_t)((n + kBsBins - 1) / kBsBins) * (kBsThreads / 32) * na * p.g.nz;
   }
+  for (size_t i = 0; i < (size_t)na * L; ++i) st->lutmax = std::max(st->lutmax, std::fabs(p.g.lut[i]));
+  TOMO_CUDA(cudaMalloc(&st->vmax, sizeof(unsigned) * (size_t)std::max(1, p.g.nz)));
+  if (sizeof(float) * (size_t)L > 48 * 1024)
+    TOMO_CUDA(cudaFuncSetAttribute(bs_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * L)));
+  // residual partials of the fused solvers: one per warp of the general forward
+  p.fwd_warps = (size_t)((n + kBsBins - 1) / kBsBins) * (kBsThreads / 32) * na * p.g.nz;
   p.g.lut = nullptr;
   return TOMO_OK;
 }
@@ -656,12 +643,12 @@ int bs_setup(Plan &p) {
 int bs_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const FwdEpi &ep) {
   const BsConst k = make_const(p);
   BsState &st = *(BsState *)p.ext;
-  if (st.pow2) {
+  if (st.pow2 && !ep.ordered) {
     const int n = k.n, tiles = (n + 2 * kBsFrame + 31) / 32, split = bs_fwd_split(n), bins = 128 / split;
     bs_frame_kernel<<<dim3(tiles, tiles, p.g.nz), dim3(32, 8), 0, s>>>(d_img, st.rows, st.cols, n);
     auto fn = split == 4 ? bs_forward_pow2_kernel<4> : bs_forward_pow2_kernel<2>;
     fn<<<dim3((n + bins - 1) / bins, k.na, p.g.nz), 128, sizeof(float) * (st.entries + 1), s>>>(
-        st.rows, st.cols, d_sino, (const float2 *)p.d_angles, (const float *)p.d_aux, st.entries, k, ep);
+        st.rows, st.cols, d_sino, (const float2 *)p.d_angles, (const float *)p.d_aux, st.entries, k);
     TOMO_CUDA(cudaGetLastError());
     return TOMO_OK;
   }
@@ -679,17 +666,17 @@ int bs_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
 int bs_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const AdjEpi &ep) {
   const BsConst k = make_const(p);
   BsState &st = *(BsState *)p.ext;
-  if (st.pow2) {
+  if (st.pow2 && !ep.ordered) {
     const int n = k.n, nz = p.g.nz;
     bs_expand_kernel<<<k.na * nz, 256, 0, s>>>(d_sino, st.S4, n, st.pads, st.w2);
     const dim3 grid((n + kBsTW - 1) / kBsTW * st.Q, (n + kBsTH - 1) / kBsTH, nz);
     const size_t smem = sizeof(float4) * 2 * (size_t)k.lut_step;
     auto fn = (n & 1) ? bs_adjoint_pow2_kernel<true> : bs_adjoint_pow2_kernel<false>;
     fn<<<grid, kBsThreads4, smem, s>>>(d_sino, st.S4, st.lut4, (const float *)p.d_aux, d_img, (const float2 *)p.d_angles, k,
-                                       st.pads, st.w2, st.Q, st.partial, ep);
+                                       st.pads, st.w2, st.Q, st.partial);
     if (st.Q > 1) {
       const size_t total = (size_t)nz * n * n;
-      bs_adj_sum_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(st.partial, st.Q, total, d_img, ep);
+      bs_adj_sum_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(st.partial, st.Q, total, d_img);
     }
     TOMO_CUDA(cudaGetLastError());
     return TOMO_OK;

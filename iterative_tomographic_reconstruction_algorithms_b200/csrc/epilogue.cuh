@@ -25,6 +25,10 @@
 
 namespace tomo {
 
+// `ordered`: the kernels that have a faster order of their sums for a plain
+// application keep to the reference's (one chain per bin or pixel).  The
+// solvers ask for it: their residuals are 64-bit sums over what the projectors
+// return, iterated on, and stay what they were to the last digits.
 enum EpiOp : int { EPI_NONE = 0, EPI_SIRT = 1, EPI_MLEM = 2, EPI_SPS = 3 };
 
 // np.spacing(1) as the reference adds it: to a float32 array (MLEM, stored
@@ -36,7 +40,8 @@ struct FwdEpi {
   int op = EPI_NONE;
   const float *b = nullptr;  // measured sinogram, same layout as the output
   const float *w = nullptr;  // SIRT: R = 1/(A 1); SPS: w = exp(-b / max b)
-  double *resid = nullptr;   // per-warp partial sums of (A x - b)^2, or null
+  double *resid = nullptr;   // per-warp partial sums of (A x - b)^2, or null (ordered kernels only)
+  bool ordered = false;
 };
 
 struct AdjEpi {
@@ -44,6 +49,7 @@ struct AdjEpi {
   const float *x = nullptr;    // current iterate (may alias the output)
   const float *aux = nullptr;  // SIRT: C = 1/(A^T 1); MLEM: 1/(A^T 1); SPS: den
   unsigned *sps_max = nullptr; // SPS: ordered-int maximum of the unclipped update
+  bool ordered = false;
 };
 
 __device__ __forceinline__ unsigned float_to_ordered(float f) {

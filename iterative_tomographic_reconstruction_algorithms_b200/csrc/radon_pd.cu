@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(256) pd_frame_kernel(const float *__restrict__
 // 32-bit atomics per product, and bounded the forward: 1.57 ms at 768^2 x 720,
 // now 0.97 (2048^2 x 1800: 25.2, now 14.8).  Bound now by instruction issue (52
 // per bin and line).
-template <bool ROWS, int DIR>
+template <bool ROWS, int DIR, bool ORD>
 __device__ __forceinline__ double pd_fwd_bin(const float *__restrict__ L, int w, float s, float c, int b, int n, int nh,
                                              int i0, int i1) {
   const float fnh = (float)nh, fb = (float)b, bm = fb - 1.0f, bp = fb + 1.0f;
@@ -123,10 +123,26 @@ __device__ __forceinline__ double pd_fwd_bin(const float *__restrict__ L, int w,
     const float2 Ts = unpack(T1), wa = unpack(add2(T1, nbm)), wb = unpack(add2(add2(t1, nbp), nh2));  // wb: -weight
     const float2 w2 = unpack(add2(add2(t2, nbp), nh2));                                               // -weight
     // below b the first of wa, -wb is the smaller one, above the second
-    const float w1x = fminf(wa.x, -wb.x), w1y = fminf(wa.y, -wb.y);
-    float p = 0.0f;
+    float w1x = fminf(wa.x, -wb.x), w1y = fminf(wa.y, -wb.y);
     const float a0 = __ldg(va), a1 = __ldg(va + DIR), a2 = __ldg(va + 2 * DIR);
     const float b0 = __ldg(vb), b1 = __ldg(vb + DIR), b2 = __ldg(vb + 2 * DIR);
+    if (ORD) {
+      // every product rounded as the reference rounds it, their exact sum; an
+      // integral T puts its weight, |(t + T) - nh|, into that bin
+      const float2 n1 = unpack(t1), T2 = unpack(add2(nh2, t2));
+      if (Ts.x == fb) w1x = fabsf(__fsub_rn(__fadd_rn(-n1.x, fb), fnh));
+      if (Ts.y == fb) w1y = fabsf(__fsub_rn(__fadd_rn(-n1.y, fb), fnh));
+      double r = 0.0, q = 0.0;
+      if (w0.x > 0.0f) r += (double)__fmul_rn(w0.x, a0);
+      r += (double)__fmul_rn(w1x, a1);
+      if (T2.x < bp) r += (double)__fmul_rn(fabsf(w2.x), a2);
+      if (w0.y > 0.0f) q += (double)__fmul_rn(w0.y, b0);
+      q += (double)__fmul_rn(w1y, b1);
+      if (T2.y < bp) q += (double)__fmul_rn(fabsf(w2.y), b2);
+      acc += r + q;
+      continue;
+    }
+    float p = 0.0f;
     if (w0.x > 0.0f) p = w0.x * a0;
     if (Ts.x != fb) p = fmaf(w1x, a1, p);
     if (w2.x < 0.0f) p = fmaf(-w2.x, a2, p);
@@ -142,14 +158,16 @@ __device__ __forceinline__ double pd_fwd_bin(const float *__restrict__ L, int w,
 // pixels.  SPLIT > 1, for small images, whose bins alone are too few warps to
 // hide a line's latency: one angle, its lines shared by SPLIT warps, whose sums
 // are added in order.  The split depends on n alone (pd_fwd_split), so a plan
-// for some of the angles or several slices gives the same bits.
+// for some of the angles or several slices gives the same bits.  SPLIT = 0: as 1
+// in the solvers' form (epilogue.cuh), the exact sum of the rounded products.
 constexpr int kPdAng = 4;
 
 template <int SPLIT>
 __global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : kPdAng)) pd_forward_kernel(
     const float *__restrict__ rows, const float *__restrict__ cols, float *__restrict__ sino, const PdAngle *__restrict__ tab,
     int n, int nh, int na, FwdEpi ep) {
-  __shared__ double part[SPLIT > 1 ? SPLIT : 1][32];
+  constexpr int kParts = SPLIT > 1 ? SPLIT : 1;
+  __shared__ double part[kParts][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, v = SPLIT > 1 ? blockIdx.y : blockIdx.y * kPdAng + warp;
   const int B0 = blockIdx.x * 32, b = B0 + lane, w = n + 2 * kPdFrame;
   const size_t z = blockIdx.z;
@@ -169,14 +187,14 @@ __global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : kPdAng)) pd_forward_
     }
     if (SPLIT > 1) {
       const int len = max(0, i1 - i0);
-      i1 = i0 + len * (warp + 1) / SPLIT;
-      i0 += len * warp / SPLIT;
+      i1 = i0 + len * (warp + 1) / kParts;
+      i0 += len * warp / kParts;
     }
     const float *L = (by_rows ? rows : cols) + z * (size_t)n * w;
     if (by_rows)
-      acc = s < 0.0f ? pd_fwd_bin<true, 1>(L, w, s, c, b, n, nh, i0, i1) : pd_fwd_bin<true, -1>(L, w, s, c, b, n, nh, i0, i1);
+      acc = s < 0.0f ? pd_fwd_bin<true, 1, SPLIT == 0>(L, w, s, c, b, n, nh, i0, i1) : pd_fwd_bin<true, -1, SPLIT == 0>(L, w, s, c, b, n, nh, i0, i1);
     else
-      acc = c < 0.0f ? pd_fwd_bin<false, 1>(L, w, s, c, b, n, nh, i0, i1) : pd_fwd_bin<false, -1>(L, w, s, c, b, n, nh, i0, i1);
+      acc = c < 0.0f ? pd_fwd_bin<false, 1, SPLIT == 0>(L, w, s, c, b, n, nh, i0, i1) : pd_fwd_bin<false, -1, SPLIT == 0>(L, w, s, c, b, n, nh, i0, i1);
   }
   if (SPLIT > 1) {
     part[warp][lane] = acc;
@@ -212,7 +230,9 @@ __global__ void __launch_bounds__(256) pd_expand_kernel(const float *__restrict_
 
 // Adjoint: a lane holds 4 x 4 pixels of a 32 x 16 tile; the Q warps of a block
 // sum Q contiguous shares of the angles, added in order through shared memory
-// (Q depends on n alone, so the result does not depend on the device).
+// (Q depends on n alone, so the result does not depend on the device).  Q = 1 is
+// the solvers' form (epilogue.cuh): one chain in the reference's order, integral
+// T included, with a row of 4 pixels per lane (R = 1) for small images.
 //
 // Per sub-sample: t and T as the reference rounds them, the pair at floor(T)
 // in one 8-byte read, and its two weights.  An integral T puts nothing into
@@ -223,18 +243,18 @@ __global__ void __launch_bounds__(256) pd_expand_kernel(const float *__restrict_
 // which halves the instructions (scalar ones: 0.57 ms against 0.51).  A thread
 // per pixel with four reads, bounds tests and the sign rule per sub-sample took
 // 1.52 ms at 768^2 x 720 and 25.5 at 2048^2 x 1800; this one 0.51 and 7.8.
-template <int Q>
+template <int Q, int R>
 __global__ void __launch_bounds__(32 * Q) pd_adjoint_kernel(const float2 *__restrict__ pairs, float *__restrict__ img,
                                                             const PdAngle *__restrict__ tab, int n, int nh, int na, int pads,
                                                             int w2, AdjEpi ep) {
-  __shared__ float part[(Q - 1) * 16][32];
+  __shared__ float part[Q > 1 ? (Q - 1) * 4 * R : 1][32];
   const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
-  const int b0 = blockIdx.x * 32 + 4 * (lane & 7), a0 = blockIdx.y * 16 + 4 * (lane >> 3);
+  const int b0 = blockIdx.x * 32 + 4 * (lane & 7), a0 = blockIdx.y * 4 * R + R * (lane >> 3);
   const size_t z = blockIdx.z;
   const float fnh = (float)nh;
-  float acc[4][4];
+  float acc[R][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < R; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
   const int u0 = (int)((long long)na * q / Q), u1 = (int)((long long)na * (q + 1) / Q);
@@ -253,7 +273,7 @@ __global__ void __launch_bounds__(32 * Q) pd_adjoint_kernel(const float2 *__rest
 #pragma unroll
       for (int j = 0; j < 4; ++j) xs[j] = mul2(f2(x0 + (float)j - 0.25f, x0 + (float)j + 0.25f), ns);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < R; ++i) {
         const F2 y = f2(y0 - (float)i - 0.25f, y0 - (float)i + 0.25f);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -266,6 +286,15 @@ __global__ void __launch_bounds__(32 * Q) pd_adjoint_kernel(const float2 *__rest
           const float2 fs = unpack(fd);
           const float2 Sa = __ldg(row + __float_as_int(fs.x)), Sb = __ldg(row + __float_as_int(fs.y));
           const float2 wu = unpack(rsub2(add2(fd, nmagic), T));
+          if (Q == 1) {
+            const float2 Tv = unpack(T), t = unpack(nt);
+            const float2 uf = unpack(add2(add2_ru(T, magic), nmagic));  // ceil(T)
+            acc[i][j] = __fmaf_rn(fabsf(__fsub_rn(__fadd_rn(-t.x, uf.x), fnh)), Sa.x, acc[i][j]);
+            if (Tv.x != uf.x) acc[i][j] = __fmaf_rn(wu.x, Sa.y, acc[i][j]);
+            acc[i][j] = __fmaf_rn(fabsf(__fsub_rn(__fadd_rn(-t.y, uf.y), fnh)), Sb.x, acc[i][j]);
+            if (Tv.y != uf.y) acc[i][j] = __fmaf_rn(wu.y, Sb.y, acc[i][j]);
+            continue;
+          }
           const float2 wl = unpack(add2(add2(nt, rsub2(fd, magic1)), nh2));  // -(t + (floor(T) + 1) - nh)
           if (wu.x != 0.0f) acc[i][j] = __fmaf_rn(-wl.x, Sa.x, __fmaf_rn(wu.x, Sa.y, acc[i][j]));
           if (wu.y != 0.0f) acc[i][j] = __fmaf_rn(-wl.y, Sb.x, __fmaf_rn(wu.y, Sb.y, acc[i][j]));
@@ -275,25 +304,25 @@ __global__ void __launch_bounds__(32 * Q) pd_adjoint_kernel(const float2 *__rest
   }
   if (q > 0)
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) part[(q - 1) * 16 + 4 * i + j][lane] = acc[i][j];
+      for (int j = 0; j < 4; ++j) part[(q - 1) * 4 * R + 4 * i + j][lane] = acc[i][j];
   __syncthreads();
   if (q > 0) return;
 #pragma unroll
   for (int r = 0; r < Q - 1; ++r)
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] += part[r * 16 + 4 * i + j][lane];
+      for (int j = 0; j < 4; ++j) acc[i][j] += part[r * 4 * R + 4 * i + j][lane];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < R; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int R = a0 + i, C = b0 + j;
-      const bool live = R < n && C < n;
+      const int y = a0 + i, x = b0 + j;
+      const bool live = y < n && x < n;
       // 0.5: the two coinciding quarter-weight sub-samples
-      adj_store(ep, 0.5f * acc[i][j], live, z * (size_t)n * n + (live ? (size_t)R * n + C : 0), img);
+      adj_store(ep, 0.5f * acc[i][j], live, z * (size_t)n * n + (live ? (size_t)y * n + x : 0), img);
     }
 }
 
@@ -346,8 +375,7 @@ int pd_setup(Plan &p) {
   st->rows = (float *)(st->pairs + pairs);
   st->cols = st->rows + framed;
   // residual partials of the fused solvers: one per warp of the forward launch
-  p.fwd_warps = (size_t)((p.g.n + 31) / 32) * p.g.nz *
-                (pd_fwd_split(p.g.n) > 1 ? na : (na + kPdAng - 1) / kPdAng * kPdAng);
+  p.fwd_warps = (size_t)((p.g.n + 31) / 32) * ((na + kPdAng - 1) / kPdAng) * kPdAng * p.g.nz;
   return TOMO_OK;
 }
 
@@ -356,8 +384,8 @@ int pd_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
   PdState &st = *(PdState *)p.ext;
   const int tiles = (n + 2 * kPdFrame + 31) / 32;
   pd_frame_kernel<<<dim3(tiles, tiles, nz), dim3(32, 8), 0, s>>>(d_img, st.rows, st.cols, n);
-  const int split = pd_fwd_split(n), warps = split > 1 ? split : kPdAng;
-  auto fn = split == 8 ? pd_forward_kernel<8> : split == 4 ? pd_forward_kernel<4> : pd_forward_kernel<1>;
+  const int split = ep.ordered ? 0 : pd_fwd_split(n), warps = split > 1 ? split : kPdAng;
+  auto fn = split == 8 ? pd_forward_kernel<8> : split == 4 ? pd_forward_kernel<4> : split == 1 ? pd_forward_kernel<1> : pd_forward_kernel<0>;
   fn<<<dim3((n + 31) / 32, split > 1 ? na : (na + kPdAng - 1) / kPdAng, nz), 32 * warps, 0, s>>>(
       st.rows, st.cols, d_sino, (const PdAngle *)p.d_angles, n, p.nh, na, ep);
   TOMO_CUDA(cudaGetLastError());
@@ -368,10 +396,14 @@ int pd_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
   PdState &st = *(PdState *)p.ext;
   pd_expand_kernel<<<na * nz, 256, 0, s>>>(d_sino, st.pairs, n, st.pads, st.w2);
-  const int Q = pd_adj_warps(n);
-  auto fn = Q == 4 ? pd_adjoint_kernel<4> : Q == 8 ? pd_adjoint_kernel<8> : pd_adjoint_kernel<16>;
-  fn<<<dim3((n + 31) / 32, (n + 15) / 16, nz), 32 * Q, 0, s>>>(st.pairs, d_img, (const PdAngle *)p.d_angles, n, p.nh, na,
-                                                               st.pads, st.w2, ep);
+  const int Q = ep.ordered ? 1 : pd_adj_warps(n), R = ep.ordered && n <= 1024 ? 1 : 4;
+  auto fn = R == 1    ? pd_adjoint_kernel<1, 1>
+            : Q == 1  ? pd_adjoint_kernel<1, 4>
+            : Q == 4  ? pd_adjoint_kernel<4, 4>
+            : Q == 8  ? pd_adjoint_kernel<8, 4>
+                      : pd_adjoint_kernel<16, 4>;
+  fn<<<dim3((n + 31) / 32, (n + 4 * R - 1) / (4 * R), nz), 32 * Q, 0, s>>>(
+      st.pairs, d_img, (const PdAngle *)p.d_angles, n, p.nh, na, st.pads, st.w2, ep);
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
 }

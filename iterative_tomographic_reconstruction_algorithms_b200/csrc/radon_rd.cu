@@ -282,7 +282,7 @@ __global__ void rd_frame_kernel(const float *__restrict__ in, float *__restrict_
   }
 }
 
-// Forward over slices z0 + blockIdx.z; Q and QT hold the chunk's slices
+// Ordered forward over slices z0 + blockIdx.z; Q and QT hold the chunk's slices
 // framed (rd_frame_kernel).  A block is kBins bins of kFwdAngles consecutive
 // angles (threadIdx.y): the walks of neighbouring angles cover nearly the same
 // pixels at nearly the same time, so its warps share L1 lines.  kBins = 128,
@@ -334,6 +334,57 @@ __global__ void __launch_bounds__(kBins * kFwdAngles, 1024 / (kBins * kFwdAngles
   double r2 = 0.0;
   if (live) sino[e] = fwd_apply(ep, acc, e, r2);
   fwd_resid_commit(ep, r2, (z * na + v) * (gridDim.x * (kBins / 32)) + b / 32);
+}
+
+// The forward of a plain application: a block is 32 bins x 5 sub-rays of an
+// angle, a warp one sub-ray of the bins, whose five sums are added in sub-ray
+// order (the walks of a bin's sub-rays cover nearly the same pixels at nearly
+// the same time, so the warps share L1 lines; two or three angles to a block: no
+// faster).  One thread for all five walks of a bin leaves small images waiting
+// for one long chain of steps: 0.54 ms at 256^2 x 304, here 0.25; 513^2 x 400
+// 1.44, here 1.16; 2048^2 x 1800, bound by ALU issue either way, 78.8, here
+// 75.7.  rd_forward_kernel keeps that one chain, the reference's, for the solvers.
+__global__ void __launch_bounds__(160, 6) rd_forward_split_kernel(
+    const float *__restrict__ img, const float *__restrict__ Q, const float *__restrict__ QT,
+    float *__restrict__ sino, const RdAngle *__restrict__ tab, const float *__restrict__ toff, int n, int nh, int na,
+    int z0) {
+  __shared__ float part[5][32];
+  const int lane = threadIdx.x, r = threadIdx.y;
+  const int b = blockIdx.x * 32 + lane, v = blockIdx.y;
+  const size_t z = (size_t)z0 + blockIdx.z;
+  const bool live = b < n;
+  float acc = 0.0f;
+  if (live) {
+    const RdAngle *g = tab + v;
+    const float *I = img + z * (size_t)n * n;
+    if (g->mode == 1) {  // |s| < 1e-7: bin n-1-i <- column i, i >= 1 (radon_rd.c:96-105)
+      const int i = n - 1 - b;
+      if (r == 0 && i >= 1)
+        for (int j = 0; j < n; ++j) acc += __ldg(I + (size_t)j * n + i);
+    } else if (g->mode == 2) {  // |c| < 1e-7: bin i <- row i (:108-117)
+      if (r == 0)
+        for (int j = 0; j < n; ++j) acc += __ldg(I + (size_t)b * n + j);
+    } else {
+      const int m = n + 3;
+      const bool tr = g->tr != 0;
+      const float *P = (tr ? QT : Q) + (size_t)blockIdx.z * m * m;
+      const int sA = tr ? 1 : m, sB = tr ? m : 1;
+      RdGather gat{P, 0.0f, 0.0f, 0.0f};
+      const RdGeom s = rd_geom_of(tab, v, toff, 6 * b + r + 1, n, nh);
+      const float rx = __frcp_rn(s.ex), ry = __frcp_rn(s.ey);
+      if (rd_walk_framed(s, nh, rx, ry))
+        rd_walk_loop<false>(s, n, nh, sA, sB, 1, rx, ry, gat);
+      else
+        gat = rd_walk_safe(s, n, nh, sA, sB, 1, rx, ry, gat);
+      acc = fmaf(gat.w, gat.xv, gat.acc);
+    }
+  }
+  part[r][lane] = acc;
+  __syncthreads();
+  if (r > 0) return;  // whole warps
+#pragma unroll
+  for (int q = 1; q < 5; ++q) acc += part[q][lane];
+  if (live) sino[(z * na + v) * (size_t)n + b] = acc;
 }
 
 // Flag bytes of non-finite credits (nonfinite_flag: 1 +inf, 2 -inf, 4 NaN),
@@ -523,6 +574,11 @@ int rd_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
     const int zc = std::min(chunk, nz - z0);
     rd_frame_kernel<<<dim3((m + 31) / 32, (m + 31) / 32, zc), dim3(32, 8), 0, s>>>(d_img + (size_t)z0 * n * n, Q,
                                                                                      QT, n);
+    if (!ep.ordered) {
+      rd_forward_split_kernel<<<dim3((n + 31) / 32, na, zc), dim3(32, 5), 0, s>>>(
+          d_img, Q, QT, d_sino, (const RdAngle *)p.d_angles, (const float *)p.d_aux, n, p.nh, na, z0);
+      continue;
+    }
     const int rows = (na + kFwdAngles - 1) / kFwdAngles, w128 = (n + 127) / 128;
     // 128-bin blocks once there are 8 or more per SM, else 32-bin ones
     if ((size_t)w128 * rows * zc >= (size_t)148 * 8)

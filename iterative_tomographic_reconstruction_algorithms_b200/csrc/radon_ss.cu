@@ -63,15 +63,16 @@ __global__ void __launch_bounds__(256) ss_frame_kernel(const float *__restrict__
 // factor wt is applied once.  SPLIT warps share a ray's steps and are added in
 // order: small images have too few rays to hide a step's latency (256^2 x 200:
 // 61 us unsplit, now 18; 768^2 x 720: 0.58 ms unsplit, 0.38 by two); the split
-// depends on n alone (ss_fwd_split).
+// depends on n alone (ss_fwd_split).  SPLIT = 0 is the solvers' form
+// (epilogue.cuh): one chain, the weight wt w rounded before each product.
 // 4 x 641^2 x 600: 1.28 ms with bounds tests and weights per step, now 0.78;
 // 2048^2 x 1800: 9.6, now 6.3.
 template <int SPLIT>
 __global__ void __launch_bounds__(128) ss_forward_kernel(const float *__restrict__ rows, const float *__restrict__ cols,
                                                          float *__restrict__ sino, const SsAngle *__restrict__ tab,
                                                          const int2 *__restrict__ lim, int n, int nh, int na, FwdEpi ep) {
-  __shared__ float part[SPLIT][128 / SPLIT];
-  constexpr int kRays = 128 / SPLIT;
+  __shared__ float part[SPLIT > 1 ? SPLIT : 1][128];
+  constexpr int kParts = SPLIT > 1 ? SPLIT : 1, kRays = 128 / kParts;
   const int lane = threadIdx.x % kRays, q = threadIdx.x / kRays;  // kRays is a multiple of 32: q is warp-uniform
   const int kt = blockIdx.x * kRays + lane;  // t + nh
   const int v = blockIdx.y;
@@ -82,8 +83,8 @@ __global__ void __launch_bounds__(128) ss_forward_kernel(const float *__restrict
   int m0 = max(L.x, -nh), m1 = min(L.y, n - nh);  // rays that miss the square may leave it
   if (SPLIT > 1) {
     const int len = max(0, m1 - m0), s0 = m0;
-    m0 = s0 + len * q / SPLIT;
-    m1 = s0 + len * (q + 1) / SPLIT;
+    m0 = s0 + len * q / kParts;
+    m1 = s0 + len * (q + 1) / kParts;
   }
   const int w = n + 2 * kSsFrame;
   const float ft = (float)(kt - nh), lo = (float)(-nh) - 2.0f, hi = (float)(n - nh) + 1.0f;
@@ -93,10 +94,12 @@ __global__ void __launch_bounds__(128) ss_forward_kernel(const float *__restrict
   for (int m = m0; m < m1; ++m, nm -= 1.0f, row += w) {
     const float f = fminf(fmaxf(__fmul_rn(__fmaf_rn(nm, g.a, ft), g.rb), lo), hi);
     const float fd = __fadd_rd(f, kSsMagic);  // floor(f), as a float among the integers and in its bits
-    const float wq = __fsub_rn(f, __fsub_rn(fd, kSsMagic));
+    const float fl = __fsub_rn(fd, kSsMagic), wq = __fsub_rn(f, fl);
     const float *p = row + __float_as_int(fd);
-    acc = fmaf(__fsub_rn(1.0f, wq), __ldg(p), acc);  // 1 - w is exactly (floor(f) + 1) - f
-    acc = fmaf(wq, __ldg(p + 1), acc);
+    // (floor(f) + 1) - f is 1 - w exactly, except in the last bits of |f| < 1
+    const float w1 = SPLIT ? __fsub_rn(1.0f, wq) : __fsub_rn(__fadd_rn(fl, 1.0f), f);
+    acc = fmaf(SPLIT ? w1 : __fmul_rn(g.wt, w1), __ldg(p), acc);
+    acc = fmaf(SPLIT ? wq : __fmul_rn(g.wt, wq), __ldg(p + 1), acc);
   }
   if (SPLIT > 1) {
     part[q][lane] = acc;
@@ -104,7 +107,7 @@ __global__ void __launch_bounds__(128) ss_forward_kernel(const float *__restrict
     if (q > 0) return;  // warp-uniform
     for (int k = 1; k < SPLIT; ++k) acc += part[k][lane];
   }
-  acc *= g.wt;
+  if (SPLIT) acc *= g.wt;
   double r2 = 0.0;
   const size_t e = z * (size_t)na * n + (size_t)g.out_row * n + kt;
   if (live) sino[e] = fwd_apply(ep, acc, e, r2);
@@ -115,25 +118,27 @@ __global__ void __launch_bounds__(128) ss_forward_kernel(const float *__restrict
 int ss_fwd_split(int n) { return n > 448 ? 2 : 4; }
 
 // Sinogram rows as pairs in the order of the angles, entry e = t + nh + pads of
-// angle v: wt {S_t, S_t+1}, 0 outside the rays.
+// angle v: wt {S_t, S_t+1} (without wt: ordered), 0 outside the rays.
 __global__ void __launch_bounds__(256) ss_expand_kernel(const float *__restrict__ sino, float2 *__restrict__ out,
                                                         const SsAngle *__restrict__ tab, int n, int nh, int na, int pads,
-                                                        int w2) {
+                                                        int w2, bool ordered) {
   const int v = blockIdx.x;
   const size_t z = blockIdx.y;
   const SsAngle g = tab[v];
+  const float wt = ordered ? 1.0f : g.wt;
   const float *src = sino + (z * na + g.out_row) * (size_t)n;
   float2 *dst = out + (z * na + v) * (size_t)w2;
   for (int e = threadIdx.x; e < w2; e += blockDim.x) {
     const int t = e - pads;
-    dst[e] = make_float2(t >= 0 && t < 2 * nh ? g.wt * __ldg(src + t) : 0.0f,
-                         t + 1 >= 0 && t + 1 < 2 * nh ? g.wt * __ldg(src + t + 1) : 0.0f);
+    dst[e] = make_float2(t >= 0 && t < 2 * nh ? wt * __ldg(src + t) : 0.0f,
+                         t + 1 >= 0 && t + 1 < 2 * nh ? wt * __ldg(src + t + 1) : 0.0f);
   }
 }
 
 // Adjoint: a lane holds 4 x 4 pixels of a 32 x 16 tile; warp q of a block's Q
 // sums every Q-th angle from q on (the costlier angles near an axis go to all),
-// and the sums are added in order.  Q depends on n alone.
+// and the sums are added in order.  Q depends on n alone.  Q = 1 is the solvers'
+// form (epilogue.cuh): one chain, the weight wt w rounded before each product.
 //
 // At a pixel's major coordinate m the rays' minor coordinates f(t) = fma(-m, a,
 // t) * rb lie |rb| = 1 / |cb| >= 1 apart, so a ray within 1 of the pixel's minor
@@ -157,11 +162,19 @@ __device__ __forceinline__ bool ss_in_limits(const int2 *__restrict__ lrow, int 
   return (t >= -nh) & (t < nh) & (m >= l.x) & (m < l.y);
 }
 
-template <bool STEEP, bool EDGE, bool NEAR>
+// Weight of a ray at f to the pixel at c, below 0 out of reach.  ORD: as f -
+// floor f or floor f + 1 - f, which differ in the last bits where |f| < 1.
+template <bool ORD>
+__device__ __forceinline__ float ss_weight(float f, float c) {
+  if (ORD) return fminf(__fsub_rn(__fadd_rn(c, 1.0f), f), __fsub_rn(f, __fsub_rn(c, 1.0f)));
+  return 1.0f - fabsf(__fsub_rn(f, c));
+}
+
+template <bool STEEP, bool EDGE, bool NEAR, bool ORD>
 __device__ __forceinline__ void ss_adj_angle(const SsAngle &g, const float2 *__restrict__ row, const int2 *__restrict__ lrow,
                                              int a0, int b0, int nh, float (&acc)[4][4]) {
   const int M0 = (STEEP ? a0 : b0) - nh, C0 = (STEEP ? b0 : a0) - nh;  // major and minor coordinates of the block
-  const float cb = 1.0f / g.rb;
+  const float cb = 1.0f / g.rb, wt = g.wt;
   const F2 rb = f2(g.rb), a = f2(g.a), step = f2(0.0f, 1.0f);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {  // along the major axis
@@ -174,19 +187,19 @@ __device__ __forceinline__ void ss_adj_angle(const SsAngle &g, const float2 *__r
       const float2 S = __ldg(row + __float_as_int(fm));
       const F2 t = add2(f2(__fsub_rn(fm, kSsMagic)), step);
       const float2 f = unpack(mul2(fma2(nm, a, t), rb));  // scalar from here: see f32x2.cuh
-      const float h0 = 1.0f - fabsf(__fsub_rn(f.x, c)), h1 = 1.0f - fabsf(__fsub_rn(f.y, c));
+      const float h0 = ss_weight<ORD>(f.x, c), h1 = ss_weight<ORD>(f.y, c);
       const int ti = __float_as_int(fm) - kSsMagicBits;
       float &o = STEEP ? acc[i][j] : acc[j][i];
       if (NEAR) {
-        const float h = 1.0f - fabsf(__fsub_rn(__fmul_rn(__fmaf_rn(-m, g.a, __fsub_rn(fm, kSsMagic) - 1.0f), g.rb), c));
-        if (h > 0.0f && (!EDGE || ss_in_limits(lrow, ti - 1, M0 + i, nh))) o = fmaf(h, __ldg(row + __float_as_int(fm) - 1).x, o);
+        const float h = ss_weight<ORD>(__fmul_rn(__fmaf_rn(-m, g.a, __fsub_rn(fm, kSsMagic) - 1.0f), g.rb), c);
+        if (h > 0.0f && (!EDGE || ss_in_limits(lrow, ti - 1, M0 + i, nh))) o = fmaf(ORD ? __fmul_rn(wt, h) : h, __ldg(row + __float_as_int(fm) - 1).x, o);
       }
       const bool in0 = EDGE ? ss_in_limits(lrow, ti, M0 + i, nh) : true, in1 = EDGE ? ss_in_limits(lrow, ti + 1, M0 + i, nh) : true;
-      if ((h0 > 0.0f) & in0) o = fmaf(h0, S.x, o);
-      if ((h1 > 0.0f) & in1) o = fmaf(h1, S.y, o);
+      if ((h0 > 0.0f) & in0) o = fmaf(ORD ? __fmul_rn(wt, h0) : h0, S.x, o);
+      if ((h1 > 0.0f) & in1) o = fmaf(ORD ? __fmul_rn(wt, h1) : h1, S.y, o);
       if (NEAR) {
-        const float h = 1.0f - fabsf(__fsub_rn(__fmul_rn(__fmaf_rn(-m, g.a, __fsub_rn(fm, kSsMagic) + 2.0f), g.rb), c));
-        if (h > 0.0f && (!EDGE || ss_in_limits(lrow, ti + 2, M0 + i, nh))) o = fmaf(h, __ldg(row + __float_as_int(fm) + 1).y, o);
+        const float h = ss_weight<ORD>(__fmul_rn(__fmaf_rn(-m, g.a, __fsub_rn(fm, kSsMagic) + 2.0f), g.rb), c);
+        if (h > 0.0f && (!EDGE || ss_in_limits(lrow, ti + 2, M0 + i, nh))) o = fmaf(ORD ? __fmul_rn(wt, h) : h, __ldg(row + __float_as_int(fm) + 1).y, o);
       }
     }
   }
@@ -196,7 +209,7 @@ template <int Q>
 __global__ void __launch_bounds__(32 * Q) ss_adjoint_kernel(const float2 *__restrict__ pairs, float *__restrict__ img,
                                                             const SsAngle *__restrict__ tab, const int2 *__restrict__ lim,
                                                             int n, int nh, int na, int pads, int w2, AdjEpi ep) {
-  __shared__ float part[(Q - 1) * 16][32];
+  __shared__ float part[Q > 1 ? (Q - 1) * 16 : 1][32];
   const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
   // the tiles of the border take longest: both border rows of tiles first
   const int by = blockIdx.y == 0 ? 0 : blockIdx.y == 1 ? gridDim.y - 1 : blockIdx.y - 1;
@@ -218,14 +231,14 @@ __global__ void __launch_bounds__(32 * Q) ss_adjoint_kernel(const float2 *__rest
       const SsAngle g = tab[u];
       const bool nr = fabsf(g.rb) * near < 1.0f;
       if (nr) {
-        if (g.steep) ss_adj_angle<true, true, true>(g, row, lrow, a0, b0, nh, acc);
-        else ss_adj_angle<false, true, true>(g, row, lrow, a0, b0, nh, acc);
+        if (g.steep) ss_adj_angle<true, true, true, Q == 1>(g, row, lrow, a0, b0, nh, acc);
+        else ss_adj_angle<false, true, true, Q == 1>(g, row, lrow, a0, b0, nh, acc);
       } else if (edge) {
-        if (g.steep) ss_adj_angle<true, true, false>(g, row, lrow, a0, b0, nh, acc);
-        else ss_adj_angle<false, true, false>(g, row, lrow, a0, b0, nh, acc);
+        if (g.steep) ss_adj_angle<true, true, false, Q == 1>(g, row, lrow, a0, b0, nh, acc);
+        else ss_adj_angle<false, true, false, Q == 1>(g, row, lrow, a0, b0, nh, acc);
       } else {
-        if (g.steep) ss_adj_angle<true, false, false>(g, row, lrow, a0, b0, nh, acc);
-        else ss_adj_angle<false, false, false>(g, row, lrow, a0, b0, nh, acc);
+        if (g.steep) ss_adj_angle<true, false, false, Q == 1>(g, row, lrow, a0, b0, nh, acc);
+        else ss_adj_angle<false, false, false, Q == 1>(g, row, lrow, a0, b0, nh, acc);
       }
     }
   }
@@ -327,9 +340,8 @@ int ss_setup(Plan &p) {
   TOMO_CUDA(cudaMalloc(&st->pairs, sizeof(float2) * pairs + 2 * sizeof(float) * framed));
   st->rows = (float *)(st->pairs + pairs);
   st->cols = st->rows + framed;
-  // residual partials of the fused solvers: one per 32 rays
-  const int rays = 128 / ss_fwd_split(n);
-  p.fwd_warps = (size_t)((n + rays - 1) / rays) * (rays / 32) * na * p.g.nz;
+  // residual partials of the fused solvers: one per warp of the ordered forward
+  p.fwd_warps = (size_t)((n + 127) / 128) * 4 * na * p.g.nz;
   return TOMO_OK;
 }
 
@@ -338,8 +350,8 @@ int ss_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
   SsState &st = *(SsState *)p.ext;
   const int tiles = (n + 2 * kSsFrame + 31) / 32;
   ss_frame_kernel<<<dim3(tiles, tiles, nz), dim3(32, 8), 0, s>>>(d_img, st.rows, st.cols, n);
-  const int split = ss_fwd_split(n), rays = 128 / split;
-  auto fn = split == 4 ? ss_forward_kernel<4> : ss_forward_kernel<2>;
+  const int split = ep.ordered ? 0 : ss_fwd_split(n), rays = 128 / std::max(split, 1);
+  auto fn = split == 4 ? ss_forward_kernel<4> : split == 2 ? ss_forward_kernel<2> : ss_forward_kernel<0>;
   fn<<<dim3((n + rays - 1) / rays, na, nz), 128, 0, s>>>(st.rows, st.cols, d_sino, (const SsAngle *)p.d_angles,
                                                          (const int2 *)p.d_aux, n, nh, na, ep);
   TOMO_CUDA(cudaGetLastError());
@@ -349,9 +361,10 @@ int ss_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
 int ss_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const AdjEpi &ep) {
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
   SsState &st = *(SsState *)p.ext;
-  ss_expand_kernel<<<dim3(na, nz), 256, 0, s>>>(d_sino, st.pairs, (const SsAngle *)p.d_angles, n, p.nh, na, st.pads, st.w2);
-  const int Q = ss_adj_warps(n);
-  auto fn = Q == 4 ? ss_adjoint_kernel<4> : Q == 8 ? ss_adjoint_kernel<8> : ss_adjoint_kernel<16>;
+  ss_expand_kernel<<<dim3(na, nz), 256, 0, s>>>(d_sino, st.pairs, (const SsAngle *)p.d_angles, n, p.nh, na, st.pads, st.w2,
+                                               ep.ordered);
+  const int Q = ep.ordered ? 1 : ss_adj_warps(n);
+  auto fn = Q == 1 ? ss_adjoint_kernel<1> : Q == 4 ? ss_adjoint_kernel<4> : Q == 8 ? ss_adjoint_kernel<8> : ss_adjoint_kernel<16>;
   fn<<<dim3((n + 31) / 32, (n + 15) / 16, nz), 32 * Q, 0, s>>>(st.pairs, d_img, (const SsAngle *)p.d_angles,
                                                                (const int2 *)p.d_aux, n, p.nh, na, st.pads, st.w2, ep);
   TOMO_CUDA(cudaGetLastError());

@@ -140,11 +140,13 @@ static int solver_iteration(Solver &S, float *x, cudaStream_t st) {
   Plan &p = *S.p;
   const size_t ni = image_elems(p);
   FwdEpi fe;
+  fe.ordered = true;
   fe.op = S.algo == TOMO_ALGO_SIRT ? EPI_SIRT : (S.algo == TOMO_ALGO_MLEM ? EPI_MLEM : EPI_SPS);
   fe.b = S.b;
   fe.w = S.aux_f;
   fe.resid = S.part;
   AdjEpi ae;
+  ae.ordered = true;
   ae.op = fe.op;
   ae.x = x;
   ae.aux = S.aux_a;
@@ -205,25 +207,28 @@ int tomo_solver_create(tomo_plan *plan, int algo, const float *d_b, void *stream
   SOLVER_CUDA(cudaMemsetAsync(S.counter, 0, sizeof(int), st));
   SOLVER_CUDA(cudaMalloc(&ones_i, sizeof(float) * ni));
   SOLVER_CUDA(cudaMalloc(&ones_s, sizeof(float) * ns));
+  FwdEpi plain_f;
+  AdjEpi plain_a;
+  plain_f.ordered = plain_a.ordered = true;
   fill_kernel<<<grid_for(ni), 256, 0, st>>>(ones_i, ni, 1.0f);
   fill_kernel<<<grid_for(ns), 256, 0, st>>>(ones_s, ns, 1.0f);
   if (algo == TOMO_ALGO_SIRT) {
     // R = 1/(A 1), C = 1/(A^T 1)   (art.py:227-237)
-    if ((rc = plan_forward(p, ones_i, S.y, st, FwdEpi()))) return bail(rc);
+    if ((rc = plan_forward(p, ones_i, S.y, st, plain_f))) return bail(rc);
     recip_guard_kernel<<<grid_for(ns), 256, 0, st>>>(S.y, S.aux_f, ns);
-    if ((rc = plan_adjoint(p, ones_s, S.aux_a, st, AdjEpi()))) return bail(rc);
+    if ((rc = plan_adjoint(p, ones_s, S.aux_a, st, plain_a))) return bail(rc);
     recip_guard_kernel<<<grid_for(ni), 256, 0, st>>>(S.aux_a, S.aux_a, ni);
   } else if (algo == TOMO_ALGO_MLEM) {
     // 1/d with d = A^T 1   (sir.py:215-217, 283)
-    if ((rc = plan_adjoint(p, ones_s, S.aux_a, st, AdjEpi()))) return bail(rc);
+    if ((rc = plan_adjoint(p, ones_s, S.aux_a, st, plain_a))) return bail(rc);
     recip_guard_kernel<<<grid_for(ni), 256, 0, st>>>(S.aux_a, S.aux_a, ni);
   } else {
     // w = exp(-b / max b), den = A^T(w * A 1)   (sir.py:365-384)
     SOLVER_CUDA(cudaMemsetAsync(S.sps_max, 0, sizeof(unsigned), st));
     max_kernel<<<grid_for(ns), 256, 0, st>>>(d_b, ns, S.sps_max);
-    if ((rc = plan_forward(p, ones_i, S.y, st, FwdEpi()))) return bail(rc);
+    if ((rc = plan_forward(p, ones_i, S.y, st, plain_f))) return bail(rc);
     sps_weights_kernel<<<grid_for(ns), 256, 0, st>>>(d_b, S.sps_max, S.aux_f, S.y, ns);
-    if ((rc = plan_adjoint(p, S.y, S.aux_a, st, AdjEpi()))) return bail(rc);
+    if ((rc = plan_adjoint(p, S.y, S.aux_a, st, plain_a))) return bail(rc);
   }
   SOLVER_CUDA(cudaGetLastError());
   SOLVER_CUDA(cudaStreamSynchronize(st));
