@@ -155,14 +155,11 @@ __global__ void __launch_bounds__(128) dd_forward_kernel(
 // ---------------------------------------------------------------------------
 // Instances
 // ---------------------------------------------------------------------------
-constexpr int kGrpDet = 127;              // detectors per forward item (128 boundaries, 4 per lane)
-#ifndef FWD_UNROLL
-#define FWD_UNROLL 2
-#endif
-constexpr int kFwdUnroll = FWD_UNROLL;  // image lines per unrolled step of the forward
-constexpr int kTileW = 32, kTileH = 16;   // pixels per adjoint item (4x4 per lane, 8x4 lanes)
+constexpr int kGrpDet = 127;              // detectors per forward item (128 boundaries, 4 x 32)
+constexpr int kTileW = 32;                // an adjoint item is 32 x 4R pixels, R x 4 per lane (8x4 lanes)
 constexpr int kScanThreads = 256;
-constexpr int kColWarps = 4, kColRows = 16;
+constexpr int kPrepWarps = kScanThreads / 32;  // warps of the pre-pass kernels
+constexpr int kColParts = 4, kColRows = 8;     // parts a column is summed in; rows staged at a time
 // Adding 1.5 * 2^23 rounds a float of magnitude < 2^22 to an integer held in
 // the low mantissa bits: int = bits - kMagicBits.
 constexpr float kMagic = 12582912.0f;
@@ -269,12 +266,11 @@ __device__ __forceinline__ double block_exclusive_scan(double x, double &carry, 
 
 // Row lines: work[sl + line*(n+2) + 1 + kk] = {S(kk), L[kk]}, kk in [-1, n],
 // S(kk) = sum_{j<kk} L[j], L the image row; guards {0, 0} and {S(n), 0}.
-__global__ void __launch_bounds__(kScanThreads) dd_row_prefix_kernel(const DdInst *__restrict__ inst,
-                                                                     int ninst, const float *__restrict__ img,
-                                                                     double2 *__restrict__ work) {
-  __shared__ double wsum[kScanThreads / 32];
-  __shared__ double carry_s;
-  const long long b = blockIdx.x;
+struct RowSmem {
+  double wsum[kPrepWarps], carry;
+};
+__device__ __forceinline__ void dd_row_prefix(RowSmem &S, long long b, const DdInst *__restrict__ inst, int ninst,
+                                              const float *__restrict__ img, double2 *__restrict__ work) {
   const DdInst &I = inst[find_inst(inst, ninst, b, &DdInst::r0)];
   const int n = I.n, line = (int)(b - I.r0);
   const float *src = img + I.img + (size_t)line * n;
@@ -283,7 +279,7 @@ __global__ void __launch_bounds__(kScanThreads) dd_row_prefix_kernel(const DdIns
   for (int base = 0; base < n; base += kScanThreads) {
     const int k = base + threadIdx.x;
     const float v = k < n ? __ldg(src + k) : 0.0f;
-    const double ex = block_exclusive_scan((double)v, carry, wsum, &carry_s);
+    const double ex = block_exclusive_scan((double)v, carry, S.wsum, &S.carry);
     if (k < n) dst[k] = make_double2(ex, (double)v);
   }
   if (threadIdx.x == 0) {
@@ -292,49 +288,73 @@ __global__ void __launch_bounds__(kScanThreads) dd_row_prefix_kernel(const DdIns
   }
 }
 
-// Column lines (line c = image column c), 32 columns per block: each warp
-// sums a quarter of the rows, then rescans its rows 16 at a time through
-// shared memory so that each column line is written contiguously.
-__global__ void __launch_bounds__(32 * kColWarps) dd_col_prefix_kernel(const DdInst *__restrict__ inst,
-                                                                       int ninst, const float *__restrict__ img,
-                                                                       double2 *__restrict__ work) {
-  __shared__ double tot[kColWarps][32];
-  __shared__ double2 tile[kColWarps][kColRows][33];
-  const long long b = blockIdx.x;
+// Column lines (line c = image column c).  A column's sums run in kColParts
+// parts of its rows, each part from the total of those before it.  A block
+// writes one part of 32 columns: its first warps total the parts (a lane per
+// column), then every warp takes an eighth of the block's rows, walks the part
+// up to it without storing, and rescans its rows kColRows at a time through
+// shared memory so that each column line is written contiguously.  The chain of
+// additions is the same as one warp's per part, at an eighth of its latency.
+struct ColSmem {
+  double tot[kColParts][32], run[kPrepWarps][kColRows][33];
+  float val[kPrepWarps][kColRows][33];
+};
+__device__ __forceinline__ double dd_col_sum(const float *__restrict__ im, int n, int col, int r0, int r1, double t) {
+  if (col < n) {
+    int r = r0;
+    for (; r + 16 <= r1; r += 16) {
+      float v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) v[u] = __ldg(im + (size_t)(r + u) * n + col);
+#pragma unroll
+      for (int u = 0; u < 16; ++u) t += (double)v[u];
+    }
+#pragma unroll 1
+    for (; r < r1; ++r) t += (double)__ldg(im + (size_t)r * n + col);
+  }
+  return t;
+}
+__device__ __forceinline__ void dd_col_prefix(ColSmem &S, long long b4, const DdInst *__restrict__ inst, int ninst,
+                                              const float *__restrict__ img, double2 *__restrict__ work) {
+  const long long b = b4 / kColParts;
+  const int part = (int)(b4 % kColParts);
   const DdInst &I = inst[find_inst(inst, ninst, b, &DdInst::c0)];
   const int n = I.n, c0 = (int)(b - I.c0) * 32;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int col = c0 + lane;
   const float *im = img + I.img;
   double2 *SLc = work + I.sl + (size_t)n * (n + 2) + 1;
-  const int ch = (n + kColWarps - 1) / kColWarps;
-  const int r0 = min(w * ch, n), r1 = min(r0 + ch, n);
-  double t = 0.0;
-  if (col < n)
-    for (int r = r0; r < r1; ++r) t += (double)__ldg(im + (size_t)r * n + col);
-  tot[w][lane] = t;
+  const int ch = (n + kColParts - 1) / kColParts;
+  if (w < kColParts) S.tot[w][lane] = dd_col_sum(im, n, col, min(w * ch, n), min(w * ch + ch, n), 0.0);
   __syncthreads();
   double run = 0.0, total = 0.0;
-  for (int u = 0; u < kColWarps; ++u) {
-    if (u < w) run += tot[u][lane];
-    total += tot[u][lane];
+  for (int u = 0; u < kColParts; ++u) {
+    if (u < part) run += S.tot[u][lane];
+    total += S.tot[u][lane];
   }
+  const int p0 = min(part * ch, n), p1 = min(p0 + ch, n);
+  const int sub = (ch + kPrepWarps - 1) / kPrepWarps;
+  const int r0 = min(p0 + w * sub, p1), r1 = min(r0 + sub, p1);
+  run = dd_col_sum(im, n, col, p0, r0, run);
   for (int rb = r0; rb < r1; rb += kColRows) {
+#pragma unroll
     for (int rr = 0; rr < kColRows; ++rr) {
       const int r = rb + rr;
       const float v = (col < n && r < r1) ? __ldg(im + (size_t)r * n + col) : 0.0f;
-      tile[w][rr][lane] = make_double2(run, (double)v);
+      S.run[w][rr][lane] = run;
+      S.val[w][rr][lane] = v;
       run += (double)v;
     }
     __syncwarp();
-    for (int cc2 = 0; cc2 < 16; ++cc2) {
-      const int cc = 2 * cc2 + (lane >> 4), rr = lane & 15;
+#pragma unroll
+    for (int c4 = 0; c4 < 32; c4 += 32 / kColRows) {
+      const int cc = c4 + lane / kColRows, rr = lane % kColRows;
       const int cg = c0 + cc, r = rb + rr;
-      if (cg < n && r < r1) SLc[(size_t)cg * (n + 2) + r] = tile[w][rr][cc];
+      if (cg < n && r < r1) SLc[(size_t)cg * (n + 2) + r] = make_double2(S.run[w][rr][cc], (double)S.val[w][rr][cc]);
     }
     __syncwarp();
   }
-  if (w == 0 && col < n) {
+  if (part == 0 && w == 0 && col < n) {
     SLc[(size_t)col * (n + 2) - 1] = make_double2(0.0, 0.0);
     SLc[(size_t)col * (n + 2) + n] = make_double2(total, 0.0);
   }
@@ -344,16 +364,13 @@ __global__ void __launch_bounds__(32 * kColWarps) dd_col_prefix_kernel(const DdI
 // [-pads, n + pads)) holds {S_m, S_m+1}, the values (0 outside [0, n)) of the
 // two detectors a pixel starting in detector m can overlap.  (The boundary
 // D_m+1 between them is recomputed from m where it is needed.)
-__global__ void __launch_bounds__(kScanThreads) dd_sino_expand_kernel(const DdInst *__restrict__ inst,
-                                                                      int ninst, const float *__restrict__ sino,
-                                                                      double2 *__restrict__ work) {
-  const long long b = blockIdx.x;
+__device__ __forceinline__ void dd_sino_expand(long long b, const DdInst *__restrict__ inst, int ninst,
+                                               const float *__restrict__ sino, double2 *__restrict__ work) {
   const DdInst &I = inst[find_inst(inst, ninst, b, &DdInst::s0)];
-  const int v = (int)(b - I.s0), n = I.n, nh = I.nh, pads = I.pads, w2 = I.w2;
+  const int v = (int)(b - I.s0), n = I.n, pads = I.pads, w2 = I.w2;
   const DdAngle g = I.ang[v];
   const float *src = sino + I.sino + (size_t)g.out_row * n;
   float2 *dst = (float2 *)(work + I.as) + (size_t)v * w2;
-  (void)nh;
   for (int e = threadIdx.x; e < w2; e += blockDim.x) {
     const int m = e - pads;
     const float s0 = (m >= 0 && m < n) ? __ldg(src + m) : 0.0f;
@@ -363,23 +380,25 @@ __global__ void __launch_bounds__(kScanThreads) dd_sino_expand_kernel(const DdIn
 }
 
 // ---------------------------------------------------------------------------
-// Forward: a warp item is 127 detectors of one angle; lane l holds the lower
+// Forward: an item is 127 detectors of one angle; lane l holds the lower
 // boundaries of detectors B0 + 32 j + l (j = 0..3), and T_j = sum over lines of
 // F(boundary).  The dropped pieces and the binade corrections come from
 // dd_fwd_corr_kernel's row; keeping them out of this loop leaves it 64
 // registers (with them inline: 76, and 24 instead of 32 warps per SM).
 // ---------------------------------------------------------------------------
+template <int J>
 __device__ __forceinline__ void dd_fwd_lines(int ia, int ib, const double2 *__restrict__ SL, int ws, float k,
-                                             int n, int nh, const float (&Dlo)[4], const float (&lo_nh)[4],
-                                             double (&T)[4]) {
+                                             int n, int nh, const float (&Dlo)[J], const float (&lo_nh)[J],
+                                             double (&T)[J]) {
+  constexpr int kUnroll = J == 4 ? 2 : 8;  // lines per step: 8 loads in flight per lane either way
   float y = (float)(ia - nh) + 0.5f;
   const double2 *sl = SL + (size_t)ia * ws;
   const float nlim = (float)n + 0.25f, cmn = kMagic + (float)nh;
-#pragma unroll kFwdUnroll
+#pragma unroll kUnroll
   for (int i = ia; i < ib; ++i) {
     const float q = __fmul_rn(y, k);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < J; ++j) {
       // kk = floor(D + nh + q) clamped to [-1, n], as a float and an int:
       // t + 1.5 * 2^23 rounded down lies where floats are the integers, so
       // f = 1.5 * 2^23 + floor(t) exactly, and its bits give kk
@@ -493,13 +512,14 @@ __device__ __forceinline__ bool dd_fwd_crossing(const float *__restrict__ V, int
 // meeting it, the overlap pieces of the detector with the line's pixels, from
 // the same float boundaries as the reference, the dropped last piece skipped
 // (radon_dd.c:125-189), summed in double.
+template <int J>
 __device__ __forceinline__ void dd_fwd_exact(const double2 *__restrict__ SL, int ws, float k, float r, int n, int nh,
-                                          int B0, int mEnd, int lane, double (&T)[4]) {
+                                          int B0, int j0, int mEnd, int lane, double (&T)[J]) {
   const float Dn = det_bound(n, nh, r);
 #pragma unroll 1
-  for (int t = 0; t < 4; ++t) {
-    const int m = B0 + 32 * t + lane;
-    if (32 * t + lane >= kGrpDet || m >= mEnd) continue;
+  for (int t = 0; t < J; ++t) {
+    const int m = B0 + 32 * (j0 + t) + lane;
+    if (32 * (j0 + t) + lane >= kGrpDet || m >= mEnd) continue;
     const float Dlo = det_bound(m, nh, r), Dhi = det_bound(m + 1, nh, r);
     int i0, i1;
     dd_line_range(-(double)nh - (double)Dhi, (double)(n - nh) - (double)Dlo, (double)k, n, nh, i0, i1);
@@ -527,29 +547,72 @@ __device__ __forceinline__ void dd_fwd_exact(const double2 *__restrict__ SL, int
   }
 }
 
+__device__ __forceinline__ bool dd_wide(float k, int nh) {
+  return fabsf(k) * (float)(nh + 1) + (float)(nh + 2) >= 4194304.0f;
+}
+
+constexpr int kCorrRow = 4096;    // rows longer than this are added in global memory
+constexpr int kDropChunk = 1024;  // dropped pieces staged at a time
+
+// 32 staged pieces starting at t0 (key, amount; key < 0: none): each key's
+// pieces summed in their order, the sum left with the first of them and the
+// others' keys set to -1.  The batches of a chunk are summed by different warps;
+// dd_drop_apply then takes the sums from the targets, batch after batch.
+__device__ __forceinline__ void dd_drop_batch(int *key, double *amt, int t0, int lane) {
+  const int k = key[t0 + lane];
+  const unsigned grp = __match_any_sync(0xffffffffu, k);
+  const bool first = k >= 0 && lane == __ffs(grp) - 1;
+  double sum = 0.0;
+  if (first)
+    for (unsigned mk = grp; mk;) {
+      double a[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        a[u] = mk ? amt[t0 + __ffs(mk) - 1] : 0.0;
+        mk &= mk - 1;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) sum += a[u];
+    }
+  __syncwarp();
+  key[t0 + lane] = first ? k : -1;
+  amt[t0 + lane] = sum;
+}
+// One warp: R[key * step] -= sum for the chunk's batches in order (a batch's keys differ).
+__device__ __forceinline__ void dd_drop_apply(const int *key, const double *amt, int count, float *R, size_t step,
+                                              int lane) {
+  int k = key[lane];
+  double a = amt[lane];
+  for (int t0 = 0; t0 < count; t0 += 32) {
+    const int k0 = k;
+    const double a0 = a;
+    if (t0 + 32 < count) {
+      k = key[t0 + 32 + lane];
+      a = amt[t0 + 32 + lane];
+    }
+    if (k0 >= 0) R[k0 * step] = __double2float_rn((double)R[k0 * step] - a0);
+    __syncwarp();
+  }
+}
+
 // The binade corrections and the dropped pieces of every angle into the float
 // rows X[v][m] that the forward adds where it stores: one block per angle of
 // every instance, its warps taking the crossings in turn (dd_fwd_crossing);
 // the crossings' sums are added into the row in crossing order through shared
 // memory, then each line's dropped piece in line order, so the result is
-// deterministic.  A launch of its own, so that the forward's register budget
-// is that of its main loop.
-__device__ __forceinline__ bool dd_wide(float k, int nh) {
-  return fabsf(k) * (float)(nh + 1) + (float)(nh + 2) >= 4194304.0f;
-}
-
-constexpr int kCorrWarps = 8, kCorrRow = 4096;  // rows longer than kCorrRow are added in global memory
-constexpr int kDropChunk = 1024;                 // lines whose dropped pieces are staged at a time
-
-__global__ void __launch_bounds__(32 * kCorrWarps) dd_fwd_corr_kernel(const DdInst *__restrict__ inst, int ninst,
-                                                                      const float *__restrict__ img,
-                                                                      double2 *__restrict__ work) {
-  __shared__ double sums[kNumCrossings][4];
-  __shared__ int smc[kNumCrossings];
-  __shared__ float row[kCorrRow];
-  __shared__ int ddet[kDropChunk];
-  __shared__ double damt[kDropChunk];
-  const long long b = blockIdx.x;
+// deterministic.  Out of the forward, whose register budget is then that of
+// its main loop.  Bound by latency, not by work: a few hundred blocks of short
+// dependent chains.  So everything but the last additions runs in parallel: a
+// thread per (crossing, detector), which takes the later crossings of the same
+// detector along, and a warp per 32 lines' pieces (one thread and one warp for
+// all of them: 31 us at 256^2 x 304, 88 at 768^2 x 720).
+struct CorrSmem {
+  double amt[kDropChunk], sums[kNumCrossings][4];
+  int key[kDropChunk], smc[kNumCrossings];
+  float row[kCorrRow];
+};
+__device__ __forceinline__ void dd_fwd_corr(CorrSmem &S, long long b, const DdInst *__restrict__ inst, int ninst,
+                                            const float *__restrict__ img, double2 *__restrict__ work) {
   const DdInst &I = inst[find_inst(inst, ninst, b, &DdInst::s0)];
   const int v = (int)(b - I.s0), n = I.n, nh = I.nh;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -560,80 +623,99 @@ __global__ void __launch_bounds__(32 * kCorrWarps) dd_fwd_corr_kernel(const DdIn
   // 17 MB that stay in L2, where the prefix tables' values (134 MB) would not
   const float *V = img + I.img;
   const int si = g.mode == DD_ROWS ? n : 1, sj = g.mode == DD_ROWS ? 1 : n;
-  for (int c = warp; c < kNumCrossings; c += kCorrWarps) {
-    int mc = 0;
-    double a[4] = {0.0, 0.0, 0.0, 0.0};
-    const bool used = lines && dd_fwd_crossing(V, si, sj, g.k, g.r, n, nh, c, lane, mc, a);
-    if (lane == 0) {
-      smc[c] = used ? mc : INT_MIN;
-#pragma unroll
-      for (int t = 0; t < 4; ++t) sums[c][t] = a[t];
-    }
-  }
   const bool in_smem = n <= kCorrRow;
-  for (int m = threadIdx.x; m < n; m += blockDim.x) {
-    if (in_smem) row[m] = 0.0f;
-    else X[m] = 0.0f;
-  }
-  __syncthreads();
-  float *R = in_smem ? row : X;
-  if (threadIdx.x == 0) {
-    for (int c = 0; c < kNumCrossings; ++c) {
-      if (smc[c] == INT_MIN) continue;
-      for (int t = 0; t < 4; ++t) {
-        const int m = smc[c] - 1 + t;
-        if (m >= 0 && m < n) R[m] += (float)sums[c][t];
+  float *R = in_smem ? S.row : X;
+  for (int m = threadIdx.x; m < n; m += kScanThreads) R[m] = 0.0f;
+  if (lines) {
+    for (int c = warp; c < kNumCrossings; c += kPrepWarps) {
+      int mc = 0;
+      double a[4] = {0.0, 0.0, 0.0, 0.0};
+      const bool used = dd_fwd_crossing(V, si, sj, g.k, g.r, n, nh, c, lane, mc, a);
+      if (lane == 0) {
+        S.smc[c] = used ? mc : INT_MIN / 2;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) S.sums[c][t] = a[t];
       }
     }
-  }
-  // The piece of every line the reference never credits (dd_dropped_piece),
-  // subtracted from its detector, line after line by one thread.
-  if (lines) {
+    __syncthreads();
+    if (threadIdx.x < 4 * kNumCrossings) {
+      const int c0 = threadIdx.x >> 2, m = S.smc[c0] - 1 + (threadIdx.x & 3);
+      if (m >= 0 && m < n) {
+        bool owner = true;  // no earlier crossing reaches m
+        for (int c = 0; c < c0; ++c) owner = owner && (unsigned)(m - S.smc[c] + 1) > 3u;
+        if (owner) {
+          float x = 0.0f;
+          for (int c = c0; c < kNumCrossings; ++c) {
+            const int t = m - S.smc[c] + 1;
+            if ((unsigned)t <= 3u) x += (float)S.sums[c][t];
+          }
+          R[m] = x;
+        }
+      }
+    }
+    // The piece of every line the reference never credits (dd_dropped_piece),
+    // subtracted from its detector in line order.
     for (int i0 = 0; i0 < n; i0 += kDropChunk) {
+      const int count = min(kDropChunk, (n - i0 + 31) & ~31);
       __syncthreads();
-      for (int t = threadIdx.x; t < kDropChunk && i0 + t < n; t += blockDim.x) {
+      for (int t = threadIdx.x; t < count; t += kScanThreads) {
         const int i = i0 + t;
         const float q = __fmul_rn(__fadd_rn((float)(i - nh), 0.5f), g.k);
         DdDrop d;
         int det = -1;
         double amt = 0.0;
-        if (dd_dropped_piece(q, g.r, n, nh, d)) {
+        if (i < n && dd_dropped_piece(q, g.r, n, nh, d)) {
           det = d.det;
           amt = (double)d.gap * (double)__ldg(V + (size_t)i * si + (size_t)d.pix * sj);
         }
-        ddet[t] = det;
-        damt[t] = amt;
+        S.key[t] = det;
+        S.amt[t] = amt;
+        __syncwarp();
+        dd_drop_batch(S.key, S.amt, t - lane, lane);  // the 32 lines of this warp
       }
       __syncthreads();
-      // warp 0, 32 lines at a time: the lanes with the same detector form a
-      // group whose lowest lane subtracts the group's pieces summed in line
-      // order; different groups touch different detectors, and the batches
-      // go in line order
-      if (warp == 0)
-        for (int t0 = 0; t0 < kDropChunk && i0 + t0 < n; t0 += 32) {
-          const int t = t0 + lane;
-          const int det = i0 + t < n ? ddet[t] : -1;
-          const unsigned grp = __match_any_sync(0xffffffffu, det);
-          if (det >= 0 && lane == __ffs(grp) - 1) {
-            double sum = 0.0;
-            for (unsigned mk = grp; mk; mk &= mk - 1) sum += damt[t0 + __ffs(mk) - 1];
-            R[det] = __double2float_rn((double)R[det] - sum);
-          }
-          __syncwarp();
-        }
+      if (warp == 0) dd_drop_apply(S.key, S.amt, count, R, 1, lane);
     }
   }
   __syncthreads();
   if (in_smem)
-    for (int m = threadIdx.x; m < n; m += blockDim.x) X[m] = row[m];
+    for (int m = threadIdx.x; m < n; m += kScanThreads) X[m] = R[m];
 }
 
+// The forward's pre-passes, independent of one another, in one launch: a block
+// per angle (corrections), per part of 32 columns, and per row, the longest
+// chains first.
+union FwdPrepSmem {
+  CorrSmem corr;
+  ColSmem col;
+  RowSmem row;
+};
+__global__ void __launch_bounds__(kScanThreads) dd_fwd_prep_kernel(const DdInst *__restrict__ inst, int ninst,
+                                                                   unsigned corr_blocks, unsigned col_blocks,
+                                                                   const float *__restrict__ img,
+                                                                   double2 *__restrict__ work) {
+  __shared__ __align__(16) char smem[sizeof(FwdPrepSmem)];
+  FwdPrepSmem &S = *reinterpret_cast<FwdPrepSmem *>(smem);
+  unsigned b = blockIdx.x;
+  if (b < corr_blocks) {
+    dd_fwd_corr(S.corr, b, inst, ninst, img, work);
+  } else if ((b -= corr_blocks) < col_blocks) {
+    dd_col_prefix(S.col, b, inst, ninst, img, work);
+  } else {
+    dd_row_prefix(S.row, b - col_blocks, inst, ninst, img, work);
+  }
+}
+
+// One item.  J = 4: a warp holds all its boundaries.  J = 1: the block's four
+// warps hold 32 each and hand the sums to the first through Ts; the lines, and
+// the order of every sum, are the same, so the result is too.
+template <int J>
 __device__ __forceinline__ void dd_fwd_item(const DdInst &I, int v, int grp, int lane,
                                             const double2 *__restrict__ work, float *__restrict__ sino,
-                                            const FwdEpi &ep, long long slot) {
+                                            const FwdEpi &ep, long long slot, double (*Ts)[32]) {
   const DdAngle g = I.ang[v];
   const int n = I.n, nh = I.nh, ws = n + 2;
-  const int B0 = grp * kGrpDet;
+  const int B0 = grp * kGrpDet, j0 = J == 4 ? 0 : (int)(threadIdx.x >> 5);
   const double2 *SLr = work + I.sl + 1, *SLc = SLr + (size_t)n * ws;
   float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   if (g.mode == DD_ROWSUM || g.mode == DD_COLSUM) {
@@ -647,26 +729,37 @@ __device__ __forceinline__ void dd_fwd_item(const DdInst &I, int v, int grp, int
   } else if (g.mode == DD_ROWS || g.mode == DD_COLS) {
     const double2 *SL = g.mode == DD_ROWS ? SLr : SLc;
     const float r = g.r, k = g.k;
-    float Dlo[4], lo_nh[4];
+    float Dlo[J], lo_nh[J];
+    double Tj[J];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      Dlo[j] = det_bound(B0 + 32 * j + lane, nh, r);
+    for (int j = 0; j < J; ++j) {
+      Dlo[j] = det_bound(B0 + 32 * (j0 + j) + lane, nh, r);
       lo_nh[j] = __fadd_rn(Dlo[j], (float)nh);
+      Tj[j] = 0.0;
     }
     const int mEnd = min(B0 + kGrpDet, n);
     const double DA = (double)det_bound(B0, nh, r), DB = (double)det_bound(mEnd, nh, r);
     const double kd = (double)k, PN = (double)(n - nh);
     int i0, i1;
     dd_line_range(-(double)nh - DB, PN - DA, kd, n, nh, i0, i1);
-    if (dd_wide(k, nh)) {
-      // |P| reaches 2^22: pieces walked exactly (rare near-axis angles)
-      double T[4] = {0.0, 0.0, 0.0, 0.0};
-      dd_fwd_exact(SL, ws, k, r, n, nh, B0, mEnd, lane, T);
+    const bool wide = dd_wide(k, nh);
+    // |P| reaches 2^22: pieces walked exactly (rare near-axis angles)
+    if (wide) dd_fwd_exact<J>(SL, ws, k, r, n, nh, B0, j0, mEnd, lane, Tj);
+    else dd_fwd_lines<J>(i0, i1 + 1, SL, ws, k, n, nh, Dlo, lo_nh, Tj);
+    double T[4];
+    if (J == 1) {
+      Ts[j0][lane] = Tj[0];
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) T[j] = Ts[j][lane];
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) T[j] = Tj[j < J ? j : 0];
+    }
+    if (wide) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[j] = (float)T[j];
     } else {
-      double T[4] = {0.0, 0.0, 0.0, 0.0};
-      dd_fwd_lines(i0, i1 + 1, SL, ws, k, n, nh, Dlo, lo_nh, T);
       // the upper boundary of detector B0 + 32 j + l is lane l+1's j-th, or lane 0's (j+1)-th
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -681,6 +774,7 @@ __device__ __forceinline__ void dd_fwd_item(const DdInst &I, int v, int grp, int
       }
     }
   }
+  if (J == 1 && j0 > 0) return;
   double r2 = 0.0;
   const size_t row = (size_t)I.sino + (size_t)g.out_row * n;
 #pragma unroll
@@ -716,6 +810,26 @@ __device__ __forceinline__ int centre_out(int gi, int ngrp) {
   return (gi & 1) ? c + ((gi + 1) >> 1) : c - (gi >> 1);
 }
 
+// Items run all angles on row lines (every detector group) before those on
+// column lines, so that the warps in flight read one of the two prefix
+// tables at a time (each about half of L2 at 2048^2).
+__device__ __forceinline__ const DdInst &fwd_locate(const DdInst *__restrict__ inst, int ninst, long long item, int &v,
+                                                    int &grp) {
+  const DdInst &I = inst[find_inst(inst, ninst, item, &DdInst::f0)];
+  const int local = (int)(item - I.f0), nRg = I.nRf * I.ngrp;
+  int gi;
+  if (local < nRg) {
+    gi = local / I.nRf;
+    v = __ldg(I.fperm + local % I.nRf);
+  } else {
+    const int l2 = local - nRg, nCf = I.na - I.nRf;
+    gi = l2 / nCf;
+    v = __ldg(I.fperm + I.nRf + l2 % nCf);
+  }
+  grp = centre_out(gi, I.ngrp);
+  return I;
+}
+
 template <int W, bool BLOCK>
 __global__ void __launch_bounds__(32 * W) dd_fwd_kernel(const DdInst *__restrict__ inst, int ninst,
                                                          long long nitems, unsigned long long *__restrict__ ctr,
@@ -727,28 +841,26 @@ __global__ void __launch_bounds__(32 * W) dd_fwd_kernel(const DdInst *__restrict
     const long long item = fetch_item<BLOCK>(ctr, W, &base_s);
     if (item - (BLOCK ? (threadIdx.x >> 5) : 0) >= nitems) break;  // block-uniform under BLOCK
     if (item < nitems) {
-      const DdInst &I = inst[find_inst(inst, ninst, item, &DdInst::f0)];
-      // items run all angles on row lines (every detector group) before those on
-      // column lines, so that the warps in flight read one of the two prefix
-      // tables at a time (each about half of L2 at 2048^2)
-      const int local = (int)(item - I.f0), nRg = I.nRf * I.ngrp;
-      int gi, v;
-      if (local < nRg) {
-        gi = local / I.nRf;
-        v = __ldg(I.fperm + local % I.nRf);
-      } else {
-        const int l2 = local - nRg, nCf = I.na - I.nRf;
-        gi = l2 / nCf;
-        v = __ldg(I.fperm + I.nRf + l2 % nCf);
-      }
-      dd_fwd_item(I, v, centre_out(gi, I.ngrp), lane, work, sino, ep, item);
+      int v, grp;
+      const DdInst &I = fwd_locate(inst, ninst, item, v, grp);
+      dd_fwd_item<4>(I, v, grp, lane, work, sino, ep, item, nullptr);
     }
   }
 }
 
+// A block of four warps per item, for plans whose items are few (dd_build).
+__global__ void __launch_bounds__(128) dd_fwd_split_kernel(const DdInst *__restrict__ inst, int ninst,
+                                                           const double2 *__restrict__ work,
+                                                           float *__restrict__ sino, FwdEpi ep) {
+  __shared__ double Ts[4][32];
+  int v, grp;
+  const DdInst &I = fwd_locate(inst, ninst, blockIdx.x, v, grp);
+  dd_fwd_item<1>(I, v, grp, threadIdx.x & 31, work, sino, ep, blockIdx.x, Ts);
+}
+
 // ---------------------------------------------------------------------------
-// Adjoint: a warp item is a 32x16 pixel tile; lane l holds the 4x4 pixels at
-// rows a0..a0+3 and columns b0..b0+3.  Per angle and line each pixel [P0, P1]
+// Adjoint: an item is a 32 x 4R pixel tile; lane l holds the R x 4 pixels at
+// rows a0..a0+R-1 and columns b0..b0+3.  Per angle and line each pixel [P0, P1]
 // overlaps the detector a holding P0 and possibly a+1 (detectors are at least
 // one pixel wide): (min(D_a+1, P1) - P0) S_a + (P1 - min(D_a+1, P1)) S_a+1,
 // the reference's two gaps, both accumulated by FMA.
@@ -767,95 +879,136 @@ __device__ __forceinline__ void dd_adj_pixel(float P0, float P1, float z, float 
   acc = __fmaf_rn(__fsub_rn(P1, m), t.y, acc);
 }
 
-template <bool COLS>
+template <bool COLS, int R>
 __device__ __forceinline__ void dd_adj_pass(const float4 *__restrict__ tab, int cnt,
                                             const float2 *__restrict__ AS, int a0, int b0, int n, int nh,
-                                            float (&acc)[4][4]) {
+                                            float (&acc)[R][4]) {
+  constexpr int NL = COLS ? 4 : R, NP = COLS ? R : 4;  // lines, pixels of a line
   const int l0 = COLS ? b0 : a0, k0 = COLS ? a0 : b0;
   const float y0 = (float)(l0 - nh) + 0.5f;
-  float x[5];
+  float x[NP + 1];
 #pragma unroll
-  for (int j = 0; j < 5; ++j) x[j] = (float)(k0 - nh + j);
+  for (int j = 0; j <= NP; ++j) x[j] = (float)(k0 - nh + j);
   const float cm = kMagic + (float)nh, cm1 = cm - 1.0f;
-#pragma unroll 1
+  constexpr int kUnroll = R == 4 ? 1 : 2;
+#pragma unroll kUnroll
   for (int u = 0; u < cnt; ++u) {
     const float4 e = __ldg(tab + u);
     const float r = e.x, k = e.y, z = e.z;
     const float2 *rowm = AS + __float_as_int(e.w) - kMagicBits;
 #pragma unroll
-    for (int li = 0; li < 4; ++li) {
+    for (int li = 0; li < NL; ++li) {
       const float q = __fmul_rn(__fadd_rn(y0, (float)li), k);
-      float P[5];
+      float P[NP + 1];
 #pragma unroll
-      for (int j = 0; j < 5; ++j) P[j] = __fsub_rn(x[j], q);
+      for (int j = 0; j <= NP; ++j) P[j] = __fsub_rn(x[j], q);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) dd_adj_pixel(P[j], P[j + 1], z, r, cm, cm1, rowm, COLS ? acc[j][li] : acc[li][j]);
+      for (int j = 0; j < NP; ++j) dd_adj_pixel(P[j], P[j + 1], z, r, cm, cm1, rowm, COLS ? acc[j][li] : acc[li][j]);
     }
   }
 }
 
 // The adjoint's dropped pieces (the last piece of each line and angle that
 // the reference never credits, dd_dropped_piece), as an image C that the
-// adjoint adds where it stores: a warp per line (an image row for the angles
-// on rows, a column for those on columns), 32 angles at a time; the lanes
-// whose pieces fall on the same pixel form a group whose lowest lane
-// subtracts their sum, taken in angle order, from C.  The row launch zeroes
-// its lines first and runs before the column launch, so every pixel gets its
-// pieces in one fixed order.  Out of the adjoint's main loop, which then holds
+// adjoint adds where it stores: a block per line (an image row for the angles
+// on rows, a column for those on columns), a warp per 32 angles, whose pieces
+// that fall on the same pixel are summed in angle order (dd_drop_batch); one
+// warp then takes the sums from the pixels, batch after batch.  The rows are
+// zeroed first and are done before the columns, so every pixel gets its pieces
+// in one fixed order.  One warp per line, which did all of it, left the GPU
+// waiting on its chain: 12 + 12 us at 256^2 x 304, 25 + 25 at 768^2 x 720.  Out of the adjoint's main loop, which then holds
 // 64 registers (with the pieces inline: 80, and 24 instead of 32 warps per SM).
+struct DropSmem {
+  double amt[kDropChunk];
+  int key[kDropChunk];
+  float row[kCorrRow];
+};
 template <bool COLS>
-__global__ void __launch_bounds__(32) dd_adj_drop_kernel(const DdInst *__restrict__ inst, int ninst,
-                                                         double2 *__restrict__ work) {
-  __shared__ double samt[32];
-  const long long b = blockIdx.x;
+__device__ __forceinline__ void dd_adj_drop(DropSmem &S, long long b, const DdInst *__restrict__ inst, int ninst,
+                                            const float *__restrict__ sino, double2 *__restrict__ work) {
   const DdInst &I = inst[find_inst(inst, ninst, b, &DdInst::r0)];
-  const int l = (int)(b - I.r0), n = I.n, nh = I.nh, lane = threadIdx.x;
-  float *C = reinterpret_cast<float *>(work + I.xs);
+  const int l = (int)(b - I.r0), n = I.n, nh = I.nh, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const size_t si = COLS ? 1 : (size_t)n, sp = COLS ? (size_t)n : 1;  // pixel p of line l: C[l si + p sp]
+  float *C = reinterpret_cast<float *>(work + I.xs) + (size_t)l * si;
+  const bool in_smem = n <= kCorrRow;
   if (!COLS)
-    for (int p = lane; p < n; p += 32) C[(size_t)l * n + p] = 0.0f;
-  __syncwarp();
+    for (int p = threadIdx.x; p < n; p += kScanThreads) (in_smem ? S.row : C)[p] = 0.0f;
   const float4 *tab = I.tab + (COLS ? I.nR : 0);
   const int cnt = COLS ? I.nC : I.nR;
-  const float2 *AS = (const float2 *)(work + I.as) + I.pads;
   const float y = __fadd_rn((float)(l - nh), 0.5f);
-  for (int u0 = 0; u0 < cnt; u0 += 32) {
-    const int u = u0 + lane;
-    int pix = -1;
-    float amt = 0.0f;
-    if (u < cnt) {
-      const float4 e = __ldg(tab + u);
-      DdDrop d;
-      if (dd_dropped_piece(__fmul_rn(y, e.y), e.x, n, nh, d)) {
-        pix = d.pix;
-        amt = __fmul_rn(d.gap, __ldg(&(AS + __float_as_int(e.w))[d.det].x));
+  for (int u0 = 0; u0 < cnt; u0 += kDropChunk) {
+    const int count = min(kDropChunk, (cnt - u0 + 31) & ~31);
+    __syncthreads();
+    for (int t = threadIdx.x; t < count; t += kScanThreads) {
+      const int u = u0 + t;
+      int pix = -1;
+      float amt = 0.0f;
+      if (u < cnt) {
+        const float4 e = __ldg(tab + u);
+        DdDrop d;
+        if (dd_dropped_piece(__fmul_rn(y, e.y), e.x, n, nh, d)) {
+          pix = d.pix;
+          const int out_row = I.na - 1 - __float_as_int(e.w) / I.w2;
+          amt = __fmul_rn(d.gap, __ldg(sino + I.sino + (size_t)out_row * n + d.det));
+        }
+      }
+      S.key[t] = pix;
+      S.amt[t] = (double)amt;
+      __syncwarp();
+      dd_drop_batch(S.key, S.amt, t - lane, lane);
+      // a column's touched pixels come into shared memory and go back below
+      const int k = S.key[t];
+      if (COLS && in_smem && k >= 0) S.row[k] = C[(size_t)k * sp];
+    }
+    __syncthreads();
+    if (warp == 0) {
+      if (in_smem) dd_drop_apply(S.key, S.amt, count, S.row, 1, lane);
+      else dd_drop_apply(S.key, S.amt, count, C, sp, lane);
+    }
+    if (COLS && in_smem) {
+      __syncthreads();
+      for (int t = threadIdx.x; t < count; t += kScanThreads) {
+        const int k = S.key[t];
+        if (k >= 0) C[(size_t)k * sp] = S.row[k];
       }
     }
-    samt[lane] = (double)amt;
-    __syncwarp();
-    const unsigned grp = __match_any_sync(0xffffffffu, pix);
-    if (pix >= 0 && lane == __ffs(grp) - 1) {
-      double sum = 0.0;
-      for (unsigned mk = grp; mk; mk &= mk - 1) sum += samt[__ffs(mk) - 1];
-      float *c = C + (size_t)l * si + (size_t)pix * sp;
-      *c = __double2float_rn((double)*c - sum);
-    }
-    __syncwarp();
+  }
+  if (!COLS && in_smem) {
+    __syncthreads();
+    for (int p = threadIdx.x; p < n; p += kScanThreads) C[p] = S.row[p];
   }
 }
 
-// One item = one 32x16 tile, worked on by 4 warps: warp `quarter` sums the
+// The adjoint's pre-passes: the row lines' dropped pieces and the sinogram
+// tables in one launch, then the columns' pieces.
+__global__ void __launch_bounds__(kScanThreads) dd_adj_prep_kernel(const DdInst *__restrict__ inst, int ninst,
+                                                                   unsigned drop_blocks, const float *__restrict__ sino,
+                                                                   double2 *__restrict__ work) {
+  __shared__ DropSmem S;
+  const unsigned b = blockIdx.x;
+  if (b < drop_blocks) dd_adj_drop<false>(S, b, inst, ninst, sino, work);
+  else dd_sino_expand(b - drop_blocks, inst, ninst, sino, work);
+}
+__global__ void __launch_bounds__(kScanThreads) dd_adj_col_drop_kernel(const DdInst *__restrict__ inst, int ninst,
+                                                                       const float *__restrict__ sino,
+                                                                       double2 *__restrict__ work) {
+  __shared__ DropSmem S;
+  dd_adj_drop<true>(S, blockIdx.x, inst, ninst, sino, work);
+}
+
+// One item = one tile of 32 x 4R pixels (R = 4, or 1 for plans of few tiles:
+// dd_adj_rows), worked on by 4 warps: warp `quarter` sums the
 // angles [quarter T / 4, (quarter + 1) T / 4) of the ROWS-then-COLS order (T =
 // nR + nC), and the tile's first warp adds the quarters in order, then the
 // row / column sums, then stores.  The split never depends on the launch
 // shape, so every shape gives the same bits.
-template <int TB>
+template <int TB, int R>
 __global__ void __launch_bounds__(128 * TB) dd_adj_kernel(const DdInst *__restrict__ inst, int ninst,
                                                            long long nitems, unsigned long long *__restrict__ ctr,
                                                            const double2 *__restrict__ work,
                                                            float *__restrict__ img, AdjEpi ep) {
   __shared__ long long base_s;
-  __shared__ float part[TB][3][16][32];  // quarters 1..3 of each tile
+  __shared__ float part[TB][3][4 * R][32];  // quarters 1..3 of each tile
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tile = warp >> 2, quarter = warp & 3;
   for (;;) {
@@ -865,9 +1018,9 @@ __global__ void __launch_bounds__(128 * TB) dd_adj_kernel(const DdInst *__restri
     __syncthreads();
     if (first >= nitems) break;  // block-uniform
     const long long item = first + tile;
-    float acc[4][4];
+    float acc[R][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
     const DdInst *Ip = nullptr;
@@ -878,7 +1031,7 @@ __global__ void __launch_bounds__(128 * TB) dd_adj_kernel(const DdInst *__restri
       const DdInst &I = *Ip;
       const int local = (int)(item - I.a0);
       b0 = (local % I.tx) * kTileW + 4 * (lane & 7);
-      a0 = (local / I.tx) * kTileH + 4 * (lane >> 3);
+      a0 = (local / I.tx) * (4 * R) + R * (lane >> 3);
       // lanes whose block starts outside the image (n not a multiple of 4)
       // only take part in the epilogue's warp reductions
       inside = a0 < I.n && b0 < I.n;
@@ -887,14 +1040,14 @@ __global__ void __launch_bounds__(128 * TB) dd_adj_kernel(const DdInst *__restri
         const int u0 = (int)((long long)T * quarter / 4), u1 = (int)((long long)T * (quarter + 1) / 4);
         const float2 *AS = (const float2 *)(work + I.as) + I.pads;
         const int r0 = min(u0, I.nR), r1 = min(u1, I.nR);
-        if (r1 > r0) dd_adj_pass<false>(I.tab + r0, r1 - r0, AS, a0, b0, I.n, I.nh, acc);
+        if (r1 > r0) dd_adj_pass<false, R>(I.tab + r0, r1 - r0, AS, a0, b0, I.n, I.nh, acc);
         const int c0 = max(u0, I.nR), c1 = max(u1, I.nR);
-        if (c1 > c0) dd_adj_pass<true>(I.tab + c0, c1 - c0, AS, a0, b0, I.n, I.nh, acc);
+        if (c1 > c0) dd_adj_pass<true, R>(I.tab + c0, c1 - c0, AS, a0, b0, I.n, I.nh, acc);
       }
     }
     if (quarter > 0) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) part[tile][quarter - 1][4 * i + j][lane] = acc[i][j];
     }
@@ -905,7 +1058,7 @@ __global__ void __launch_bounds__(128 * TB) dd_adj_kernel(const DdInst *__restri
 #pragma unroll
       for (int q = 0; q < 3; ++q)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < R; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) acc[i][j] += part[tile][q][4 * i + j][lane];
       const float2 *AS = (const float2 *)(work + I.as) + I.pads;
@@ -913,14 +1066,14 @@ __global__ void __launch_bounds__(128 * TB) dd_adj_kernel(const DdInst *__restri
         const int2 e = __ldg(I.tabS + t);
         const float2 *row = AS + e.y;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < R; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) acc[i][j] += __ldg(&row[e.x == DD_ROWSUM ? a0 + i : b0 + j].x);
       }
       // the dropped pieces (dd_adj_drop_kernel)
       const float *Cimg = reinterpret_cast<const float *>(work + I.xs);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int a = a0 + i, b = b0 + j;
@@ -984,6 +1137,7 @@ namespace {
 
 // Per-plan state: the instance table, the geometry tables of every distinct
 // geometry, the persistent kernels' work counters and the tuned launch shape.
+constexpr int kSplitCfg = 6;  // kDdCfg's block of four warps per item
 struct DdState {
   std::vector<DdInst> inst;  // scheduling order (largest work first)
   DdInst *d_inst = nullptr;
@@ -991,7 +1145,8 @@ struct DdState {
   unsigned long long *d_ctr = nullptr;  // [0] forward items, [1] adjoint items
   long long fwd_items = 0, adj_items = 0, row_blocks = 0, col_blocks = 0, sino_blocks = 0;
   double updates = 0.0;  // pixel x angle updates per application
-  int wf = 1, wa = 1;    // launch shape (kDdCfg index) of the forward / adjoint kernels
+  int R = 4;             // pixel rows per lane of the adjoint
+  int wf = kSplitCfg, wa = 1;    // launch shape (kDdCfg index) of the forward / adjoint kernels
   int grid_f = 0, grid_a = 0;
   std::vector<size_t> img_off, sino_off;  // packed offsets in the caller's order (count + 1)
   std::string tuning;
@@ -1010,36 +1165,47 @@ using FwdFn = void (*)(const DdInst *, int, long long, unsigned long long *, con
 using AdjFn = void (*)(const DdInst *, int, long long, unsigned long long *, const double2 *, float *,
                       AdjEpi);
 // Launch shapes the autotuner chooses from.  Forward: warps per block x
-// fetch mode.  Adjoint: tiles per block (4 warps each).
+// fetch mode, or a block of four warps per item (fwd null).  Adjoint: tiles per
+// block (4 warps each).
 struct DdCfg {
   int W;
-  bool block;
+  char mode;  // w: a warp fetches its item, b: a block W items, s: an item's boundaries split over the warps
   FwdFn fwd;
 };
 const DdCfg kDdCfg[] = {
-    {2, false, dd_fwd_kernel<2, false>}, {4, false, dd_fwd_kernel<4, false>}, {8, false, dd_fwd_kernel<8, false>},
-    {2, true, dd_fwd_kernel<2, true>},   {4, true, dd_fwd_kernel<4, true>},   {8, true, dd_fwd_kernel<8, true>},
+    {2, 'w', dd_fwd_kernel<2, false>}, {4, 'w', dd_fwd_kernel<4, false>}, {8, 'w', dd_fwd_kernel<8, false>},
+    {2, 'b', dd_fwd_kernel<2, true>},   {4, 'b', dd_fwd_kernel<4, true>},   {8, 'b', dd_fwd_kernel<8, true>},
+    {4, 's', nullptr},  // dd_fwd_split_kernel
 };
 constexpr int kNumCfg = (int)(sizeof(kDdCfg) / sizeof(kDdCfg[0]));
+static_assert(kNumCfg == kSplitCfg + 1, "the split shape is the last");
 struct AdjCfg {
   int TB;
-  AdjFn adj;
+  AdjFn adj[2];  // R = 1, 4
 };
-const AdjCfg kAdjCfg[] = {{1, dd_adj_kernel<1>}, {2, dd_adj_kernel<2>}, {4, dd_adj_kernel<4>}};
+const AdjCfg kAdjCfg[] = {{1, {dd_adj_kernel<1, 1>, dd_adj_kernel<1, 4>}},
+                          {2, {dd_adj_kernel<2, 1>, dd_adj_kernel<2, 4>}},
+                          {4, {dd_adj_kernel<4, 1>, dd_adj_kernel<4, 4>}}};
 constexpr int kNumAdj = (int)(sizeof(kAdjCfg) / sizeof(kAdjCfg[0]));
 int num_cfg(bool fwd) { return fwd ? kNumCfg : kNumAdj; }
 std::string cfg_name(int c, bool fwd = true) {
   if (!fwd) return "t" + std::to_string(kAdjCfg[c].TB);
-  return "w" + std::to_string(kDdCfg[c].W) + (kDdCfg[c].block ? "b" : "w");
+  return "w" + std::to_string(kDdCfg[c].W) + kDdCfg[c].mode;
 }
 int cfg_threads(int c, bool fwd) { return fwd ? 32 * kDdCfg[c].W : 128 * kAdjCfg[c].TB; }
 
 // Persistent grid: as many blocks as fit on the device at once.
-int dd_grid(int c, bool fwd, int *grid) {
+AdjFn adj_fn(const DdState &S, int c) { return kAdjCfg[c].adj[S.R == 4 ? 1 : 0]; }
+int dd_grid(const DdState &S, int c, bool fwd, int *grid) {
   int dev = 0, sms = 0, nb = 0;
   TOMO_CUDA(cudaGetDevice(&dev));
   TOMO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const void *k = fwd ? (const void *)kDdCfg[c].fwd : (const void *)kAdjCfg[c].adj;
+  if (fwd && !kDdCfg[c].fwd) {
+    if (S.fwd_items > INT_MAX) return fail(TOMO_EINVAL, "dd: too many forward items for one block each");
+    *grid = (int)S.fwd_items;
+    return TOMO_OK;
+  }
+  const void *k = fwd ? (const void *)kDdCfg[c].fwd : (const void *)adj_fn(S, c);
   TOMO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, cfg_threads(c, fwd), 0));
   *grid = std::max(1, nb) * sms;
   return TOMO_OK;
@@ -1047,9 +1213,13 @@ int dd_grid(int c, bool fwd, int *grid) {
 
 int dd_launch_fwd(const DdState &S, int c, int grid, const double2 *work, float *sino, cudaStream_t s,
                   const FwdEpi &ep) {
+  if (!kDdCfg[c].fwd) {
+    dd_fwd_split_kernel<<<grid, 128, 0, s>>>(S.d_inst, (int)S.inst.size(), work, sino, ep);
+    TOMO_CUDA(cudaGetLastError());
+    return TOMO_OK;
+  }
   TOMO_CUDA(cudaMemsetAsync(S.d_ctr, 0, sizeof(unsigned long long), s));
-  kDdCfg[c].fwd<<<grid, 32 * kDdCfg[c].W, 0, s>>>(S.d_inst, (int)S.inst.size(), S.fwd_items, S.d_ctr, work,
-                                                    sino, ep);
+  kDdCfg[c].fwd<<<grid, 32 * kDdCfg[c].W, 0, s>>>(S.d_inst, (int)S.inst.size(), S.fwd_items, S.d_ctr, work, sino, ep);
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
 }
@@ -1057,7 +1227,7 @@ int dd_launch_fwd(const DdState &S, int c, int grid, const double2 *work, float 
 int dd_launch_adj(const DdState &S, int c, int grid, const double2 *work, float *img, cudaStream_t s,
                   const AdjEpi &ep) {
   TOMO_CUDA(cudaMemsetAsync(S.d_ctr + 1, 0, sizeof(unsigned long long), s));
-  kAdjCfg[c].adj<<<grid, cfg_threads(c, false), 0, s>>>(S.d_inst, (int)S.inst.size(), S.adj_items,
+  adj_fn(S, c)<<<grid, cfg_threads(c, false), 0, s>>>(S.d_inst, (int)S.inst.size(), S.adj_items,
                                                          S.d_ctr + 1, work, img, ep);
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
@@ -1076,6 +1246,7 @@ constexpr double kTuneMinUpdates = 5e7;  // below this the default shape is used
 // buffer is touched.  The choice does not change any result (each output is
 // owned by one lane whatever the shape), only the time.
 int dd_autotune(Plan &p, DdState &S) {
+  if (S.fwd_items > INT_MAX) S.wf = 1;
   const auto key = std::make_tuple(S.fwd_items, S.adj_items, (int)S.inst.size(), S.inst[0].n, S.inst[0].na);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1105,7 +1276,8 @@ int dd_autotune(Plan &p, DdState &S) {
       log += dir == 0 ? "fwd" : "; adj";
       for (int c = 0; c < num_cfg(dir == 0) && rc == TOMO_OK; ++c) {
         int grid = 0;
-        if ((rc = dd_grid(c, dir == 0, &grid))) break;
+        if (dir == 0 && c == kSplitCfg && S.fwd_items > INT_MAX) continue;
+        if ((rc = dd_grid(S, c, dir == 0, &grid))) break;
         float ms = 0.0f;
         for (int rep = 0; rep < 3 && rc == TOMO_OK; ++rep) {
           cudaEventRecord(e0, st);
@@ -1137,10 +1309,10 @@ int dd_autotune(Plan &p, DdState &S) {
     g_tuned[key] = std::make_pair(S.wf, S.wa);
   }
   if (S.tuning.empty()) S.tuning = "default (small workload)";
-  int rc = dd_grid(S.wf, true, &S.grid_f);
-  if (!rc) rc = dd_grid(S.wa, false, &S.grid_a);
+  int rc = dd_grid(S, S.wf, true, &S.grid_f);
+  if (!rc) rc = dd_grid(S, S.wa, false, &S.grid_a);
   S.tuning = "fwd " + cfg_name(S.wf) + ", adj " + cfg_name(S.wa, false) +
-             " (forward w<warps/block> + b: block fetch, w: warp fetch; adjoint t<tiles/block>)" +
+             " (forward w<warps/block> + b: block fetch, w: warp fetch, s: a block per item; adjoint t<tiles/block>)" +
              ", grids " + std::to_string(S.grid_f) + "/" + std::to_string(S.grid_a) + " (" + S.tuning + ")";
   return rc;
 }
@@ -1157,6 +1329,15 @@ int dd_build(Plan &p, const DdGeo *geo, int count) {
   auto *S = new DdState();
   p.ext = S;
   p.ext_free = dd_state_free;
+  long long tiles = 0;  // of 32 x 16 pixels
+  for (int gi = 0; gi < count; ++gi) {
+    const long long n = geo[gi].n;
+    tiles += (long long)geo[gi].nz * ((n + kTileW - 1) / kTileW) * ((n + 15) / 16);
+  }
+  // rows of 4 pixels per lane for plans of few tiles, where blocks of 4 x 4 leave
+  // warps idle: 256^2 x 304 (128 tiles) 131 -> 53 us, 513^2 x 400 (561 tiles) 170
+  // -> 97; at 768^2 x 720 (1152 tiles) 281 with 4 x 4, 305 with rows
+  S->R = tiles <= 768 ? 1 : 4;
   // host tables per geometry, packed into one device buffer
   struct GeoTabs {
     size_t ang, tab, tabS, fperm;
@@ -1240,7 +1421,7 @@ int dd_build(Plan &p, const DdGeo *geo, int count) {
       I.nS = t.nS;
       I.ngrp = (G.n + kGrpDet - 1) / kGrpDet;
       I.tx = (G.n + kTileW - 1) / kTileW;
-      I.ty = (G.n + kTileH - 1) / kTileH;
+      I.ty = (G.n + 4 * S->R - 1) / (4 * S->R);
       I.ang = (const DdAngle *)(tb + t.ang);
       I.tab = (const float4 *)(tb + t.tab);
       I.tabS = (const int2 *)(tb + t.tabS);
@@ -1290,7 +1471,7 @@ int dd_build(Plan &p, const DdGeo *geo, int count) {
     S->sino_blocks += I.na;
     S->inst.push_back(I);
   }
-  if (S->row_blocks > 2147483647LL || S->sino_blocks > 2147483647LL)
+  if (S->row_blocks + S->sino_blocks + kColParts * S->col_blocks > 2147483647LL)
     return fail(TOMO_EINVAL, "dd: batch too large for one launch");
   TOMO_CUDA(cudaMalloc(&S->d_inst, sizeof(DdInst) * S->inst.size()));
   TOMO_CUDA(cudaMemcpy(S->d_inst, S->inst.data(), sizeof(DdInst) * S->inst.size(), cudaMemcpyHostToDevice));
@@ -1345,8 +1526,8 @@ int dd_set_tuning(Plan &p, const char *fwd, const char *adj) {
                                                 " shape '" + name + "'");
     (dir == 0 ? wf : wa) = found;
   }
-  int rc = dd_grid(wf, true, &S.grid_f);
-  if (!rc) rc = dd_grid(wa, false, &S.grid_a);
+  int rc = dd_grid(S, wf, true, &S.grid_f);
+  if (!rc) rc = dd_grid(S, wa, false, &S.grid_a);
   if (rc) return rc;
   S.wf = wf;
   S.wa = wa;
@@ -1358,9 +1539,9 @@ int dd_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
   const DdState &S = *(const DdState *)p.ext;
   double2 *work = (double2 *)p.d_scratch;
   const int ni = (int)S.inst.size();
-  dd_row_prefix_kernel<<<(unsigned)S.row_blocks, kScanThreads, 0, s>>>(S.d_inst, ni, d_img, work);
-  dd_col_prefix_kernel<<<(unsigned)S.col_blocks, 32 * kColWarps, 0, s>>>(S.d_inst, ni, d_img, work);
-  dd_fwd_corr_kernel<<<(unsigned)S.sino_blocks, 32 * kCorrWarps, 0, s>>>(S.d_inst, ni, d_img, work);
+  const unsigned corr = (unsigned)S.sino_blocks, cols = (unsigned)(kColParts * S.col_blocks);
+  dd_fwd_prep_kernel<<<corr + cols + (unsigned)S.row_blocks, kScanThreads, 0, s>>>(S.d_inst, ni, corr, cols, d_img,
+                                                                                  work);
   TOMO_CUDA(cudaGetLastError());
   return dd_launch_fwd(S, S.wf, S.grid_f, work, d_sino, s, ep);
 }
@@ -1369,9 +1550,9 @@ int dd_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const
   const DdState &S = *(const DdState *)p.ext;
   double2 *work = (double2 *)p.d_scratch;
   const int ni = (int)S.inst.size();
-  dd_sino_expand_kernel<<<(unsigned)S.sino_blocks, kScanThreads, 0, s>>>(S.d_inst, ni, d_sino, work);
-  dd_adj_drop_kernel<false><<<(unsigned)S.row_blocks, 32, 0, s>>>(S.d_inst, ni, work);
-  dd_adj_drop_kernel<true><<<(unsigned)S.row_blocks, 32, 0, s>>>(S.d_inst, ni, work);
+  const unsigned rows = (unsigned)S.row_blocks;
+  dd_adj_prep_kernel<<<rows + (unsigned)S.sino_blocks, kScanThreads, 0, s>>>(S.d_inst, ni, rows, d_sino, work);
+  dd_adj_col_drop_kernel<<<rows, kScanThreads, 0, s>>>(S.d_inst, ni, d_sino, work);
   TOMO_CUDA(cudaGetLastError());
   return dd_launch_adj(S, S.wa, S.grid_a, work, d_img, s, ep);
 }
