@@ -42,6 +42,11 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
   return r;
 }
+__device__ __forceinline__ F2 fma2_rd(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
 // c - a, rounded once
 __device__ __forceinline__ F2 rsub2(F2 a, F2 c) { return fma2(a, f2(-1.0f), c); }
 

@@ -59,6 +59,7 @@
 #include <vector>
 
 #include "epilogue.cuh"
+#include "f32x2.cuh"
 #include "tomo_internal.cuh"
 
 namespace tomo {
@@ -156,7 +157,7 @@ __global__ void __launch_bounds__(128) dd_forward_kernel(
 // Instances
 // ---------------------------------------------------------------------------
 constexpr int kGrpDet = 127;              // detectors per forward item (128 boundaries, 4 x 32)
-constexpr int kTileW = 32;                // an adjoint item is 32 x 4R pixels, R x 4 per lane (8x4 lanes)
+constexpr int kTileW = 32;                // columns of an adjoint item, one per lane
 constexpr int kScanThreads = 256;
 constexpr int kPrepWarps = kScanThreads / 32;  // warps of the pre-pass kernels
 constexpr int kColParts = 4, kColRows = 8;     // parts a column is summed in; rows staged at a time
@@ -859,52 +860,79 @@ __global__ void __launch_bounds__(128) dd_fwd_split_kernel(const DdInst *__restr
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint: an item is a 32 x 4R pixel tile; lane l holds the R x 4 pixels at
-// rows a0..a0+R-1 and columns b0..b0+3.  Per angle and line each pixel [P0, P1]
-// overlaps the detector a holding P0 and possibly a+1 (detectors are at least
-// one pixel wide): (min(D_a+1, P1) - P0) S_a + (P1 - min(D_a+1, P1)) S_a+1,
-// the reference's two gaps, both accumulated by FMA.
+// Adjoint: an item is a 32 x NR pixel tile; lane l holds the NR pixels of column
+// b0 + l.  Per angle and line each pixel [P0, P1] overlaps the detector a holding
+// P0 and possibly a+1 (detectors are at least one pixel wide):
+// (min(D_a+1, P1) - P0) S_a + (P1 - min(D_a+1, P1)) S_a+1, the reference's two
+// gaps, both accumulated by FMA.  A lane holds a column, so that a load of the warp
+// covers 32 neighbouring pixels' entries (2.75 cache wavefronts; with 4 x 4 pixels
+// per lane 3.65), and takes two rows at a time as packed pairs (13 instead of 15
+// instructions per pixel and angle).  2048^2 x 1800: 4.39 -> 4.17 ms.  Touching the
+// next angle's entries ahead cost more than it gave.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void dd_adj_pixel(float P0, float P1, float z, float r, float cm, float cm1,
-                                             const float2 *__restrict__ rowm, float &acc) {
-  // f = cm + floor(P0 z) exactly: rounded down in [2^23, 2^24), where floats
-  // are the integers; a = floor(P0 z + nh) is f's bits minus kMagicBits (rowm
-  // is the row base minus kMagicBits entries)
-  const float f = __fmaf_rd(P0, z, cm);
-  const float2 t = __ldg(rowm + __float_as_int(f));  // {S_a, S_a+1}
-  // D_a+1 = (a + 1 - nh) r, with a + 1 - nh = f - (kMagic + nh - 1) exactly
-  const float D1 = __fmul_rn(__fsub_rn(f, cm1), r);
-  const float m = fminf(D1, P1);
-  acc = __fmaf_rn(__fsub_rn(m, P0), t.x, acc);
-  acc = __fmaf_rn(__fsub_rn(P1, m), t.y, acc);
+// Two pixels of a column: a = floor(P0 z + nh) is the bits of f = cm + floor(P0 z)
+// (rounded down in [2^23, 2^24), where floats are the integers) minus kMagicBits;
+// rowm is the angle's row minus kMagicBits entries.  D_a+1 = (a + 1 - nh) r, with
+// a + 1 - nh = f - (kMagic + nh - 1) exactly.
+__device__ __forceinline__ void dd_adj_pair(F2 P0, F2 P1, F2 z, F2 r, F2 cm, F2 ncm1,
+                                            const float2 *__restrict__ rowm, float &acc0, float &acc1) {
+  const F2 f = fma2_rd(P0, z, cm);
+  const float2 fs = unpack(f);
+  const float2 t0 = __ldg(rowm + __float_as_int(fs.x)), t1 = __ldg(rowm + __float_as_int(fs.y));  // {S_a, S_a+1}
+  const float2 D1 = unpack(mul2(add2(f, ncm1), r)), p1 = unpack(P1);
+  const F2 m = f2(fminf(D1.x, p1.x), fminf(D1.y, p1.y));
+  const float2 ga = unpack(rsub2(P0, m)), gb = unpack(rsub2(m, P1));
+  acc0 = __fmaf_rn(ga.x, t0.x, acc0);
+  acc0 = __fmaf_rn(gb.x, t0.y, acc0);
+  acc1 = __fmaf_rn(ga.y, t1.x, acc1);
+  acc1 = __fmaf_rn(gb.y, t1.y, acc1);
 }
 
-template <bool COLS, int R>
-__device__ __forceinline__ void dd_adj_pass(const float4 *__restrict__ tab, int cnt,
-                                            const float2 *__restrict__ AS, int a0, int b0, int n, int nh,
-                                            float (&acc)[R][4]) {
-  constexpr int NL = COLS ? 4 : R, NP = COLS ? R : 4;  // lines, pixels of a line
-  const int l0 = COLS ? b0 : a0, k0 = COLS ? a0 : b0;
-  const float y0 = (float)(l0 - nh) + 0.5f;
-  float x[NP + 1];
+// COLS = false: the lines are the image's rows; -q of every row comes from qs,
+// where the warp has computed 32 / NR angles' at once (a lane a row).
+template <int NR>
+__device__ __forceinline__ void dd_adj_rows(const float4 *__restrict__ tab, int cnt, const float2 *__restrict__ AS,
+                                            int a0, int b, int nh, float *qs, float (&acc)[NR]) {
+  constexpr int kAng = 32 / NR;
+  const int lane = threadIdx.x & 31;
+  const float y = (float)(a0 + lane % NR - nh) + 0.5f;
+  const F2 x0 = f2((float)(b - nh)), x1 = f2((float)(b - nh + 1));
+  const F2 cm = f2(kMagic + (float)nh), ncm1 = f2(-(kMagic + (float)nh - 1.0f));
+  for (int u0 = 0; u0 < cnt; u0 += kAng) {
+    __syncwarp();
+    qs[lane] = -__fmul_rn(y, __ldg(tab + min(u0 + lane / NR, cnt - 1)).y);
+    __syncwarp();
 #pragma unroll
-  for (int j = 0; j <= NP; ++j) x[j] = (float)(k0 - nh + j);
-  const float cm = kMagic + (float)nh, cm1 = cm - 1.0f;
-  constexpr int kUnroll = R == 4 ? 1 : 2;
+    for (int t = 0; t < kAng; ++t) {
+      if (u0 + t >= cnt) break;
+      const float4 e = __ldg(tab + u0 + t);
+      const F2 r = f2(e.x), z = f2(e.z);
+      const float2 *rowm = AS + __float_as_int(e.w) - kMagicBits;
+#pragma unroll
+      for (int i = 0; i < NR; i += 2) {
+        const float2 q = *reinterpret_cast<const float2 *>(qs + t * NR + i);
+        const F2 nq = f2(q.x, q.y);
+        dd_adj_pair(add2(x0, nq), add2(x1, nq), z, r, cm, ncm1, rowm, acc[i], acc[i + 1]);
+      }
+    }
+  }
+}
+// COLS: the lane's column is the line.
+template <int NR>
+__device__ __forceinline__ void dd_adj_cols(const float4 *__restrict__ tab, int cnt, const float2 *__restrict__ AS,
+                                            int a0, int b, int nh, float (&acc)[NR]) {
+  const float y = (float)(b - nh) + 0.5f, x = (float)(a0 - nh);
+  const F2 cm = f2(kMagic + (float)nh), ncm1 = f2(-(kMagic + (float)nh - 1.0f));
+  constexpr int kUnroll = NR == 16 ? 1 : 4;
 #pragma unroll kUnroll
   for (int u = 0; u < cnt; ++u) {
     const float4 e = __ldg(tab + u);
-    const float r = e.x, k = e.y, z = e.z;
+    const F2 r = f2(e.x), z = f2(e.z), nq = f2(-__fmul_rn(y, e.y));
     const float2 *rowm = AS + __float_as_int(e.w) - kMagicBits;
 #pragma unroll
-    for (int li = 0; li < NL; ++li) {
-      const float q = __fmul_rn(__fadd_rn(y0, (float)li), k);
-      float P[NP + 1];
-#pragma unroll
-      for (int j = 0; j <= NP; ++j) P[j] = __fsub_rn(x[j], q);
-#pragma unroll
-      for (int j = 0; j < NP; ++j) dd_adj_pixel(P[j], P[j + 1], z, r, cm, cm1, rowm, COLS ? acc[j][li] : acc[li][j]);
-    }
+    for (int i = 0; i < NR; i += 2)
+      dd_adj_pair(add2(f2(x + i, x + (i + 1)), nq), add2(f2(x + (i + 1), x + (i + 2)), nq), z, r, cm, ncm1, rowm,
+                  acc[i], acc[i + 1]);
   }
 }
 
@@ -996,19 +1024,22 @@ __global__ void __launch_bounds__(kScanThreads) dd_adj_col_drop_kernel(const DdI
   dd_adj_drop<true>(S, blockIdx.x, inst, ninst, sino, work);
 }
 
-// One item = one tile of 32 x 4R pixels (R = 4, or 1 for plans of few tiles:
-// dd_adj_rows), worked on by 4 warps: warp `quarter` sums the
+// One item = one tile of 32 x NR pixels (NR = 16, or 4 for plans of few tiles:
+// dd_build), worked on by 4 warps: warp `quarter` sums the
 // angles [quarter T / 4, (quarter + 1) T / 4) of the ROWS-then-COLS order (T =
 // nR + nC), and the tile's first warp adds the quarters in order, then the
 // row / column sums, then stores.  The split never depends on the launch
 // shape, so every shape gives the same bits.
-template <int TB, int R>
-__global__ void __launch_bounds__(128 * TB) dd_adj_kernel(const DdInst *__restrict__ inst, int ninst,
+// Registers held to 64, 32 warps per SM: at 80 the waits for loads show (2048^2
+// x 1800: 5.0 ms); at 48 the loads in flight get fewer (4.5).
+template <int TB, int NR>
+__global__ void __launch_bounds__(128 * TB, 8 / TB) dd_adj_kernel(const DdInst *__restrict__ inst, int ninst,
                                                            long long nitems, unsigned long long *__restrict__ ctr,
                                                            const double2 *__restrict__ work,
                                                            float *__restrict__ img, AdjEpi ep) {
   __shared__ long long base_s;
-  __shared__ float part[TB][3][4 * R][32];  // quarters 1..3 of each tile
+  __shared__ float part[TB][3][NR][32];  // quarters 1..3 of each tile
+  __shared__ __align__(16) float qs[4 * TB][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tile = warp >> 2, quarter = warp & 3;
   for (;;) {
@@ -1018,38 +1049,32 @@ __global__ void __launch_bounds__(128 * TB) dd_adj_kernel(const DdInst *__restri
     __syncthreads();
     if (first >= nitems) break;  // block-uniform
     const long long item = first + tile;
-    float acc[R][4];
+    float acc[NR];
 #pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    for (int i = 0; i < NR; ++i) acc[i] = 0.0f;
     const DdInst *Ip = nullptr;
-    int a0 = 0, b0 = 0;
-    bool inside = false;
+    int a0 = 0, aT = 0, b = 0;
     if (item < nitems) {
       Ip = &inst[find_inst(inst, ninst, item, &DdInst::a0)];
       const DdInst &I = *Ip;
       const int local = (int)(item - I.a0);
-      b0 = (local % I.tx) * kTileW + 4 * (lane & 7);
-      a0 = (local / I.tx) * (4 * R) + R * (lane >> 3);
-      // lanes whose block starts outside the image (n not a multiple of 4)
-      // only take part in the epilogue's warp reductions
-      inside = a0 < I.n && b0 < I.n;
-      if (inside) {
-        const int T = I.nR + I.nC;
-        const int u0 = (int)((long long)T * quarter / 4), u1 = (int)((long long)T * (quarter + 1) / 4);
-        const float2 *AS = (const float2 *)(work + I.as) + I.pads;
-        const int r0 = min(u0, I.nR), r1 = min(u1, I.nR);
-        if (r1 > r0) dd_adj_pass<false, R>(I.tab + r0, r1 - r0, AS, a0, b0, I.n, I.nh, acc);
-        const int c0 = max(u0, I.nR), c1 = max(u1, I.nR);
-        if (c1 > c0) dd_adj_pass<true, R>(I.tab + c0, c1 - c0, AS, a0, b0, I.n, I.nh, acc);
-      }
+      b = (local % I.tx) * kTileW + lane;
+      // a tile across the lower edge takes the rows above it along, a lane
+      // beyond the right edge the last column; neither stores them
+      aT = (local / I.tx) * NR;
+      a0 = max(0, min(aT, I.n - NR));
+      const int bc = min(b, I.n - 1);
+      const int T = I.nR + I.nC;
+      const int u0 = (int)((long long)T * quarter / 4), u1 = (int)((long long)T * (quarter + 1) / 4);
+      const float2 *AS = (const float2 *)(work + I.as) + I.pads;
+      const int r0 = min(u0, I.nR), r1 = min(u1, I.nR);
+      if (r1 > r0) dd_adj_rows<NR>(I.tab + r0, r1 - r0, AS, a0, bc, I.nh, qs[warp], acc);
+      const int c0 = max(u0, I.nR), c1 = max(u1, I.nR);
+      if (c1 > c0) dd_adj_cols<NR>(I.tab + c0, c1 - c0, AS, a0, bc, I.nh, acc);
     }
     if (quarter > 0) {
 #pragma unroll
-      for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) part[tile][quarter - 1][4 * i + j][lane] = acc[i][j];
+      for (int i = 0; i < NR; ++i) part[tile][quarter - 1][i][lane] = acc[i];
     }
     __syncthreads();
     if (quarter == 0 && Ip) {
@@ -1058,29 +1083,24 @@ __global__ void __launch_bounds__(128 * TB) dd_adj_kernel(const DdInst *__restri
 #pragma unroll
       for (int q = 0; q < 3; ++q)
 #pragma unroll
-        for (int i = 0; i < R; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] += part[tile][q][4 * i + j][lane];
+        for (int i = 0; i < NR; ++i) acc[i] += part[tile][q][i][lane];
       const float2 *AS = (const float2 *)(work + I.as) + I.pads;
-      for (int t = 0; inside && t < I.nS; ++t) {  // row / column sums (|sin| or |cos| < 1e-7)
+      for (int t = 0; t < I.nS; ++t) {  // row / column sums (|sin| or |cos| < 1e-7)
         const int2 e = __ldg(I.tabS + t);
         const float2 *row = AS + e.y;
 #pragma unroll
-        for (int i = 0; i < R; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] += __ldg(&row[e.x == DD_ROWSUM ? a0 + i : b0 + j].x);
+        for (int i = 0; i < NR; ++i) acc[i] += __ldg(&row[e.x == DD_ROWSUM ? a0 + i : min(b, n - 1)].x);
       }
-      // the dropped pieces (dd_adj_drop_kernel)
+      // the dropped pieces (dd_adj_drop)
       const float *Cimg = reinterpret_cast<const float *>(work + I.xs);
 #pragma unroll
-      for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int a = a0 + i, b = b0 + j;
-          const bool live = inside && a < n && b < n;
-          if (live) acc[i][j] += __ldg(Cimg + (size_t)a * n + b);
-          adj_store(ep, acc[i][j], live, (size_t)I.img + (size_t)(live ? a : 0) * n + (live ? b : 0), img);
-        }
+      for (int i = 0; i < NR; ++i) {
+        const int a = a0 + i;
+        const bool live = a >= aT && a < n && b < n;
+        const size_t p = (size_t)(live ? a : 0) * n + (live ? b : 0);
+        if (live) acc[i] += __ldg(Cimg + p);
+        adj_store(ep, acc[i], live, (size_t)I.img + p, img);
+      }
     }
     __syncthreads();  // part[] is rewritten by the next item
   }
@@ -1145,7 +1165,7 @@ struct DdState {
   unsigned long long *d_ctr = nullptr;  // [0] forward items, [1] adjoint items
   long long fwd_items = 0, adj_items = 0, row_blocks = 0, col_blocks = 0, sino_blocks = 0;
   double updates = 0.0;  // pixel x angle updates per application
-  int R = 4;             // pixel rows per lane of the adjoint
+  int NR = 16;           // pixel rows of an adjoint tile
   int wf = kSplitCfg, wa = 1;    // launch shape (kDdCfg index) of the forward / adjoint kernels
   int grid_f = 0, grid_a = 0;
   std::vector<size_t> img_off, sino_off;  // packed offsets in the caller's order (count + 1)
@@ -1181,11 +1201,11 @@ constexpr int kNumCfg = (int)(sizeof(kDdCfg) / sizeof(kDdCfg[0]));
 static_assert(kNumCfg == kSplitCfg + 1, "the split shape is the last");
 struct AdjCfg {
   int TB;
-  AdjFn adj[2];  // R = 1, 4
+  AdjFn adj[2];  // NR = 4, 16
 };
-const AdjCfg kAdjCfg[] = {{1, {dd_adj_kernel<1, 1>, dd_adj_kernel<1, 4>}},
-                          {2, {dd_adj_kernel<2, 1>, dd_adj_kernel<2, 4>}},
-                          {4, {dd_adj_kernel<4, 1>, dd_adj_kernel<4, 4>}}};
+const AdjCfg kAdjCfg[] = {{1, {dd_adj_kernel<1, 4>, dd_adj_kernel<1, 16>}},
+                          {2, {dd_adj_kernel<2, 4>, dd_adj_kernel<2, 16>}},
+                          {4, {dd_adj_kernel<4, 4>, dd_adj_kernel<4, 16>}}};
 constexpr int kNumAdj = (int)(sizeof(kAdjCfg) / sizeof(kAdjCfg[0]));
 int num_cfg(bool fwd) { return fwd ? kNumCfg : kNumAdj; }
 std::string cfg_name(int c, bool fwd = true) {
@@ -1195,7 +1215,7 @@ std::string cfg_name(int c, bool fwd = true) {
 int cfg_threads(int c, bool fwd) { return fwd ? 32 * kDdCfg[c].W : 128 * kAdjCfg[c].TB; }
 
 // Persistent grid: as many blocks as fit on the device at once.
-AdjFn adj_fn(const DdState &S, int c) { return kAdjCfg[c].adj[S.R == 4 ? 1 : 0]; }
+AdjFn adj_fn(const DdState &S, int c) { return kAdjCfg[c].adj[S.NR == 16 ? 1 : 0]; }
 int dd_grid(const DdState &S, int c, bool fwd, int *grid) {
   int dev = 0, sms = 0, nb = 0;
   TOMO_CUDA(cudaGetDevice(&dev));
@@ -1330,14 +1350,17 @@ int dd_build(Plan &p, const DdGeo *geo, int count) {
   p.ext = S;
   p.ext_free = dd_state_free;
   long long tiles = 0;  // of 32 x 16 pixels
+  int least = 32767;
   for (int gi = 0; gi < count; ++gi) {
     const long long n = geo[gi].n;
+    least = std::min(least, geo[gi].n);
     tiles += (long long)geo[gi].nz * ((n + kTileW - 1) / kTileW) * ((n + 15) / 16);
   }
-  // rows of 4 pixels per lane for plans of few tiles, where blocks of 4 x 4 leave
-  // warps idle: 256^2 x 304 (128 tiles) 131 -> 53 us, 513^2 x 400 (561 tiles) 170
-  // -> 97; at 768^2 x 720 (1152 tiles) 281 with 4 x 4, 305 with rows
-  S->R = tiles <= 768 ? 1 : 4;
+  // 4 pixels per lane for plans of few tiles, where 16 leave warps idle: the adjoint
+  // at 256^2 x 304 (128 tiles) 136 us with 16, 57 with 4; 513^2 x 400 (561 tiles) 177
+  // and 106; 768^2 x 720 (1152 tiles) 298 and 306.  (A tile may not be higher than
+  // the image: its last rows are moved up to lie inside.)
+  S->NR = tiles <= 768 || least < 16 ? 4 : 16;
   // host tables per geometry, packed into one device buffer
   struct GeoTabs {
     size_t ang, tab, tabS, fperm;
@@ -1421,7 +1444,7 @@ int dd_build(Plan &p, const DdGeo *geo, int count) {
       I.nS = t.nS;
       I.ngrp = (G.n + kGrpDet - 1) / kGrpDet;
       I.tx = (G.n + kTileW - 1) / kTileW;
-      I.ty = (G.n + 4 * S->R - 1) / (4 * S->R);
+      I.ty = (G.n + S->NR - 1) / S->NR;
       I.ang = (const DdAngle *)(tb + t.ang);
       I.tab = (const float4 *)(tb + t.tab);
       I.tabS = (const int2 *)(tb + t.tabS);
