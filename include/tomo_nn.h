@@ -44,6 +44,12 @@ int tomo_nn_gemm(const void *A, int lda, const void *B, int ldb, int M, int N, i
 int tomo_nn_conv3x3(const void *X, int batch, int H, int W, int Cin, const void *Wt, int Cout, float *Yf,
                     void *Yb, const float *bias, int relu, void *stream);
 
+/* The same without bias, in BF16, its result kept where mask (BF16, laid out
+ * like Yb) is > 0 and 0 elsewhere: an input gradient that goes on through the
+ * ReLU which made that input. */
+int tomo_nn_conv3x3_masked(const void *X, int batch, int H, int W, int Cin, const void *Wt, int Cout, const void *mask,
+                           void *Yb, void *stream);
+
 /* Weight and bias gradients of a convolution with `taps` = 9 (3x3, pad 1) or
  * 1 (1x1): dW [Cout][taps][Cin] = sum over pixels p of dY[p][co] x
  * im2col(X)[p][(tap, ci)], db[Cout] = sum_p dY[p][co] (db may be NULL); X
@@ -62,6 +68,32 @@ int tomo_nn_prepare_weights(const float *W, int Cout, int Cin, int taps, void *W
 
 /* ReLU backward in place on BF16 arrays: dY[i] = Y[i] > 0 ? dY[i] : 0. */
 int tomo_nn_relu_bwd(const void *Y, void *dY, size_t n, void *stream);
+
+/* 2x2 max-pooling: X [batch][2h][2w][C] -> Y [batch][h][w][C], BF16 (as all of
+ * the following, with C a multiple of 8 and pointers 16-byte aligned). */
+int tomo_nn_pool(const void *X, int batch, int h, int w, int C, void *Y, void *stream);
+
+/* Gradient of X from those of its pooling dP [batch][h][w][C] and of X used
+ * directly, dS [batch][2h][2w][lds] (its first C channels; lds a multiple of 8),
+ * through the ReLU that made X: dZ = X > 0 ? dS + (dP where X is its window's
+ * first maximum) : 0. */
+int tomo_nn_pool_bwd(const void *X, const void *dP, const void *dS, int lds, int batch, int h, int w, int C, void *dZ,
+                     void *stream);
+
+/* Y [batch][2h][2w][Cu + Cs] = X [batch][h][w][Cu] upsampled by 2 (nearest)
+ * beside S [batch][2h][2w][Cs]. */
+int tomo_nn_upcat(const void *X, const void *S, int batch, int h, int w, int Cu, int Cs, void *Y, void *stream);
+
+/* Gradient of that X from the first C of dY's ldy channels, through the ReLU
+ * that made X: dX = X > 0 ? the sum over X's four pixels : 0. */
+int tomo_nn_up_bwd(const void *dY, int ldy, const void *X, int batch, int h, int w, int C, void *dX, void *stream);
+
+/* dZ [P][8] = BF16 of dY [P] in channel 0, zeros in the others. */
+int tomo_nn_pad8(const float *dY, long long P, void *dZ, void *stream);
+
+/* Input gradient of a 1x1 convolution with 8 outputs, through the ReLU that
+ * made its input: dX [P][C] = X > 0 ? dZ [P][8] . Wt [C][8]^T : 0; C <= 1024. */
+int tomo_nn_head_bwd(const void *dZ, const void *Wt, const void *X, long long P, int C, void *dX, void *stream);
 
 /* One Adam step on FP32 parameters p with gradient g and moments m, v
  * (step >= 1; bias-corrected; no weight decay). */

@@ -47,6 +47,7 @@ constexpr int kDrainSpins = 1 << 22;
 
 struct ConvArgs {
   const float *bias;
+  const __nv_bfloat16 *mask;  // outputs stand where it is > 0 (0 elsewhere); laid out like Yb
   float *Yf;
   __nv_bfloat16 *Yb;
   unsigned *status;
@@ -140,6 +141,22 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_tc_kernel(ConvArgs g, co
           if (!in) continue;
           if (g.Yb) {
             __nv_bfloat16 *d = g.Yb + o + c0;
+            if (g.mask) {
+              const __nv_bfloat16 *k = g.mask + o + c0;
+              if (g.vec) {
+                const uint4 a = __ldg((const uint4 *)k), b = c0 + 8 < nv ? __ldg((const uint4 *)(k + 8)) : a;
+                const unsigned w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  if (!(__uint_as_float(w[i] << 16) > 0.0f)) v[2 * i] = 0.0f;
+                  if (!(__uint_as_float(w[i] & 0xffff0000u) > 0.0f)) v[2 * i + 1] = 0.0f;
+                }
+              } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                  if (c0 + i < nv && !(__bfloat162float(k[i]) > 0.0f)) v[i] = 0.0f;
+              }
+            }
             if (g.vec) {  // nv is a multiple of 8
               unsigned w[8];
 #pragma unroll
@@ -317,13 +334,14 @@ int up1k(int b) { return (b + 1023) / 1024 * 1024; }
 }  // namespace
 
 int conv_launch(const __nv_bfloat16 *X, int batch, int H, int W, int Cin, const __nv_bfloat16 *Wt, int Cout, float *Yf,
-                __nv_bfloat16 *Yb, const float *bias, int relu, unsigned *status, int spins, cudaStream_t s) {
+                __nv_bfloat16 *Yb, const float *bias, int relu, const __nv_bfloat16 *mask, unsigned *status, int spins, cudaStream_t s) {
   if (batch < 1 || H < 1 || W < 1 || Cin < 8 || Cin % 8 || Cout < 1) return NN_EINVAL;
   if ((long long)batch * H * W > 0x7fffffffLL) return NN_EINVAL;
-  if ((Yf == nullptr) == (Yb == nullptr)) return NN_EINVAL;
+  if ((Yf == nullptr) == (Yb == nullptr) || (mask && !Yb)) return NN_EINVAL;
   if (((uintptr_t)X | (uintptr_t)Wt) & 15) return NN_EINVAL;  // TMA sources
   ConvArgs g{};
   g.bias = bias;
+  g.mask = mask;
   g.Yf = Yf;
   g.Yb = Yb;
   g.status = status;
@@ -375,7 +393,7 @@ int conv_launch(const __nv_bfloat16 *X, int batch, int H, int W, int Cin, const 
   g.cols = 32;
   while (g.cols < 2 * g.T * g.BN) g.cols *= 2;
   g.ngroups = (g.ntiles + g.T - 1) / g.T;
-  g.vec = Yb ? Cout % 8 == 0 && ((uintptr_t)Yb & 15) == 0 : Cout % 4 == 0 && ((uintptr_t)Yf & 15) == 0;
+  g.vec = Yb ? Cout % 8 == 0 && (((uintptr_t)Yb | (uintptr_t)mask) & 15) == 0 : Cout % 4 == 0 && ((uintptr_t)Yf & 15) == 0;
   CUtensorMap mx, mw;
   {
     const unsigned long long d[4] = {(unsigned long long)Cin, (unsigned long long)W, (unsigned long long)H,

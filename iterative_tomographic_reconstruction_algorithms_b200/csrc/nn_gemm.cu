@@ -60,11 +60,11 @@ __global__ void __launch_bounds__(kThreads) gemm_tc_kernel(GemmArgs g) {
   constexpr int kStageA = BM * BK * 2, kStageB = BN * BK * 2;
   unsigned char *sA[2] = {smem, smem + kStageA + kStageB};
   unsigned char *sB[2] = {smem + kStageA, smem + 2 * kStageA + kStageB};
-  uint64_t *bars = (uint64_t *)(smem + 2 * (kStageA + kStageB));
+  const int nkb = (g.K + BK - 1) / BK;
+  uint64_t *bars = (uint64_t *)(smem + (nkb > 1 ? 2 : 1) * (kStageA + kStageB));
   uint32_t *tmem_slot = (uint32_t *)(bars + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  const int nkb = (g.K + BK - 1) / BK;
 
   if (warp == 0) {  // TMEM accumulator: BN columns x 128 lanes of FP32
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)),
@@ -163,7 +163,8 @@ __global__ void __launch_bounds__(kThreads) gemm_tc_kernel(GemmArgs g) {
 
 template <int BN>
 int launch_bn(const GemmArgs &g, cudaStream_t s) {
-  const size_t smem = 2 * (size_t)(BM * BK * 2 + BN * BK * 2) + 64;
+  // one K block needs one stage: more CTAs to an SM
+  const size_t smem = (g.K > BK ? 2 : 1) * (size_t)(BM * BK * 2 + BN * BK * 2) + 64;
   if (cudaFuncSetAttribute(gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return NN_ECUDA;

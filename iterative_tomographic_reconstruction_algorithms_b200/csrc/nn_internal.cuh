@@ -31,7 +31,8 @@ int gemm_launch(const GemmArgs &g, cudaStream_t s);
 
 // 3x3 convolution, stride 1, zero padding 1, NHWC (nn_conv.cu).
 int conv_launch(const __nv_bfloat16 *X, int batch, int H, int W, int Cin, const __nv_bfloat16 *Wt, int Cout, float *Yf,
-                __nv_bfloat16 *Yb, const float *bias, int relu, unsigned *status, int spins, cudaStream_t s);
+                __nv_bfloat16 *Yb, const float *bias, int relu, const __nv_bfloat16 *mask, unsigned *status, int spins,
+                cudaStream_t s);
 
 // BF16 tensor map of `rank` dimensions (innermost first; strides in bytes from
 // the second on) whose boxes have rows of rb = 16, 32, 64 or 128 bytes, stored

@@ -123,7 +123,15 @@ int tomo_nn_gemm(const void *A, int lda, const void *B, int ldb, int M, int N, i
 int tomo_nn_conv3x3(const void *X, int batch, int H, int W, int Cin, const void *Wt, int Cout, float *Yf,
                     void *Yb, const float *bias, int relu, void *stream) {
   return conv_launch((const __nv_bfloat16 *)X, batch, H, W, Cin, (const __nv_bfloat16 *)Wt, Cout, Yf, (__nv_bfloat16 *)Yb,
-                     bias, relu, status_ptr(), g_wait_spins.load(), (cudaStream_t)stream);
+                     bias, relu, nullptr, status_ptr(), g_wait_spins.load(), (cudaStream_t)stream);
+}
+
+int tomo_nn_conv3x3_masked(const void *X, int batch, int H, int W, int Cin, const void *Wt, int Cout, const void *mask,
+                           void *Yb, void *stream) {
+  if (!mask) return NN_EINVAL;
+  return conv_launch((const __nv_bfloat16 *)X, batch, H, W, Cin, (const __nv_bfloat16 *)Wt, Cout, nullptr,
+                     (__nv_bfloat16 *)Yb, nullptr, 0, (const __nv_bfloat16 *)mask, status_ptr(), g_wait_spins.load(),
+                     (cudaStream_t)stream);
 }
 
 size_t tomo_nn_wgrad_workspace(int batch, int H, int W, int Cin, int Cout, int taps) {

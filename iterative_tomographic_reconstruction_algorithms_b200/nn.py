@@ -39,6 +39,13 @@ def _load():
     lib.tomo_nn_wgrad_workspace.restype = sz
     lib.tomo_nn_wgrad.argtypes = [vp, vp, i, i, i, i, i, i, vp, vp, vp, sz, vp]
     lib.tomo_nn_prepare_weights.argtypes = [vp, i, i, i, vp, vp, vp]
+    lib.tomo_nn_conv3x3_masked.argtypes = [vp, i, i, i, i, vp, i, vp, vp, vp]
+    lib.tomo_nn_pool.argtypes = [vp, i, i, i, i, vp, vp]
+    lib.tomo_nn_pool_bwd.argtypes = [vp, vp, vp, i, i, i, i, i, vp, vp]
+    lib.tomo_nn_upcat.argtypes = [vp, vp, i, i, i, i, i, vp, vp]
+    lib.tomo_nn_up_bwd.argtypes = [vp, i, vp, i, i, i, i, vp, vp]
+    lib.tomo_nn_pad8.argtypes = [vp, ctypes.c_longlong, vp, vp]
+    lib.tomo_nn_head_bwd.argtypes = [vp, vp, vp, ctypes.c_longlong, i, vp, vp]
     lib.tomo_nn_relu_bwd.argtypes = [vp, vp, sz, vp]
     lib.tomo_nn_adam.argtypes = [vp, vp, vp, vp, sz, f, f, f, f, i, vp]
     lib.tomo_nn_status.argtypes = [ctypes.POINTER(ctypes.c_uint)]
@@ -121,59 +128,123 @@ def prepare_weights(W, with_transpose=True):
     return Wb, Wd
 
 
+def _conv3x3_dx(dZ, Wd, X=None):
+    """Input gradient [B, H, W, Cin]; with X, where the input X is > 0 (through the ReLU that made it)."""
+    B, H, W, Cin = dZ.shape
+    Cout = Wd.shape[0]
+    if X is None:
+        return conv3x3(dZ, Wd.reshape(Cout, 3, 3, Cin))
+    out = torch.empty((B, H, W, Cout), dtype=torch.bfloat16, device=dZ.device)
+    _check(lib.tomo_nn_conv3x3_masked(_p(dZ), B, H, W, Cin, _p(Wd), Cout, _p(X), _p(out), _stream(dZ)),
+           "tomo_nn_conv3x3_masked")
+    return out
+
+
+def _bf16(d):
+    return d.to(torch.bfloat16).contiguous()
+
+
+# The network's layers.  A layer's incoming gradient has already gone through
+# the ReLU at its output: whoever consumes that output has it at hand and
+# applies it while writing the gradient.
+
 class _Conv3x3(torch.autograd.Function):
-    """3x3 convolution + bias (+ ReLU) with the tensor-core kernels in both directions."""
+    """3x3 convolution + bias + ReLU; mask_dx: the input is a ReLU's output."""
 
     @staticmethod
-    def forward(ctx, X, W, b, relu, need_dx):
+    def forward(ctx, X, W, b, need_dx, mask_dx):
         Wb, Wd = prepare_weights(W.detach().reshape(W.shape[0], 9, W.shape[-1]), with_transpose=need_dx)
-        Y = conv3x3(X, Wb.reshape(W.shape), b.detach(), relu=relu)
-        ctx.save_for_backward(X, Y, Wd if need_dx else None)
-        ctx.relu, ctx.need_dx = relu, need_dx
+        Y = conv3x3(X, Wb.reshape(W.shape), b.detach(), relu=True)
+        ctx.save_for_backward(X, Wd if need_dx else None)
+        ctx.need_dx, ctx.mask_dx = need_dx, mask_dx
         return Y
 
     @staticmethod
     def backward(ctx, dY):
-        X, Y, Wd = ctx.saved_tensors
-        dZ = dY.to(torch.bfloat16).contiguous()
-        if ctx.relu:
-            _check(lib.tomo_nn_relu_bwd(_p(Y), _p(dZ), dZ.numel(), _stream(dZ)), "tomo_nn_relu_bwd")
+        X, Wd = ctx.saved_tensors
+        dZ = _bf16(dY)
         dW, db = wgrad(X, dZ, 9)
-        dX = None
-        if ctx.need_dx:
-            dX = conv3x3(dZ, Wd.reshape(Wd.shape[0], 3, 3, Wd.shape[-1]))
+        dX = _conv3x3_dx(dZ, Wd, X if ctx.mask_dx else None) if ctx.need_dx else None
         return dX, dW.reshape(dW.shape[0], 3, 3, dW.shape[-1]), db, None, None
 
 
-class _Conv1x1(torch.autograd.Function):
-    """1x1 convolution + bias, FP32 output (the network's last layer)."""
+class _Conv3x3Pool(torch.autograd.Function):
+    """3x3 convolution + bias + ReLU of a ReLU's output, and its 2x2 max-pooling."""
 
     @staticmethod
     def forward(ctx, X, W, b):
-        Bn, H, Wd_, Cin = X.shape
+        Wb, Wd = prepare_weights(W.detach().reshape(W.shape[0], 9, W.shape[-1]))
+        Y = conv3x3(X, Wb.reshape(W.shape), b.detach(), relu=True)
+        B, H, W_, C = Y.shape
+        P = torch.empty((B, H // 2, W_ // 2, C), dtype=torch.bfloat16, device=Y.device)
+        _check(lib.tomo_nn_pool(_p(Y), B, H // 2, W_ // 2, C, _p(P), _stream(Y)), "tomo_nn_pool")
+        ctx.save_for_backward(X, Y, Wd)
+        return Y, P
+
+    @staticmethod
+    def backward(ctx, dS, dP):
+        X, Y, Wd = ctx.saved_tensors
+        B, H, W, C = Y.shape
+        dP, dS = _bf16(dP), dS.to(torch.bfloat16)
+        ld = dS.stride(2)
+        # the skip's gradient comes as a slice of the concatenation's channels
+        if dS.stride() != (H * W * ld, W * ld, ld, 1) or ld < C or ld % 8 or dS.data_ptr() % 16:
+            dS, ld = dS.contiguous(), C
+        dZ = torch.empty_like(Y)
+        _check(lib.tomo_nn_pool_bwd(_p(Y), _p(dP), _p(dS), ld, B, H // 2, W // 2, C, _p(dZ), _stream(Y)),
+               "tomo_nn_pool_bwd")
+        dW, db = wgrad(X, dZ, 9)
+        return _conv3x3_dx(dZ, Wd, X), dW.reshape(dW.shape[0], 3, 3, dW.shape[-1]), db
+
+
+class _UpCat(torch.autograd.Function):
+    """A ReLU's output upsampled by 2 (nearest) beside the skip's channels."""
+
+    @staticmethod
+    def forward(ctx, X, S):
+        B, h, w, Cu = X.shape
+        Cs = S.shape[-1]
+        Y = torch.empty((B, 2 * h, 2 * w, Cu + Cs), dtype=torch.bfloat16, device=X.device)
+        _check(lib.tomo_nn_upcat(_p(X), _p(S), B, h, w, Cu, Cs, _p(Y), _stream(X)), "tomo_nn_upcat")
+        ctx.save_for_backward(X)
+        return Y
+
+    @staticmethod
+    def backward(ctx, dY):
+        X, = ctx.saved_tensors
+        B, h, w, Cu = X.shape
+        d = _bf16(dY)
+        dX = torch.empty_like(X)
+        _check(lib.tomo_nn_up_bwd(_p(d), d.shape[-1], _p(X), B, h, w, Cu, _p(dX), _stream(d)), "tomo_nn_up_bwd")
+        return dX, d[..., Cu:]
+
+
+class _Head(torch.autograd.Function):
+    """First output of a 1x1 convolution with 8 outputs on a ReLU's output, + bias, FP32 [B, H, W]."""
+
+    @staticmethod
+    def forward(ctx, X, W, b):
+        Bn, H, W_, Cin = X.shape
         Wb, Wt = prepare_weights(W.detach().reshape(W.shape[0], 1, Cin), with_transpose=True)
-        Y = gemm(X.reshape(-1, Cin), Wb.reshape(W.shape[0], Cin), bias=b.detach())
+        Y = gemm(X.reshape(-1, Cin), Wb.reshape(W.shape[0], Cin)[:1], bias=b.detach())
         ctx.save_for_backward(X, Wt)
-        return Y.reshape(Bn, H, Wd_, W.shape[0])
+        return Y.reshape(Bn, H, W_)
 
     @staticmethod
     def backward(ctx, dY):
         X, Wt = ctx.saved_tensors
         Bn, H, W_, Cin = X.shape
-        dZ = dY.to(torch.bfloat16).contiguous()
+        d = dY.to(torch.float32).contiguous()
+        dZ = torch.empty((Bn, H, W_, 8), dtype=torch.bfloat16, device=X.device)
+        _check(lib.tomo_nn_pad8(_p(d), d.numel(), _p(dZ), _stream(d)), "tomo_nn_pad8")
         dW, db = wgrad(X, dZ, 1)
-        dX = gemm(dZ.reshape(-1, dZ.shape[-1]), Wt.reshape(Cin, -1), out_dtype=torch.bfloat16)
-        return dX.reshape(X.shape), dW.reshape(dW.shape[0], Cin), db
-
-
-def _pool(x):
-    # NHWC view as channels-last NCHW for max-pooling
-    return torch.nn.functional.max_pool2d(x.permute(0, 3, 1, 2), 2).permute(0, 2, 3, 1).contiguous()
-
-
-def _up(x):
-    return torch.nn.functional.interpolate(x.permute(0, 3, 1, 2), scale_factor=2, mode="nearest") \
-        .permute(0, 2, 3, 1).contiguous()
+        if Cin <= 1024:
+            dX = torch.empty_like(X)
+            _check(lib.tomo_nn_head_bwd(_p(dZ), _p(Wt), _p(X), d.numel(), Cin, _p(dX), _stream(d)), "tomo_nn_head_bwd")
+        else:  # its weights no longer fit that kernel's shared memory
+            dX = gemm(dZ.reshape(-1, 8), Wt.reshape(Cin, 8), out_dtype=torch.bfloat16).reshape(X.shape)
+            _check(lib.tomo_nn_relu_bwd(_p(X), _p(dX), dX.numel(), _stream(d)), "tomo_nn_relu_bwd")
+        return dX, dW.reshape(dW.shape[0], Cin), db
 
 
 class UNet(torch.nn.Module):
@@ -212,28 +283,28 @@ class UNet(torch.nn.Module):
     def forward(self, x, extra=None):
         """``extra``: optional further input channels, FP32 [B, H, W] or [B, H, W, k] (k <= 7)."""
         B, H, W = x.shape
+        if H % 2 ** (self.levels - 1) or W % 2 ** (self.levels - 1):
+            raise RuntimeError(f"sides {H} x {W} are not multiples of {2 ** (self.levels - 1)}")
         h = torch.zeros((B, H, W, self.CIN), dtype=torch.bfloat16, device=x.device)
         h[..., 0] = x.to(torch.bfloat16)
         if extra is not None:
             e = extra if extra.dim() == 4 else extra[..., None]
             h[..., 1:1 + e.shape[-1]] = e.to(torch.bfloat16)
         skips = []
-        first = True
         for lvl in range(self.levels):
             w1, b1, w2, b2 = self.enc[4 * lvl:4 * lvl + 4]
-            h = _Conv3x3.apply(h, w1, b1, True, not first)
-            h = _Conv3x3.apply(h, w2, b2, True, True)
-            first = False
+            h = _Conv3x3.apply(h, w1, b1, lvl > 0, False)
             if lvl < self.levels - 1:
-                skips.append(h)
-                h = _pool(h)
+                skip, h = _Conv3x3Pool.apply(h, w2, b2)
+                skips.append(skip)
+            else:
+                h = _Conv3x3.apply(h, w2, b2, True, True)
         for j in range(self.levels - 1):
             w1, b1, w2, b2 = self.dec[4 * j:4 * j + 4]
-            h = torch.cat([_up(h), skips[-1 - j]], dim=-1)
-            h = _Conv3x3.apply(h, w1, b1, True, True)
+            h = _UpCat.apply(h, skips[-1 - j])
+            h = _Conv3x3.apply(h, w1, b1, True, False)
             h = _Conv3x3.apply(h, w2, b2, True, True)
-        out = _Conv1x1.apply(h, self.head_w, self.head_b)
-        return x + out[..., 0]
+        return x + _Head.apply(h, self.head_w, self.head_b)
 
 
 class Adam:
