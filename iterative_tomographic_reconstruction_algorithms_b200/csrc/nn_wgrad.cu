@@ -24,8 +24,8 @@
 // clock and SM in 128-byte rows, those copies 15.
 //
 // Measured at 4 x 192^2, 128 -> 128 channels: 1.28 ms when the im2col matrix
-// was written out, 0.17 with 16-byte copies, now 0.097; 4 x 768^2, 32 -> 32:
-// 6.19, 0.69, 0.42; 4 x 192^2, 384 -> 128: 3.42, 0.86, 0.20.
+// was written out, 0.17 with 16-byte copies, now 0.052; 4 x 768^2, 32 -> 32:
+// 6.19, 0.69, 0.18; 4 x 192^2, 384 -> 128: 3.42, 0.86, 0.14.
 //
 // Work split: a CTA owns up to 128 output channels, some of the (tap row,
 // channel block) units that fit its 512 TMEM columns, and one of S contiguous
@@ -67,6 +67,8 @@ struct WgradArgs {
   int U, G, upg;                   // units, groups of them, units of a group
   int rb, chb, nblk, ndx, nmma;    // bytes of X's rows, their channels, channel blocks; taps of an MMA and its N
   int gw, strip_bytes, unit_bytes; // pixels of a strip, bytes of a strip and of a unit's strips
+  int seg;                         // 64 pixels may go over the end of a row: two strips
+  int kpm, blk_bytes;              // 64-pixel blocks of a stage, bytes of one
   int rby, chby, nby, yblk;        // the same of dY: rows, channels, blocks of a CTA's output channels, bytes of one
   // wgrad_gather_kernel
   int ntap, NB, Nb, Mb, sxc, syc;  // taps per group; input-channel blocks and their width; output rows staged
@@ -85,17 +87,25 @@ __device__ __forceinline__ void store_part(const WgradArgs &g, int co, size_t e,
   }
 }
 
-__global__ void __launch_bounds__(192) wgrad_tma_kernel(WgradArgs g, const __grid_constant__ CUtensorMap mx,
+// Warps by role.  A single warp gets an MMA out every 80 clocks and a TMA box
+// every 250 here, and each stage's barriers cost it some 400, so the work is
+// spread: up to four warps issue MMAs, each those of some units (their
+// accumulators are apart), warps 4 and 6 load the input's even and odd units, warp
+// 5 the output gradient, and a stage is up to 4 blocks of 64 pixels.
+// 4 x 768^2, 32 -> 32 channels: 0.36 ms with one warp each and a block per stage,
+// 0.18 now; 96 -> 32: 0.64 and 0.40.
+// SEG: blocks of 64 pixels that may go over the end of a row, in two strips then.
+template <bool SEG>
+__global__ void __launch_bounds__(224) wgrad_tma_kernel(WgradArgs g, const __grid_constant__ CUtensorMap mx,
                                                         const __grid_constant__ CUtensorMap my) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t full[kMaxStages], empty[kMaxStages], done;
+  __shared__ uint64_t xfull[2][kMaxStages], yfull[kMaxStages], empty[kMaxStages], done[4];
   __shared__ uint32_t tmem_slot;
   __shared__ int gave_up;
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int tg = blockIdx.x % g.G, m0 = (blockIdx.x / g.G) * 128;
-  const int u0 = tg * g.upg, nu = min(g.upg, g.U - u0);
+  const int u0 = tg * g.upg, nu = min(g.upg, g.U - u0), nissue = min(nu, 4);
   const int t0 = (int)((long long)g.nkb * blockIdx.y / g.S), t1 = (int)((long long)g.nkb * (blockIdx.y + 1) / g.S);
-  const int nby = min(g.nby, (g.ldY - m0 + g.chby - 1) / g.chby);
   const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u;  // swizzle period
 
   if (warp == 5) {
@@ -105,10 +115,12 @@ __global__ void __launch_bounds__(192) wgrad_tma_kernel(WgradArgs g, const __gri
   }
   if (tid == 0) {
     for (int s = 0; s < g.nst; ++s) {
-      mbar_init(smem_u32(&full[s]), 1);
-      mbar_init(smem_u32(&empty[s]), 1);
+      mbar_init(smem_u32(&xfull[0][s]), 1);
+      mbar_init(smem_u32(&xfull[1][s]), 1);
+      mbar_init(smem_u32(&yfull[s]), 1);
+      mbar_init(smem_u32(&empty[s]), nissue);
     }
-    mbar_init(smem_u32(&done), 1);
+    for (int w = 0; w < 4; ++w) mbar_init(smem_u32(&done[w]), 1);
     gave_up = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -119,39 +131,89 @@ __global__ void __launch_bounds__(192) wgrad_tma_kernel(WgradArgs g, const __gri
   const uint32_t y_off = g.upg * g.unit_bytes;
   bool ok = true;
 
-  if (warp == 4) {  // loads
+  if (warp >= 4) {  // loads, by one thread each, whose loops are kept short: coordinates are stepped, not divided out
     if (lane == 0) {
-      const int halo = g.ndx >> 1, hw = g.H * g.W, nstrip = kKP / g.gw;
-      const uint32_t bytes = nu * nstrip * (g.gw + 2 * halo) * g.rb + nby * kKP * g.rby;
+      uint64_t *full = warp == 5 ? yfull : xfull[warp == 6];
+      const int nst = g.nst;
       Ring r;
       int it = 0;
-      for (int t = t0; t < t1; ++t, ++it, r.next(g.nst)) {
-        if (it >= g.nst) ok = role_wait(&empty[r.s], r.ph ^ 1u, g.spins, &gave_up);
-        if (!ok) break;
-        const uint32_t bar = smem_u32(&full[r.s]), st = base + r.s * g.stage_bytes;
-        mbar_expect(bar, bytes);
-        for (int q = 0; q < nstrip; ++q) {
-          const int p = t * kKP + q * g.gw;
-          int b = 0, y = 0, x = p;
-          if (halo) {  // pixels from P on lie in images that do not exist: zero
-            b = fast_div(p, g.fhw);
-            const int rem = p - b * hw;
-            y = fast_div(rem, g.fw);
-            x = rem - y * g.W;
+      if (warp != 5) {  // units 0, 2, .. or 1, 3, ..
+        const int half = warp == 6, mine = (nu + 1 - half) >> 1;
+        const int halo = g.ndx >> 1, nstrip = kKP / g.gw, gw = g.gw, W = g.W, H = g.H, chb = g.chb;
+        const int nblk = g.nblk, sb = g.strip_bytes, ub = 2 * g.unit_bytes;
+        const uint32_t bytes = mine * (gw + 2 * halo) * g.rb;  // of a strip
+        const int dyu = (u0 + half) / nblk, cu = (u0 + half - dyu * nblk) * chb, cend = nblk * chb;
+        // the next strip's first pixel; from P on it lies in images that do not exist: zero
+        int x = t0 * kKP, y = 0, b = 0;
+        if (halo) {
+          b = fast_div(x, g.fhw);
+          x -= b * H * W;
+          y = fast_div(x, g.fw);
+          x -= y * W;
+        }
+        auto strips = [&](uint32_t dst, int xs, uint32_t bar) {
+          int yy = y + dyu - halo, c = cu;
+          dst += half * g.unit_bytes;
+          for (int u = 0; u < mine; ++u, dst += ub) {
+            tma_load4(dst, &mx, c, xs - halo, yy, b, bar);
+            c += 2 * chb;
+            while (c >= cend) c -= cend, ++yy;
           }
-          int dy = u0 / g.nblk, c = u0 - dy * g.nblk;
-          for (int u = 0; u < nu; ++u) {
-            tma_load4(st + u * g.unit_bytes + q * g.strip_bytes, &mx, c * g.chb, x - halo, y + dy - halo, b, bar);
-            if (++c == g.nblk) c = 0, ++dy;
+        };
+        auto next_row = [&] {
+          if (++y == H) y = 0, ++b;
+        };
+        for (int t = t0; t < t1; ++it, r.next(nst)) {
+          if (it >= nst) ok = role_wait(&empty[r.s], r.ph ^ 1u, g.spins, &gave_up);
+          if (!ok) break;
+          const uint32_t bar = smem_u32(&full[r.s]);
+          uint32_t st = base + r.s * g.stage_bytes;
+          const int te = min(t + g.kpm, t1);
+          if (SEG) {
+            int count = te - t;
+            for (int k = t, xx = x; k < te; ++k)
+              if ((xx += kKP) >= W) xx -= W, count += xx > 0;
+            mbar_expect(bar, count * bytes);
+            for (; t < te; ++t, st += g.blk_bytes) {
+              strips(st, x, bar);
+              if ((x += kKP) >= W) {  // the rest, from the next row's first pixel
+                x -= W;
+                next_row();
+                if (x > 0) strips(st + sb, 0, bar);
+              }
+            }
+          } else {
+            mbar_expect(bar, (te - t) * nstrip * bytes);
+            for (; t < te; ++t, st += g.blk_bytes)
+              for (int q = 0; q < nstrip; ++q) {
+                strips(st + q * sb, x, bar);
+                x += gw;
+                if (halo && x >= W) {
+                  x = 0;
+                  next_row();
+                }
+              }
           }
         }
-        for (int c = 0; c < nby; ++c) tma_load3(st + y_off + c * g.yblk, &my, m0 + c * g.chby, t * kKP, 0, bar);
+      } else {
+        const int nby = min(g.nby, (g.ldY - m0 + g.chby - 1) / g.chby);
+        const uint32_t bytes = nby * kKP * g.rby;
+        for (int t = t0; t < t1; ++it, r.next(nst)) {
+          if (it >= nst) ok = role_wait(&empty[r.s], r.ph ^ 1u, g.spins, &gave_up);
+          if (!ok) break;
+          const uint32_t bar = smem_u32(&full[r.s]);
+          uint32_t st = base + r.s * g.stage_bytes + y_off;
+          const int te = min(t + g.kpm, t1);
+          mbar_expect(bar, (te - t) * bytes);
+          for (; t < te; ++t, st += g.blk_bytes)
+            for (int c = 0; c < nby; ++c) tma_load3(st + c * g.yblk, &my, m0 + c * g.chby, t * kKP, 0, bar);
+        }
       }
       // copies still in flight (after a wait that gave up nobody else waits for them)
-      for (int k = max(0, it - g.nst); k < it; ++k)
-        if (!mbar_wait(smem_u32(&full[k % g.nst]), (k / g.nst) & 1, kDrainSpins)) ok = false;
+      for (int k = max(0, it - nst); k < it; ++k)
+        if (!mbar_wait(smem_u32(&full[k % nst]), (k / nst) & 1, kDrainSpins)) ok = false;
     }
-  } else if (warp == 5) {  // MMAs
+  } else if (warp < nissue) {  // MMAs of units warp, warp + 4, ...
     const uint32_t idesc = instr_desc_mn(g.nmma, g.mrows);
     // K groups of 8 pixels follow one another, or, in strips of 8, lie a strip
     // apart; N blocks (taps) one pixel apart
@@ -162,27 +224,40 @@ __global__ void __launch_bounds__(192) wgrad_tma_kernel(WgradArgs g, const __gri
     Ring r;
     bool issued = false;
     uint32_t more = 0;
-    for (int t = t0; t < t1; ++t, r.next(g.nst)) {
-      ok = warp_wait(&full[r.s], r.ph, g.spins, &gave_up);
+    int x = SEG ? t0 * kKP - fast_div(t0 * kKP, g.fw) * g.W : 0;
+    for (int t = t0; t < t1; r.next(g.nst)) {
+      ok = warp_wait(&xfull[warp & 1][r.s], r.ph, g.spins, &gave_up) && warp_wait(&yfull[r.s], r.ph, g.spins, &gave_up);
       if (!ok) break;
       tc_fence_after();
-      const uint32_t st = base + r.s * g.stage_bytes;
-      const uint64_t da = dy0 + ((st + y_off) >> 4);
-      uint64_t db = dx0 + (st >> 4);
-      uint32_t d = tmem;
-      for (int u = 0; u < nu; ++u) {
-        mma_warp<4>(d, da, db, idesc, more, sa, sb);
-        d += g.nmma;
-        db += g.unit_bytes >> 4;
+      uint32_t st = base + r.s * g.stage_bytes;
+      for (const int te = min(t + g.kpm, t1); t < te; ++t, st += g.blk_bytes) {
+        const uint64_t da = dy0 + ((st + y_off) >> 4);
+        const int c = SEG ? (g.W - x) >> 3 : 8;  // K groups up to the end of the row
+        if (SEG && c < kKP / 8) {
+          // the others lie in the second strip; the MMA across the end has its two a strip apart
+          const uint32_t back = g.strip_bytes - c * kg;
+          const uint32_t over = back + kg;
+          const uint64_t dxo = g.rb == 16 ? smem_desc_rb(0, over, 16, 16) : smem_desc_rb(0, g.rb, over, g.rb);
+          for (int u = warp; u < nu; u += 4)
+            for (int j = 0; j < 4; ++j) {
+              const uint32_t at = st + u * g.unit_bytes + 2 * j * kg + (2 * j >= c ? back : 0);
+              mma_warp<1>(tmem + u * g.nmma, da + j * sa, (2 * j + 1 == c ? dxo : dx0) + (at >> 4), idesc,
+                          more | (j > 0));
+            }
+        } else {
+          for (int u = warp; u < nu; u += 4)
+            mma_warp<4>(tmem + u * g.nmma, da, dx0 + ((st + u * g.unit_bytes) >> 4), idesc, more, sa, sb);
+        }
+        if (SEG && (x += kKP) >= g.W) x -= g.W;
+        more = 1;
       }
       mma_commit_warp(smem_u32(&empty[r.s]));
       issued = true;
-      more = 1;
     }
     // every MMA issued so far, also on the way out of a wait that gave up
     if (issued) {
-      mma_commit_warp(smem_u32(&done));
-      if (!mbar_wait(smem_u32(&done), 0, kDrainSpins)) ok = false;
+      mma_commit_warp(smem_u32(&done[warp]));
+      if (!mbar_wait(smem_u32(&done[warp]), 0, kDrainSpins)) ok = false;
     }
   }
   if (!ok) atomicOr(&gave_up, 1);
@@ -362,8 +437,8 @@ __global__ void wgrad_reduce_kernel(const float *__restrict__ part, int S, size_
 }
 
 // Bias gradient: block b sums its range of pixels of dY [P][C] per channel.  A
-// thread takes 8 channels of every (threads / (C/8))-th pixel, in double, so
-// the sum's own rounding stays below the result's; the block's threads and
+// thread takes 8 channels of every (threads / (C/8))-th pixel, 16 of them in float
+// (8 significant bits each) and those sums in double; the block's threads and
 // then the blocks (colsum_final_kernel) are added in order.
 constexpr int kColThreads = 256, kColBlocks = 592;
 
@@ -472,9 +547,13 @@ WgradArgs wgrad_plan(int batch, int H, int W, int Cin, int Cout, int taps) {
     g.nby = (std::min(g.ldY, 128) + g.chby - 1) / g.chby;
     g.yblk = kKP * g.rby;
     const int halo = g.ndx >> 1;
-    g.gw = taps == 1 || W % 64 == 0 ? 64 : W % 16 == 0 ? 16 : 8;
+    // a strip of 64 pixels, and a second one where a row ends among them; images
+    // narrower than that take strips of 16 or 8 (a TMA box costs some 250 clocks,
+    // whatever its rows: 4 x 760^2, 32 -> 32 in strips of 8 took 1.02 ms, now 0.24)
+    g.gw = taps == 1 || W >= 64 ? 64 : W % 16 == 0 ? 16 : 8;
+    g.seg = taps == 9 && W >= 64 && W % 64;
     g.strip_bytes = ((g.gw + 2 * halo) * g.rb + 1023) / 1024 * 1024;
-    g.unit_bytes = kKP / g.gw * g.strip_bytes;
+    g.unit_bytes = (g.seg ? 2 : kKP / g.gw) * g.strip_bytes;
     for (;; --g.upg) {  // two stages at least
       g.stage_bytes = g.upg * g.unit_bytes + g.nby * g.yblk;
       // an MMA reads mrows rows of dY whatever Cout: blocks behind the staged
@@ -509,6 +588,12 @@ WgradArgs wgrad_plan(int batch, int H, int W, int Cin, int Cout, int taps) {
   // two CTAs to an SM when there are more than one for each
   int budget = ctas > kSms && 2 * g.cols <= 512 ? kSmemMax / 2 - 1024 : kSmemMax;
   if (3 * g.stage_bytes + g.tail_bytes > budget) budget = kSmemMax;
+  // A stage of the TMA kernel is up to 4 blocks, as long as there are three
+  // stages (32 -> 32 at 768^2: 331 us with one, 267 with two, 235 with four).
+  g.blk_bytes = g.stage_bytes;
+  g.kpm = 1;
+  while (g.rb && g.kpm < 4 && 3 * 2 * g.kpm * g.blk_bytes + g.tail_bytes <= budget) g.kpm *= 2;
+  g.stage_bytes = g.kpm * g.blk_bytes;
   g.nst = std::min(kMaxStages, (budget - g.tail_bytes) / g.stage_bytes);
   return g;
 }
@@ -577,9 +662,9 @@ int wgrad_launch(const __nv_bfloat16 *X, const __nv_bfloat16 *dY, int batch, int
     const unsigned long long dy[3] = {ul, up, 1}, sy[2] = {2 * ul, 2 * ul * up};
     const unsigned by[3] = {(unsigned)g.chby, kKP, 1};
     if (int rc = make_tensor_map(&my, dY, 3, dy, sy, by, g.rby)) return rc;
-    if (cudaFuncSetAttribute(wgrad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return NN_ECUDA;
-    wgrad_tma_kernel<<<dim3(MB * g.G, g.S), 192, smem, s>>>(g, mx, my);
+    auto fn = g.seg ? wgrad_tma_kernel<true> : wgrad_tma_kernel<false>;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return NN_ECUDA;
+    fn<<<dim3(MB * g.G, g.S), 224, smem, s>>>(g, mx, my);
   } else {
     const int lag = g.nst >= 7 ? 5 : g.nst >= 5 ? 3 : g.nst >= 3 ? 2 : 1;
     auto fn = lag == 5   ? wgrad_gather_kernel<5>

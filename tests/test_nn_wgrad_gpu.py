@@ -42,3 +42,12 @@ def test_wgrad_tile_edges(cuda, B, H, W, Cin, Cout, taps):
     Yo = torch.empty(dY.numel() + 1, dtype=torch.bfloat16, device="cuda")[1:].view(dY.shape)
     off, _ = nn.wgrad(Xo.copy_(X), Yo.copy_(dY), taps)
     assert torch.equal(off, dW)
+
+
+@pytest.mark.parametrize("B,H,W,Cin,Cout", [
+    (1, 5, 64, 32, 32), (1, 5, 72, 32, 32), (2, 9, 88, 8, 40), (1, 7, 120, 64, 64), (1, 3, 200, 96, 130), (2, 4, 136, 16, 24),
+    (3, 11, 80, 48, 16), (1, 1, 104, 8, 8), (2, 2, 760, 32, 32)])
+def test_wgrad_rows_ending_among_a_block(cuda, B, H, W, Cin, Cout):
+    """64-pixel blocks that go over the end of a row at each multiple of 8; fewer than 100
+    groups of 16 pixels per accumulator, as above."""
+    test_wgrad_tile_edges(cuda, B, H, W, Cin, Cout, 9)
