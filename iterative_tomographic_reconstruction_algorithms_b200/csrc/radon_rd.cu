@@ -12,7 +12,7 @@
 // to the pixel it steps INTO (x index -> image row) if that pixel has row and
 // column in [1, n-1]; it stops after the first step with alpha > 1.
 //
-// Both directions run the same walks (rd_walk_loop), one thread per (bin, angle,
+// Both directions run the same walks (rd_walk_free, rd_walk_checked), one thread per (bin, angle,
 // slice) replaying its bin's five sub-rays (the adjoint, on grids too small to
 // fill the GPU, one thread per sub-ray):
 //   forward  gathers 0.2 l x[pixel] into the bin, in walk order;
@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "f32x2.cuh"
 #include "fixed_sum.cuh"
 #include "tomo_internal.cuh"
 
@@ -148,9 +149,9 @@ __device__ __forceinline__ float rd_alpha_mf(float m, float f, float e, float r)
 // offset in the image the caller reads or writes (sA = row stride, sB = 1
 // row-major; sA = 1, sB = row stride transposed), l the length credited.
 //
-// Two forms.  Checked (Safe): ok as above, and the walk stops after 4n + 16
+// Two forms.  rd_walk_checked: ok as above, and the walk stops after 4n + 16
 // steps: a zero or tiny extent makes that axis' alphas infinite or NaN, on
-// which the reference never ends.  Unchecked (Safe false), for walks with
+// which the reference never ends.  rd_walk_free, for walks with
 // |1/e| <= 2^64 on both axes, where each step raises the stepped axis' next
 // alpha by about 1/|e| (far above the float spacing of alphas <= 1) and no
 // alpha is inf or NaN, so a walk ends after at most |ex| + |ey| + 4 steps;
@@ -164,9 +165,9 @@ __device__ __forceinline__ float rd_alpha_mf(float m, float f, float e, float r)
 // c <= nh - 1/2 and the pixel stepped into, c + 3/2, is <= nh + 1; step 0
 // goes to round(p1x) + 1 <= nh + 1; and round(p1x) >= -nh.  The same for
 // dx = -1 and for y.)
-template <bool Safe, class Visit>
-__device__ __forceinline__ void rd_walk_loop(const RdGeom &s, int n, int nh, int sA, int sB, int pad, float rx,
-                                             float ry, Visit &visit) {
+template <class Visit>
+__device__ __forceinline__ void rd_walk_checked(const RdGeom &s, int n, int nh, int sA, int sB, int pad, float rx,
+                                                float ry, Visit &visit) {
   const float incr = __fsqrt_rn(__fmaf_rn(s.ex, s.ex, __fmul_rn(s.ey, s.ey)));
   const float hx = s.dx > 0 ? 0.5f : -0.5f, hy = s.dy > 0 ? 0.5f : -0.5f;
   const float fdx = hx + hx, fdy = hy + hy;
@@ -184,23 +185,72 @@ __device__ __forceinline__ void rd_walk_loop(const RdGeom &s, int n, int nh, int
   int off = (s.ii0 + nh + pad) * sA + (s.jj0 + nh + pad) * sB;
   const int ox = s.dx * sA, oy = s.dy * sB;
   float alpha = 0.0f, alpha_old = 0.0f;
-  for (int it = Safe ? 4 * n + 16 : 1; alpha <= 1.0f && it > 0; it -= Safe ? 1 : 0) {
+  for (int it = 4 * n + 16; alpha <= 1.0f && it > 0; --it) {
     // x step if ax < ay, y step if ax > ay, both if equal (radon_rd.c:45-58);
-    // a NaN crossing would never advance the reference: stop.  Written
-    // without branches on the step kind, so the lanes of a warp stay together:
-    // one new crossing parameter (two on a diagonal step).
+    // a NaN crossing would never advance the reference: stop.
     const bool sx = ax <= ay, sy = ay <= ax;
-    if (Safe && !(sx || sy)) break;
+    if (!(sx || sy)) break;
     alpha = sx ? ax : ay;
     mx = sx ? __fadd_rn(mx, fdx) : mx;
     my = sy ? __fadd_rn(my, fdy) : my;
     off += (sx ? ox : 0) + (sy ? oy : 0);
-    const float a1 = rd_alpha_mf(sx ? mx : my, sx ? fx : fy, sx ? s.ex : s.ey, sx ? rx : ry);
-    ax = sx ? a1 : ax;
-    ay = sx ? ay : a1;
-    if (sx && sy) ay = rd_alpha_mf(my, fy, s.ey, ry);
+    if (sx) ax = rd_alpha_mf(mx, fx, s.ex, rx);
+    if (sy) ay = rd_alpha_mf(my, fy, s.ey, ry);
     const float l = __fmul_rn(__fsub_rn(alpha, alpha_old), incr);
-    visit(!Safe || (fabsf(__fadd_rn(mx, kx)) <= lim && fabsf(__fadd_rn(my, ky)) <= lim), off, l);
+    visit(fabsf(__fadd_rn(mx, kx)) <= lim && fabsf(__fadd_rn(my, ky)) <= lim, off, l);
+    alpha_old = alpha;
+  }
+}
+
+// Both axes' next crossings are computed every step, as one packed pair: the axis
+// that did not step gets its value again, and nothing has to be selected between
+// the axes (compares and selects go at half the rate of additions).  Forward at
+// 768^2 x 720 with selects and one crossing per step 4.33 ms, now 4.04, 3.96 with
+// the gather two steps ahead; at 2048^2 x 1800 75.7, 70.4, 68.9.  The adjoint is
+// bound by its reductions (83 % of L1's throughput) and takes as long either way.
+// nz is a -0 the compiler does not know: a product that goes into an addition
+// must be rounded first, and h r + nz is (a mul2 would be contracted).
+// q2 -+ d (rd_alpha_mf) are one fma each, of q1 2^-38 with q1's sign: the two
+// then change places, and only their equality counts; the product is exact,
+// |q1| being 0 or far above 2^-80.
+template <class Visit>
+__device__ __forceinline__ void rd_walk_free(const RdGeom &s, int nh, int sA, int sB, int pad, float rx, float ry,
+                                             float nz, Visit &visit) {
+  const float incr = __fsqrt_rn(__fmaf_rn(s.ex, s.ex, __fmul_rn(s.ey, s.ey)));
+  const float hx = s.dx > 0 ? 0.5f : -0.5f, hy = s.dy > 0 ? 0.5f : -0.5f;
+  const float Px = rintf(s.p1x), Py = rintf(s.p1y);
+  const F2 nf = f2(__fsub_rn(Px, s.p1x), __fsub_rn(Py, s.p1y)), fd = f2(hx + hx, hy + hy);
+  const F2 r = f2(rx, ry), ne = f2(-s.ex, -s.ey), nzz = f2(nz), up = f2(0x1p-38f), dn = f2(-0x1p-38f);
+  // numerators of the next x and y crossings, m - f, m stepped exactly by +-1
+  F2 m = f2(__fsub_rn(__fadd_rn((float)s.ii0, hx), Px), __fsub_rn(__fadd_rn((float)s.jj0, hy), Py));
+  int off = (s.ii0 + nh + pad) * sA + (s.jj0 + nh + pad) * sB;
+  const int ox = s.dx * sA, oy = s.dy * sB;
+  float ax, ay;
+  auto crossings = [&] {
+    const F2 h = add2(m, nf), l = rsub2(rsub2(m, h), nf);
+    const F2 q1 = fma2(h, r, nzz);
+    const F2 q2 = mul2(add2(fma2(q1, ne, h), l), r);
+    const float2 lo = unpack(add2(q1, fma2(q1, dn, q2))), hi = unpack(add2(q1, fma2(q1, up, q2)));
+    ax = lo.x;
+    ay = lo.y;
+    if (lo.x != hi.x || lo.y != hi.y) {
+      const float2 hs = unpack(h), ls = unpack(l);
+      if (lo.x != hi.x) ax = rd_alpha_div(hs.x, ls.x, s.ex);
+      if (lo.y != hi.y) ay = rd_alpha_div(hs.y, ls.y, s.ey);
+    }
+  };
+  crossings();
+  float alpha = 0.0f, alpha_old = 0.0f;
+#pragma unroll 2
+  while (alpha <= 1.0f) {
+    // x step if ax < ay, y step if ax > ay, both if equal (radon_rd.c:45-58)
+    const bool sx = ax <= ay, sy = ay <= ax;
+    alpha = sx ? ax : ay;
+    m = fma2(f2(sx ? 1.0f : 0.0f, sy ? 1.0f : 0.0f), fd, m);
+    if (sx) off += ox;
+    if (sy) off += oy;
+    crossings();
+    visit(true, off, __fmul_rn(__fsub_rn(alpha, alpha_old), incr));
     alpha_old = alpha;
   }
 }
@@ -215,18 +265,31 @@ __device__ __forceinline__ bool rd_walk_framed(const RdGeom &s, int nh, float rx
 }
 
 // The forward's credits along walks: acc += 0.2 l x[pixel] in walk order,
-// each credit added one step after its load is issued, so the load is in
-// flight during the next step; a step outside [1, n-1]^2 adds 0 * 0 (checked
+// each credit added kAhead steps after its load is issued, so the load is in
+// flight meanwhile (two: three and four need moves or registers, 4.3 ms at
+// 768^2 x 720); a step outside [1, n-1]^2 adds 0 * 0 (checked
 // walks) or w * 0 from the frame (acc is never -0, so that leaves it
 // unchanged).
 struct RdGather {
+  static constexpr int kAhead = 2;
   const float *P;
-  float acc, w, xv;
+  float acc, w[kAhead], xv[kAhead];
   __device__ __forceinline__ void operator()(bool ok, int off, float l) {
     const float x = ok ? __ldg(P + off) : 0.0f;
-    acc = fmaf(w, xv, acc);
-    w = ok ? 0.2f * l : 0.0f;
-    xv = x;
+    acc = fmaf(w[0], xv[0], acc);
+#pragma unroll
+    for (int i = 0; i + 1 < kAhead; ++i) {
+      w[i] = w[i + 1];
+      xv[i] = xv[i + 1];
+    }
+    w[kAhead - 1] = ok ? 0.2f * l : 0.0f;
+    xv[kAhead - 1] = x;
+  }
+  __device__ __forceinline__ float sum() const {
+    float a = acc;
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) a = fmaf(w[i], xv[i], a);
+    return a;
   }
 };
 
@@ -249,13 +312,13 @@ struct RdScatter {
 // out of the register budget of the unchecked loop.
 __device__ __noinline__ RdGather rd_walk_safe(RdGeom s, int n, int nh, int sA, int sB, int pad, float rx, float ry,
                                               RdGather v) {
-  rd_walk_loop<true>(s, n, nh, sA, sB, pad, rx, ry, v);
+  rd_walk_checked(s, n, nh, sA, sB, pad, rx, ry, v);
   return v;
 }
 
 __device__ __noinline__ void rd_walk_safe(RdGeom s, int n, int nh, int sA, int sB, int pad, float rx, float ry,
                                           RdScatter v) {
-  rd_walk_loop<true>(s, n, nh, sA, sB, pad, rx, ry, v);
+  rd_walk_checked(s, n, nh, sA, sB, pad, rx, ry, v);
 }
 
 // Framed copies of slice blockIdx.z for the forward's walks: Q (row-major)
@@ -297,7 +360,7 @@ template <int kBins>
 __global__ void __launch_bounds__(kBins * kFwdAngles, 1024 / (kBins * kFwdAngles)) rd_forward_kernel(
     const float *__restrict__ img, const float *__restrict__ Q, const float *__restrict__ QT,
     float *__restrict__ sino, const RdAngle *__restrict__ tab, const float *__restrict__ toff, int n, int nh, int na,
-    int z0, FwdEpi ep) {
+    int z0, float nz, FwdEpi ep) {
   const int b = blockIdx.x * kBins + threadIdx.x;
   const int v = blockIdx.y * kFwdAngles + threadIdx.y;
   if (v >= na) return;  // whole warps
@@ -318,16 +381,16 @@ __global__ void __launch_bounds__(kBins * kFwdAngles, 1024 / (kBins * kFwdAngles
     const bool tr = g.tr != 0;
     const float *P = (tr ? QT : Q) + (size_t)blockIdx.z * m * m;
     const int sA = tr ? 1 : m, sB = tr ? m : 1;
-    RdGather gat{P, 0.0f, 0.0f, 0.0f};
+    RdGather gat{P, 0.0f, {}, {}};
     for (int r = 1; r <= 5; ++r) {
       const RdGeom s = rd_geom_of(tab, v, toff, 6 * b + r, n, nh);
       const float rx = __frcp_rn(s.ex), ry = __frcp_rn(s.ey);
       if (rd_walk_framed(s, nh, rx, ry))
-        rd_walk_loop<false>(s, n, nh, sA, sB, 1, rx, ry, gat);
+        rd_walk_free(s, nh, sA, sB, 1, rx, ry, nz, gat);
       else
         gat = rd_walk_safe(s, n, nh, sA, sB, 1, rx, ry, gat);
     }
-    acc = fmaf(gat.w, gat.xv, gat.acc);
+    acc = gat.sum();
   }
   // store through the epilogue; residual slot as in one launch over all slices
   const size_t e = (z * na + v) * (size_t)n + (live ? b : 0);
@@ -341,13 +404,12 @@ __global__ void __launch_bounds__(kBins * kFwdAngles, 1024 / (kBins * kFwdAngles
 // order (the walks of a bin's sub-rays cover nearly the same pixels at nearly
 // the same time, so the warps share L1 lines; two or three angles to a block: no
 // faster).  One thread for all five walks of a bin leaves small images waiting
-// for one long chain of steps: 0.54 ms at 256^2 x 304, here 0.25; 513^2 x 400
-// 1.44, here 1.16; 2048^2 x 1800, bound by ALU issue either way, 78.8, here
-// 75.7.  rd_forward_kernel keeps that one chain, the reference's, for the solvers.
+// for one long chain of steps: 0.49 ms at 256^2 x 304, here 0.23; 513^2 x 400
+// 1.32, here 1.05.  rd_forward_kernel keeps that one chain, the reference's, for the solvers.
 __global__ void __launch_bounds__(160, 6) rd_forward_split_kernel(
     const float *__restrict__ img, const float *__restrict__ Q, const float *__restrict__ QT,
     float *__restrict__ sino, const RdAngle *__restrict__ tab, const float *__restrict__ toff, int n, int nh, int na,
-    int z0) {
+    int z0, float nz) {
   __shared__ float part[5][32];
   const int lane = threadIdx.x, r = threadIdx.y;
   const int b = blockIdx.x * 32 + lane, v = blockIdx.y;
@@ -369,14 +431,14 @@ __global__ void __launch_bounds__(160, 6) rd_forward_split_kernel(
       const bool tr = g->tr != 0;
       const float *P = (tr ? QT : Q) + (size_t)blockIdx.z * m * m;
       const int sA = tr ? 1 : m, sB = tr ? m : 1;
-      RdGather gat{P, 0.0f, 0.0f, 0.0f};
+      RdGather gat{P, 0.0f, {}, {}};
       const RdGeom s = rd_geom_of(tab, v, toff, 6 * b + r + 1, n, nh);
       const float rx = __frcp_rn(s.ex), ry = __frcp_rn(s.ey);
       if (rd_walk_framed(s, nh, rx, ry))
-        rd_walk_loop<false>(s, n, nh, sA, sB, 1, rx, ry, gat);
+        rd_walk_free(s, nh, sA, sB, 1, rx, ry, nz, gat);
       else
         gat = rd_walk_safe(s, n, nh, sA, sB, 1, rx, ry, gat);
-      acc = fmaf(gat.w, gat.xv, gat.acc);
+      acc = gat.sum();
     }
   }
   part[r][lane] = acc;
@@ -411,7 +473,7 @@ __device__ __noinline__ void rd_scatter_nonfinite(float y, const RdAngle *__rest
       auto flag = [&](bool ok, int off, float l) {
         if (ok) rd_flag(Fl, (size_t)off, __fmul_rn(0.2f * l, y));
       };
-      rd_walk_loop<true>(s, n, nh, n, 1, 0, __frcp_rn(s.ex), __frcp_rn(s.ey), flag);
+      rd_walk_checked(s, n, nh, n, 1, 0, __frcp_rn(s.ex), __frcp_rn(s.ey), flag);
     }
   }
 }
@@ -438,7 +500,7 @@ template <bool kSplit>
 __global__ void __launch_bounds__(128) rd_scatter_kernel(
     const float *__restrict__ sino, unsigned long long *__restrict__ accf, unsigned long long *__restrict__ accT,
     unsigned long long *__restrict__ lines, unsigned *__restrict__ flags, const RdAngle *__restrict__ tab,
-    const float *__restrict__ toff, int n, int nh, int na, const unsigned *__restrict__ smax) {
+    const float *__restrict__ toff, int n, int nh, int na, const unsigned *__restrict__ smax, float nz) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = kSplit ? t / 5 : t;
   const int r0 = kSplit ? t - 5 * b + 1 : 1, r1 = kSplit ? r0 : 5;
@@ -473,7 +535,7 @@ __global__ void __launch_bounds__(128) rd_scatter_kernel(
     const RdGeom s = rd_geom_of(tab, v, toff, 6 * b + r, n, nh);
     const float rx = __frcp_rn(s.ex), ry = __frcp_rn(s.ey);
     if (rd_walk_framed(s, nh, rx, ry))
-      rd_walk_loop<false>(s, n, nh, sA, sB, 1, rx, ry, add);
+      rd_walk_free(s, nh, sA, sB, 1, rx, ry, nz, add);
     else
       rd_walk_safe(s, n, nh, sA, sB, 1, rx, ry, add);
   }
@@ -576,17 +638,17 @@ int rd_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
                                                                                      QT, n);
     if (!ep.ordered) {
       rd_forward_split_kernel<<<dim3((n + 31) / 32, na, zc), dim3(32, 5), 0, s>>>(
-          d_img, Q, QT, d_sino, (const RdAngle *)p.d_angles, (const float *)p.d_aux, n, p.nh, na, z0);
+          d_img, Q, QT, d_sino, (const RdAngle *)p.d_angles, (const float *)p.d_aux, n, p.nh, na, z0, -0.0f);
       continue;
     }
     const int rows = (na + kFwdAngles - 1) / kFwdAngles, w128 = (n + 127) / 128;
     // 128-bin blocks once there are 8 or more per SM, else 32-bin ones
     if ((size_t)w128 * rows * zc >= (size_t)148 * 8)
       rd_forward_kernel<128><<<dim3(w128, rows, zc), dim3(128, kFwdAngles), 0, s>>>(
-          d_img, Q, QT, d_sino, (const RdAngle *)p.d_angles, (const float *)p.d_aux, n, p.nh, na, z0, ep);
+          d_img, Q, QT, d_sino, (const RdAngle *)p.d_angles, (const float *)p.d_aux, n, p.nh, na, z0, -0.0f, ep);
     else
       rd_forward_kernel<32><<<dim3(4 * w128, rows, zc), dim3(32, kFwdAngles), 0, s>>>(
-          d_img, Q, QT, d_sino, (const RdAngle *)p.d_angles, (const float *)p.d_aux, n, p.nh, na, z0, ep);
+          d_img, Q, QT, d_sino, (const RdAngle *)p.d_angles, (const float *)p.d_aux, n, p.nh, na, z0, -0.0f, ep);
   }
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
@@ -615,11 +677,11 @@ int rd_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const
     if ((size_t)n * na * zc >= (size_t)148 * 1024)
       rd_scatter_kernel<false><<<dim3((n + 127) / 128, na, zc), 128, 0, s>>>(
           d_sino + (size_t)z0 * per_sino, accf, accT, lines, flags, (const RdAngle *)p.d_angles,
-          (const float *)p.d_aux, n, p.nh, na, smax + z0);
+          (const float *)p.d_aux, n, p.nh, na, smax + z0, -0.0f);
     else
       rd_scatter_kernel<true><<<dim3((5 * n + 127) / 128, na, zc), 128, 0, s>>>(
           d_sino + (size_t)z0 * per_sino, accf, accT, lines, flags, (const RdAngle *)p.d_angles,
-          (const float *)p.d_aux, n, p.nh, na, smax + z0);
+          (const float *)p.d_aux, n, p.nh, na, smax + z0, -0.0f);
     rd_finalize_kernel<<<dim3((n + 31) / 32, (n + 31) / 32, zc), dim3(32, 8), 0, s>>>(
         accf, accT, lines, flags, d_img, n, z0, na, smax + z0, ep);
   }
