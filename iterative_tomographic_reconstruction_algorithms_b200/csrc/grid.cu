@@ -40,7 +40,7 @@
 // H; the 2-D DFT with sign -1; the forward's deapodisation, crop and flip.
 //
 // Only the 2-D transform uses cuFFT; the per-projection 1-D transforms are a
-// mixed-radix Stockham FFT in shared memory (radix 4/2/3/5/7 and generic odd
+// mixed-radix Stockham FFT in shared memory (radix 8/4/2/3/5/7 and generic odd
 // primes; Govindaraju et al., SC'08 formulation).
 #include <cufft.h>
 #include <cstring>
@@ -70,6 +70,8 @@ struct GridState {
   float2 *filt_b = nullptr;   // adjoint filter [pdim/2]
   float2 *tw = nullptr;       // exp(-2 pi i t / pdim), t < pdim
   float2 *sorted = nullptr;   // adjoint gather: (polar angle, angle index as float bits), sorted
+  int *start = nullptr;       // adjoint gather: where to look for an angle in sorted, by bucket
+  int nbuck = 0;
   float4 *sc4 = nullptr;      // adjoint gather: per angle (sin, cos, 1/cos, 1/sin)
   float2 *H = nullptr;        // [nz][pdim][pdim]
   float2 *rows = nullptr;     // [nz][na][pdim]
@@ -93,65 +95,109 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// In-place (ping-pong) Stockham FFT of one row in shared memory, sign -1.
-// Returns the buffer holding the result.
+// Place of element i of a row in shared memory: one float2 of padding after every
+// 16 spreads the strided stores of the first passes over the banks.
+__device__ __forceinline__ int fft_at(int i) { return i + (i >> 4); }
+size_t fft_smem(int n) { return 2 * sizeof(float2) * (size_t)(n + n / 16 + 1); }
+
+// Radix-4 butterfly, sign -1, of v[0], v[S], v[2S], v[3S].
+template <int S>
+__device__ __forceinline__ void dft4(const float2 *v, float2 *o) {
+  const float2 s0 = make_float2(v[0].x + v[2 * S].x, v[0].y + v[2 * S].y);
+  const float2 d0 = make_float2(v[0].x - v[2 * S].x, v[0].y - v[2 * S].y);
+  const float2 s1 = make_float2(v[S].x + v[3 * S].x, v[S].y + v[3 * S].y);
+  const float2 d1 = make_float2(v[S].x - v[3 * S].x, v[S].y - v[3 * S].y);
+  o[0] = make_float2(s0.x + s1.x, s0.y + s1.y);
+  o[2] = make_float2(s0.x - s1.x, s0.y - s1.y);
+  o[1] = make_float2(d0.x + d1.y, d0.y - d1.x);  // d0 - i d1
+  o[3] = make_float2(d0.x - d1.y, d0.y + d1.x);  // d0 + i d1
+}
+
+// One pass of radix R of the row's Stockham FFT, Ns the product of the radices
+// before it.  R is a template parameter so that the butterfly stays in registers
+// (as a loop bound it put them in local memory, and the twiddles' indices took
+// 64-bit remainders that are never needed: r jm span < N).
+template <int R>
+__device__ __forceinline__ void fft_pass(const float2 *a, float2 *b, int N, int Ns, const float2 *__restrict__ tw) {
+  const int NR = N / R, span = NR / Ns;
+  const unsigned inv = Ns > 1 ? (unsigned)((0x100000000ull + Ns - 1) / Ns) : 0u;  // j / Ns, j < 2^13
+  for (int j = threadIdx.x; j < NR; j += blockDim.x) {
+    const int jq = Ns > 1 ? (int)__umulhi((unsigned)j, inv) : j, jm = j - jq * Ns;
+    float2 v[R], o[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      v[r] = a[fft_at(j + r * NR)];
+      if (r && Ns > 1) v[r] = cmul(v[r], __ldg(tw + r * jm * span));
+    }
+    if constexpr (R == 2) {
+      o[0] = make_float2(v[0].x + v[1].x, v[0].y + v[1].y);
+      o[1] = make_float2(v[0].x - v[1].x, v[0].y - v[1].y);
+    } else if constexpr (R == 4) {
+      dft4<1>(v, o);
+    } else if constexpr (R == 8) {
+      constexpr float c8 = 0.70710678118654752f;
+      float2 e[4], d[4];
+      dft4<2>(v, e);
+      dft4<2>(v + 1, d);
+      const float2 w[4] = {d[0], make_float2(c8 * (d[1].x + d[1].y), c8 * (d[1].y - d[1].x)),
+                           make_float2(d[2].y, -d[2].x), make_float2(c8 * (d[3].y - d[3].x), -c8 * (d[3].x + d[3].y))};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        o[k] = make_float2(e[k].x + w[k].x, e[k].y + w[k].y);
+        o[k + 4] = make_float2(e[k].x - w[k].x, e[k].y - w[k].y);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        o[k] = v[0];
+#pragma unroll
+        for (int q = 1; q < R; ++q) {
+          const float2 t = cmul(v[q], __ldg(tw + NR * ((q * k) % R)));
+          o[k].x += t.x;
+          o[k].y += t.y;
+        }
+      }
+    }
+    const int base = jq * Ns * R + jm;
+#pragma unroll
+    for (int r = 0; r < R; ++r) b[fft_at(base + r * Ns)] = o[r];
+  }
+}
+
+// The same for a prime radix without a butterfly: the sums straight from the input.
+__device__ void fft_pass_prime(const float2 *a, float2 *b, int R, int N, int Ns, const float2 *__restrict__ tw) {
+  const int NR = N / R, span = NR / Ns;
+  for (int j = threadIdx.x; j < NR; j += blockDim.x) {
+    const int jm = j % Ns, base = (j / Ns) * Ns * R + jm;
+    for (int k = 0; k < R; ++k) {
+      float2 acc = make_float2(0, 0);
+      for (int q = 0; q < R; ++q) {
+        float2 x = a[fft_at(j + q * NR)];
+        if (q) x = cmul(x, __ldg(tw + q * jm * span));
+        const float2 t = cmul(x, __ldg(tw + NR * (int)(((long long)q * k) % R)));
+        acc.x += t.x;
+        acc.y += t.y;
+      }
+      b[fft_at(base + k * Ns)] = acc;
+    }
+  }
+}
+
+// Stockham FFT of one row in shared memory (a, scratch b, both laid out by
+// fft_at), sign -1.  Returns the buffer holding the result.
+// 1500 rows of 4096: 198 us with radix-4 passes through local memory, now 80.
 __device__ float2 *stockham(float2 *a, float2 *b, const FftConst &c, const float2 *__restrict__ tw) {
-  const int N = c.n;
   int Ns = 1;
   for (int s = 0; s < c.nfac; ++s) {
     const int R = c.fac[s];
-    const int NR = N / R, span = N / (Ns * R);
-    for (int j = threadIdx.x; j < NR; j += blockDim.x) {
-      const int jm = j % Ns;
-      float2 v[16];
-      float2 out[16];
-      if (R <= 16) {
-        for (int r = 0; r < R; ++r) {
-          float2 x = a[j + r * NR];
-          if (r) x = cmul(x, __ldg(tw + ((long long)r * jm * span) % N));
-          v[r] = x;
-        }
-        if (R == 2) {
-          out[0] = make_float2(v[0].x + v[1].x, v[0].y + v[1].y);
-          out[1] = make_float2(v[0].x - v[1].x, v[0].y - v[1].y);
-        } else if (R == 4) {
-          const float2 s0 = make_float2(v[0].x + v[2].x, v[0].y + v[2].y);
-          const float2 d0 = make_float2(v[0].x - v[2].x, v[0].y - v[2].y);
-          const float2 s1 = make_float2(v[1].x + v[3].x, v[1].y + v[3].y);
-          const float2 d1 = make_float2(v[1].x - v[3].x, v[1].y - v[3].y);
-          out[0] = make_float2(s0.x + s1.x, s0.y + s1.y);
-          out[2] = make_float2(s0.x - s1.x, s0.y - s1.y);
-          out[1] = make_float2(d0.x + d1.y, d0.y - d1.x);  // d0 - i d1
-          out[3] = make_float2(d0.x - d1.y, d0.y + d1.x);  // d0 + i d1
-        } else {
-          for (int k = 0; k < R; ++k) {
-            float2 acc = v[0];
-            for (int q = 1; q < R; ++q) {
-              const float2 w = __ldg(tw + ((long long)(N / R) * ((q * k) % R)) % N);
-              const float2 t = cmul(v[q], w);
-              acc.x += t.x;
-              acc.y += t.y;
-            }
-            out[k] = acc;
-          }
-        }
-        const int base = (j / Ns) * Ns * R + jm;
-        for (int r = 0; r < R; ++r) b[base + r * Ns] = out[r];
-      } else {  // large prime radix: generic DFT straight from the input
-        const int base = (j / Ns) * Ns * R + jm;
-        for (int k = 0; k < R; ++k) {
-          float2 acc = make_float2(0, 0);
-          for (int q = 0; q < R; ++q) {
-            float2 x = a[j + q * NR];
-            if (q) x = cmul(x, __ldg(tw + ((long long)q * jm * span) % N));
-            const float2 w = __ldg(tw + ((long long)(N / R) * ((q * k) % R)) % N);
-            const float2 t = cmul(x, w);
-            acc.x += t.x;
-            acc.y += t.y;
-          }
-          b[base + k * Ns] = acc;
-        }
-      }
+    switch (R) {
+      case 2: fft_pass<2>(a, b, c.n, Ns, tw); break;
+      case 3: fft_pass<3>(a, b, c.n, Ns, tw); break;
+      case 4: fft_pass<4>(a, b, c.n, Ns, tw); break;
+      case 5: fft_pass<5>(a, b, c.n, Ns, tw); break;
+      case 7: fft_pass<7>(a, b, c.n, Ns, tw); break;
+      case 8: fft_pass<8>(a, b, c.n, Ns, tw); break;
+      default: fft_pass_prime(a, b, R, c.n, Ns, tw);
     }
     __syncthreads();
     float2 *t = a;
@@ -245,15 +291,15 @@ __global__ void __launch_bounds__(kFftThreads) grid_fft_fwd_kernel(
     const float2 *__restrict__ rows, float *__restrict__ sino, const float2 *__restrict__ tw,
     FftConst c, int na, int npix, int padleft, float inv_pdim, FwdEpi ep) {
   extern __shared__ float2 sm[];
-  float2 *a = sm, *b = sm + c.n;
+  float2 *a = sm, *b = sm + fft_at(c.n) + 1;
   const size_t row = blockIdx.x;  // z * na + n
   const float2 *src = rows + row * c.n;
-  for (int i = threadIdx.x; i < c.n; i += blockDim.x) a[i] = src[i];
+  for (int i = threadIdx.x; i < c.n; i += blockDim.x) a[fft_at(i)] = src[i];
   __syncthreads();
   const float2 *o = stockham(a, b, c, tw);
   double r2 = 0.0;
   for (int k = threadIdx.x; k < npix; k += blockDim.x) {
-    const float acc = __fmul_rn(inv_pdim, o[padleft + k].x);
+    const float acc = __fmul_rn(inv_pdim, o[fft_at(padleft + k)].x);
     const size_t e = row * npix + k;
     float out = acc;
     if (ep.op != EPI_NONE) {
@@ -279,7 +325,7 @@ __global__ void __launch_bounds__(kFftThreads) grid_fft_adj_kernel(
     const float2 *__restrict__ filt, FftConst c, int npix, int padleft, int pdim_h,
     int radon_degree, float tmp2) {
   extern __shared__ float2 sm[];
-  float2 *a = sm, *b = sm + c.n;
+  float2 *a = sm, *b = sm + fft_at(c.n) + 1;
   const size_t row = blockIdx.x;
   const float *src = sino + row * npix;
   const int padright = padleft + npix;
@@ -288,17 +334,17 @@ __global__ void __launch_bounds__(kFftThreads) grid_fft_adj_kernel(
     if (i < padleft) v = radon_degree ? 0.0f : src[0];
     else if (i < padright) v = src[i - padleft];
     else v = radon_degree ? 0.0f : src[npix - 1];
-    a[i] = make_float2(v, 0.0f);
+    a[fft_at(i)] = make_float2(v, 0.0f);
   }
   __syncthreads();
   const float2 *o = stockham(a, b, c, tw);
   float4 *dst = cd + row * pdim_h;
   for (int j = threadIdx.x; j < pdim_h; j += blockDim.x) {
     const float2 f = filt[j];
-    const float2 t2 = make_float2(__fmul_rn(tmp2, o[j].x), __fmul_rn(tmp2, o[j].y));
+    const float2 oj = o[fft_at(j)], t2 = make_float2(__fmul_rn(tmp2, oj.x), __fmul_rn(tmp2, oj.y));
     float4 r;
     if (j != 0) {
-      const float2 t3 = make_float2(__fmul_rn(tmp2, o[c.n - j].x), __fmul_rn(tmp2, o[c.n - j].y));
+      const float2 om = o[fft_at(c.n - j)], t3 = make_float2(__fmul_rn(tmp2, om.x), __fmul_rn(tmp2, om.y));
       r.x = __fmaf_rn(f.x, t3.x, -__fmul_rn(f.y, t3.y));
       r.y = __fmaf_rn(f.x, t3.y, __fmul_rn(f.y, t3.x));
       const float ci = -f.y;
@@ -322,23 +368,23 @@ __global__ void __launch_bounds__(kFftThreads) grid_fft_adj_matched_kernel(
     const float *__restrict__ sino, float4 *__restrict__ cd, const float2 *__restrict__ tw,
     const float2 *__restrict__ filt, FftConst c, int npix, int padleft, int pdim_h, float scale) {
   extern __shared__ float2 sm[];
-  float2 *a = sm, *b = sm + c.n;
+  float2 *a = sm, *b = sm + fft_at(c.n) + 1;
   const size_t row = blockIdx.x;
   const float *src = sino + row * npix;
   for (int i = threadIdx.x; i < c.n; i += blockDim.x) {
     const int k = i - padleft;
-    a[i] = make_float2(k >= 0 && k < npix ? __fmul_rn(scale, src[k]) : 0.0f, 0.0f);
+    a[fft_at(i)] = make_float2(k >= 0 && k < npix ? __fmul_rn(scale, src[k]) : 0.0f, 0.0f);
   }
   __syncthreads();
   const float2 *o = stockham(a, b, c, tw);
   float4 *dst = cd + row * pdim_h;
   for (int w = threadIdx.x; w < pdim_h; w += blockDim.x) {
-    const float2 f = filt[w], d = o[w];                       // rho^[pdim - w] = o[w]
+    const float2 f = filt[w], d = o[fft_at(w)];                       // rho^[pdim - w] = o[w]
     float4 r;
     r.x = __fmaf_rn(f.x, d.x, -__fmul_rn(f.y, d.y));
     r.y = __fmaf_rn(f.x, d.y, __fmul_rn(f.y, d.x));
     if (w != 0) {
-      const float2 m = o[c.n - w];                            // rho^[w] = o[pdim - w]
+      const float2 m = o[fft_at(c.n - w)];                            // rho^[w] = o[pdim - w]
       r.z = __fmaf_rn(f.x, m.x, __fmul_rn(f.y, m.y));        // conj(f) m
       r.w = __fmaf_rn(f.x, m.y, -__fmul_rn(f.y, m.x));
     } else {
@@ -391,126 +437,164 @@ struct GatherArgs {
   const float4 *sc4;      // per angle (sin, cos, 1/cos, 1/sin)
   const float2 *sorted;   // (polar angle, angle index as float bits), ascending
   const float *lut;
+  const int *start;       // [nbuck + 3] first sorted index that an angle of bucket b can have
+  int nbuck;
   int pdim, pdim_h, na, interp, centre;  // centre: half-size of the box done by warps
   float h, tbl;
 };
 
+// The samples whose window holds point (tu, tv): the sum of their direct values,
+// which belongs to that point, and of their mirror values, which belongs to
+// (pdim - tu, pdim - tv).  A point and its mirror point are therefore done
+// together, each window walked once.
+struct Gathered {
+  float2 direct, mirror;
+};
 template <int STRIDE>
-__device__ __forceinline__ void gather_point(const GatherArgs &A, int IU, int IV, size_t z, int lane, float &hr,
-                                             float &hi) {
+__device__ __forceinline__ Gathered gather_window(const GatherArgs &A, int tu, int tv, size_t z, int lane) {
+  Gathered s{make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
   const float4 *cdz = A.cd + z * (size_t)A.na * A.pdim_h;
-  const int pdim = A.pdim, pdim_h = A.pdim_h, na = A.na;
+  const int pdim_h = A.pdim_h, na = A.na;
   const float h = A.h, fph = (float)pdim_h;
   const float reach = h * 1.41421356f + 1.0f;
-  for (int mirror = 0; mirror < 2; ++mirror) {
-    // the window point the sample must contain, and its offset from the centre
-    const int tu = mirror ? pdim - IU : IU, tv = mirror ? pdim - IV : IV;
-    if (mirror && (IU == 0 || IV == 0)) continue;  // targets pdim - 0 are outside the grid
-    const float ftu = (float)tu, ftv = (float)tv;
-    const float du = (float)(tu - pdim_h), dv = (float)(tv - pdim_h);
-    const float rho = sqrtf(du * du + dv * dv);
-    const bool windowed = rho > reach + 1.0f;
-    int a0 = 0;
-    float phi = 0.0f, dmax = 0.0f;
-    if (windowed) {
-      phi = atan2f(dv, du);
-      if (phi < 0.0f) phi += 6.2831853f;
-      dmax = asinf(fminf(1.0f, reach / rho)) + 1e-3f;
-      // first sorted angle >= phi - dmax (with wrap-around)
-      float lo = phi - dmax;
-      if (lo < 0.0f) lo += 6.2831853f;
-      int l = 0, r = na;
-      while (l < r) {
-        const int m = (l + r) >> 1;
-        if (A.sorted[m].x < lo) l = m + 1;
-        else r = m;
-      }
-      a0 = l;
+  const float ftu = (float)tu, ftv = (float)tv;
+  const float du = (float)(tu - pdim_h), dv = (float)(tv - pdim_h);  // offset from the centre
+  const float rho = sqrtf(du * du + dv * dv);
+  if (rho > fph + reach) return s;  // beyond every sample's window
+  const bool windowed = rho > reach + 1.0f;
+  int a0 = 0;
+  float phi = 0.0f, dmax = 0.0f;
+  if (windowed) {
+    phi = atan2f(dv, du);
+    if (phi < 0.0f) phi += 6.2831853f;
+    dmax = asinf(fminf(1.0f, reach / rho)) + 1e-3f;
+    // first sorted angle >= phi - dmax (with wrap-around), between the bounds of
+    // its bucket (a rounding of the bucket's index is covered by one more on each side)
+    float lo = phi - dmax;
+    if (lo < 0.0f) lo += 6.2831853f;
+    const int b = min((int)(lo * ((float)A.nbuck / 6.2831853f)), A.nbuck - 1);
+    int l = __ldg(A.start + b), r = __ldg(A.start + b + 3);
+    while (l < r) {
+      const int m = (l + r) >> 1;
+      if (__ldg(A.sorted + m).x < lo) l = m + 1;
+      else r = m;
     }
-    const float wbase = mirror ? 1.0f : 0.0f;
-    // the in-window angles are a prefix of the cyclic order from a0
-    for (int t = lane; t < na; t += STRIDE) {
-      int si = a0 + t;
-      if (si >= na) si -= na;
-      const float2 e = A.sorted[si];
-      if (windowed) {
-        // Stop once past the window.  The test is looser than the window by
-        // far more than the float rounding of lo = phi - dmax and of e.x - phi:
-        // the search starts at the first angle >= lo, which the exact test
-        // could judge just outside and so end the scan before the window.
-        // Which samples count is decided below, per sample, whatever this.
-        float dphi = fabsf(e.x - phi);
-        dphi = fminf(dphi, 6.2831853f - dphi);
-        if (dphi > dmax + 1e-5f) break;  // left the window
-      }
-      const int n = __float_as_int(e.y);
-      const float4 ang = A.sc4[n];  // SIN, COS, 1/COS, 1/SIN
-      const float SIN = ang.x, COS = ang.y;
-      const float tt = du * COS + dv * SIN;  // along-ray position of the target
-      float lo = tt - reach, hi2 = tt + reach;
-      if (fabsf(COS) >= 1e-2f) {
-        const float a = (du - h) * ang.z, b = (du + h) * ang.z;
-        lo = fmaxf(lo, fminf(a, b) - 1.0f);
-        hi2 = fminf(hi2, fmaxf(a, b) + 1.0f);
-      }
-      if (fabsf(SIN) >= 1e-2f) {
-        const float a = (dv - h) * ang.w, b = (dv + h) * ang.w;
-        lo = fmaxf(lo, fminf(a, b) - 1.0f);
-        hi2 = fminf(hi2, fmaxf(a, b) + 1.0f);
-      }
-      lo = fmaxf(ceilf(lo), wbase);
-      hi2 = fminf(floorf(hi2), (float)(pdim_h - 1));
-      if (lo > hi2) continue;
-      int w = (int)lo;
-      for (float wf = lo; wf <= hi2; wf += 1.0f, ++w) {
-        const float U = __fmaf_rn(COS, wf, fph), V = __fmaf_rn(SIN, wf, fph);
-        const float ua = __fsub_rn(U, h), va = __fsub_rn(V, h);
-        if (ua <= -1.0f || va <= -1.0f) continue;  // the reference skips this sample entirely
-        if (ua > ftu || __fadd_rn(h, U) < ftu || va > ftv || __fadd_rn(V, h) < ftv) continue;
-        const float rt = lut_eval_fast(A.lut, __fmul_rn(fabsf(__fsub_rn(U, ftu)), A.tbl), A.interp);
-        const float wk = lut_eval_fast(A.lut, __fmul_rn(fabsf(__fsub_rn(V, ftv)), A.tbl), A.interp);
-        const float conv = __fmul_rn(rt, wk);
-        const float4 c = cdz[(size_t)n * pdim_h + w];
-        if (!mirror) {
-          hr = __fmaf_rn(conv, c.x, hr);
-          hi = __fmaf_rn(conv, c.y, hi);
-        } else if (tu != 0 && tv != 0 && w != 0) {
-          hr = __fmaf_rn(conv, c.z, hr);
-          hi = __fmaf_rn(conv, c.w, hi);
-        }
+    a0 = l;
+  }
+  // the in-window angles are a prefix of the cyclic order from a0
+  for (int t = lane; t < na; t += STRIDE) {
+    int si = a0 + t;
+    if (si >= na) si -= na;
+    const float2 e = __ldg(A.sorted + si);
+    if (windowed) {
+      // Stop once past the window.  The test is looser than the window by
+      // far more than the float rounding of lo = phi - dmax and of e.x - phi:
+      // the search starts at the first angle >= lo, which the exact test
+      // could judge just outside and so end the scan before the window.
+      // Which samples count is decided below, per sample, whatever this.
+      float dphi = fabsf(e.x - phi);
+      dphi = fminf(dphi, 6.2831853f - dphi);
+      if (dphi > dmax + 1e-5f) break;  // left the window
+    }
+    const int n = __float_as_int(e.y);
+    const float4 ang = __ldg(A.sc4 + n);  // SIN, COS, 1/COS, 1/SIN
+    const float SIN = ang.x, COS = ang.y;
+    const float tt = du * COS + dv * SIN;  // along-ray position of the target
+    float lo = tt - reach, hi2 = tt + reach;
+    if (fabsf(COS) >= 1e-2f) {
+      const float a = (du - h) * ang.z, b = (du + h) * ang.z;
+      lo = fmaxf(lo, fminf(a, b) - 1.0f);
+      hi2 = fminf(hi2, fmaxf(a, b) + 1.0f);
+    }
+    if (fabsf(SIN) >= 1e-2f) {
+      const float a = (dv - h) * ang.w, b = (dv + h) * ang.w;
+      lo = fmaxf(lo, fminf(a, b) - 1.0f);
+      hi2 = fminf(hi2, fmaxf(a, b) + 1.0f);
+    }
+    lo = fmaxf(ceilf(lo), 0.0f);
+    hi2 = fminf(floorf(hi2), (float)(pdim_h - 1));
+    if (lo > hi2) continue;
+    int w = (int)lo;
+    const float4 *c0 = cdz + (size_t)n * pdim_h;
+#pragma unroll 2
+    for (float wf = lo; wf <= hi2; wf += 1.0f, ++w) {
+      const float4 c = __ldg(c0 + w);
+      const float U = __fmaf_rn(COS, wf, fph), V = __fmaf_rn(SIN, wf, fph);
+      const float ua = __fsub_rn(U, h), va = __fsub_rn(V, h);
+      if (ua <= -1.0f || va <= -1.0f) continue;  // the reference skips this sample entirely
+      if (ua > ftu || __fadd_rn(h, U) < ftu || va > ftv || __fadd_rn(V, h) < ftv) continue;
+      const float rt = lut_eval_fast(A.lut, __fmul_rn(fabsf(__fsub_rn(U, ftu)), A.tbl), A.interp);
+      const float wk = lut_eval_fast(A.lut, __fmul_rn(fabsf(__fsub_rn(V, ftv)), A.tbl), A.interp);
+      const float conv = __fmul_rn(rt, wk);
+      s.direct.x = __fmaf_rn(conv, c.x, s.direct.x);
+      s.direct.y = __fmaf_rn(conv, c.y, s.direct.y);
+      if (w != 0) {
+        s.mirror.x = __fmaf_rn(conv, c.z, s.mirror.x);
+        s.mirror.y = __fmaf_rn(conv, c.w, s.mirror.y);
       }
     }
   }
+  return s;
 }
 
-// One thread per Cartesian point outside the central box.
+__device__ __forceinline__ float2 gather_sum(float2 direct, float2 mirror) {
+  return make_float2(__fadd_rn(direct.x, mirror.x), __fadd_rn(direct.y, mirror.y));
+}
+
+// One thread per Cartesian point outside the central box and its mirror point
+// (points of row 0 and column 0 have none: targets pdim - 0 are outside the
+// grid).  4096^2, 1500 angles: 0.98 ms a thread per point, which walked the
+// point's window and the mirror point's and searched all angles for each; now
+// 0.52, bound by the issue of the samples' tests and weights.
 __global__ void __launch_bounds__(128) grid_gather_kernel(GatherArgs A) {
   const int IV = blockIdx.x * blockDim.x + threadIdx.x;
-  const int IU = blockIdx.y;
+  const int IU = blockIdx.y;  // 0 .. pdim / 2
   const size_t z = blockIdx.z;
-  if (IV >= A.pdim) return;
-  if (abs(IU - A.pdim_h) <= A.centre && abs(IV - A.pdim_h) <= A.centre) return;  // grid_gather_centre_kernel
-  float hr = 0.0f, hi = 0.0f;
-  gather_point<1>(A, IU, IV, z, 0, hr, hi);
-  A.H[z * (size_t)A.pdim * A.pdim + (size_t)IU * A.pdim + IV] = make_float2(hr, hi);
+  const int pdim = A.pdim, pdim_h = A.pdim_h;
+  if (IV >= pdim) return;
+  if (abs(IU - pdim_h) <= A.centre && abs(IV - pdim_h) <= A.centre) return;  // grid_gather_centre_kernel
+  float2 *H = A.H + z * (size_t)pdim * pdim;
+  if (IU == 0 || IV == 0) {
+    H[(size_t)IU * pdim + IV] = gather_window<1>(A, IU, IV, z, 0).direct;
+    if (IU > 0 && IU < pdim_h) H[(size_t)(pdim - IU) * pdim] = gather_window<1>(A, pdim - IU, 0, z, 0).direct;
+    return;
+  }
+  if (IU == pdim_h && IV > pdim_h) return;
+  const Gathered p = gather_window<1>(A, IU, IV, z, 0), q = gather_window<1>(A, pdim - IU, pdim - IV, z, 0);
+  H[(size_t)IU * pdim + IV] = gather_sum(p.direct, q.mirror);
+  H[(size_t)(pdim - IU) * pdim + (pdim - IV)] = gather_sum(q.direct, p.mirror);
 }
 
-// One warp per point of the central box, where every angle's first samples
-// overlap and a point gathers thousands of them: lanes take every 32nd angle
-// and the partial sums are combined by a fixed butterfly (deterministic).
+// One block per point of the central box and its mirror point: every angle's
+// first samples overlap there and a point gathers thousands of them, so threads
+// take every 128th angle and the partial sums are combined by a fixed butterfly
+// and then warp after warp (deterministic).  A warp per pair is one wave of
+// long chains: 110 us at 4096^2, 1500 angles; a block 46.
 __global__ void __launch_bounds__(128) grid_gather_centre_kernel(GatherArgs A) {
-  const int side = 2 * A.centre + 1;
-  const int p = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  __shared__ float4 part[4];
+  const int side = 2 * A.centre + 1, p = blockIdx.x;
   const size_t z = blockIdx.y;
-  if (p >= side * side) return;  // warp-uniform
   const int IU = A.pdim_h - A.centre + p / side, IV = A.pdim_h - A.centre + p % side;
-  float hr = 0.0f, hi = 0.0f;
-  gather_point<32>(A, IU, IV, z, lane, hr, hi);
+  const int MU = A.pdim - IU, MV = A.pdim - IV;
+  const Gathered s = gather_window<128>(A, IU, IV, z, threadIdx.x), m = gather_window<128>(A, MU, MV, z, threadIdx.x);
+  float2 a = gather_sum(s.direct, m.mirror), b = gather_sum(m.direct, s.mirror);
   for (int off = 16; off; off >>= 1) {
-    hr = __fadd_rn(hr, __shfl_xor_sync(0xffffffffu, hr, off));
-    hi = __fadd_rn(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+    a.x = __fadd_rn(a.x, __shfl_xor_sync(0xffffffffu, a.x, off));
+    a.y = __fadd_rn(a.y, __shfl_xor_sync(0xffffffffu, a.y, off));
+    b.x = __fadd_rn(b.x, __shfl_xor_sync(0xffffffffu, b.x, off));
+    b.y = __fadd_rn(b.y, __shfl_xor_sync(0xffffffffu, b.y, off));
   }
-  if (lane == 0) A.H[z * (size_t)A.pdim * A.pdim + (size_t)IU * A.pdim + IV] = make_float2(hr, hi);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = make_float4(a.x, a.y, b.x, b.y);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 4; ++w) {
+      a = gather_sum(a, make_float2(part[w].x, part[w].y));
+      b = gather_sum(b, make_float2(part[w].z, part[w].w));
+    }
+    float2 *H = A.H + z * (size_t)A.pdim * A.pdim;
+    H[(size_t)IU * A.pdim + IV] = a;
+    H[(size_t)MU * A.pdim + MV] = b;
+  }
 }
 
 // Adjoint step 4: deapodise, crop and flip (gridrec_v4_backproj.c:440-491).
@@ -535,6 +619,7 @@ __global__ void __launch_bounds__(256) grid_extract_kernel(const float2 *__restr
 // ---- host helpers ----
 std::vector<int> factorize(int n) {
   std::vector<int> f;
+  while (n % 8 == 0) { f.push_back(8); n /= 8; }
   while (n % 4 == 0) { f.push_back(4); n /= 4; }
   while (n % 2 == 0) { f.push_back(2); n /= 2; }
   for (int p = 3; n > 1; p += 2)
@@ -655,6 +740,7 @@ static void grid_free(void *ext) {
   cudaFree(g->filt_b);
   cudaFree(g->tw);
   cudaFree(g->sorted);
+  cudaFree(g->start);
   cudaFree(g->sc4);
   cudaFree(g->H);
   cudaFree(g->rows);
@@ -726,6 +812,15 @@ int grid_setup(Plan &p) {
     std::memcpy(&idx, &order[n].second, sizeof(int));
     sorted[n] = make_float2(order[n].first, idx);
   }
+  // start[b] = first sorted angle >= the lower end of bucket b - 1 (b = 0: 0)
+  g->nbuck = 64;
+  while (g->nbuck < 2 * na && g->nbuck < (1 << 20)) g->nbuck *= 2;
+  std::vector<int> start(g->nbuck + 3);
+  for (int b = 0, i = 0; b < g->nbuck + 3; ++b) {
+    const double end = (b - 1) * (6.283185307179586 / g->nbuck);
+    while (i < na && b <= g->nbuck && sorted[i].x < end) ++i;
+    start[b] = b > g->nbuck ? na : i;
+  }
   // forward centring filter (gridrec_v4_forwproj.c:182-205)
   float ctr_f = (float)(npix * 0.5);
   if (pdim != npix) ctr_f += (float)g->padleft;
@@ -760,6 +855,7 @@ int grid_setup(Plan &p) {
   if ((rc = up((void **)&g->deapod, G.grid_deapod, sizeof(float) * (size_t)pdim * pdim))) return rc;
   if ((rc = up((void **)&g->sc, sc.data(), sizeof(float2) * na))) return rc;
   if ((rc = up((void **)&g->sorted, sorted.data(), sizeof(float2) * na))) return rc;
+  if ((rc = up((void **)&g->start, start.data(), sizeof(int) * start.size()))) return rc;
   if ((rc = up((void **)&g->sc4, sc4.data(), sizeof(float4) * na))) return rc;
   if ((rc = up((void **)&g->filt_f, ff.data(), sizeof(float2) * ff.size()))) return rc;
   if ((rc = up((void **)&g->filt_b, fb.data(), sizeof(float2) * fb.size()))) return rc;
@@ -772,7 +868,7 @@ int grid_setup(Plan &p) {
       CUFFT_SUCCESS)
     return fail(TOMO_ECUDA, "grid: cufftPlanMany failed");
   g->have_fft = true;
-  const int smem = (int)(2 * sizeof(float2) * pdim);
+  const int smem = (int)fft_smem(pdim);
   TOMO_CUDA(cudaFuncSetAttribute(grid_fft_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   TOMO_CUDA(cudaFuncSetAttribute(grid_fft_adj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   TOMO_CUDA(cudaFuncSetAttribute(grid_fft_adj_matched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -799,7 +895,7 @@ int grid_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, con
   dim3 pb(128), pg((g.pdim_h + 127) / 128, na, nz);
   grid_polar_kernel<<<pg, pb, 0, s>>>(g.H, g.rows, g.sc, g.filt_f, g.lut, pdim, g.pdim_h, na, g.h_f,
                                       g.tbl_f, g.interp);
-  const int smem = (int)(2 * sizeof(float2) * pdim);
+  const int smem = (int)fft_smem(pdim);
   grid_fft_fwd_kernel<<<na * nz, kFftThreads, smem, s>>>(g.rows, d_sino, g.tw, fft_const(g), na, npix,
                                                          g.padleft, g.inv_pdim, ep);
   TOMO_CUDA(cudaGetLastError());
@@ -809,7 +905,7 @@ int grid_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, con
 int grid_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const AdjEpi &ep) {
   GridState &g = *(GridState *)p.ext;
   const int npix = p.g.n, na = p.g.na, nz = p.g.nz, pdim = g.pdim;
-  const int smem = (int)(2 * sizeof(float2) * pdim);
+  const int smem = (int)fft_smem(pdim);
   if (g.matched)
     grid_fft_adj_matched_kernel<<<na * nz, kFftThreads, smem, s>>>(d_sino, g.cd, g.tw, g.filt_f, fft_const(g),
                                                                    npix, g.padleft, g.pdim_h, g.inv_pdim);
@@ -817,12 +913,12 @@ int grid_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, con
     grid_fft_adj_kernel<<<na * nz, kFftThreads, smem, s>>>(d_sino, g.cd, g.tw, g.filt_b, fft_const(g), npix,
                                                            g.padleft, g.pdim_h, g.radon_degree,
                                                            (float)(1.0 / pdim));
-  GatherArgs ga{g.cd, g.H, g.sc4, g.sorted, g.lut, pdim, g.pdim_h, na, g.interp, 0,
+  GatherArgs ga{g.cd, g.H, g.sc4, g.sorted, g.lut, g.start, g.nbuck, pdim, g.pdim_h, na, g.interp, 0,
                 g.matched ? g.h_f : g.h_b, g.matched ? g.tbl_f : g.tbl_b};
   ga.centre = std::min(kGatherCentre, g.pdim_h - 1);
   const int side = 2 * ga.centre + 1;
-  grid_gather_centre_kernel<<<dim3((side * side + 3) / 4, nz), 128, 0, s>>>(ga);
-  dim3 gb(128), gg((pdim + 127) / 128, pdim, nz);
+  grid_gather_centre_kernel<<<dim3(side * side / 2 + 1, nz), 128, 0, s>>>(ga);
+  dim3 gb(128), gg((pdim + 127) / 128, g.pdim_h + 1, nz);
   grid_gather_kernel<<<gg, gb, 0, s>>>(ga);
   if (cufftSetStream(g.fft2, s) != CUFFT_SUCCESS ||
       cufftExecC2C(g.fft2, (cufftComplex *)g.H, (cufftComplex *)g.H, g.matched ? CUFFT_FORWARD : CUFFT_INVERSE) !=
