@@ -8,8 +8,8 @@
 // by 10 dy + dx, with 8-row groups one patch row apart, so nine descriptors
 // read all nine taps from the one copy.
 //
-// A persistent CTA per SM, warps by role: one stages patches, one weights, one
-// issues the MMAs, two sets of four run the epilogue, each out of its own one
+// A persistent CTA per SM, warps by role: one stages patches, one weights, one or
+// two issue the MMAs, two sets of four run the epilogue, each out of its own one
 // of two TMEM accumulator sets.  Weights that fit beside three patches stay in
 // shared memory for all of a CTA's tiles; others stream through a ring, and
 // then two M tiles share each stage where their patches fit: a 128-pixel tile
@@ -20,7 +20,7 @@
 // launch, so a layer's result does not depend on it (above 384 channels the
 // channels are taken 384 at a time).
 //
-// Measured, 4 images: 32 -> 32 channels at 768^2 0.99 -> 0.144 ms, 128 -> 128
+// Measured, 4 images: 32 -> 32 channels at 768^2 0.99 -> 0.132 ms, 128 -> 128
 // at 192^2 0.45 -> 0.049 ms (895 TFLOP/s), 256 -> 256 at 96^2 0.32 -> 0.046 ms.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -38,7 +38,7 @@ constexpr int kTW = 8, kTH = 16;             // output pixels of an M tile
 constexpr int kPW = kTW + 2, kPH = kTH + 2;  // its input patch
 constexpr int kPatch = kPW * kPH;
 constexpr int kEpiWarps = 8;                 // two sets of four
-constexpr int kConvThreads = (kEpiWarps + 3) * 32;
+constexpr int kConvThreads = (kEpiWarps + 4) * 32;
 constexpr int kMaxSlots = 8, kMaxW = 8;
 constexpr int kMaxPass = 384;                // channels of a patch
 constexpr int kSms = 148;
@@ -57,6 +57,7 @@ struct ConvArgs {
   FastDiv ftx, fty;         // tiles of a row, rows of tiles of an image
   int NB, BN;               // output-channel blocks and their width
   int T, NS, NW, resident;  // tiles per group, patch slots, weight stages
+  int issuers;              // warps that issue MMAs
   int npass, cpp;           // channel passes, channels per pass
   int rb, chb, kch;         // bytes of a row, its channels, channels of a weight stage (chb, or 16 when rows hold 8)
   int nblk, wblks, kblk16;  // channel blocks of a pass, weight blocks of a stage, bytes / 16 from a stage's patch block to the next
@@ -72,7 +73,7 @@ template <int KS, bool RES>
 __global__ void __launch_bounds__(kConvThreads, 1) conv_tc_kernel(ConvArgs g, const __grid_constant__ CUtensorMap mx,
                                                                   const __grid_constant__ CUtensorMap mw) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t pfull[kMaxSlots], pempty[kMaxSlots], wfull[kMaxW], wempty[kMaxW], afull[2], aempty[2], done;
+  __shared__ uint64_t pfull[kMaxSlots], pempty[kMaxSlots], wfull[kMaxW], wempty[kMaxW], afull[2], aempty[2], done[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int gave_up;
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // swizzle period
@@ -101,7 +102,8 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_tc_kernel(ConvArgs g, co
       mbar_init(smem_u32(&afull[s]), 1);
       mbar_init(smem_u32(&aempty[s]), 128);
     }
-    mbar_init(smem_u32(&done), 1);
+    mbar_init(smem_u32(&done[0]), 1);
+    mbar_init(smem_u32(&done[1]), 1);
     gave_up = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -239,7 +241,8 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_tc_kernel(ConvArgs g, co
           if (!mbar_wait(smem_u32(&wfull[k % g.NW]), (k / g.NW) & 1, kDrainSpins)) ok = false;
       }
     }
-  } else {  // MMAs
+  } else if (warp - (kEpiWarps + 2) < g.issuers) {  // MMAs; of two warps each takes every other tile
+    const int step = RES ? g.issuers : 1, me = warp - (kEpiWarps + 2);
     const uint32_t idesc = instr_desc(g.BN);
     // descriptors of address 0; rows of 16 bytes hold 8 k, and the other 8 of
     // an MMA lie in the next block
@@ -247,10 +250,15 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_tc_kernel(ConvArgs g, co
     const uint64_t dw0 = smem_desc_rb(0, g.rb == 16 ? g.wblk : 16, 8 * g.rb, g.rb);
     Ring pr, wr, ar;  // patch slots, weight stages, accumulator sets
     bool issued = false;
-    for (int grp = grp0; grp < g.ngroups && ok; grp += gstep, ar.next(2)) {
+    if (me == 1) {
+      pr.next(g.NS);
+      ar.next(2);
+    }
+    const int first = grp0 + me * gstep;
+    for (int grp = first; grp < g.ngroups && ok; grp += step * gstep) {
       const int tc = min(g.T, g.ntiles - grp * g.T);
       if (grp >= grp0 + 2 * gstep) ok = warp_wait(&aempty[ar.s], ar.ph ^ 1u, g.spins, &gave_up);
-      if (ok && g.resident && grp == grp0) ok = warp_wait(&wfull[0], 0, g.spins, &gave_up);
+      if (ok && g.resident && grp == first) ok = warp_wait(&wfull[0], 0, g.spins, &gave_up);
       const uint32_t acc = tmem + (uint32_t)(ar.s * g.T * g.BN);
       for (int p = 0; p < g.npass && ok; ++p) {
         Ring slot[2];
@@ -313,11 +321,16 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_tc_kernel(ConvArgs g, co
         if (tc > 1) mma_commit_warp(smem_u32(&pempty[slot[1].s]));
       }
       if (ok) mma_commit_warp(smem_u32(&afull[ar.s]));
+      ar.next(2);
+      if (step == 2) {  // the other warp's tile
+        pr.next(g.NS);
+        ar.next(2);
+      }
     }
     // every MMA issued so far, also on the way out of a wait that gave up
     if (issued) {
-      mma_commit_warp(smem_u32(&done));
-      if (!mbar_wait(smem_u32(&done), 0, kDrainSpins)) ok = false;
+      mma_commit_warp(smem_u32(&done[me]));
+      if (!mbar_wait(smem_u32(&done[me]), 0, kDrainSpins)) ok = false;
     }
   }
   if (!ok) atomicOr(&gave_up, 1);
@@ -381,7 +394,12 @@ int conv_launch(const __nv_bfloat16 *X, int batch, int H, int W, int Cin, const 
     g.T = 1;
     g.NW = 1;
     g.NS = std::min(kMaxSlots, (budget - wres) / g.slot_bytes);
+    // MMAs of 32 columns end faster than one warp issues them; wider ones lose by
+    // being mixed (4 x 768^2, 32 -> 32: 148 us with one warp, 132 with two; 32 -> 96:
+    // 182, 246; 8 -> 32: 83, 87)
+    g.issuers = g.BN <= 32 && Cin > 8 ? 2 : 1;
   } else {
+    g.issuers = 1;
     // two tiles to a weight stage, once there are two for every SM
     g.T = g.npass == 1 && 2 * g.slot_bytes + 2 * g.stage_bytes <= budget && (long long)g.ntiles * g.NB >= 2 * kSms ? 2 : 1;
     g.NS = std::min(2 * g.T, (budget - 2 * g.stage_bytes) / g.slot_bytes);
