@@ -426,20 +426,10 @@ __global__ void __launch_bounds__(kWgThreads) wgrad_gather_kernel(WgradArgs g) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(g.cols));
 }
 
-// dW[i] = sum_s part[s][i], s ascending (part is [S][n]).
-__global__ void wgrad_reduce_kernel(const float *__restrict__ part, int S, size_t n, float *__restrict__ dW) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float acc = 0.0f;
-#pragma unroll 8
-  for (int s = 0; s < S; ++s) acc += __ldg(part + (size_t)s * n + i);
-  dW[i] = acc;
-}
-
 // Bias gradient: block b sums its range of pixels of dY [P][C] per channel.  A
 // thread takes 8 channels of every (threads / (C/8))-th pixel, 16 of them in float
 // (8 significant bits each) and those sums in double; the block's threads and
-// then the blocks (colsum_final_kernel) are added in order.
+// then the blocks (wgrad_reduce_kernel) are added in order.
 constexpr int kColThreads = 256, kColBlocks = 592;
 
 __global__ void __launch_bounds__(kColThreads) colsum_kernel(const __nv_bfloat16 *__restrict__ Y, long long P, int C,
@@ -454,7 +444,7 @@ __global__ void __launch_bounds__(kColThreads) colsum_kernel(const __nv_bfloat16
     if (r < rows) {
       for (long long p = p0 + r; p < p1; p += 16 * rows) {  // 16 pixels in float, then double
         float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll 4
+#pragma unroll 8
         for (int k = 0; k < 16; ++k) {
           const long long q = p + (long long)k * rows;
           if (q < p1) {
@@ -483,15 +473,28 @@ __global__ void __launch_bounds__(kColThreads) colsum_kernel(const __nv_bfloat16
   }
 }
 
-// db[c] = sum over blocks of part[b][c]: a warp per channel, lanes 32 blocks
-// apart, then a fixed butterfly (one thread per channel was a chain of 592
-// loads, 32 us).
-__global__ void __launch_bounds__(128) colsum_final_kernel(const double *__restrict__ part, int nblk, int C, int ld,
+// dW[i] = sum_s part[s][i], s ascending (part is [S][n]), in the first nw blocks;
+// the others take db[c] = sum over blocks b of cpart[b][c], a warp per channel,
+// lanes 32 blocks apart, then a fixed butterfly (one thread per channel was a
+// chain of 592 loads, 32 us).
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restrict__ part, int S, size_t n,
+                                                           float *__restrict__ dW, int nw,
+                                                           const double *__restrict__ cpart, int nblk, int C, int ld,
                                                            float *__restrict__ db) {
-  const int c = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if ((int)blockIdx.x < nw) {
+    const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    float acc = 0.0f;
+#pragma unroll 8
+    for (int s = 0; s < S; ++s) acc += __ldg(part + (size_t)s * n + i);
+    dW[i] = acc;
+    return;
+  }
+  const int c = (blockIdx.x - nw) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (c >= C) return;  // warp-uniform
   double s = 0.0;
-  for (int b = lane; b < nblk; b += 32) s += part[(size_t)b * ld + c];
+#pragma unroll 4
+  for (int b = lane; b < nblk; b += 32) s += __ldg(cpart + (size_t)b * ld + c);
   for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) db[c] = (float)s;
 }
@@ -675,13 +678,10 @@ int wgrad_launch(const __nv_bfloat16 *X, const __nv_bfloat16 *dY, int batch, int
     fn<<<dim3(MB * g.NB * g.G, g.S), kWgThreads, smem, s>>>(g);
   }
   const size_t nout = (size_t)taps * Cin * Cout;
-  wgrad_reduce_kernel<<<(unsigned)((nout + 255) / 256), 256, 0, s>>>(g.part, g.S, nout, dW);
-  if (db) {
-    double *cp = (double *)(w + ww.colsum);
-    const int nblk = (int)std::min<long long>(kColBlocks, std::max<long long>(1, P / 64));
-    colsum_kernel<<<nblk, kColThreads, 0, s>>>(dY, P, g.ldY, cp);
-    colsum_final_kernel<<<(Cout + 3) / 4, 128, 0, s>>>(cp, nblk, Cout, g.ldY, db);
-  }
+  double *cp = (double *)(w + ww.colsum);
+  const int nblk = (int)std::min<long long>(kColBlocks, std::max<long long>(1, P / 64)), nw = (int)((nout + 255) / 256);
+  if (db) colsum_kernel<<<nblk, kColThreads, 0, s>>>(dY, P, g.ldY, cp);
+  wgrad_reduce_kernel<<<nw + (db ? (Cout + 7) / 8 : 0), 256, 0, s>>>(g.part, g.S, nout, dW, nw, cp, nblk, Cout, g.ldY, db);
   return cudaGetLastError() == cudaSuccess ? NN_OK : NN_ECUDA;
 }
 
