@@ -28,7 +28,7 @@
 //            for pixels straddling a binade of P (|P| = 2^e), whose width
 //            differs by a rounding of q: those are added per line, and the
 //            dropped last piece of every line is subtracted, by a kernel of
-//            their own (dd_fwd_corr_kernel) into a float row per angle that
+//            their own (dd_fwd_corr) into a float row per angle that
 //            the forward adds where it stores.  Angles whose coordinates
 //            reach 2^22 walk the pieces instead (dd_fwd_exact).
 //   adjoint  a pixel is at most one detector wide (r >= 1), so it overlaps the
@@ -36,16 +36,17 @@
 //            float gaps, as the reference forms them, from one 8-byte table
 //            entry {S_a, S_a+1} per angle and the boundary D_a+1 recomputed.
 // The dropped last piece is subtracted where it falls (dd_dropped_piece):
-// forward in dd_fwd_corr_kernel, adjoint in the pixel loop.
+// forward in dd_fwd_corr, adjoint in dd_adj_drop.
 //
 // Work is described by a table of instances (one per slice, or per geometry
-// of an uneven batch) and consumed by persistent kernels: each warp takes the
-// next work item (forward: 127 detectors of one angle; adjoint: a 16x8 pixel
-// tile over all angles) from a device counter, finds its instance by binary
-// search and runs it.  Every output element is owned by one lane and its sum
-// order is fixed, so results do not depend on scheduling and are
-// deterministic.  Warps per block and the fetch mode are chosen per plan by timing the
-// candidates (dd_autotune).  The projection arithmetic of the solvers
+// of an uneven batch).  An item (forward: 127 detectors of one angle; adjoint: a
+// tile of 32 x 16 or 32 x 4 pixels over all angles) finds its instance by binary
+// search; the adjoint's kernel is persistent and takes the next items from a
+// device counter, the forward's either that or a block per item.  Every output
+// element is owned by one lane and its sum order is fixed, so results do not
+// depend on scheduling and are deterministic.  The shapes of the launches are
+// chosen per plan by timing the candidates (dd_autotune).  The projection
+// arithmetic of the solvers
 // (epilogue.cuh) is applied where the result is stored.
 #include <algorithm>
 #include <climits>
@@ -384,7 +385,7 @@ __device__ __forceinline__ void dd_sino_expand(long long b, const DdInst *__rest
 // Forward: an item is 127 detectors of one angle; lane l holds the lower
 // boundaries of detectors B0 + 32 j + l (j = 0..3), and T_j = sum over lines of
 // F(boundary).  The dropped pieces and the binade corrections come from
-// dd_fwd_corr_kernel's row; keeping them out of this loop leaves it 64
+// dd_fwd_corr's row; keeping them out of this loop leaves it 64
 // registers (with them inline: 76, and 24 instead of 32 warps per SM).
 // ---------------------------------------------------------------------------
 template <int J>
@@ -469,36 +470,44 @@ __device__ __forceinline__ bool dd_fwd_crossing(const float *__restrict__ V, int
   }
 #pragma unroll
   for (int t = 0; t < 4; ++t) a[t] = 0.0;
-#pragma unroll 1
+  // Without branches, so that the lines of an unrolled step overlap (with loops
+  // and early ends each waited for its pixel: all pre-passes at 768^2 x 720 57 us,
+  // now 49; 2048^2 x 1800 245, 227).  lo[t] = D + nh of detectors mc - 1 .. mc + 3.
+  float lo[5];
+#pragma unroll
+  for (int t = 0; t < 5; ++t) lo[t] = __fadd_rn(det_bound(mc - 1 + t, nh, r), fnh);
+#pragma unroll 4
   for (int i = ia + lane; i <= ib; i += 32) {
     const float q = __fmul_rn(__fadd_rn((float)(i - nh), 0.5f), k);
-    int j = (int)floor((double)B + (double)q) + nh - 1;
-    // j with P_j < B <= P_j+1 (B > 0) or P_j <= B < P_j+1 (B < 0)
-    if (!sg) {
-      for (int it = 0; it < 4 && pix_bound(j, nh, q) >= B; ++it) --j;
-      for (int it = 0; it < 4 && pix_bound(j + 1, nh, q) < B; ++it) ++j;
-    } else {
-      for (int it = 0; it < 4 && pix_bound(j, nh, q) > B; ++it) --j;
-      for (int it = 0; it < 4 && pix_bound(j + 1, nh, q) <= B; ++it) ++j;
+    // x = j - nh with P_j < B <= P_j+1 (B > 0) or P_j <= B < P_j+1 (B < 0), P_j =
+    // RN(x - q): floor(B + q) - 1 or one of its neighbours, P's rounding being 1/4
+    // at most; steps of 1 are exact in float
+    float x = floorf(__fadd_rn(B, q)) - 1.0f;
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+      const float P = __fsub_rn(x, q);
+      if (sg ? P > B : P >= B) x -= 1.0f;
     }
-    if (j < 0 || j >= n) continue;
-    const float Pj = pix_bound(j, nh, q), Pj1 = pix_bound(j + 1, nh, q);
+#pragma unroll
+    for (int it = 0; it < 3; ++it) {
+      const float P = __fsub_rn(x + 1.0f, q);
+      if (sg ? P <= B : P < B) x += 1.0f;
+    }
+    const int j = (int)x + nh;
+    const float Pj = __fsub_rn(x, q), Pj1 = __fsub_rn(x + 1.0f, q);
     const bool at = sg ? (Pj <= B && B < Pj1 && (e == 0 || Pj1 <= 0.5f * B))
                        : (Pj < B && B <= Pj1 && (e == 0 || Pj >= 0.5f * B));
-    if (!at) continue;
     const float delta = __fsub_rn(__fsub_rn(Pj1, Pj), 1.0f);
-    if (delta == 0.0f) continue;
-    // the detector m with kk_m <= j < kk_m+1, among mc-1 .. mc+2
-    int m = mc;
-    for (int it = 0; it < 4; ++it) {
-      if (dd_fwd_kk(__fadd_rn(det_bound(m, nh, r), fnh), q, nlim) > j) --m;
-      else if (dd_fwd_kk(__fadd_rn(det_bound(m + 1, nh, r), fnh), q, nlim) <= j) ++m;
-      else break;
-    }
-    const double amt = (double)delta * (double)__ldg(V + (size_t)i * si + (size_t)j * sj);
+    const bool use = at && j >= 0 && j < n && delta != 0.0f;
+    // the detector m with kk_m <= j < kk_m+1, among mc-1 .. mc+2: how many kk <= j
+    int m = -1;
+#pragma unroll
+    for (int t = 0; t < 5; ++t) m += dd_fwd_kk(lo[t], q, nlim) <= j ? 1 : 0;
+    const float v = use ? __ldg(V + (size_t)i * si + (size_t)j * sj) : 0.0f;
+    const double amt = (double)delta * (double)v;
 #pragma unroll
     for (int t = 0; t < 4; ++t)
-      if (m == mc - 1 + t) a[t] += amt;
+      if (use && m == t) a[t] += amt;
   }
 #pragma unroll
   for (int t = 0; t < 4; ++t)
