@@ -3,10 +3,10 @@
 The network maps a cheap reconstruction (2 SIRT iterations) to a start close
 to the converged SIRT result; the plain solver then continues from it.  All
 convolutions -- forward, input gradient and weight gradient -- are the
-hand-written tcgen05 BF16 kernels of ``libtomo_nn.so`` (``csrc/nn_gemm.cu``,
-``csrc/nn_ops.cu``) with FP32 accumulation and FP32 master weights; pooling,
-upsampling and concatenation are layout operations left to torch.  Activations
-are BF16 NHWC.
+hand-written tcgen05 BF16 kernels of ``libtomo_nn.so`` (``csrc/nn_conv.cu``,
+``csrc/nn_wgrad.cu``, ``csrc/nn_gemm.cu``) with FP32 accumulation and FP32 master
+weights; pooling, upsampling beside the skip connection and their gradients are
+passes of its own (``csrc/nn_resample.cu``).  Activations are BF16 NHWC.
 
 Layers (``UNet(levels=4, base=32)``): per level two 3x3 convolutions + ReLU,
 2x2 max-pooling down, nearest 2x upsampling up with the skip connection
