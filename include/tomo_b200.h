@@ -29,6 +29,8 @@
  *
  * Thread safety: a plan may be used from one host thread at a time; distinct
  * plans are independent.  The drop-in entry points serialise internally.
+ * Streams: calls of one plan may come on any streams, also captured ones; they
+ * share the plan's buffers, so each waits for the one enqueued before it.
  */
 #ifndef TOMO_B200_H
 #define TOMO_B200_H

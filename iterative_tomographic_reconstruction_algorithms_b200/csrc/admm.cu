@@ -604,7 +604,8 @@ int tomo_admm_create(tomo_plan *plan, int reg, const float *d_b, const tomo_admm
   V.atb = A.atb;
   V.q = A.q;
   // A^T b once (every CG start uses it)
-  int rc = plan_adjoint(p, d_b, A.atb, st, AdjEpi());
+  PlanUse use(p, st);
+  int rc = use.end(use.error() ? use.error() : plan_adjoint(p, d_b, A.atb, st, AdjEpi()));
   if (rc) {
     admm_free(A);
     delete h;
@@ -627,6 +628,8 @@ int tomo_admm_run(tomo_admm *h, float *d_x, int iters, int reset, double *stats,
   cudaStream_t caller = (cudaStream_t)stream, st = A.own;
   TOMO_CUDA(cudaEventRecord(A.ev_in, caller));
   TOMO_CUDA(cudaStreamWaitEvent(st, A.ev_in, 0));
+  PlanUse use(*A.p, st);
+  if (use.error()) return use.error();
   TOMO_CUDA(cudaMemsetAsync(A.counter, 0, sizeof(int), st));
   A.V.x = d_x;
   const size_t ni = image_elems(*A.p);
@@ -671,6 +674,7 @@ int tomo_admm_run(tomo_admm *h, float *d_x, int iters, int reset, double *stats,
       if (rc) return rc;
     }
   }
+  if (int rc = use.end(TOMO_OK)) return rc;
   TOMO_CUDA(cudaEventRecord(A.ev_out, st));
   TOMO_CUDA(cudaStreamWaitEvent(caller, A.ev_out, 0));
   if (stats && iters > 0) {

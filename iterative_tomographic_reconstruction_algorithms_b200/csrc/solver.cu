@@ -210,6 +210,8 @@ int tomo_solver_create(tomo_plan *plan, int algo, const float *d_b, void *stream
   FwdEpi plain_f;
   AdjEpi plain_a;
   plain_f.ordered = plain_a.ordered = true;
+  PlanUse use(p, st);
+  if ((rc = use.error())) return bail(rc);
   fill_kernel<<<grid_for(ni), 256, 0, st>>>(ones_i, ni, 1.0f);
   fill_kernel<<<grid_for(ns), 256, 0, st>>>(ones_s, ns, 1.0f);
   if (algo == TOMO_ALGO_SIRT) {
@@ -231,6 +233,7 @@ int tomo_solver_create(tomo_plan *plan, int algo, const float *d_b, void *stream
     if ((rc = plan_adjoint(p, S.y, S.aux_a, st, plain_a))) return bail(rc);
   }
   SOLVER_CUDA(cudaGetLastError());
+  if ((rc = use.end(rc))) return bail(rc);
   SOLVER_CUDA(cudaStreamSynchronize(st));
   cudaFree(ones_i);
   cudaFree(ones_s);
@@ -249,6 +252,8 @@ int tomo_solver_run(tomo_solver *solver, float *d_x, int iters, double *residual
   // order the solver's stream after the caller's work, and the caller's after ours
   TOMO_CUDA(cudaEventRecord(S.ev_in, caller));
   TOMO_CUDA(cudaStreamWaitEvent(st, S.ev_in, 0));
+  PlanUse use(*S.p, st);
+  if (use.error()) return use.error();
   TOMO_CUDA(cudaMemsetAsync(S.counter, 0, sizeof(int), st));
   if (use_graph && iters > 0) {
     if (!S.exec || S.graph_x != d_x) {
@@ -277,6 +282,7 @@ int tomo_solver_run(tomo_solver *solver, float *d_x, int iters, double *residual
       if (rc) return rc;
     }
   }
+  if (int rc = use.end(TOMO_OK)) return rc;
   TOMO_CUDA(cudaEventRecord(S.ev_out, st));
   TOMO_CUDA(cudaStreamWaitEvent(caller, S.ev_out, 0));
   if (residuals && iters > 0) {

@@ -45,6 +45,9 @@ static void release(Plan &p) {
   if (p.d_in) cudaFree(p.d_in);
   if (p.d_out) cudaFree(p.d_out);
   if (p.host_stream) cudaStreamDestroy(p.host_stream);
+  if (p.used) cudaEventDestroy(p.used);
+  if (p.used_capture) cudaEventDestroy(p.used_capture);
+  p.used = p.used_capture = nullptr;
   if (p.h_stage) cudaFreeHost(p.h_stage);
   for (cudaEvent_t e : p.stage_events) cudaEventDestroy(e);
   p.stage_events.clear();
@@ -54,6 +57,46 @@ static void release(Plan &p) {
   p.d_angles = p.d_aux = nullptr;
   p.d_scratch = p.d_in = p.d_out = nullptr;
   p.host_stream = nullptr;
+}
+
+static int create_events(Plan &p) {
+  TOMO_CUDA(cudaEventCreateWithFlags(&p.used, cudaEventDisableTiming));
+  TOMO_CUDA(cudaEventCreateWithFlags(&p.used_capture, cudaEventDisableTiming));
+  return TOMO_OK;
+}
+
+static int use_begin(Plan &p, cudaStream_t s, bool *capturing) {
+  cudaStreamCaptureStatus st;
+  unsigned long long id = 0;
+  TOMO_CUDA(cudaStreamGetCaptureInfo(s, &st, &id));
+  *capturing = st != cudaStreamCaptureStatusNone;
+  if (!*capturing) {
+    TOMO_CUDA(cudaStreamWaitEvent(s, p.used, 0));
+  } else if (p.capture_id != id) {
+    TOMO_CUDA(cudaStreamWaitEvent(s, p.used, cudaEventWaitExternal));
+    p.capture_id = id;
+  } else {
+    TOMO_CUDA(cudaStreamWaitEvent(s, p.used_capture, 0));
+  }
+  return TOMO_OK;
+}
+
+PlanUse::PlanUse(Plan &p, cudaStream_t s) : p_(p), s_(s) {
+  p.use_mu.lock();
+  rc_ = use_begin(p, s, &capturing_);
+  open_ = rc_ == TOMO_OK;
+  if (!open_) p.use_mu.unlock();
+}
+
+int PlanUse::end(int rc) {
+  if (open_) {
+    open_ = false;
+    cudaError_t e = cudaEventRecordWithFlags(p_.used, s_, capturing_ ? cudaEventRecordExternal : cudaEventRecordDefault);
+    if (e == cudaSuccess && capturing_) e = cudaEventRecord(p_.used_capture, s_);
+    p_.use_mu.unlock();
+    if (e != cudaSuccess) rc_ = cuda_fail(e, "recording a plan's use");
+  }
+  return rc ? rc : rc_;
 }
 
 static int validate(const tomo_geom *g) {
@@ -150,6 +193,7 @@ int tomo_plan_create(const tomo_geom *geom, tomo_plan **out) {
     default:
       rc = fail(TOMO_EINVAL, "unsupported kind");
   }
+  if (!rc) rc = create_events(p);
   if (rc) {
     release(p);
     delete tp;
@@ -181,6 +225,7 @@ int tomo_plan_create_batch(const tomo_geom *geoms, int count, tomo_plan **out) {
   p.nh = (int)(p.g.n * 0.5);
   cudaGetDevice(&p.device);
   int rc = dd_setup_batch(p, geoms, count);
+  if (!rc) rc = create_events(p);
   if (rc) {
     release(p);
     delete tp;
@@ -229,12 +274,14 @@ int tomo_plan_destroy(tomo_plan *plan) {
 
 int tomo_forward(tomo_plan *plan, const float *d_image, float *d_sino, void *stream) {
   if (!plan || !d_image || !d_sino) return fail(TOMO_EINVAL, "tomo_forward: NULL argument");
-  return plan_forward(plan->p, d_image, d_sino, (cudaStream_t)stream, FwdEpi());
+  PlanUse use(plan->p, (cudaStream_t)stream);
+  return use.end(use.error() ? use.error() : plan_forward(plan->p, d_image, d_sino, (cudaStream_t)stream, FwdEpi()));
 }
 
 int tomo_adjoint(tomo_plan *plan, const float *d_sino, float *d_image, void *stream) {
   if (!plan || !d_image || !d_sino) return fail(TOMO_EINVAL, "tomo_adjoint: NULL argument");
-  return plan_adjoint(plan->p, d_sino, d_image, (cudaStream_t)stream, AdjEpi());
+  PlanUse use(plan->p, (cudaStream_t)stream);
+  return use.end(use.error() ? use.error() : plan_adjoint(plan->p, d_sino, d_image, (cudaStream_t)stream, AdjEpi()));
 }
 
 static int ensure_host_buffers(Plan &p) {

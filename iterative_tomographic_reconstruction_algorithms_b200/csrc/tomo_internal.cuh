@@ -5,6 +5,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -89,6 +90,11 @@ struct Plan {
   std::vector<cudaEvent_t> stage_events;
   cudaStream_t host_stream = nullptr;
   int device = 0;
+  // order between calls that use the plan's buffers (PlanUse)
+  cudaEvent_t used = nullptr;         // recorded behind the last one
+  cudaEvent_t used_capture = nullptr; // the same among the calls of one capture,
+  unsigned long long capture_id = 0;  // this one
+  std::mutex use_mu;                  // held while a call enqueues its work
   // distance-driven layout (radon_dd.cu)
   int dd_pads = 0, dd_w = 0, dd_wl = 0, dd_nR = 0, dd_nC = 0, dd_nS = 0;
   // warps of the forward launch that write residual partial sums (solver.cu)
@@ -99,6 +105,27 @@ struct Plan {
   // kind-specific state owned by the plan (gridding), freed with ext_free
   void *ext = nullptr;
   void (*ext_free)(void *) = nullptr;
+};
+
+// A plan's tables and scratch serve one call at a time.  A call (anything that
+// enqueues plan_forward or plan_adjoint) opens a PlanUse on its stream, which
+// makes the stream wait for the plan's last call if that came on another one, and
+// closes it with end(): calls on several streams then run one after another, as on
+// one.  In a stream capture the wait and the record become nodes of the graph, so
+// its replays take their turn too; calls on several streams of one capture
+// depend on one another.  While it is open no other host thread enqueues.
+class PlanUse {
+ public:
+  PlanUse(Plan &p, cudaStream_t s);
+  ~PlanUse() { end(0); }
+  int error() const { return rc_; }  // of the wait: enqueue nothing then
+  int end(int rc);                   // rc, or the error of the wait or the record
+
+ private:
+  Plan &p_;
+  cudaStream_t s_;
+  int rc_ = 0;
+  bool open_ = false, capturing_ = false;
 };
 
 size_t image_elems(const Plan &p);
