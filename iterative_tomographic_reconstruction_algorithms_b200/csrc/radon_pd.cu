@@ -72,42 +72,44 @@ __global__ void __launch_bounds__(256) pd_frame_kernel(const float *__restrict__
 // above its rounding: a fourth pixel would lie past b - 1.05 + 3 sigma > b + 1).
 // Each is evaluated with the reference's arithmetic: the first lies below b
 // (floor(T) = b - 1, weight T - floor(T)), the third above (floor(T) = b,
-// weight (t + ceil(T)) - nh), the second on either side; an integral T puts
-// nothing into either bin.  Six products of a line are added in float, lines
-// in double, rounded once: deterministic, and as close to the exact sum as the
-// 64-bit fixed-point sums in shared memory that this replaces.  Those took two
-// 32-bit atomics per product, and bounded the forward: 1.57 ms at 768^2 x 720,
-// now 0.97 (2048^2 x 1800: 25.2, now 14.8).  Bound now by instruction issue (52
-// per bin and line).
-template <bool ROWS, int DIR, bool ORD>
-__device__ __forceinline__ double pd_fwd_bin(const float *__restrict__ L, int w, float s, float c, int b, int n, int nh,
-                                             int i0, int i1) {
-  const float fnh = (float)nh, fb = (float)b, bm = fb - 1.0f, bp = fb + 1.0f;
-  const float k = ROWS ? s : c, o = ROWS ? c : s;  // t along the line, across lines
-  const float inv = 1.0f / k, slope = -o * inv;
-  // position (pixel index) at which T = b - 1: base + slope * (line coordinate)
-  float base[2];
-#pragma unroll
-  for (int e = 0; e < 2; ++e) base[e] = (fnh - bm) * inv + fnh - 0.5f - (e ? 0.25f : -0.25f) - DIR * 0.05f;
-  const float lo = DIR > 0 ? -4.0f : -2.0f, hi = DIR > 0 ? (float)(n + 1) : (float)(n + 3);
-  const float *line = L + (size_t)i0 * w + kPdFrame - kPdMagicBits;
-  float lc = (float)i0 - fnh + 0.5f;  // the line's own coordinate
-  double acc = 0.0;
-  // both sub-samples at once, as pairs; nt = -t
-  const F2 base2 = f2(base[0], base[1]), slope2 = f2(slope), magic = f2(kPdMagic), nmagic = f2(-kPdMagic);
-  const F2 off = f2(0.25f - fnh, 0.75f - fnh), dir = f2((float)DIR), d2 = f2(-0.25f, 0.25f), nh2 = f2(fnh);
-  const F2 ns = f2(-s), nc = f2(-c), nbm = f2(-bm), nbp = f2(-bp);
-#pragma unroll 2
-  for (int i = i0; i < i1; ++i, line += w, lc += 1.0f) {
-    const F2 l = add2(f2(lc), d2);
-    const float2 ps = unpack(fma2(slope2, l, base2));
-    const F2 pos = f2(fminf(fmaxf(ps.x, lo), hi), fminf(fmaxf(ps.y, lo), hi));
-    const F2 fm = DIR > 0 ? add2_ru(pos, magic) : add2_rd(pos, magic);  // next pixels in DIR
-    const float2 fs = unpack(fm);
-    const float *va = line + __float_as_int(fs.x), *vb = line + __float_as_int(fs.y);
-    const F2 u0 = add2(add2(fm, nmagic), off);  // their coordinates along the line, exactly
+// weight (t + ceil(T)) - nh), the second on either side; an integral T puts |(t +
+// T) - nh|, the rounding of t, and 0 into bin T.
+//
+// The products are added in double and rounded once: deterministic, and as close
+// to their exact sum as the 64-bit fixed-point sums in shared memory that this
+// replaces.  Those took two 32-bit atomics per product, and bounded the forward:
+// 1.57 ms at 768^2 x 720, now 1.03 (2048^2 x 1800: 25.2, now 16.4).  Bound by
+// issue and the FP32 pipe.  (Adding a line's products in
+// float first takes 0.95 and 14.6, but keeps 24 bits of the sum, and reaches
+// infinity next to the largest float where the bin is finite.)
+
+// A bin and its angle, as both loops use them.
+template <bool ROWS, int DIR>
+struct PdBin {
+  float fnh, fb, bm, bp;
+  F2 base2, slope2, ns, nc, nh2, nbm, nbp, off, dir;
+  __device__ __forceinline__ PdBin(float s, float c, int b, int nh) {
+    fnh = (float)nh;
+    fb = (float)b;
+    bm = fb - 1.0f;
+    bp = fb + 1.0f;
+    const float k = ROWS ? s : c, o = ROWS ? c : s;  // t along the line, across lines
+    const float inv = 1.0f / k;
+    // position (pixel index) at which T = b - 1: base + slope * (line coordinate)
+    const float at = (fnh - bm) * inv + fnh - 0.5f;
+    base2 = f2(at + 0.25f - DIR * 0.05f, at - 0.25f - DIR * 0.05f);
+    slope2 = f2(-o * inv);
+    ns = f2(-s);
+    nc = f2(-c);
+    nh2 = f2(fnh);
+    nbm = f2(-bm);
+    nbp = f2(-bp);
+    off = f2(0.25f - fnh, 0.75f - fnh);
+    dir = f2((float)DIR);
+  }
+  // -t of the three pixels from coordinate u0 (along the line) on
+  __device__ __forceinline__ void nt(F2 l, F2 u0, F2 &t0, F2 &t1, F2 &t2) const {
     const F2 u1 = add2(u0, dir), u2 = add2(u1, dir);
-    F2 t0, t1, t2;
     if (ROWS) {
       t0 = fma2(nc, l, mul2(u0, ns));
       t1 = fma2(nc, l, mul2(u1, ns));
@@ -118,39 +120,109 @@ __device__ __forceinline__ double pd_fwd_bin(const float *__restrict__ L, int w,
       t1 = fma2(nc, u1, xs);
       t2 = fma2(nc, u2, xs);
     }
-    const float2 w0 = unpack(add2(add2(nh2, t0), nbm));
-    const F2 T1 = add2(nh2, t1);
-    const float2 Ts = unpack(T1), wa = unpack(add2(T1, nbm)), wb = unpack(add2(add2(t1, nbp), nh2));  // wb: -weight
-    const float2 w2 = unpack(add2(add2(t2, nbp), nh2));                                               // -weight
-    // below b the first of wa, -wb is the smaller one, above the second
-    float w1x = fminf(wa.x, -wb.x), w1y = fminf(wa.y, -wb.y);
+  }
+  // an integral T's weight |(t + T) - nh|
+  __device__ __forceinline__ float on_bin(float nt) const { return fabsf(__fsub_rn(__fadd_rn(-nt, fb), fnh)); }
+};
+
+// Every product as the reference rounds it, added in double.
+template <bool ROWS, int DIR>
+__device__ __forceinline__ double pd_fwd_exact(const float *__restrict__ L, int w, float s, float c, int b, int n, int nh,
+                                               int i0, int i1) {
+  const PdBin<ROWS, DIR> B(s, c, b, nh);
+  const float lo = DIR > 0 ? -4.0f : -2.0f, hi = DIR > 0 ? (float)(n + 1) : (float)(n + 3);
+  const float *line = L + (size_t)i0 * w + kPdFrame - kPdMagicBits;
+  float lc = (float)i0 - B.fnh + 0.5f;  // the line's own coordinate
+  double acc = 0.0;
+#pragma unroll 2
+  for (int i = i0; i < i1; ++i, line += w, lc += 1.0f) {
+    const F2 l = add2(f2(lc), f2(-0.25f, 0.25f));
+    const float2 ps = unpack(fma2(B.slope2, l, B.base2));
+    const F2 pos = f2(fminf(fmaxf(ps.x, lo), hi), fminf(fmaxf(ps.y, lo), hi));
+    const F2 fm = DIR > 0 ? add2_ru(pos, f2(kPdMagic)) : add2_rd(pos, f2(kPdMagic));  // next pixels in DIR
+    const float2 fs = unpack(fm);
+    const float *va = line + __float_as_int(fs.x), *vb = line + __float_as_int(fs.y);
+    F2 t0, t1, t2;
+    B.nt(l, add2(add2(fm, f2(-kPdMagic)), B.off), t0, t1, t2);
+    const float2 w0 = unpack(add2(add2(B.nh2, t0), B.nbm));
+    const F2 T1 = add2(B.nh2, t1);
+    const float2 Ts = unpack(T1), wa = unpack(add2(T1, B.nbm)), wb = unpack(add2(add2(t1, B.nbp), B.nh2));  // wb: -weight
+    const float2 w2 = unpack(add2(add2(t2, B.nbp), B.nh2));                                                 // -weight
+    const float2 n1 = unpack(t1), T2 = unpack(add2(B.nh2, t2));
     const float a0 = __ldg(va), a1 = __ldg(va + DIR), a2 = __ldg(va + 2 * DIR);
     const float b0 = __ldg(vb), b1 = __ldg(vb + DIR), b2 = __ldg(vb + 2 * DIR);
-    if (ORD) {
-      // every product rounded as the reference rounds it, their exact sum; an
-      // integral T puts its weight, |(t + T) - nh|, into that bin
-      const float2 n1 = unpack(t1), T2 = unpack(add2(nh2, t2));
-      if (Ts.x == fb) w1x = fabsf(__fsub_rn(__fadd_rn(-n1.x, fb), fnh));
-      if (Ts.y == fb) w1y = fabsf(__fsub_rn(__fadd_rn(-n1.y, fb), fnh));
-      double r = 0.0, q = 0.0;
-      if (w0.x > 0.0f) r += (double)__fmul_rn(w0.x, a0);
-      r += (double)__fmul_rn(w1x, a1);
-      if (T2.x < bp) r += (double)__fmul_rn(fabsf(w2.x), a2);
-      if (w0.y > 0.0f) q += (double)__fmul_rn(w0.y, b0);
-      q += (double)__fmul_rn(w1y, b1);
-      if (T2.y < bp) q += (double)__fmul_rn(fabsf(w2.y), b2);
-      acc += r + q;
-      continue;
-    }
-    float p = 0.0f;
-    if (w0.x > 0.0f) p = w0.x * a0;
-    if (Ts.x != fb) p = fmaf(w1x, a1, p);
-    if (w2.x < 0.0f) p = fmaf(-w2.x, a2, p);
-    if (w0.y > 0.0f) p = fmaf(w0.y, b0, p);
-    if (Ts.y != fb) p = fmaf(w1y, b1, p);
-    if (w2.y < 0.0f) p = fmaf(-w2.y, b2, p);
-    acc += (double)p;
+    // below b the first of wa, -wb is the smaller one, above the second
+    float px = __fmul_rn(fminf(wa.x, -wb.x), a1), py = __fmul_rn(fminf(wa.y, -wb.y), b1);
+    if (Ts.x == B.fb) px = __fmaf_rn(0.0f, a1, __fmul_rn(B.on_bin(n1.x), a1));
+    if (Ts.y == B.fb) py = __fmaf_rn(0.0f, b1, __fmul_rn(B.on_bin(n1.y), b1));
+    double r = 0.0, q = 0.0;
+    if (w0.x > 0.0f) r += (double)__fmul_rn(w0.x, a0);
+    r += (double)px;
+    if (T2.x < B.bp) r += (double)__fmul_rn(fabsf(w2.x), a2);
+    if (w0.y > 0.0f) q += (double)__fmul_rn(w0.y, b0);
+    q += (double)py;
+    if (T2.y < B.bp) q += (double)__fmul_rn(fabsf(w2.y), b2);
+    acc += r + q;
   }
+  return acc;
+}
+
+// Out of the register budget of the loop that falls back to it.
+template <bool ROWS, int DIR>
+__device__ __noinline__ double pd_fwd_again(const float *__restrict__ L, int w, float s, float c, int b, int n, int nh, int i0,
+                                            int i1) {
+  return pd_fwd_exact<ROWS, DIR>(L, w, s, c, b, n, nh, i0, i1);
+}
+
+// The same with the two sub-samples' weights of a pixel added first (both are
+// multiples of the spacing of T, so their sum is exact for T >= 2): four pixels,
+// products and conversions to double per line instead of six (1.35 ms at 768^2 x
+// 720 with six).  A sum that is not finite, as one weight's zero or two weights'
+// overflow can make it, is left to pd_fwd_exact.
+template <bool ROWS, int DIR>
+__device__ __forceinline__ double pd_fwd_bin(const float *__restrict__ L, int w, float s, float c, int b, int n, int nh,
+                                             int i0, int i1) {
+  const PdBin<ROWS, DIR> B(s, c, b, nh);
+  // the four pixels from the next one on, or from the one above it, stay in the frame
+  const float lo = DIR > 0 ? -4.0f : -1.0f, hi = DIR > 0 ? (float)n : (float)(n + 2);
+  const float *line = L + (size_t)i0 * w + kPdFrame - kPdMagicBits;
+  float lc = (float)i0 - B.fnh + 0.5f;
+  double acc = 0.0;
+#pragma unroll 2
+  for (int i = i0; i < i1; ++i, line += w, lc += 1.0f) {
+    const F2 l = add2(f2(lc), f2(-0.25f, 0.25f));
+    const float2 ps = unpack(fma2(B.slope2, l, B.base2));
+    const float pos = fminf(fmaxf(ps.y, lo), hi);
+    const float fy = DIR > 0 ? __fadd_ru(pos, kPdMagic) : __fadd_rd(pos, kPdMagic);  // next pixel in DIR
+    // The first sub-sample crosses 0 to 1 pixels above the second: its next
+    // pixel is taken to be the same or the one above it (a rounding's pixel more
+    // or less at the start is within the 0.05)
+    const float iy = __fsub_rn(fy, kPdMagic), up = iy + 1.0f;
+    const bool same = DIR > 0 ? ps.x <= iy : ps.x < up;
+    const float *v = line + __float_as_int(fy) + (DIR < 0 && !same ? 1 : 0);
+    const float v0 = __ldg(v), v1 = __ldg(v + DIR), v2 = __ldg(v + 2 * DIR), v3 = __ldg(v + 3 * DIR);
+    F2 t0, t1, t2;
+    B.nt(l, add2(f2(same ? iy : up, iy), B.off), t0, t1, t2);
+    const float2 T0 = unpack(add2(B.nh2, t0)), T2 = unpack(add2(B.nh2, t2));
+    const F2 T1 = add2(B.nh2, t1);
+    const float2 Ts = unpack(T1), wa = unpack(add2(T1, B.nbm));
+    // above b the weight of bin floor(T) is -((nt + ceil(T)) + nh)
+    const F2 nce = f2(Ts.x == B.fb ? -B.fb : -B.bp, Ts.y == B.fb ? -B.fb : -B.bp);
+    const float2 wb = unpack(add2(add2(t1, nce), B.nh2));
+    // the first and the third weight are 0 for a pixel out of reach: a saturating
+    // sum, and a test, for (t + ceil(T)) - nh is not 0 when T is b + 1
+    const float x0 = __saturatef(__fsub_rn(T0.x, B.bm)), y0 = __saturatef(__fsub_rn(T0.y, B.bm));
+    const float2 w2 = unpack(add2(add2(t2, B.nbp), B.nh2));  // -weight
+    const float x2 = T2.x < B.bp ? -w2.x : 0.0f, y2 = T2.y < B.bp ? -w2.y : 0.0f;
+    const float x1 = fminf(wa.x, fabsf(wb.x)), y1 = fminf(wa.y, fabsf(wb.y));
+    // e: the sub-sample that starts first, g: the other
+    const float e0 = DIR > 0 ? y0 : x0, e1 = DIR > 0 ? y1 : x1, e2 = DIR > 0 ? y2 : x2;
+    const float g0 = DIR > 0 ? x0 : y0, g1 = DIR > 0 ? x1 : y1, g2 = DIR > 0 ? x2 : y2;
+    const float p0 = __fmul_rn(e0 + (same ? g0 : 0.0f), v0), p1 = __fmul_rn(e1 + (same ? g1 : g0), v1);
+    const float p2 = __fmul_rn(e2 + (same ? g2 : g1), v2), p3 = __fmul_rn(same ? 0.0f : g2, v3);
+    acc += ((double)p0 + (double)p1) + ((double)p2 + (double)p3);
+  }
+  if (!(fabs(acc) < INFINITY)) acc = pd_fwd_again<ROWS, DIR>(L, w, s, c, b, n, nh, i0, i1);
   return acc;
 }
 
@@ -159,11 +231,11 @@ __device__ __forceinline__ double pd_fwd_bin(const float *__restrict__ L, int w,
 // hide a line's latency: one angle, its lines shared by SPLIT warps, whose sums
 // are added in order.  The split depends on n alone (pd_fwd_split), so a plan
 // for some of the angles or several slices gives the same bits.  SPLIT = 0: as 1
-// in the solvers' form (epilogue.cuh), the exact sum of the rounded products.
+// in the solvers' form (epilogue.cuh), pd_fwd_exact.
 constexpr int kPdAng = 4;
 
 template <int SPLIT>
-__global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : kPdAng)) pd_forward_kernel(
+__global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : kPdAng), 32 / (SPLIT > 1 ? SPLIT : kPdAng)) pd_forward_kernel(
     const float *__restrict__ rows, const float *__restrict__ cols, float *__restrict__ sino, const PdAngle *__restrict__ tab,
     int n, int nh, int na, FwdEpi ep) {
   constexpr int kParts = SPLIT > 1 ? SPLIT : 1;
@@ -191,10 +263,10 @@ __global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : kPdAng)) pd_forward_
       i0 += len * warp / kParts;
     }
     const float *L = (by_rows ? rows : cols) + z * (size_t)n * w;
-    if (by_rows)
-      acc = s < 0.0f ? pd_fwd_bin<true, 1, SPLIT == 0>(L, w, s, c, b, n, nh, i0, i1) : pd_fwd_bin<true, -1, SPLIT == 0>(L, w, s, c, b, n, nh, i0, i1);
-    else
-      acc = c < 0.0f ? pd_fwd_bin<false, 1, SPLIT == 0>(L, w, s, c, b, n, nh, i0, i1) : pd_fwd_bin<false, -1, SPLIT == 0>(L, w, s, c, b, n, nh, i0, i1);
+#define PD_BIN(R, D) (SPLIT ? pd_fwd_bin<R, D>(L, w, s, c, b, n, nh, i0, i1) : pd_fwd_exact<R, D>(L, w, s, c, b, n, nh, i0, i1))
+    if (by_rows) acc = s < 0.0f ? PD_BIN(true, 1) : PD_BIN(true, -1);
+    else acc = c < 0.0f ? PD_BIN(false, 1) : PD_BIN(false, -1);
+#undef PD_BIN
   }
   if (SPLIT > 1) {
     part[warp][lane] = acc;
@@ -231,18 +303,21 @@ __global__ void __launch_bounds__(256) pd_expand_kernel(const float *__restrict_
 // Adjoint: a lane holds 4 x 4 pixels of a 32 x 16 tile; the Q warps of a block
 // sum Q contiguous shares of the angles, added in order through shared memory
 // (Q depends on n alone, so the result does not depend on the device).  Q = 1 is
-// the solvers' form (epilogue.cuh): one chain in the reference's order, integral
-// T included, with a row of 4 pixels per lane (R = 1) for small images.
+// the solvers' form (epilogue.cuh), one chain in the reference's order, with a
+// row of 4 pixels per lane (R = 1) for small images.
 //
 // Per sub-sample: t and T as the reference rounds them, the pair at floor(T)
-// in one 8-byte read, and its two weights.  An integral T puts nothing into
-// either bin: its weights are the rounding of t, and are skipped.
+// in one 8-byte read, and its two weights, which carry the factor 1/2 of the two
+// coinciding quarter-weight sub-samples (scaling by it rounds nothing; without it
+// the sums would reach infinity at half the largest float).  An integral T, where
+// floor and ceil are one bin, is rare and takes the branch.
 //
 // Bound by L1 (70 % of its rate) and FP32 (65 %): 9 operations and 2 FMAs per
 // sub-sample, whose table pairs hit L1.  The two sub-samples go as f32x2 pairs,
 // which halves the instructions (scalar ones: 0.57 ms against 0.51).  A thread
 // per pixel with four reads, bounds tests and the sign rule per sub-sample took
-// 1.52 ms at 768^2 x 720 and 25.5 at 2048^2 x 1800; this one 0.51 and 7.8.
+// 1.52 ms at 768^2 x 720 and 25.5 at 2048^2 x 1800; this one 0.51 and 8.1.
+constexpr int kPdGrp = 2;  // pixels that share the test for an integral T
 template <int Q, int R>
 __global__ void __launch_bounds__(32 * Q) pd_adjoint_kernel(const float2 *__restrict__ pairs, float *__restrict__ img,
                                                             const PdAngle *__restrict__ tab, int n, int nh, int na, int pads,
@@ -260,7 +335,8 @@ __global__ void __launch_bounds__(32 * Q) pd_adjoint_kernel(const float2 *__rest
   const int u0 = (int)((long long)na * q / Q), u1 = (int)((long long)na * (q + 1) / Q);
   if (a0 < n && b0 < n) {
     const float x0 = (float)b0 - fnh + 0.5f, y0 = (float)(n - 1 - a0) - fnh + 0.5f;  // rows go up in y
-    const F2 nh2 = f2(fnh), magic = f2(kPdMagic), nmagic = f2(-kPdMagic), magic1 = f2(kPdMagic - 1.0f);
+    const F2 nh2 = f2(fnh), magic = f2(kPdMagic), half = f2(0.5f), nhalf = f2(-0.5f), hnh = f2(0.5f * fnh);
+    const F2 hm = f2(0.5f * kPdMagic), hm1 = f2(0.5f * (kPdMagic - 1.0f));
     // row base minus the bits of the magic floor
     const float2 *row = pairs + (z * na + u0) * (size_t)w2 + pads - kPdMagicBits;
 #pragma unroll 1
@@ -276,28 +352,46 @@ __global__ void __launch_bounds__(32 * Q) pd_adjoint_kernel(const float2 *__rest
       for (int i = 0; i < R; ++i) {
         const F2 y = f2(y0 - (float)i - 0.25f, y0 - (float)i + 0.25f);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const F2 nt = fma2(nc, y, xs[j]);
-          const F2 T = add2(nh2, nt);
+        for (int j0 = 0; j0 < 4; j0 += kPdGrp) {
+        float2 wu[kPdGrp], wl[kPdGrp], Sa[kPdGrp], Sb[kPdGrp];
+        F2 nt[kPdGrp];
+#pragma unroll
+        for (int j = 0; j < kPdGrp; ++j) {
+          nt[j] = fma2(nc, y, xs[j0 + j]);
+          const F2 T = add2(nh2, nt[j]);
           // floor(T) without the conversion pipe: T + 1.5 * 2^23 rounded down
           // lies where floats are the integers (|T| < 2^22), and its bits give
           // the integer
           const F2 fd = add2_rd(T, magic);
           const float2 fs = unpack(fd);
-          const float2 Sa = __ldg(row + __float_as_int(fs.x)), Sb = __ldg(row + __float_as_int(fs.y));
-          const float2 wu = unpack(rsub2(add2(fd, nmagic), T));
-          if (Q == 1) {
-            const float2 Tv = unpack(T), t = unpack(nt);
-            const float2 uf = unpack(add2(add2_ru(T, magic), nmagic));  // ceil(T)
-            acc[i][j] = __fmaf_rn(fabsf(__fsub_rn(__fadd_rn(-t.x, uf.x), fnh)), Sa.x, acc[i][j]);
-            if (Tv.x != uf.x) acc[i][j] = __fmaf_rn(wu.x, Sa.y, acc[i][j]);
-            acc[i][j] = __fmaf_rn(fabsf(__fsub_rn(__fadd_rn(-t.y, uf.y), fnh)), Sb.x, acc[i][j]);
-            if (Tv.y != uf.y) acc[i][j] = __fmaf_rn(wu.y, Sb.y, acc[i][j]);
-            continue;
+          Sa[j] = __ldg(row + __float_as_int(fs.x));
+          Sb[j] = __ldg(row + __float_as_int(fs.y));
+          // halves of the reference's weights T - floor(T) and, negative, (t + ceil(T)) - nh
+          wu[j] = unpack(fma2(T, half, fma2(fd, nhalf, hm)));
+          wl[j] = unpack(add2(fma2(nt[j], half, fma2(fd, nhalf, hm1)), hnh));
+        }
+        float least = fminf(wu[0].x, wu[0].y);
+#pragma unroll
+        for (int j = 1; j < kPdGrp; ++j) least = fminf(least, fminf(wu[j].x, wu[j].y));
+        if (least == 0.0f) {  // an integral T: floor and ceil are one bin
+#pragma unroll
+          for (int j = 0; j < kPdGrp; ++j) {
+            const float2 t = unpack(nt[j]);
+            if (wu[j].x == 0.0f) {
+              wl[j].x = -0.5f * fabsf(__fsub_rn(__fadd_rn(-t.x, __fadd_rn(fnh, t.x)), fnh));
+              Sa[j].y = Sa[j].x;
+            }
+            if (wu[j].y == 0.0f) {
+              wl[j].y = -0.5f * fabsf(__fsub_rn(__fadd_rn(-t.y, __fadd_rn(fnh, t.y)), fnh));
+              Sb[j].y = Sb[j].x;
+            }
           }
-          const float2 wl = unpack(add2(add2(nt, rsub2(fd, magic1)), nh2));  // -(t + (floor(T) + 1) - nh)
-          if (wu.x != 0.0f) acc[i][j] = __fmaf_rn(-wl.x, Sa.x, __fmaf_rn(wu.x, Sa.y, acc[i][j]));
-          if (wu.y != 0.0f) acc[i][j] = __fmaf_rn(-wl.y, Sb.x, __fmaf_rn(wu.y, Sb.y, acc[i][j]));
+        }
+#pragma unroll
+        for (int j = 0; j < kPdGrp; ++j) {
+          acc[i][j0 + j] = __fmaf_rn(wu[j].x, Sa[j].y, __fmaf_rn(-wl[j].x, Sa[j].x, acc[i][j0 + j]));
+          acc[i][j0 + j] = __fmaf_rn(wu[j].y, Sb[j].y, __fmaf_rn(-wl[j].y, Sb[j].x, acc[i][j0 + j]));
+        }
         }
       }
     }
@@ -321,8 +415,7 @@ __global__ void __launch_bounds__(32 * Q) pd_adjoint_kernel(const float2 *__rest
     for (int j = 0; j < 4; ++j) {
       const int y = a0 + i, x = b0 + j;
       const bool live = y < n && x < n;
-      // 0.5: the two coinciding quarter-weight sub-samples
-      adj_store(ep, 0.5f * acc[i][j], live, z * (size_t)n * n + (live ? (size_t)y * n + x : 0), img);
+      adj_store(ep, acc[i][j], live, z * (size_t)n * n + (live ? (size_t)y * n + x : 0), img);
     }
 }
 

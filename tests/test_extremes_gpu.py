@@ -1,0 +1,65 @@
+"""The projector pairs at the ends of the float range: values next to the largest
+float whose projections are finite, and infinite values that meet a weight of
+exactly 0, against the FP64 oracle (the reference's float geometry and bin
+decisions, summed in FP64).
+
+Tolerance of the large values: all terms have one sign, so relative errors add.
+Forward: every product is rounded (2^-24), their sum once more.  Adjoint: a pixel
+adds up to 8 products in float.  9 x 2^-24 in both.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BIG = 3.2e38  # the largest float is 3.4e38
+REL = 9 * 2.0 ** -24
+
+
+def _pair(oper, n, deg, oracle):
+    from iterative_tomographic_reconstruction_algorithms_b200 import class_projectors_radon as cpr
+    tp = cpr.projectors(n, np.array(deg), oper=oper)
+    return tp, lambda d, a: oracle.radon(oper, d, a, tp.angles)
+
+
+def _compare(torch, fn, ref, a):
+    got = fn(torch.from_numpy(a).cuda()).cpu().numpy()
+    for test in (np.isnan, np.isposinf, np.isneginf):
+        assert np.array_equal(test(got), test(ref)), test.__name__
+    fin = np.isfinite(ref)
+    assert np.all(np.abs(got[fin] - ref[fin]) <= REL * np.abs(ref[fin]) + 1e-30)
+    return fin
+
+
+@pytest.mark.parametrize("oper,n", [("pd", 40), ("pd", 330), ("pd", 641)])
+def test_values_next_to_the_largest_float(cuda, oracle, oper, n):
+    tp, orc = _pair(oper, n, [20.0, 61.0, 100.0, 155.0], oracle)
+    for place in ((n // 2 + 3, n // 3), (n // 4, n // 2)):
+        x = np.zeros((n, n), np.float32)
+        x[place] = BIG
+        assert _compare(cuda, tp.A, orc(0, x), x).all()
+    for place in ((0, n // 2 + 5), (1, n // 3), (3, n // 2 - 1)):
+        y = np.zeros((4, n), np.float32)
+        y[place] = BIG
+        assert _compare(cuda, tp.At, orc(1, y), y).all()
+
+
+@pytest.mark.parametrize("oper,n", [("pd", 32), ("pd", 33), ("pd", 450)])
+def test_infinite_values_at_zero_weights(cuda, oracle, oper, n):
+    """At 45 degrees (pd) the pixels of the diagonal land on a bin's centre exactly, where the
+    other neighbour has weight 0: 0 x infinity is NaN."""
+    deg = [20.0, 45.0, 100.0]
+    tp, orc = _pair(oper, n, deg, oracle)
+    x = np.zeros((n, n), np.float32)
+    x[n - 1 - n // 3, n // 3] = np.inf
+    ref = orc(0, x)
+    assert np.isnan(ref).any()
+    _compare(cuda, tp.A, ref, x)
+    for sign in (1.0, -1.0):
+        y = np.zeros((3, n), np.float32)
+        y[:, n // 2] = sign * np.inf
+        ref = orc(1, y)
+        assert np.isnan(ref).any()
+        _compare(cuda, tp.At, ref, y)
