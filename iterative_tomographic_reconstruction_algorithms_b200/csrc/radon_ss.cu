@@ -96,8 +96,7 @@ __global__ void __launch_bounds__(128) ss_forward_kernel(const float *__restrict
     const float fd = __fadd_rd(f, kSsMagic);  // floor(f), as a float among the integers and in its bits
     const float fl = __fsub_rn(fd, kSsMagic), wq = __fsub_rn(f, fl);
     const float *p = row + __float_as_int(fd);
-    // (floor(f) + 1) - f is 1 - w exactly, except in the last bits of |f| < 1
-    const float w1 = SPLIT ? __fsub_rn(1.0f, wq) : __fsub_rn(__fadd_rn(fl, 1.0f), f);
+    const float w1 = __fsub_rn(__fadd_rn(fl, 1.0f), f);  // not 1 - wq: that loses the last bits of |f| < 1
     acc = fmaf(SPLIT ? w1 : __fmul_rn(g.wt, w1), __ldg(p), acc);
     acc = fmaf(SPLIT ? wq : __fmul_rn(g.wt, wq), __ldg(p + 1), acc);
   }
@@ -118,16 +117,21 @@ __global__ void __launch_bounds__(128) ss_forward_kernel(const float *__restrict
 int ss_fwd_split(int n) { return n > 448 ? 2 : 4; }
 
 // Sinogram rows as pairs in the order of the angles, entry e = t + nh + pads of
-// angle v: wt {S_t, S_t+1} (without wt: ordered), 0 outside the rays.
+// angle v: wt {S_t, S_t+1}, 0 outside the rays.  A row where one of these is not
+// finite keeps {S_t, S_t+1} and is marked in raw[z][v] (as all are: ordered).
 __global__ void __launch_bounds__(256) ss_expand_kernel(const float *__restrict__ sino, float2 *__restrict__ out,
-                                                        const SsAngle *__restrict__ tab, int n, int nh, int na, int pads,
-                                                        int w2, bool ordered) {
+                                                        int *__restrict__ raw, const SsAngle *__restrict__ tab, int n, int nh,
+                                                        int na, int pads, int w2, bool ordered) {
   const int v = blockIdx.x;
   const size_t z = blockIdx.y;
   const SsAngle g = tab[v];
-  const float wt = ordered ? 1.0f : g.wt;
   const float *src = sino + (z * na + g.out_row) * (size_t)n;
   float2 *dst = out + (z * na + v) * (size_t)w2;
+  bool bad = ordered;
+  for (int t = threadIdx.x; t < 2 * nh; t += blockDim.x) bad |= !(fabsf(g.wt * __ldg(src + t)) < INFINITY);
+  bad = __syncthreads_or(bad);
+  if (threadIdx.x == 0) raw[z * na + v] = bad;
+  const float wt = bad ? 1.0f : g.wt;
   for (int e = threadIdx.x; e < w2; e += blockDim.x) {
     const int t = e - pads;
     dst[e] = make_float2(t >= 0 && t < 2 * nh ? wt * __ldg(src + t) : 0.0f,
@@ -143,18 +147,26 @@ __global__ void __launch_bounds__(256) ss_expand_kernel(const float *__restrict_
 // At a pixel's major coordinate m the rays' minor coordinates f(t) = fma(-m, a,
 // t) * rb lie |rb| = 1 / |cb| >= 1 apart, so a ray within 1 of the pixel's minor
 // coordinate c is within |cb| <= 1 of the crossing t* of c: it is floor(t*) or
-// the next.  Each has weight wt (1 - |f - c|), exactly the forward's (f - floor
-// f or floor f + 1 - f).  A rounding of t* across an integer loses nothing while
-// |cb| < 1 by more than that rounding (below n 2^-22 in all); the few angles
-// nearer to an axis (NEAR) look at the rays before and behind too.  The two
+// the next.  It reaches c if f is in [c - 1, c + 1), with the forward's weight wt (f
+// - floor f) or wt (floor f + 1 - f), which are wt (1 - |f - c|) (to 2^-25 where f
+// has bits below those of c = +-1).  A rounding of t* across an integer loses
+// nothing while |cb| < 1 by more than that rounding (below n 2^-22 in all); the few
+// angles nearer to an axis (NEAR) look at the rays before and behind too.  The two
 // rays come as one pair, evaluated as packed operations.
+//
+// For finite values a ray with weight 0 can be passed by, and wt be applied to the
+// value; an infinite value makes NaN of a weight of 0, and wt S may overflow where
+// wt w S does not.  The rows where that matters are marked (raw) and go through
+// ss_adj_raw.
 //
 // The ray's own limits (EDGE) matter only next to the border: at a pixel 4 or
 // more inside the square both rays are inside it.
 //
 // Bound by FP32 and issue.  Candidate rays checked one by one against their
 // limits, each credited to 4 pixels by 8 tests, took 3.53 ms at 4 x 641^2 x
-// 600 and 18.1 at 2048^2 x 1800; this takes 1.22 and 6.5.
+// 600 and 18.1 at 2048^2 x 1800; this takes 1.24 and 6.7 (with the reference's two
+// forms of the weight in every mode 1.88 and 9.6).
+
 // Whether ray t passes major coordinate m (without branches: the loads of a
 // block's rays overlap).
 __device__ __forceinline__ bool ss_in_limits(const int2 *__restrict__ lrow, int t, int m, int nh) {
@@ -162,12 +174,25 @@ __device__ __forceinline__ bool ss_in_limits(const int2 *__restrict__ lrow, int 
   return (t >= -nh) & (t < nh) & (m >= l.x) & (m < l.y);
 }
 
-// Weight of a ray at f to the pixel at c, below 0 out of reach.  ORD: as f -
-// floor f or floor f + 1 - f, which differ in the last bits where |f| < 1.
-template <bool ORD>
-__device__ __forceinline__ float ss_weight(float f, float c) {
-  if (ORD) return fminf(__fsub_rn(__fadd_rn(c, 1.0f), f), __fsub_rn(f, __fsub_rn(c, 1.0f)));
-  return 1.0f - fabsf(__fsub_rn(f, c));
+// o += wt w S for the ray at f and the pixel at c, if it reaches it and `in`, as the
+// reference has it: wt w is rounded, and a weight of 0 counts.
+__device__ __forceinline__ void ss_credit(float &o, float f, float c, float wt, float S, bool in) {
+  const float u = __fsub_rn(f, c - 1.0f), v = __fsub_rn(c + 1.0f, f);
+  if ((u >= 0.0f) & (v > 0.0f) & in) o = fmaf(__fmul_rn(wt, fminf(u, v)), S, o);
+}
+
+// o + a marked row's credits to pixel (R, C); row: its pair at t = -nh.
+__device__ __noinline__ float ss_adj_raw(float o, const SsAngle *__restrict__ tab, const float2 *__restrict__ row,
+                                         const int2 *__restrict__ lrow, int R, int C, int nh) {
+  const SsAngle g = *tab;
+  const int mi = (g.steep ? R : C) - nh, ci = (g.steep ? C : R) - nh;
+  const float m = (float)mi, c = (float)ci, t0 = floorf(fmaf(c, 1.0f / g.rb, m * g.a));
+#pragma unroll 1
+  for (int k = -1; k <= 2; ++k) {
+    const int t = (int)t0 + k;
+    ss_credit(o, __fmul_rn(__fmaf_rn(-m, g.a, t0 + (float)k), g.rb), c, g.wt, __ldg(row + nh + t).x, ss_in_limits(lrow, t, mi, nh));
+  }
+  return o;
 }
 
 template <bool STEEP, bool EDGE, bool NEAR, bool ORD>
@@ -187,26 +212,36 @@ __device__ __forceinline__ void ss_adj_angle(const SsAngle &g, const float2 *__r
       const float2 S = __ldg(row + __float_as_int(fm));
       const F2 t = add2(f2(__fsub_rn(fm, kSsMagic)), step);
       const float2 f = unpack(mul2(fma2(nm, a, t), rb));  // scalar from here: see f32x2.cuh
-      const float h0 = ss_weight<ORD>(f.x, c), h1 = ss_weight<ORD>(f.y, c);
       const int ti = __float_as_int(fm) - kSsMagicBits;
       float &o = STEEP ? acc[i][j] : acc[j][i];
-      if (NEAR) {
-        const float h = ss_weight<ORD>(__fmul_rn(__fmaf_rn(-m, g.a, __fsub_rn(fm, kSsMagic) - 1.0f), g.rb), c);
-        if (h > 0.0f && (!EDGE || ss_in_limits(lrow, ti - 1, M0 + i, nh))) o = fmaf(ORD ? __fmul_rn(wt, h) : h, __ldg(row + __float_as_int(fm) - 1).x, o);
-      }
+      // as the reference has it (ORD), or on finite rows that hold wt S
+      auto credit = [&](float f, float S, bool in) {
+        if (ORD) {
+          ss_credit(o, f, c, wt, S, in);
+        } else {
+          const float h = 1.0f - fabsf(__fsub_rn(f, c));
+          if ((h > 0.0f) & in) o = fmaf(h, S, o);
+        }
+      };
+      auto before_or_behind = [&](int k) {
+        const float f = __fmul_rn(__fmaf_rn(-m, g.a, __fsub_rn(fm, kSsMagic) + (float)k), g.rb);
+        credit(f, k < 0 ? __ldg(row + __float_as_int(fm) - 1).x : __ldg(row + __float_as_int(fm) + 1).y,
+               !EDGE || ss_in_limits(lrow, ti + k, M0 + i, nh));
+      };
+      if (NEAR) before_or_behind(-1);
       const bool in0 = EDGE ? ss_in_limits(lrow, ti, M0 + i, nh) : true, in1 = EDGE ? ss_in_limits(lrow, ti + 1, M0 + i, nh) : true;
-      if ((h0 > 0.0f) & in0) o = fmaf(ORD ? __fmul_rn(wt, h0) : h0, S.x, o);
-      if ((h1 > 0.0f) & in1) o = fmaf(ORD ? __fmul_rn(wt, h1) : h1, S.y, o);
-      if (NEAR) {
-        const float h = ss_weight<ORD>(__fmul_rn(__fmaf_rn(-m, g.a, __fsub_rn(fm, kSsMagic) + 2.0f), g.rb), c);
-        if (h > 0.0f && (!EDGE || ss_in_limits(lrow, ti + 2, M0 + i, nh))) o = fmaf(ORD ? __fmul_rn(wt, h) : h, __ldg(row + __float_as_int(fm) + 1).y, o);
-      }
+      credit(f.x, S.x, in0);
+      credit(f.y, S.y, in1);
+      if (NEAR) before_or_behind(2);
     }
   }
 }
 
+// 28 warps per SM at Q = 4 (72 registers) took 1.235 and 6.7 ms, 32 (64, with 12
+// bytes spilled) 1.29 and 6.8.
 template <int Q>
-__global__ void __launch_bounds__(32 * Q) ss_adjoint_kernel(const float2 *__restrict__ pairs, float *__restrict__ img,
+__global__ void __launch_bounds__(32 * Q, (Q == 1 ? 0 : Q == 4 ? 28 : 32) / Q) ss_adjoint_kernel(const float2 *__restrict__ pairs,
+                                                            const int *__restrict__ raw, float *__restrict__ img,
                                                             const SsAngle *__restrict__ tab, const int2 *__restrict__ lim,
                                                             int n, int nh, int na, int pads, int w2, AdjEpi ep) {
   __shared__ float part[Q > 1 ? (Q - 1) * 16 : 1][32];
@@ -222,6 +257,11 @@ __global__ void __launch_bounds__(32 * Q) ss_adjoint_kernel(const float2 *__rest
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
   // the tile's pixels are all 4 or more inside the square [0, 2 nh - 1]
   const bool edge = blockIdx.x * 32 < 4 || by * 16 < 4 || blockIdx.x * 32 + 36 > 2 * nh || by * 16 + 20 > 2 * nh;
+  bool marked = false;  // rows of this warp's share
+  if (Q > 1) {
+    for (int u = q + Q * lane; u < na; u += Q * 32) marked |= __ldg(raw + z * na + u) != 0;
+    marked = __any_sync(0xffffffffu, marked);
+  }
   if (a0 < n && b0 < n) {
     const float near = 1.0f - (float)n * 0x1p-22f;
     const float2 *row = pairs + (z * na + q) * (size_t)w2 + pads + nh - kSsMagicBits;
@@ -230,6 +270,7 @@ __global__ void __launch_bounds__(32 * Q) ss_adjoint_kernel(const float2 *__rest
     for (int u = q; u < na; u += Q, row += (size_t)Q * w2, lrow += (size_t)Q * 2 * nh) {
       const SsAngle g = tab[u];
       const bool nr = fabsf(g.rb) * near < 1.0f;
+      if (marked && __ldg(raw + z * na + u)) continue;
       if (nr) {
         if (g.steep) ss_adj_angle<true, true, true, Q == 1>(g, row, lrow, a0, b0, nh, acc);
         else ss_adj_angle<false, true, true, Q == 1>(g, row, lrow, a0, b0, nh, acc);
@@ -241,6 +282,16 @@ __global__ void __launch_bounds__(32 * Q) ss_adjoint_kernel(const float2 *__rest
         else ss_adj_angle<false, false, false, Q == 1>(g, row, lrow, a0, b0, nh, acc);
       }
     }
+    if (marked)
+#pragma unroll 1
+      for (int u = q; u < na; u += Q)
+        if (__ldg(raw + z * na + u))
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              acc[i][j] = ss_adj_raw(acc[i][j], tab + u, pairs + (z * na + u) * (size_t)w2 + pads, lim + (size_t)u * 2 * nh,
+                                     a0 + i, b0 + j, nh);
   }
   if (q > 0)
 #pragma unroll
@@ -271,6 +322,7 @@ int ss_adj_warps(int n) { return n > 640 ? 4 : n > 384 ? 8 : 16; }
 
 struct SsState {
   float2 *pairs = nullptr;                 // [nz][na][w2]
+  int *raw = nullptr;                      // [nz][na]
   float *rows = nullptr, *cols = nullptr;  // [nz][n][n + 2 kSsFrame]
   int pads = 0, w2 = 0;
 };
@@ -337,9 +389,10 @@ int ss_setup(Plan &p) {
   // one workspace: the adjoint's pairs, then the forward's framed copies
   const int n = p.g.n;
   const size_t pairs = (size_t)p.g.nz * na * st->w2, framed = (size_t)p.g.nz * n * (n + 2 * kSsFrame);
-  TOMO_CUDA(cudaMalloc(&st->pairs, sizeof(float2) * pairs + 2 * sizeof(float) * framed));
+  TOMO_CUDA(cudaMalloc(&st->pairs, sizeof(float2) * pairs + 2 * sizeof(float) * framed + sizeof(int) * p.g.nz * na));
   st->rows = (float *)(st->pairs + pairs);
   st->cols = st->rows + framed;
+  st->raw = (int *)(st->cols + framed);
   // residual partials of the fused solvers: one per warp of the ordered forward
   p.fwd_warps = (size_t)((n + 127) / 128) * 4 * na * p.g.nz;
   return TOMO_OK;
@@ -361,11 +414,11 @@ int ss_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
 int ss_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const AdjEpi &ep) {
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
   SsState &st = *(SsState *)p.ext;
-  ss_expand_kernel<<<dim3(na, nz), 256, 0, s>>>(d_sino, st.pairs, (const SsAngle *)p.d_angles, n, p.nh, na, st.pads, st.w2,
-                                               ep.ordered);
+  ss_expand_kernel<<<dim3(na, nz), 256, 0, s>>>(d_sino, st.pairs, st.raw, (const SsAngle *)p.d_angles, n, p.nh, na, st.pads,
+                                               st.w2, ep.ordered);
   const int Q = ep.ordered ? 1 : ss_adj_warps(n);
   auto fn = Q == 1 ? ss_adjoint_kernel<1> : Q == 4 ? ss_adjoint_kernel<4> : Q == 8 ? ss_adjoint_kernel<8> : ss_adjoint_kernel<16>;
-  fn<<<dim3((n + 31) / 32, (n + 15) / 16, nz), 32 * Q, 0, s>>>(st.pairs, d_img, (const SsAngle *)p.d_angles,
+  fn<<<dim3((n + 31) / 32, (n + 15) / 16, nz), 32 * Q, 0, s>>>(st.pairs, st.raw, d_img, (const SsAngle *)p.d_angles,
                                                                (const int2 *)p.d_aux, n, p.nh, na, st.pads, st.w2, ep);
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;

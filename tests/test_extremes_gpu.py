@@ -26,6 +26,8 @@ def _pair(oper, n, deg, oracle):
 
 def _compare(torch, fn, ref, a):
     got = fn(torch.from_numpy(a).cuda()).cpu().numpy()
+    with np.errstate(over="ignore"):
+        ref = np.where(np.isfinite(ref), ref.astype(np.float32), ref)  # beyond the largest float: infinite
     for test in (np.isnan, np.isposinf, np.isneginf):
         assert np.array_equal(test(got), test(ref)), test.__name__
     fin = np.isfinite(ref)
@@ -33,24 +35,24 @@ def _compare(torch, fn, ref, a):
     return fin
 
 
-@pytest.mark.parametrize("oper,n", [("pd", 40), ("pd", 330), ("pd", 641)])
+@pytest.mark.parametrize("oper,n", [("pd", 40), ("pd", 330), ("pd", 641), ("ss", 40), ("ss", 450), ("ss", 641)])
 def test_values_next_to_the_largest_float(cuda, oracle, oper, n):
     tp, orc = _pair(oper, n, [20.0, 61.0, 100.0, 155.0], oracle)
     for place in ((n // 2 + 3, n // 3), (n // 4, n // 2)):
         x = np.zeros((n, n), np.float32)
         x[place] = BIG
-        assert _compare(cuda, tp.A, orc(0, x), x).all()
+        assert _compare(cuda, tp.A, orc(0, x), x).sum() > 3 * n
     for place in ((0, n // 2 + 5), (1, n // 3), (3, n // 2 - 1)):
         y = np.zeros((4, n), np.float32)
         y[place] = BIG
-        assert _compare(cuda, tp.At, orc(1, y), y).all()
+        assert _compare(cuda, tp.At, orc(1, y), y).sum() > n * (n - 2)
 
 
-@pytest.mark.parametrize("oper,n", [("pd", 32), ("pd", 33), ("pd", 450)])
+@pytest.mark.parametrize("oper,n", [("pd", 32), ("pd", 33), ("pd", 450), ("ss", 32), ("ss", 33), ("ss", 450)])
 def test_infinite_values_at_zero_weights(cuda, oracle, oper, n):
     """At 45 degrees (pd) the pixels of the diagonal land on a bin's centre exactly, where the
-    other neighbour has weight 0: 0 x infinity is NaN."""
-    deg = [20.0, 45.0, 100.0]
+    other neighbour has weight 0: 0 x infinity is NaN.  At 0 degrees (ss) every ray does."""
+    deg = [20.0, 45.0, 100.0] if oper == "pd" else [0.0, 20.0, 100.0]
     tp, orc = _pair(oper, n, deg, oracle)
     x = np.zeros((n, n), np.float32)
     x[n - 1 - n // 3, n // 3] = np.inf
