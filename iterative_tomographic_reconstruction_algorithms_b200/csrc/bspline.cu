@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "f32x2.cuh"
 #include "fixed_sum.cuh"
 #include "tomo_internal.cuh"
 
@@ -255,29 +256,78 @@ __device__ __forceinline__ bool bs_special(float y) {
 // Above the rounding of fl(s + ps), |ps| <= n/sqrt(2) + 2.
 __device__ __forceinline__ float bs_near(int n) { return (float)(n + 8) * 0x1p-24f; }
 
-// The six pixels of a line and bin b, each with the number of taps that the
-// reference puts into the bin (0, 1 or 2).
+// A lane's bin and angle, as it walks lines l (ROWS: ky, else kx).
 template <bool ROWS, int DIR>
-__device__ __noinline__ float bs_fwd_taps(const float *v, const float *tab, int entries, unsigned org, float u0, float l, float C,
-                                          float S, int b, const BsConst &k) {
-  float p = 0.0f;
+struct BsLine {
+  float C, S, y, base, slope, lo, hi;
+  __device__ __forceinline__ BsLine(float C_, float S_, int b, const BsConst &k) : C(C_), S(S_), y((float)b - k.fmid) {
+    const float inv = 1.0f / (ROWS ? C : -S);  // 1 / (ps per pixel)
+    // pixel at which ps = y - 2 - 1/64
+    base = (y - 2.015625f) * inv + k.fmid;
+    slope = -(ROWS ? S : C) * inv;
+    lo = DIR > 0 ? -8.0f : -3.0f;
+    hi = DIR > 0 ? (float)(k.n + 2) : (float)(k.n + 7);
+  }
+  __device__ __forceinline__ static float coordinate(int i, const BsConst &k) {
+    return ROWS ? k.fmid - (float)i : (float)i - k.fmid;
+  }
+  // the first of the six pixels, in the magic form
+  __device__ __forceinline__ float first(float l) const {
+    const float pos = fminf(fmaxf(fmaf(slope, l, base), lo), hi);
+    return DIR > 0 ? __fadd_ru(pos, kBsMagic) : __fadd_rd(pos, kBsMagic);
+  }
+};
+
+// How many taps of a pixel at distance d, ps from the centre, the reference puts into
+// bin b (0, 1 or 2).
+__device__ __forceinline__ int bs_count(float d, float ps, int b, const BsConst &k) {
+  const float s0 = rintf(d);  // a tap on the bin is within 1 of the distance
+  int m = 0;
+#pragma unroll
+  for (int s = -1; s <= 1; ++s) {
+    const float t = s0 + (float)s;
+    m += (fabsf(t) <= 2.0f) & (bs_bin((int)t, ps, k.mid) == b);
+  }
+  return m;
+}
+
+struct BsSix {
+  float x[6];
+};
+// The products of a line's six pixels, each as often as the reference counts it.
+template <bool ROWS, int DIR>
+__device__ __noinline__ double bs_fwd_taps(BsSix s, float u0, float l, float so, float C, float S, int b, const BsConst &k) {
+  double p = 0.0;
 #pragma unroll
   for (int q = 0; q < 6; ++q) {
     const float u = u0 + (float)(q * DIR);
-    const float ps = ROWS ? __fmaf_rn(u, C, l) : __fmaf_rn(l, C, __fmul_rn(S, -u));
-    const float d = __fsub_rn((float)b - k.fmid, ps);
-    const unsigned fl = __float_as_uint(__fmaf_rd(d, k.lut_step, kBsMagic)), ce = __float_as_uint(__fmaf_ru(d, k.lut_step, kBsMagic));
-    const float wt = tab[min(fl + ce + org, (unsigned)entries)];
-    const float s0 = rintf(d);  // a tap on the bin is within 1 of the distance
-    int m = 0;
-#pragma unroll
-    for (int s = -1; s <= 1; ++s) {
-      const float t = s0 + (float)s;
-      m += (fabsf(t) <= 2.0f) & (bs_bin((int)t, ps, k.mid) == b);
-    }
-    if (wt == wt && m) p = fmaf(wt * (float)m, __ldg(v + q * DIR), p);
+    const float ps = ROWS ? __fmaf_rn(u, C, so) : __fmaf_rn(l, C, __fmul_rn(S, -u));
+    const int m = bs_count(__fsub_rn((float)b - k.fmid, ps), ps, b, k);
+    const double x = m ? (double)s.x[q] : 0.0;
+    p += x;
+    if (m == 2) p += x;
   }
   return p;
+}
+
+// All lines of a bin as the reference has them.
+template <bool ROWS, int DIR>
+__device__ __noinline__ double bs_fwd_again(const float *__restrict__ I, const float *__restrict__ L, int w, float C, float S, int b,
+                                            const BsConst &k, int i0, int i1) {
+  const BsLine<ROWS, DIR> B(C, S, b, k);
+  double acc = 0.0;
+  for (int i = i0; i < i1; ++i) {
+    const float l = BsLine<ROWS, DIR>::coordinate(i, k), fm = B.first(l);
+    const float *v = I + (size_t)i * w + kBsFrame + (__float_as_int(fm) - kBsMagicBits);
+#pragma unroll 1
+    for (int q = 0; q < 6; ++q) {
+      const float u = __fsub_rn(__fsub_rn(fm, kBsMagic), k.fmid) + (float)(q * DIR);
+      const float ps = ROWS ? __fmaf_rn(u, C, __fmul_rn(S, l)) : __fmaf_rn(l, C, __fmul_rn(S, -u));
+      const int li = bs_lut(b, ps, k), m = bs_count(__fsub_rn(B.y, ps), ps, b, k);
+      if (m && li >= 0 && li < k.lut_max) acc += (double)m * (double)__fmul_rn(__ldg(L + li), __ldg(v + q * DIR));
+    }
+  }
+  return acc;
 }
 
 // Forward: a lane owns a bin and walks the lines (ROWS: image rows, when ps
@@ -285,56 +335,62 @@ __device__ __noinline__ float bs_fwd_taps(const float *v, const float *tab, int 
 // (+ 1 table step) are among six consecutive ones, sigma = max(|C|, |S|) in
 // [0.707, 1] apart (a seventh would lie 6 x 0.707 > 4.03 behind the first).
 // The angle's table is in shared memory by half steps of the distance, with the
-// index's truncation toward zero applied: entry floor(a) + ceil(a), a = d *
-// step, needs no conversion.  MODE 1: some of the warp's bins are special, 2:
-// it holds bin 0, whose pixels count twice (the reference's truncation folds
-// the tap on bin -1 onto it).  Six products of a line are added in float, lines
-// in double, rounded once.
+// index's truncation toward zero applied and 0 where no tap counts: entry floor(a)
+// + ceil(a), a = d * step, needs no conversion.  MODE 1: some of the warp's bins are
+// special, 2: it holds bin 0, whose pixels count twice (the reference's truncation
+// folds the tap on bin -1 onto it).  Products are rounded as the reference rounds
+// them and added in double, rounded once.  A sum that is not finite, for which a
+// pixel out of reach may be the cause, is done again tap by tap.
 //
-// Bound by shared memory: six reads at the lanes' own phases, about 3.5 bank
-// conflicts each.  Adding every tap to 64-bit fixed-point sums by two
-// shared-memory atomics took 2.15 ms at 768^2 x 720 and 31.7 at 2048^2 x 1800;
-// this takes 1.46 and 22.2.
+// Bound by shared memory (six reads at the lanes' own phases, about 3.5 bank
+// conflicts each) and the conversions to double; two pixels at a time as packed
+// pairs.  Adding every tap to 64-bit fixed-point sums by two shared-memory atomics
+// took 2.15 ms at 768^2 x 720 and 31.7 at 2048^2 x 1800; this takes 1.48 and
+// 22.6 (1.66 and 25.5 pixel by pixel with NaN for the missing taps).
 template <bool ROWS, int DIR, int MODE>
-__device__ __forceinline__ double bs_fwd_bin(const float *__restrict__ L, const float *tab, int entries, int w, float C, float S,
-                                             int b, const BsConst &k, int i0, int i1) {
-  const float fmid = k.fmid, y = (float)b - fmid, step = k.lut_step;
-  const float inv = 1.0f / (ROWS ? C : -S);  // 1 / (ps per pixel)
-  // pixel at which ps = y - 2 - 1/64
-  const float base = (y - 2.015625f) * inv + fmid, slope = -(ROWS ? S : C) * inv;
-  const float lo = DIR > 0 ? -8.0f : -3.0f, hi = DIR > 0 ? (float)(k.n + 2) : (float)(k.n + 7);
-  const float *line = L + (size_t)i0 * w + kBsFrame - kBsMagicBits;
+__device__ __forceinline__ double bs_fwd_bin(const float *__restrict__ I, const float *tab, const float *__restrict__ L, int entries,
+                                             int w, float C, float S, int b, const BsConst &k, int i0, int i1) {
+  const BsLine<ROWS, DIR> B(C, S, b, k);
+  const float y = B.y;
+  const float *line = I + (size_t)i0 * w + kBsFrame - kBsMagicBits;
   const unsigned org = (unsigned)entries / 2u - 2u * (unsigned)kBsMagicBits;  // entry of distance 0
-  float lc = ROWS ? fmid - (float)i0 : (float)i0 - fmid;
+  float lc = BsLine<ROWS, DIR>::coordinate(i0, k);
   const float thr = bs_special(y) ? bs_near(k.n) : -1.0f;
-  const bool twice = b == 0;  // a tap on bin -1 folds onto bin 0, where the next tap lies
+  const F2 C2 = f2(C), S2 = f2(S), y2 = f2(y), step2 = f2(k.lut_step), magic = f2(kBsMagic);
   double acc = 0.0;
 #pragma unroll 1
   for (int i = i0; i < i1; ++i, line += w, lc += ROWS ? -1.0f : 1.0f) {
-    const float pos = fminf(fmaxf(fmaf(slope, lc, base), lo), hi);
-    const float fm = DIR > 0 ? __fadd_ru(pos, kBsMagic) : __fadd_rd(pos, kBsMagic);  // the first of the six
+    const float fm = B.first(lc);
     const float *v = line + __float_as_int(fm);
-    const float u0 = __fsub_rn(__fsub_rn(fm, kBsMagic), fmid);
-    const float so = ROWS ? __fmul_rn(S, lc) : 0.0f;
-    float p = 0.0f, near = 1.0f;
+    const float u0 = __fsub_rn(__fsub_rn(fm, kBsMagic), k.fmid), so = ROWS ? __fmul_rn(S, lc) : 0.0f;
+    BsSix s;  // the products
+    float(&x)[6] = s.x, near = 1.0f;
+    double again = 0.0;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      const float u = u0 + (float)(q * DIR);
-      const float ps = ROWS ? __fmaf_rn(u, C, so) : __fmaf_rn(lc, C, __fmul_rn(S, -u));
-      const float d = __fsub_rn(y, ps);
-      const unsigned fl = __float_as_uint(__fmaf_rd(d, step, kBsMagic)), ce = __float_as_uint(__fmaf_ru(d, step, kBsMagic));
-      const float wt = tab[min(fl + ce + org, (unsigned)entries)];  // outside: the NaN behind the table
-      const float x = __ldg(v + q * DIR);
-      if (wt == wt) p = fmaf(wt, x, p);
+    for (int q = 0; q < 6; q += 2) {
+      F2 ps;
+      if (ROWS) ps = fma2(add2(f2(u0), f2((float)(q * DIR), (float)((q + 1) * DIR))), C2, f2(so));
+      else ps = fma2(f2(lc), C2, mul2(S2, add2(f2(-u0), f2((float)(-q * DIR), (float)(-(q + 1) * DIR)))));
+      const F2 d2 = rsub2(ps, y2);
+      const float2 d = unpack(d2), fl = unpack(fma2_rd(d2, step2, magic)), ce = unpack(fma2_ru(d2, step2, magic));
+      const float wa = tab[min(__float_as_uint(fl.x) + __float_as_uint(ce.x) + org, (unsigned)entries)];
+      const float wb = tab[min(__float_as_uint(fl.y) + __float_as_uint(ce.y) + org, (unsigned)entries)];
+      x[q] = __fmul_rn(wa, __ldg(v + q * DIR));
+      x[q + 1] = __fmul_rn(wb, __ldg(v + (q + 1) * DIR));
       if (MODE > 0) {
-        const float r = fabsf(__fsub_rn(d, __fsub_rn(__fadd_rn(d, kBsMagic), kBsMagic)));
-        near = fminf(near, r);
-        if (MODE > 1 && twice && wt == wt && d > -2.0f && r > 0.0f) p = fmaf(wt, x, p);
+        auto off = [](float e) { return fabsf(__fsub_rn(e, __fsub_rn(__fadd_rn(e, kBsMagic), kBsMagic))); };
+        const float ra = off(d.x), rb = off(d.y);
+        near = fminf(near, fminf(ra, rb));
+        if (MODE > 1 && b == 0 && d.x > -2.0f && ra > 0.0f) again += (double)x[q];
+        if (MODE > 1 && b == 0 && d.y > -2.0f && rb > 0.0f) again += (double)x[q + 1];
       }
     }
-    if (MODE > 0 && near < thr) p = bs_fwd_taps<ROWS, DIR>(v, tab, entries, org, u0, ROWS ? so : lc, C, S, b, k);
-    acc += (double)p;
+    double p = (((double)x[0] + (double)x[1]) + ((double)x[2] + (double)x[3])) + ((double)x[4] + (double)x[5]);
+    if (MODE > 1) p += again;
+    if (MODE > 0 && near < thr) p = bs_fwd_taps<ROWS, DIR>(s, u0, lc, so, C, S, b, k);
+    acc += p;
   }
+  if (!(fabs(acc) < INFINITY)) acc = bs_fwd_again<ROWS, DIR>(I, L, w, C, S, b, k, i0, i1);
   return acc;
 }
 
@@ -343,10 +399,10 @@ __device__ __forceinline__ double bs_fwd_bin(const float *__restrict__ L, const 
 // better (513^2 x 400: 0.75 ms unsplit, 0.43 by four; 2048^2 x 1800 the same by
 // two).  The split is a function of n alone (bs_fwd_split).
 template <int SPLIT>
-__global__ void __launch_bounds__(128) bs_forward_pow2_kernel(const float *__restrict__ rows, const float *__restrict__ cols,
+__global__ void __launch_bounds__(128, 8) bs_forward_pow2_kernel(const float *__restrict__ rows, const float *__restrict__ cols,
                                                               float *__restrict__ sino, const float2 *__restrict__ cs,
                                                               const float *__restrict__ lut, int entries, BsConst k) {
-  extern __shared__ float tab[];  // [entries] by half steps, distances within 2 (+ 2 steps); NaN where no tap counts
+  extern __shared__ float tab[];  // [entries] by half steps, distances within 2 (+ 2 steps); 0 where no tap counts
   __shared__ double part[SPLIT][128 / SPLIT];
   constexpr int kBins = 128 / SPLIT;
   const int lane = threadIdx.x % kBins, q = threadIdx.x / kBins;
@@ -357,7 +413,7 @@ __global__ void __launch_bounds__(128) bs_forward_pow2_kernel(const float *__res
   for (int e = threadIdx.x; e <= entries; e += 128) {
     const int i2 = e - org;                    // floor(a) + ceil(a)
     const int li = (i2 >= 0 ? i2 >> 1 : -(-i2 >> 1)) + k.lut_half;  // toward zero
-    tab[e] = e < entries && li >= 0 && li < k.lut_max ? __ldg(Lv + li) : __int_as_float(0x7fffffff);
+    tab[e] = e < entries && li >= 0 && li < k.lut_max ? __ldg(Lv + li) : 0.0f;
   }
   __syncthreads();
   const float C = cs[v].x, S = cs[v].y;
@@ -381,9 +437,9 @@ __global__ void __launch_bounds__(128) bs_forward_pow2_kernel(const float *__res
   const float *L = (by_rows ? rows : cols) + z * (size_t)n * w;
   const bool spec = __any_sync(0xffffffffu, bs_special((float)b - k.fmid)), first = __any_sync(0xffffffffu, b == 0);
   double acc;
-#define BS_BIN(R, D) (first  ? bs_fwd_bin<R, D, 2>(L, tab, entries, w, C, S, b, k, i0, i1) \
-                      : spec ? bs_fwd_bin<R, D, 1>(L, tab, entries, w, C, S, b, k, i0, i1) \
-                             : bs_fwd_bin<R, D, 0>(L, tab, entries, w, C, S, b, k, i0, i1))
+#define BS_BIN(R, D) (first  ? bs_fwd_bin<R, D, 2>(L, tab, Lv, entries, w, C, S, b, k, i0, i1) \
+                      : spec ? bs_fwd_bin<R, D, 1>(L, tab, Lv, entries, w, C, S, b, k, i0, i1) \
+                             : bs_fwd_bin<R, D, 0>(L, tab, Lv, entries, w, C, S, b, k, i0, i1))
   if (by_rows) acc = C > 0.0f ? BS_BIN(true, 1) : BS_BIN(true, -1);
   else acc = S < 0.0f ? BS_BIN(false, 1) : BS_BIN(false, -1);
 #undef BS_BIN
@@ -415,11 +471,12 @@ __global__ void bs_lut4_kernel(const float *__restrict__ lut, float4 *__restrict
 
 // Sinogram rows as groups, entry e = m + pads: {S_m-1, S_m, S_m+1, S_m+2}, 0
 // outside [0, n); bin 0 twice, for the tap on bin -1 that folds onto it with
-// the same weight.
-__global__ void __launch_bounds__(256) bs_expand_kernel(const float *__restrict__ sino, float4 *__restrict__ out, int n, int pads,
-                                                        int w2) {
+// the same weight.  A row where that is not finite is marked.
+__global__ void __launch_bounds__(256) bs_expand_kernel(const float *__restrict__ sino, float4 *__restrict__ out,
+                                                        int *__restrict__ mark, int n, int pads, int w2) {
   const float *src = sino + (size_t)blockIdx.x * n;
   float4 *dst = out + (size_t)blockIdx.x * w2;
+  if (threadIdx.x == 0) mark[blockIdx.x] = !(2.0f * fabsf(__ldg(src)) < INFINITY);
   for (int e = threadIdx.x; e < w2; e += blockDim.x) {
     float v[4];
 #pragma unroll
@@ -537,12 +594,29 @@ __global__ void __launch_bounds__(kBsThreads4) bs_adjoint_pow2_kernel(const floa
   }
 }
 
-__global__ void __launch_bounds__(256) bs_adj_sum_kernel(const float *__restrict__ partial, int Q, size_t total, float *__restrict__ img) {
+// The shares of slice blockIdx.y added in order (Q = 1: nothing to add).  A slice with
+// marked rows, which may lack finite values, is done again by the reference's rule.
+__global__ void __launch_bounds__(256) bs_adj_sum_kernel(const float *__restrict__ partial, int Q, float *__restrict__ img,
+                                                         const float *__restrict__ sino, const int *__restrict__ mark,
+                                                         const float2 *__restrict__ cs, const float *__restrict__ lut, BsConst k) {
+  const size_t z = blockIdx.y, per = (size_t)k.n * k.n, total = per * gridDim.y;
+  bool marked = false;
+  for (int u = threadIdx.x; u < k.na; u += 256) marked |= __ldg(mark + z * k.na + u) != 0;
+  marked = __syncthreads_or(marked);
   const size_t p = (size_t)blockIdx.x * 256 + threadIdx.x;
-  if (p >= total) return;
+  if (p >= per || (Q == 1 && !marked)) return;
   float acc = 0.0f;
-  for (int q = 0; q < Q; ++q) acc += partial[(size_t)q * total + p];
-  img[p] = acc;
+  if (marked) {
+    const int R = (int)(p / k.n);
+    const float x = (float)((int)p - R * k.n) - k.fmid, y = k.fmid - (float)R;
+    for (int u = 0; u < k.na; ++u) {
+      const float2 g = __ldg(cs + u);
+      acc = bs_adj_taps(__fmaf_rn(x, g.x, __fmul_rn(g.y, y)), sino + (z * k.na + u) * (size_t)k.n, lut + (size_t)u * k.lut_size, k, acc);
+    }
+  } else {
+    for (int q = 0; q < Q; ++q) acc += partial[(size_t)q * total + z * per + p];
+  }
+  img[z * per + p] = acc;
 }
 
 // Shares of the angles: blocks enough for four rounds of two to an SM, since
@@ -574,6 +648,7 @@ struct BsState {
   void *work = nullptr;       // one workspace for what follows
   float4 *lut4 = nullptr, *S4 = nullptr;
   float *rows = nullptr, *cols = nullptr, *partial = nullptr;
+  int *mark = nullptr;  // [nz][na]
   int pads = 0, w2 = 0, Q = 1, entries = 0;
 };
 
@@ -611,7 +686,13 @@ int bs_setup(Plan &p) {
   p.ext_free = bs_state_free;
   const BsConst k = make_const(p);
   const int n = p.g.n, L = p.g.lut_size;
-  st->pow2 = p.g.support == 4.0f && (L & (L - 1)) == 0 && L >= 64 && L <= 2048 && n >= 4 && n <= 4096;
+  // (a table that is not finite would poison the pixels out of reach)
+  bool finite = true;
+  for (size_t i = 0; i < (size_t)na * L; ++i) {
+    st->lutmax = std::max(st->lutmax, std::fabs(p.g.lut[i]));
+    finite = finite && std::isfinite(p.g.lut[i]);
+  }
+  st->pow2 = finite && p.g.support == 4.0f && (L & (L - 1)) == 0 && L >= 64 && L <= 2048 && n >= 4 && n <= 4096;
   if (st->pow2) {
     // |ps| stays below sqrt(2) (n/2 + 1) + 4, also for a tile's pixels outside the image
     st->pads = (int)std::ceil((p.nh + 1) * 0.41422) + 64;
@@ -620,17 +701,17 @@ int bs_setup(Plan &p) {
     st->entries = 8 * (int)k.lut_step + 8;
     const size_t nz = p.g.nz, lut4 = (size_t)na * 2 * (size_t)k.lut_step, s4 = nz * na * st->w2;
     const size_t framed = nz * n * (n + 2 * kBsFrame), part = st->Q > 1 ? st->Q * nz * n * n : 0;
-    TOMO_CUDA(cudaMalloc(&st->work, sizeof(float4) * (lut4 + s4) + sizeof(float) * (2 * framed + part)));
+    TOMO_CUDA(cudaMalloc(&st->work, sizeof(float4) * (lut4 + s4) + sizeof(float) * (2 * framed + part) + sizeof(int) * nz * na));
     st->lut4 = (float4 *)st->work;
     st->S4 = st->lut4 + lut4;
     st->rows = (float *)(st->S4 + s4);
     st->cols = st->rows + framed;
     st->partial = st->cols + framed;
+    st->mark = (int *)(st->partial + part);
     bs_lut4_kernel<<<na, 256>>>((const float *)p.d_aux, st->lut4, k);
     TOMO_CUDA(cudaGetLastError());
     TOMO_CUDA(cudaStreamSynchronize(0));  // later calls may come on streams that do not wait for this one
   }
-  for (size_t i = 0; i < (size_t)na * L; ++i) st->lutmax = std::max(st->lutmax, std::fabs(p.g.lut[i]));
   TOMO_CUDA(cudaMalloc(&st->vmax, sizeof(unsigned) * (size_t)std::max(1, p.g.nz)));
   if (sizeof(float) * (size_t)L > 48 * 1024)
     TOMO_CUDA(cudaFuncSetAttribute(bs_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * L)));
@@ -668,16 +749,14 @@ int bs_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const
   BsState &st = *(BsState *)p.ext;
   if (st.pow2 && !ep.ordered) {
     const int n = k.n, nz = p.g.nz;
-    bs_expand_kernel<<<k.na * nz, 256, 0, s>>>(d_sino, st.S4, n, st.pads, st.w2);
+    bs_expand_kernel<<<k.na * nz, 256, 0, s>>>(d_sino, st.S4, st.mark, n, st.pads, st.w2);
     const dim3 grid((n + kBsTW - 1) / kBsTW * st.Q, (n + kBsTH - 1) / kBsTH, nz);
     const size_t smem = sizeof(float4) * 2 * (size_t)k.lut_step;
     auto fn = (n & 1) ? bs_adjoint_pow2_kernel<true> : bs_adjoint_pow2_kernel<false>;
     fn<<<grid, kBsThreads4, smem, s>>>(d_sino, st.S4, st.lut4, (const float *)p.d_aux, d_img, (const float2 *)p.d_angles, k,
                                        st.pads, st.w2, st.Q, st.partial);
-    if (st.Q > 1) {
-      const size_t total = (size_t)nz * n * n;
-      bs_adj_sum_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(st.partial, st.Q, total, d_img);
-    }
+    bs_adj_sum_kernel<<<dim3((unsigned)(((size_t)n * n + 255) / 256), nz), 256, 0, s>>>(
+        st.partial, st.Q, d_img, d_sino, st.mark, (const float2 *)p.d_angles, (const float *)p.d_aux, k);
     TOMO_CUDA(cudaGetLastError());
     return TOMO_OK;
   }

@@ -47,6 +47,11 @@ __device__ __forceinline__ F2 fma2_rd(F2 a, F2 b, F2 c) {
   asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
   return r;
 }
+__device__ __forceinline__ F2 fma2_ru(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rp.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
 // c - a, rounded once
 __device__ __forceinline__ F2 rsub2(F2 a, F2 c) { return fma2(a, f2(-1.0f), c); }
 

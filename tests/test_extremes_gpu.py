@@ -65,3 +65,60 @@ def test_infinite_values_at_zero_weights(cuda, oracle, oper, n):
         ref = orc(1, y)
         assert np.isnan(ref).any()
         _compare(cuda, tp.At, ref, y)
+
+
+def _bspline(n, oracle):
+    from iterative_tomographic_reconstruction_algorithms_b200 import class_projectors_bspline as cpb
+    tp = cpb.projectors(n, np.arange(24))  # 0, 45, 90 and 135 degrees among them
+    return tp, lambda d, a: oracle.bspline(d, a, tp.angles, tp.lut, tp.param_spline)
+
+
+@pytest.mark.parametrize("n", [40, 41, 300, 1100])
+def test_bspline_values_next_to_the_largest_float(cuda, oracle, n):
+    """Forward: neighbouring values that overflow a line's float sum in places where the bin is
+    finite (off by the rounding of at most 12 products).  Adjoint: bin 0, whose value counts twice."""
+    tp, orc = _bspline(n, oracle)
+    x = np.zeros((n, n), np.float32)
+    x[n // 2 + 3, n // 3:n // 3 + 6] = [3.1e38, 3.1e38, 3.1e38, -3.1e38, -3.1e38, -3.1e38]
+    ref = orc(0, x)
+    lim = float(np.finfo(np.float32).max)
+    keep = np.abs(np.abs(ref) / lim - 1) > 1e-4  # away from the edge itself
+    got = tp.A(cuda.from_numpy(x).cuda()).cpu().numpy()
+    assert np.array_equal(np.isfinite(got)[keep], (np.abs(ref) < lim)[keep])
+    fin = keep & (np.abs(ref) < lim)
+    assert np.all(np.abs(got[fin] - ref[fin]) <= 13 * 2.0 ** -24 * 3.1e38)
+    for v in (0, 3, 6, 12, 17):
+        y = np.zeros((24, n), np.float32)
+        y[v, 0] = BIG
+        fin = _compare(cuda, tp.At, orc(1, y), y)
+        assert fin.sum() > n * (n - 5)
+
+
+@pytest.mark.parametrize("n", [40, 41])
+def test_bspline_infinite_values(cuda, oracle, n):
+    tp, orc = _bspline(n, oracle)
+    rng = np.random.default_rng(n)
+    for value in (np.inf, -np.inf, np.nan):
+        x = rng.standard_normal((n, n)).astype(np.float32)
+        x[n // 3, n // 2 - 2] = value
+        y = rng.standard_normal((24, n)).astype(np.float32)
+        y[5, 0], y[7, n // 2], y[0, 1] = value, value, -value
+        for d, fn, a in ((0, tp.A, x), (1, tp.At, y)):
+            ref, got = orc(d, a), fn(cuda.from_numpy(a).cuda()).cpu().numpy()
+            for test in (np.isnan, np.isposinf, np.isneginf):
+                assert np.array_equal(test(got), test(ref)), (value, d, test.__name__)
+
+
+def test_bspline_table_that_is_not_finite(cuda, oracle):
+    """Such a table takes the general kernels, where only the taps that read it are touched."""
+    from iterative_tomographic_reconstruction_algorithms_b200 import _lib
+    n = 40
+    tp, _ = _bspline(n, oracle)
+    lut = np.array(tp.lut, np.float32)
+    lut[3, lut.shape[1] // 2 + 700] = np.nan
+    x = np.random.default_rng(1).standard_normal((n, n)).astype(np.float32)
+    ref = oracle.bspline(0, x, tp.angles, lut, tp.param_spline)
+    assert np.isnan(ref).any() and np.isfinite(ref).any()
+    plan = _lib.Plan(_lib.KIND_BSPLINE, n, tp.angles, lut=lut, lut_size=lut.shape[1], support=float(tp.param_spline[1]))
+    got = plan.forward(cuda.from_numpy(x[None]).cuda()).cpu().numpy()[0]
+    assert np.array_equal(np.isnan(got), np.isnan(ref))
