@@ -105,8 +105,9 @@ int tomo_nn_adam(float *p, const float *g, float *m, float *v, size_t n, float l
  * they give up: spins >= 0 sets the limit for later launches in this process
  * (0: give up at once, which only serves to exercise the give-up path), spins
  * < 0 restores the default of 2^22.  A kernel that gives up sets bit 0 of the
- * status word, stores nothing, and before freeing its tensor memory waits for
- * its last committed MMAs with the long default limit whatever this setting. */
+ * status word, and before freeing its tensor memory waits for its last committed
+ * MMAs with the long default limit whatever this setting.  What such a call
+ * stored is unspecified (tiles done before, sums of partial results). */
 int tomo_nn_set_wait_limit(int spins);
 
 /* Reads and clears the device status word of the current device (bit 0: a

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_tc_kernel(ConvArgs g, co
     int job = set;
     for (int grp = grp0 + set * gstep; grp < g.ngroups; grp += 2 * gstep, job += 2) {
       const int tc = min(g.T, g.ntiles - grp * g.T);
-      ok = role_wait(&afull[set], (job >> 1) & 1, g.spins, &gave_up);
+      ok = warp_wait(&afull[set], (job >> 1) & 1, g.spins, &gave_up);  // the loads below take the whole warp
       if (!ok) break;
       tc_fence_after();
       for (int t = 0; t < tc; ++t) {
@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_tc_kernel(ConvArgs g, co
         const size_t o = in ? (((size_t)b * g.H + y) * g.W + x) * g.Cout + n0 : 0;
         for (int c0 = 0; c0 < nv; c0 += 16) {
           float v[16];
+          __syncwarp();  // lanes outside the image skipped the stores
           tmem_ld16(tmem + ((uint32_t)(w4 * 32) << 16) + (uint32_t)((set * g.T + t) * g.BN + c0), v);
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
