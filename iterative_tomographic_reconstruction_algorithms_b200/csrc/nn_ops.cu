@@ -135,7 +135,9 @@ int tomo_nn_conv3x3_masked(const void *X, int batch, int H, int W, int Cin, cons
 }
 
 size_t tomo_nn_wgrad_workspace(int batch, int H, int W, int Cin, int Cout, int taps) {
-  if ((taps != 9 && taps != 1) || Cin < 8 || Cout < 1 || batch < 1 || H < 1 || W < 1) return 256;
+  if ((taps != 9 && taps != 1) || Cin < 8 || Cout < 1 || batch < 1 || H < 1 || W < 1 ||
+      (long long)H * W > 0x7fffffffLL / batch)
+    return 256;  // tomo_nn_wgrad refuses these
   return wgrad_workspace(batch, H, W, Cin, Cout, taps);
 }
 
