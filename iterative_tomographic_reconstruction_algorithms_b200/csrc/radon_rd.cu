@@ -202,12 +202,44 @@ __device__ __forceinline__ void rd_walk_checked(const RdGeom &s, int n, int nh, 
   }
 }
 
+// rd_walk_free's steps with one new crossing each (two on a diagonal step), chosen by
+// selects: the adjoint with a thread per bin, bound by its reductions, takes 0.3 to
+// 0.7 % longer with both axes' crossings (2048^2 x 1800: 99.8 ms, 100.3).  With a thread
+// per sub-ray it is the other way round (513^2 x 400: 1.595, 1.585).
+template <class Visit>
+__device__ __forceinline__ void rd_walk_select(const RdGeom &s, int nh, int sA, int sB, int pad, float rx, float ry,
+                                               Visit &visit) {
+  const float incr = __fsqrt_rn(__fmaf_rn(s.ex, s.ex, __fmul_rn(s.ey, s.ey)));
+  const float hx = s.dx > 0 ? 0.5f : -0.5f, hy = s.dy > 0 ? 0.5f : -0.5f;
+  const float fdx = hx + hx, fdy = hy + hy;
+  const float Px = rintf(s.p1x), Py = rintf(s.p1y);
+  const float fx = __fsub_rn(s.p1x, Px), fy = __fsub_rn(s.p1y, Py);
+  float mx = __fsub_rn(__fadd_rn((float)s.ii0, hx), Px), my = __fsub_rn(__fadd_rn((float)s.jj0, hy), Py);
+  float ax = rd_alpha_mf(mx, fx, s.ex, rx), ay = rd_alpha_mf(my, fy, s.ey, ry);
+  int off = (s.ii0 + nh + pad) * sA + (s.jj0 + nh + pad) * sB;
+  const int ox = s.dx * sA, oy = s.dy * sB;
+  float alpha = 0.0f, alpha_old = 0.0f;
+  while (alpha <= 1.0f) {
+    const bool sx = ax <= ay, sy = ay <= ax;
+    alpha = sx ? ax : ay;
+    mx = sx ? __fadd_rn(mx, fdx) : mx;
+    my = sy ? __fadd_rn(my, fdy) : my;
+    off += (sx ? ox : 0) + (sy ? oy : 0);
+    const float a1 = rd_alpha_mf(sx ? mx : my, sx ? fx : fy, sx ? s.ex : s.ey, sx ? rx : ry);
+    ax = sx ? a1 : ax;
+    ay = sx ? ay : a1;
+    if (sx && sy) ay = rd_alpha_mf(my, fy, s.ey, ry);
+    visit(true, off, __fmul_rn(__fsub_rn(alpha, alpha_old), incr));
+    alpha_old = alpha;
+  }
+}
+
 // Both axes' next crossings are computed every step, as one packed pair: the axis
 // that did not step gets its value again, and nothing has to be selected between
 // the axes (compares and selects go at half the rate of additions).  Forward at
 // 768^2 x 720 with selects and one crossing per step 4.33 ms, now 4.04, 3.96 with
 // the gather two steps ahead; at 2048^2 x 1800 75.7, 70.4, 68.9.  The adjoint is
-// bound by its reductions (83 % of L1's throughput) and takes as long either way.
+// bound by its reductions (83 % of L1's throughput): see rd_walk_select.
 // nz is a -0 the compiler does not know: a product that goes into an addition
 // must be rounded first, and h r + nz is (a mul2 would be contracted).
 // q2 -+ d (rd_alpha_mf) are one fma each, of q1 2^-38 with q1's sign: the two
@@ -535,7 +567,7 @@ __global__ void __launch_bounds__(128) rd_scatter_kernel(
     const RdGeom s = rd_geom_of(tab, v, toff, 6 * b + r, n, nh);
     const float rx = __frcp_rn(s.ex), ry = __frcp_rn(s.ey);
     if (rd_walk_framed(s, nh, rx, ry))
-      rd_walk_free(s, nh, sA, sB, 1, rx, ry, nz, add);
+      kSplit ? rd_walk_free(s, nh, sA, sB, 1, rx, ry, nz, add) : rd_walk_select(s, nh, sA, sB, 1, rx, ry, add);
     else
       rd_walk_safe(s, n, nh, sA, sB, 1, rx, ry, add);
   }
