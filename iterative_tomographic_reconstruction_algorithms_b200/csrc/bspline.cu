@@ -648,8 +648,8 @@ struct BsState {
   void *work = nullptr;       // one workspace for what follows
   float4 *lut4 = nullptr, *S4 = nullptr;
   float *rows = nullptr, *cols = nullptr, *partial = nullptr;
-  int *mark = nullptr;  // [nz][na]
-  int pads = 0, w2 = 0, Q = 1, entries = 0;
+  int *mark = nullptr;  // [chunk][na]
+  int pads = 0, w2 = 0, Q = 1, entries = 0, chunk = 1;
 };
 
 void bs_state_free(void *q) {
@@ -699,8 +699,11 @@ int bs_setup(Plan &p) {
     st->w2 = n + 2 * st->pads;
     st->Q = bs_adj_shares(n);
     st->entries = 8 * (int)k.lut_step + 8;
-    const size_t nz = p.g.nz, lut4 = (size_t)na * 2 * (size_t)k.lut_step, s4 = nz * na * st->w2;
-    const size_t framed = nz * n * (n + 2 * kBsFrame), part = st->Q > 1 ? st->Q * nz * n * n : 0;
+    // the weights, and the rest for a chunk of slices
+    const size_t lut4 = (size_t)na * 2 * (size_t)k.lut_step, s41 = (size_t)na * st->w2, framed1 = (size_t)n * (n + 2 * kBsFrame);
+    const size_t part1 = st->Q > 1 ? (size_t)st->Q * n * n : 0;
+    st->chunk = slice_chunk(p, sizeof(float4) * s41 + sizeof(float) * (2 * framed1 + part1) + sizeof(int) * na);
+    const size_t nz = st->chunk, s4 = nz * s41, framed = nz * framed1, part = nz * part1;
     TOMO_CUDA(cudaMalloc(&st->work, sizeof(float4) * (lut4 + s4) + sizeof(float) * (2 * framed + part) + sizeof(int) * nz * na));
     st->lut4 = (float4 *)st->work;
     st->S4 = st->lut4 + lut4;
@@ -726,10 +729,13 @@ int bs_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
   BsState &st = *(BsState *)p.ext;
   if (st.pow2 && !ep.ordered) {
     const int n = k.n, tiles = (n + 2 * kBsFrame + 31) / 32, split = bs_fwd_split(n), bins = 128 / split;
-    bs_frame_kernel<<<dim3(tiles, tiles, p.g.nz), dim3(32, 8), 0, s>>>(d_img, st.rows, st.cols, n);
     auto fn = split == 4 ? bs_forward_pow2_kernel<4> : bs_forward_pow2_kernel<2>;
-    fn<<<dim3((n + bins - 1) / bins, k.na, p.g.nz), 128, sizeof(float) * (st.entries + 1), s>>>(
-        st.rows, st.cols, d_sino, (const float2 *)p.d_angles, (const float *)p.d_aux, st.entries, k);
+    for (int z0 = 0; z0 < p.g.nz; z0 += st.chunk) {
+      const int zc = std::min(st.chunk, p.g.nz - z0);
+      bs_frame_kernel<<<dim3(tiles, tiles, zc), dim3(32, 8), 0, s>>>(d_img + (size_t)z0 * n * n, st.rows, st.cols, n);
+      fn<<<dim3((n + bins - 1) / bins, k.na, zc), 128, sizeof(float) * (st.entries + 1), s>>>(
+          st.rows, st.cols, d_sino + (size_t)z0 * k.na * n, (const float2 *)p.d_angles, (const float *)p.d_aux, st.entries, k);
+    }
     TOMO_CUDA(cudaGetLastError());
     return TOMO_OK;
   }
@@ -749,14 +755,18 @@ int bs_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const
   BsState &st = *(BsState *)p.ext;
   if (st.pow2 && !ep.ordered) {
     const int n = k.n, nz = p.g.nz;
-    bs_expand_kernel<<<k.na * nz, 256, 0, s>>>(d_sino, st.S4, st.mark, n, st.pads, st.w2);
-    const dim3 grid((n + kBsTW - 1) / kBsTW * st.Q, (n + kBsTH - 1) / kBsTH, nz);
     const size_t smem = sizeof(float4) * 2 * (size_t)k.lut_step;
     auto fn = (n & 1) ? bs_adjoint_pow2_kernel<true> : bs_adjoint_pow2_kernel<false>;
-    fn<<<grid, kBsThreads4, smem, s>>>(d_sino, st.S4, st.lut4, (const float *)p.d_aux, d_img, (const float2 *)p.d_angles, k,
-                                       st.pads, st.w2, st.Q, st.partial);
-    bs_adj_sum_kernel<<<dim3((unsigned)(((size_t)n * n + 255) / 256), nz), 256, 0, s>>>(
-        st.partial, st.Q, d_img, d_sino, st.mark, (const float2 *)p.d_angles, (const float *)p.d_aux, k);
+    for (int z0 = 0; z0 < nz; z0 += st.chunk) {
+      const int zc = std::min(st.chunk, nz - z0);
+      const float *sino = d_sino + (size_t)z0 * k.na * n;
+      float *img = d_img + (size_t)z0 * n * n;
+      bs_expand_kernel<<<k.na * zc, 256, 0, s>>>(sino, st.S4, st.mark, n, st.pads, st.w2);
+      fn<<<dim3((n + kBsTW - 1) / kBsTW * st.Q, (n + kBsTH - 1) / kBsTH, zc), kBsThreads4, smem, s>>>(
+          sino, st.S4, st.lut4, (const float *)p.d_aux, img, (const float2 *)p.d_angles, k, st.pads, st.w2, st.Q, st.partial);
+      bs_adj_sum_kernel<<<dim3((unsigned)(((size_t)n * n + 255) / 256), zc), 256, 0, s>>>(
+          st.partial, st.Q, img, sino, st.mark, (const float2 *)p.d_angles, (const float *)p.d_aux, k);
+    }
     TOMO_CUDA(cudaGetLastError());
     return TOMO_OK;
   }

@@ -52,6 +52,20 @@ struct AdjEpi {
   bool ordered = false;
 };
 
+// The same for the slices from the one whose first element is e on (slots: residual
+// slots of the slices before).
+inline FwdEpi epi_from(FwdEpi ep, size_t e, size_t slots) {
+  if (ep.b) ep.b += e;
+  if (ep.w) ep.w += e;
+  if (ep.resid) ep.resid += slots;
+  return ep;
+}
+inline AdjEpi epi_from(AdjEpi ep, size_t e) {
+  if (ep.x) ep.x += e;
+  if (ep.aux) ep.aux += e;
+  return ep;
+}
+
 __device__ __forceinline__ unsigned float_to_ordered(float f) {
   unsigned u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);

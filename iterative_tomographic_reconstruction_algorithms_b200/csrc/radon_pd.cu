@@ -421,9 +421,9 @@ __global__ void __launch_bounds__(32 * Q) pd_adjoint_kernel(const float2 *__rest
 
 // What the pair owns beside the angle table.
 struct PdState {
-  float *rows = nullptr, *cols = nullptr;  // [nz][n][n + 2 kPdFrame]
-  float2 *pairs = nullptr;    // [nz][na][w2]
-  int pads = 0, w2 = 0;
+  float *rows = nullptr, *cols = nullptr;  // [chunk][n][n + 2 kPdFrame]
+  float2 *pairs = nullptr;                 // [chunk][na][w2]
+  int pads = 0, w2 = 0, chunk = 1;
 };
 
 void pd_state_free(void *q) {
@@ -462,8 +462,10 @@ int pd_setup(Plan &p) {
   // up to 3 outside the image
   st->pads = (int)std::ceil((p.nh + 1) * 0.41422) + 12;
   st->w2 = p.g.n + 2 * st->pads;
-  // one workspace: the adjoint's pairs, then the forward's framed copies
-  const size_t pairs = (size_t)p.g.nz * na * st->w2, framed = (size_t)p.g.nz * p.g.n * (p.g.n + 2 * kPdFrame);
+  // one workspace for a chunk of slices: the adjoint's pairs, then the forward's framed copies
+  const size_t pairs1 = (size_t)na * st->w2, framed1 = (size_t)p.g.n * (p.g.n + 2 * kPdFrame);
+  st->chunk = slice_chunk(p, sizeof(float2) * pairs1 + 2 * sizeof(float) * framed1);
+  const size_t pairs = st->chunk * pairs1, framed = st->chunk * framed1;
   TOMO_CUDA(cudaMalloc(&st->pairs, sizeof(float2) * pairs + 2 * sizeof(float) * framed));
   st->rows = (float *)(st->pairs + pairs);
   st->cols = st->rows + framed;
@@ -476,11 +478,16 @@ int pd_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
   PdState &st = *(PdState *)p.ext;
   const int tiles = (n + 2 * kPdFrame + 31) / 32;
-  pd_frame_kernel<<<dim3(tiles, tiles, nz), dim3(32, 8), 0, s>>>(d_img, st.rows, st.cols, n);
   const int split = ep.ordered ? 0 : pd_fwd_split(n), warps = split > 1 ? split : kPdAng;
   auto fn = split == 8 ? pd_forward_kernel<8> : split == 4 ? pd_forward_kernel<4> : split == 1 ? pd_forward_kernel<1> : pd_forward_kernel<0>;
-  fn<<<dim3((n + 31) / 32, split > 1 ? na : (na + kPdAng - 1) / kPdAng, nz), 32 * warps, 0, s>>>(
-      st.rows, st.cols, d_sino, (const PdAngle *)p.d_angles, n, p.nh, na, ep);
+  const size_t per = (size_t)n * n, per_sino = (size_t)na * n, slots = p.fwd_warps / nz;
+  for (int z0 = 0; z0 < nz; z0 += st.chunk) {
+    const int zc = std::min(st.chunk, nz - z0);
+    pd_frame_kernel<<<dim3(tiles, tiles, zc), dim3(32, 8), 0, s>>>(d_img + z0 * per, st.rows, st.cols, n);
+    fn<<<dim3((n + 31) / 32, split > 1 ? na : (na + kPdAng - 1) / kPdAng, zc), 32 * warps, 0, s>>>(
+        st.rows, st.cols, d_sino + z0 * per_sino, (const PdAngle *)p.d_angles, n, p.nh, na,
+        epi_from(ep, z0 * per_sino, z0 * slots));
+  }
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
 }
@@ -488,15 +495,19 @@ int pd_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
 int pd_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const AdjEpi &ep) {
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
   PdState &st = *(PdState *)p.ext;
-  pd_expand_kernel<<<na * nz, 256, 0, s>>>(d_sino, st.pairs, n, st.pads, st.w2);
   const int Q = ep.ordered ? 1 : pd_adj_warps(n), R = ep.ordered && n <= 1024 ? 1 : 4;
   auto fn = R == 1    ? pd_adjoint_kernel<1, 1>
             : Q == 1  ? pd_adjoint_kernel<1, 4>
             : Q == 4  ? pd_adjoint_kernel<4, 4>
             : Q == 8  ? pd_adjoint_kernel<8, 4>
                       : pd_adjoint_kernel<16, 4>;
-  fn<<<dim3((n + 31) / 32, (n + 4 * R - 1) / (4 * R), nz), 32 * Q, 0, s>>>(
-      st.pairs, d_img, (const PdAngle *)p.d_angles, n, p.nh, na, st.pads, st.w2, ep);
+  const size_t per = (size_t)n * n, per_sino = (size_t)na * n;
+  for (int z0 = 0; z0 < nz; z0 += st.chunk) {
+    const int zc = std::min(st.chunk, nz - z0);
+    pd_expand_kernel<<<na * zc, 256, 0, s>>>(d_sino + z0 * per_sino, st.pairs, n, st.pads, st.w2);
+    fn<<<dim3((n + 31) / 32, (n + 4 * R - 1) / (4 * R), zc), 32 * Q, 0, s>>>(
+        st.pairs, d_img + z0 * per, (const PdAngle *)p.d_angles, n, p.nh, na, st.pads, st.w2, epi_from(ep, z0 * per));
+  }
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
 }

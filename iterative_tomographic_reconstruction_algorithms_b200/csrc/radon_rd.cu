@@ -616,8 +616,7 @@ size_t rd_framed(const Plan &p) { return (size_t)(p.g.n + 3) * (p.g.n + 3); }
 
 int rd_chunk(const Plan &p) {
   const size_t per = 16 * rd_framed(p) + 16 * (size_t)p.g.n + 4 * rd_flag_words(p);
-  const size_t cap = std::min<size_t>(((size_t)512 << 20) / per, 65535);
-  return (int)std::max<size_t>(1, std::min<size_t>((size_t)p.g.nz, cap));
+  return slice_chunk(p, per);
 }
 
 }  // namespace

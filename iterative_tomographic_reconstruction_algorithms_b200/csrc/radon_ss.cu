@@ -321,10 +321,10 @@ __global__ void __launch_bounds__(32 * Q, (Q == 1 ? 0 : Q == 4 ? 28 : 32) / Q) s
 int ss_adj_warps(int n) { return n > 640 ? 4 : n > 384 ? 8 : 16; }
 
 struct SsState {
-  float2 *pairs = nullptr;                 // [nz][na][w2]
-  int *raw = nullptr;                      // [nz][na]
-  float *rows = nullptr, *cols = nullptr;  // [nz][n][n + 2 kSsFrame]
-  int pads = 0, w2 = 0;
+  float2 *pairs = nullptr;                 // [chunk][na][w2]
+  int *raw = nullptr;                      // [chunk][na]
+  float *rows = nullptr, *cols = nullptr;  // [chunk][n][n + 2 kSsFrame]
+  int pads = 0, w2 = 0, chunk = 1;
 };
 
 void ss_state_free(void *q) {
@@ -386,10 +386,13 @@ int ss_setup(Plan &p) {
   // tile that lie up to 3 outside the image
   st->pads = (int)std::ceil((nh + 1) * 0.41422) + 14;
   st->w2 = 2 * nh + 2 * st->pads;
-  // one workspace: the adjoint's pairs, then the forward's framed copies
+  // one workspace for a chunk of slices: the adjoint's pairs, the forward's framed
+  // copies, the marked rows
   const int n = p.g.n;
-  const size_t pairs = (size_t)p.g.nz * na * st->w2, framed = (size_t)p.g.nz * n * (n + 2 * kSsFrame);
-  TOMO_CUDA(cudaMalloc(&st->pairs, sizeof(float2) * pairs + 2 * sizeof(float) * framed + sizeof(int) * p.g.nz * na));
+  const size_t pairs1 = (size_t)na * st->w2, framed1 = (size_t)n * (n + 2 * kSsFrame);
+  st->chunk = slice_chunk(p, sizeof(float2) * pairs1 + 2 * sizeof(float) * framed1 + sizeof(int) * na);
+  const size_t pairs = st->chunk * pairs1, framed = st->chunk * framed1;
+  TOMO_CUDA(cudaMalloc(&st->pairs, sizeof(float2) * pairs + 2 * sizeof(float) * framed + sizeof(int) * st->chunk * na));
   st->rows = (float *)(st->pairs + pairs);
   st->cols = st->rows + framed;
   st->raw = (int *)(st->cols + framed);
@@ -402,11 +405,16 @@ int ss_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
   const int n = p.g.n, na = p.g.na, nz = p.g.nz, nh = p.nh;
   SsState &st = *(SsState *)p.ext;
   const int tiles = (n + 2 * kSsFrame + 31) / 32;
-  ss_frame_kernel<<<dim3(tiles, tiles, nz), dim3(32, 8), 0, s>>>(d_img, st.rows, st.cols, n);
   const int split = ep.ordered ? 0 : ss_fwd_split(n), rays = 128 / std::max(split, 1);
   auto fn = split == 4 ? ss_forward_kernel<4> : split == 2 ? ss_forward_kernel<2> : ss_forward_kernel<0>;
-  fn<<<dim3((n + rays - 1) / rays, na, nz), 128, 0, s>>>(st.rows, st.cols, d_sino, (const SsAngle *)p.d_angles,
-                                                         (const int2 *)p.d_aux, n, nh, na, ep);
+  const size_t per = (size_t)n * n, per_sino = (size_t)na * n, slots = p.fwd_warps / nz;
+  for (int z0 = 0; z0 < nz; z0 += st.chunk) {
+    const int zc = std::min(st.chunk, nz - z0);
+    ss_frame_kernel<<<dim3(tiles, tiles, zc), dim3(32, 8), 0, s>>>(d_img + z0 * per, st.rows, st.cols, n);
+    fn<<<dim3((n + rays - 1) / rays, na, zc), 128, 0, s>>>(st.rows, st.cols, d_sino + z0 * per_sino,
+                                                           (const SsAngle *)p.d_angles, (const int2 *)p.d_aux, n, nh, na,
+                                                           epi_from(ep, z0 * per_sino, z0 * slots));
+  }
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
 }
@@ -414,12 +422,17 @@ int ss_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
 int ss_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const AdjEpi &ep) {
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
   SsState &st = *(SsState *)p.ext;
-  ss_expand_kernel<<<dim3(na, nz), 256, 0, s>>>(d_sino, st.pairs, st.raw, (const SsAngle *)p.d_angles, n, p.nh, na, st.pads,
-                                               st.w2, ep.ordered);
   const int Q = ep.ordered ? 1 : ss_adj_warps(n);
   auto fn = Q == 1 ? ss_adjoint_kernel<1> : Q == 4 ? ss_adjoint_kernel<4> : Q == 8 ? ss_adjoint_kernel<8> : ss_adjoint_kernel<16>;
-  fn<<<dim3((n + 31) / 32, (n + 15) / 16, nz), 32 * Q, 0, s>>>(st.pairs, st.raw, d_img, (const SsAngle *)p.d_angles,
-                                                               (const int2 *)p.d_aux, n, p.nh, na, st.pads, st.w2, ep);
+  const size_t per = (size_t)n * n, per_sino = (size_t)na * n;
+  for (int z0 = 0; z0 < nz; z0 += st.chunk) {
+    const int zc = std::min(st.chunk, nz - z0);
+    ss_expand_kernel<<<dim3(na, zc), 256, 0, s>>>(d_sino + z0 * per_sino, st.pairs, st.raw, (const SsAngle *)p.d_angles, n,
+                                                 p.nh, na, st.pads, st.w2, ep.ordered);
+    fn<<<dim3((n + 31) / 32, (n + 15) / 16, zc), 32 * Q, 0, s>>>(st.pairs, st.raw, d_img + z0 * per,
+                                                                 (const SsAngle *)p.d_angles, (const int2 *)p.d_aux, n, p.nh,
+                                                                 na, st.pads, st.w2, epi_from(ep, z0 * per));
+  }
   TOMO_CUDA(cudaGetLastError());
   return TOMO_OK;
 }

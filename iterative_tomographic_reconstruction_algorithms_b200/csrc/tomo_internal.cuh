@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <mutex>
@@ -127,6 +128,13 @@ class PlanUse {
   int rc_ = 0;
   bool open_ = false, capturing_ = false;
 };
+
+// Slices that go through a kind's scratch of `per` bytes a slice at a time: all, or
+// as many as 512 MiB hold (one at least).
+inline int slice_chunk(const Plan &p, size_t per) {
+  const size_t cap = std::min<size_t>(((size_t)512 << 20) / per, 65535);
+  return (int)std::max<size_t>(1, std::min<size_t>((size_t)p.g.nz, cap));
+}
 
 size_t image_elems(const Plan &p);
 size_t sino_elems(const Plan &p);
