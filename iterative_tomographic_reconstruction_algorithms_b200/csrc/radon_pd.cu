@@ -11,8 +11,8 @@
 // (fftshifted) angle order of the input.
 //
 // Evaluation order of the compiled reference (-O3 -ffast-math, read from its
-// x86-64 code), reproduced exactly: t = |fma(-c, y, x*s)|, the sign test uses
-// (x*s) * (1/c), and the first weight is |(t + ceil(T)) - nh|.
+// x86-64 code), reproduced exactly: t = |fma(-c, y, x*s)|, its sign for every angle
+// that of pd_line, and the first weight is |(t + ceil(T)) - nh|.
 //
 // Forward = gather per bin over image lines; adjoint = gather per pixel over
 // angles.  The duplicate sub-samples are evaluated once with weight 2 * 1/4.
@@ -25,7 +25,6 @@
 namespace tomo {
 namespace {
 
-constexpr double kPi = 3.141592653589793;
 constexpr float kPdMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr int kPdMagicBits = 0x4B400000;  // its bit pattern
 
@@ -442,15 +441,11 @@ int pd_setup(Plan &p) {
   const int na = p.g.na;
   std::vector<PdAngle> tab(na);
   for (int v = 0; v < na; ++v) {
-    const float theta = p.angles[v];
     float s, c;
-    sincosf(theta, &s, &c);
+    sincosf(p.angles[v], &s, &c);
     PdAngle a{};
     a.s = s;
     a.c = c;
-    a.rc = 1.0f / c;
-    a.flags = ((double)theta < kPi / 2 ? 1 : 0) | ((double)theta > kPi / 2 ? 2 : 0) |
-              (theta == 0.0f ? 4 : 0);
     tab[v] = a;
   }
   TOMO_CUDA(cudaMalloc(&p.d_angles, sizeof(PdAngle) * (size_t)na));

@@ -59,8 +59,7 @@ struct SsAngle {
 
 // Pixel-driven (radon_pd.c).
 struct PdAngle {
-  float s, c, rc;  // sin, cos, 1/c
-  int flags;       // 1: theta < pi/2, 2: theta > pi/2, 4: theta == 0
+  float s, c;  // sin, cos
 };
 
 // Ray-driven / Siddon (radon_rd.c).
