@@ -77,10 +77,10 @@ __global__ void __launch_bounds__(256) pd_frame_kernel(const float *__restrict__
 // The products are added in double and rounded once: deterministic, and as close
 // to their exact sum as the 64-bit fixed-point sums in shared memory that this
 // replaces.  Those took two 32-bit atomics per product, and bounded the forward:
-// 1.57 ms at 768^2 x 720, now 1.03 (2048^2 x 1800: 25.2, now 16.4).  Bound by
-// issue and the FP32 pipe.  (Adding a line's products in
-// float first takes 0.95 and 14.6, but keeps 24 bits of the sum, and reaches
-// infinity next to the largest float where the bin is finite.)
+// 1.57 ms at 768^2 x 720, now 0.96 (2048^2 x 1800: 25.2, now 16.2).  Bound by
+// issue and the FP32 pipe.  (Adding a line's products in float first takes a tenth
+// less, but keeps 24 bits of the sum, and reaches infinity next to the largest float
+// where the bin is finite.)
 
 // A bin and its angle, as both loops use them.
 template <bool ROWS, int DIR>
@@ -225,21 +225,21 @@ __device__ __forceinline__ double pd_fwd_bin(const float *__restrict__ L, int w,
   return acc;
 }
 
-// SPLIT = 1: a block takes 32 bins of kPdAng angles, whose warps read the same
-// pixels.  SPLIT > 1, for small images, whose bins alone are too few warps to
-// hide a line's latency: one angle, its lines shared by SPLIT warps, whose sums
-// are added in order.  The split depends on n alone (pd_fwd_split), so a plan
-// for some of the angles or several slices gives the same bits.  SPLIT = 0: as 1
-// in the solvers' form (epilogue.cuh), pd_fwd_exact.
+// A block takes 32 bins of an angle, whose lines SPLIT warps share (their sums are
+// added in order): bins alone are too few warps to hide a line's latency in small
+// images, and few enough in large ones that the blocks' ends show.  The split
+// depends on n alone (pd_fwd_split), so a plan for some of the angles or several
+// slices gives the same bits.  SPLIT = 0 is the solvers' form (epilogue.cuh),
+// pd_fwd_exact with a warp per bin, four angles to a block.
 constexpr int kPdAng = 4;
 
 template <int SPLIT>
-__global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : kPdAng), 32 / (SPLIT > 1 ? SPLIT : kPdAng)) pd_forward_kernel(
+__global__ void __launch_bounds__(32 * (SPLIT ? SPLIT : kPdAng), 32 / (SPLIT ? SPLIT : kPdAng)) pd_forward_kernel(
     const float *__restrict__ rows, const float *__restrict__ cols, float *__restrict__ sino, const PdAngle *__restrict__ tab,
     int n, int nh, int na, FwdEpi ep) {
-  constexpr int kParts = SPLIT > 1 ? SPLIT : 1;
+  constexpr int kParts = SPLIT ? SPLIT : 1;
   __shared__ double part[kParts][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, v = SPLIT > 1 ? blockIdx.y : blockIdx.y * kPdAng + warp;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, v = SPLIT ? blockIdx.y : blockIdx.y * kPdAng + warp;
   const int B0 = blockIdx.x * 32, b = B0 + lane, w = n + 2 * kPdFrame;
   const size_t z = blockIdx.z;
   const bool live = v < na && b < n;
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : kPdAng), 32 / (SPLIT
       i0 = max(0, (int)floorf(fminf(fmaxf(fminf(l0, l1) + fnh - 2.0f, 0.0f), (float)n)));
       i1 = min(n, (int)ceilf(fminf(fmaxf(fmaxf(l0, l1) + fnh + 2.0f, 0.0f), (float)n)));
     }
-    if (SPLIT > 1) {
+    if (SPLIT) {
       const int len = max(0, i1 - i0);
       i1 = i0 + len * (warp + 1) / kParts;
       i0 += len * warp / kParts;
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : kPdAng), 32 / (SPLIT
     else acc = c < 0.0f ? PD_BIN(false, 1) : PD_BIN(false, -1);
 #undef PD_BIN
   }
-  if (SPLIT > 1) {
+  if (SPLIT) {
     part[warp][lane] = acc;
     __syncthreads();
     if (warp > 0) return;
@@ -279,10 +279,14 @@ __global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : kPdAng), 32 / (SPLIT
   const size_t e = z * (size_t)na * n + (size_t)v * n + b;
   if (live) sino[e] = fwd_apply(ep, out, e, r2);
   const size_t block = ((size_t)z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  fwd_resid_commit(ep, r2, SPLIT > 1 ? block : block * kPdAng + warp);
+  fwd_resid_commit(ep, r2, SPLIT ? block : block * kPdAng + warp);
 }
 
-int pd_fwd_split(int n) { return n > 448 ? 1 : n > 320 ? 4 : 8; }
+// ms with 1 (four angles to a block), 4, 8 warps: 200^2 x 200 0.046, 0.042, 0.038; 320^2
+// x 320 0.114, 0.099, 0.097; 384^2 x 400 0.177, 0.159, 0.157; 512^2 x 500 0.353, 0.321, 0.319;
+// 768^2 x 720 1.033, 0.962, 0.966; 2048^2 x 1800 16.4, 16.2, 16.2.  Several slices do with
+// fewer (8 x 256^2 x 300: 0.402, 0.390, 0.401), but a slice has the same bits in any call.
+int pd_fwd_split(int n) { return n > 320 ? 4 : 8; }
 
 // Sinogram rows as pairs, entry e = l + pads of angle v: {S_l, S_l+1}, the two
 // bins a sub-sample with floor(T) = l is split between; bin 0 and the bins
@@ -315,7 +319,7 @@ __global__ void __launch_bounds__(256) pd_expand_kernel(const float *__restrict_
 // sub-sample, whose table pairs hit L1.  The two sub-samples go as f32x2 pairs,
 // which halves the instructions (scalar ones: 0.57 ms against 0.51).  A thread
 // per pixel with four reads, bounds tests and the sign rule per sub-sample took
-// 1.52 ms at 768^2 x 720 and 25.5 at 2048^2 x 1800; this one 0.51 and 8.1.
+// 1.52 ms at 768^2 x 720 and 25.5 at 2048^2 x 1800; this one 0.49 and 8.0.
 constexpr int kPdGrp = 2;  // pixels that share the test for an integral T
 template <int Q, int R>
 __global__ void __launch_bounds__(32 * Q) pd_adjoint_kernel(const float2 *__restrict__ pairs, float *__restrict__ img,
@@ -431,9 +435,10 @@ void pd_state_free(void *q) {
   delete st;
 }
 
-// Warps of an adjoint tile: more shares of the angles where the tiles alone
-// leave the SMs short of warps (148 x 32 of them hide the reads' latency).
-int pd_adj_warps(int n) { return n > 640 ? 4 : n > 384 ? 8 : 16; }
+// Warps of an adjoint tile.  ms with 4, 8, 16: 256^2 x 300 0.079, 0.052, 0.040; 320^2 x
+// 320 0.089, 0.071, 0.071; 512^2 x 500 0.196, 0.187, 0.192; 768^2 x 720 0.510, 0.491, 0.513;
+// 2048^2 x 1800 8.03, 8.03, 8.51.  (8 x 256^2 x 300: 0.200, 0.192, 0.212.)
+int pd_adj_warps(int n) { return n > 320 ? 8 : 16; }
 
 }  // namespace
 
@@ -473,13 +478,13 @@ int pd_forward(Plan &p, const float *d_img, float *d_sino, cudaStream_t s, const
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
   PdState &st = *(PdState *)p.ext;
   const int tiles = (n + 2 * kPdFrame + 31) / 32;
-  const int split = ep.ordered ? 0 : pd_fwd_split(n), warps = split > 1 ? split : kPdAng;
-  auto fn = split == 8 ? pd_forward_kernel<8> : split == 4 ? pd_forward_kernel<4> : split == 1 ? pd_forward_kernel<1> : pd_forward_kernel<0>;
+  const int split = ep.ordered ? 0 : pd_fwd_split(n), warps = split ? split : kPdAng;
+  auto fn = split == 8 ? pd_forward_kernel<8> : split == 4 ? pd_forward_kernel<4> : pd_forward_kernel<0>;
   const size_t per = (size_t)n * n, per_sino = (size_t)na * n, slots = p.fwd_warps / nz;
   for (int z0 = 0; z0 < nz; z0 += st.chunk) {
     const int zc = std::min(st.chunk, nz - z0);
     pd_frame_kernel<<<dim3(tiles, tiles, zc), dim3(32, 8), 0, s>>>(d_img + z0 * per, st.rows, st.cols, n);
-    fn<<<dim3((n + 31) / 32, split > 1 ? na : (na + kPdAng - 1) / kPdAng, zc), 32 * warps, 0, s>>>(
+    fn<<<dim3((n + 31) / 32, split ? na : (na + kPdAng - 1) / kPdAng, zc), 32 * warps, 0, s>>>(
         st.rows, st.cols, d_sino + z0 * per_sino, (const PdAngle *)p.d_angles, n, p.nh, na,
         epi_from(ep, z0 * per_sino, z0 * slots));
   }
@@ -493,7 +498,6 @@ int pd_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const
   const int Q = ep.ordered ? 1 : pd_adj_warps(n), R = ep.ordered && n <= 1024 ? 1 : 4;
   auto fn = R == 1    ? pd_adjoint_kernel<1, 1>
             : Q == 1  ? pd_adjoint_kernel<1, 4>
-            : Q == 4  ? pd_adjoint_kernel<4, 4>
             : Q == 8  ? pd_adjoint_kernel<8, 4>
                       : pd_adjoint_kernel<16, 4>;
   const size_t per = (size_t)n * n, per_sino = (size_t)na * n;

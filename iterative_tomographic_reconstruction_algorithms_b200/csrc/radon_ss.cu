@@ -114,6 +114,10 @@ __global__ void __launch_bounds__(128) ss_forward_kernel(const float *__restrict
   fwd_resid_commit(ep, r2, block * (kRays / 32) + lane / 32);
 }
 
+// ms with 2, 4 warps: 256^2 x 300 0.040, 0.038; 448^2 x 450 0.108, 0.099; 640^2 x 600 0.235,
+// 0.233; 768^2 x 720 0.374, 0.378; 2048^2 x 1800 6.18, 6.40; several slices want fewer (4 x 641^2
+// x 600: 0.781, 0.851; 8 x 256^2 x 300: 0.149, 0.151), but a slice has the same bits in any
+// call.
 int ss_fwd_split(int n) { return n > 448 ? 2 : 4; }
 
 // Sinogram rows as pairs in the order of the angles, entry e = t + nh + pads of
@@ -164,8 +168,8 @@ __global__ void __launch_bounds__(256) ss_expand_kernel(const float *__restrict_
 //
 // Bound by FP32 and issue.  Candidate rays checked one by one against their
 // limits, each credited to 4 pixels by 8 tests, took 3.53 ms at 4 x 641^2 x
-// 600 and 18.1 at 2048^2 x 1800; this takes 1.24 and 6.7 (with the reference's two
-// forms of the weight in every mode 1.88 and 9.6).
+// 600 and 18.1 at 2048^2 x 1800; this takes 1.16 and 6.7 (with the reference's two
+// forms of the weight in every mode half as long again).
 
 // Whether ray t passes major coordinate m (without branches: the loads of a
 // block's rays overlap).
@@ -237,8 +241,8 @@ __device__ __forceinline__ void ss_adj_angle(const SsAngle &g, const float2 *__r
   }
 }
 
-// 28 warps per SM at Q = 4 (72 registers) took 1.235 and 6.7 ms, 32 (64, with 12
-// bytes spilled) 1.29 and 6.8.
+// Q = 4: 28 warps per SM (72 registers) take 6.7 ms at 2048^2 x 1800, 32 (64, with 12
+// bytes spilled) 6.8.
 template <int Q>
 __global__ void __launch_bounds__(32 * Q, (Q == 1 ? 0 : Q == 4 ? 28 : 32) / Q) ss_adjoint_kernel(const float2 *__restrict__ pairs,
                                                             const int *__restrict__ raw, float *__restrict__ img,
@@ -316,9 +320,11 @@ __global__ void __launch_bounds__(32 * Q, (Q == 1 ? 0 : Q == 4 ? 28 : 32) / Q) s
     }
 }
 
-// Warps of an adjoint tile: more shares of the angles where the tiles alone
-// leave the SMs short of warps.
-int ss_adj_warps(int n) { return n > 640 ? 4 : n > 384 ? 8 : 16; }
+// Warps of an adjoint tile.  ms with 4, 8, 16: 256^2 x 300 0.118, 0.077, 0.058; 512^2 x 500
+// 0.271, 0.255, 0.222; 768^2 x 720 0.558, 0.536, 0.486; 1280^2 x 1024 1.69, 1.66, 1.62; 1600^2 x
+// 1400 3.32, 3.33, 3.30; 2048^2 x 1800 6.72, 6.78, 6.75; also for several slices (4 x 641^2 x
+// 600: 1.23, 1.21, 1.16).
+int ss_adj_warps(int n) { return n > 1800 ? 4 : 16; }
 
 struct SsState {
   float2 *pairs = nullptr;                 // [chunk][na][w2]
@@ -423,7 +429,7 @@ int ss_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
   SsState &st = *(SsState *)p.ext;
   const int Q = ep.ordered ? 1 : ss_adj_warps(n);
-  auto fn = Q == 1 ? ss_adjoint_kernel<1> : Q == 4 ? ss_adjoint_kernel<4> : Q == 8 ? ss_adjoint_kernel<8> : ss_adjoint_kernel<16>;
+  auto fn = Q == 1 ? ss_adjoint_kernel<1> : Q == 4 ? ss_adjoint_kernel<4> : ss_adjoint_kernel<16>;
   const size_t per = (size_t)n * n, per_sino = (size_t)na * n;
   for (int z0 = 0; z0 < nz; z0 += st.chunk) {
     const int zc = std::min(st.chunk, nz - z0);
