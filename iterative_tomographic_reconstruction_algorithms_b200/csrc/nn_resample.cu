@@ -5,7 +5,7 @@
 // convolution that they hand their gradient to (its output is what they read for
 // the pooling's argmax, or the upsampled input).  As chains of library passes
 // (upsample, cat, copies, pooling backward, add, ReLU) these were 6.9 of the 12.9
-// ms of a training step at 4 x 768^2, 32 channels, 4 levels; now 1.1.
+// ms of a training step at 4 x 768^2, 32 channels, 4 levels; now 0.66.
 //
 // Layouts: BF16, NHWC, channel counts multiples of 8, pointers 16-byte aligned.
 #include <cuda_bf16.h>

@@ -12,9 +12,9 @@
 // to the pixel it steps INTO (x index -> image row) if that pixel has row and
 // column in [1, n-1]; it stops after the first step with alpha > 1.
 //
-// Both directions run the same walks (rd_walk_free, rd_walk_checked), one thread per (bin, angle,
-// slice) replaying its bin's five sub-rays (the adjoint, on grids too small to
-// fill the GPU, one thread per sub-ray):
+// Both directions run the same walks (rd_walk_free, rd_walk_select, rd_walk_checked).  A
+// thread takes one of a bin's five sub-rays (forward of plain calls; adjoint up to
+// 600 000 bins) or all five in turn (solvers' forward; larger adjoints):
 //   forward  gathers 0.2 l x[pixel] into the bin, in walk order;
 //   adjoint  scatters 0.2 l y[bin] into a 64-bit fixed-point image with
 //            integer reductions (order-independent sums, so deterministic, of
