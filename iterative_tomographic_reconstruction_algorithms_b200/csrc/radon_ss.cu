@@ -152,8 +152,8 @@ __global__ void __launch_bounds__(256) ss_expand_kernel(const float *__restrict_
 // t) * rb lie |rb| = 1 / |cb| >= 1 apart, so a ray within 1 of the pixel's minor
 // coordinate c is within |cb| <= 1 of the crossing t* of c: it is floor(t*) or
 // the next.  It reaches c if f is in [c - 1, c + 1), with the forward's weight wt (f
-// - floor f) or wt (floor f + 1 - f), which are wt (1 - |f - c|) (to 2^-25 where f
-// has bits below those of c = +-1).  A rounding of t* across an integer loses
+// - floor f) or wt (floor f + 1 - f), which are wt (1 - |f - c|) but for the bits that f
+// has below those of c = +-1 (BOTH, ss_centre).  A rounding of t* across an integer loses
 // nothing while |cb| < 1 by more than that rounding (below n 2^-22 in all); the few
 // angles nearer to an axis (NEAR) look at the rays before and behind too.  The two
 // rays come as one pair, evaluated as packed operations.
@@ -168,8 +168,8 @@ __global__ void __launch_bounds__(256) ss_expand_kernel(const float *__restrict_
 //
 // Bound by FP32 and issue.  Candidate rays checked one by one against their
 // limits, each credited to 4 pixels by 8 tests, took 3.53 ms at 4 x 641^2 x
-// 600 and 18.1 at 2048^2 x 1800; this takes 1.16 and 6.7 (with the reference's two
-// forms of the weight in every mode half as long again).
+// 600 and 18.1 at 2048^2 x 1800; this takes 1.19 and 6.8 (with the reference's products
+// throughout half as long again).
 
 // Whether ray t passes major coordinate m (without branches: the loads of a
 // block's rays overlap).
@@ -199,7 +199,29 @@ __device__ __noinline__ float ss_adj_raw(float o, const SsAngle *__restrict__ ta
   return o;
 }
 
-template <bool STEEP, bool EDGE, bool NEAR, bool ORD>
+// What a row's credits to pixel (m, c), |c| = 1, lack: its rays' weights as f - floor f
+// or floor f + 1 - f, less those that the main loop takes, times wt S.
+__device__ __forceinline__ float ss_centre(const SsAngle &g, const float2 *__restrict__ row, const int2 *__restrict__ lrow,
+                                           int mi, int ci, int nh, bool limits, bool near) {
+  const float m = (float)mi, c = (float)ci, fm = __fadd_rd(fmaf(c, 1.0f / g.rb, m * g.a), kSsMagic), t0 = __fsub_rn(fm, kSsMagic);
+  const int ti = __float_as_int(fm) - kSsMagicBits;
+  float o = 0.0f;
+  auto ray = [&](int k, float S) {
+    const float f = __fmul_rn(__fmaf_rn(-m, g.a, t0 + (float)k), g.rb);
+    const float h = fminf(__fsub_rn(f, c - 1.0f), __fsub_rn(c + 1.0f, f)), q = 1.0f - fabsf(__fsub_rn(f, c));
+    if ((fmaxf(h, q) > 0.0f) & (!limits || ss_in_limits(lrow, ti + k, mi, nh))) o = fmaf(fmaxf(h, 0.0f) - fmaxf(q, 0.0f), S, o);
+  };
+  const float2 S = __ldg(row + nh + ti);
+  ray(0, S.x);
+  ray(1, S.y);
+  if (near) {
+    ray(-1, __ldg(row + nh + ti - 1).x);
+    ray(2, __ldg(row + nh + ti + 1).y);
+  }
+  return o;
+}
+
+template <bool STEEP, bool EDGE, bool NEAR, bool ORD, bool BOTH>
 __device__ __forceinline__ void ss_adj_angle(const SsAngle &g, const float2 *__restrict__ row, const int2 *__restrict__ lrow,
                                              int a0, int b0, int nh, float (&acc)[4][4]) {
   const int M0 = (STEEP ? a0 : b0) - nh, C0 = (STEEP ? b0 : a0) - nh;  // major and minor coordinates of the block
@@ -223,7 +245,7 @@ __device__ __forceinline__ void ss_adj_angle(const SsAngle &g, const float2 *__r
         if (ORD) {
           ss_credit(o, f, c, wt, S, in);
         } else {
-          const float h = 1.0f - fabsf(__fsub_rn(f, c));
+          const float h = BOTH ? fminf(__fsub_rn(f, c - 1.0f), __fsub_rn(c + 1.0f, f)) : 1.0f - fabsf(__fsub_rn(f, c));
           if ((h > 0.0f) & in) o = fmaf(h, S, o);
         }
       };
@@ -243,12 +265,13 @@ __device__ __forceinline__ void ss_adj_angle(const SsAngle &g, const float2 *__r
 
 // Q = 4: 28 warps per SM (72 registers) take 6.7 ms at 2048^2 x 1800, 32 (64, with 12
 // bytes spilled) 6.8.
-template <int Q>
+template <int Q, bool BOTH>
 __global__ void __launch_bounds__(32 * Q, (Q == 1 ? 0 : Q == 4 ? 28 : 32) / Q) ss_adjoint_kernel(const float2 *__restrict__ pairs,
                                                             const int *__restrict__ raw, float *__restrict__ img,
                                                             const SsAngle *__restrict__ tab, const int2 *__restrict__ lim,
                                                             int n, int nh, int na, int pads, int w2, AdjEpi ep) {
   __shared__ float part[Q > 1 ? (Q - 1) * 16 : 1][32];
+  __shared__ float centre[Q > 1 && !BOTH ? Q : 1][3][32];  // what the tile's pixels with |c| = 1 lack: two half columns, two rows
   const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
   // the tiles of the border take longest: both border rows of tiles first
   const int by = blockIdx.y == 0 ? 0 : blockIdx.y == 1 ? gridDim.y - 1 : blockIdx.y - 1;
@@ -261,13 +284,13 @@ __global__ void __launch_bounds__(32 * Q, (Q == 1 ? 0 : Q == 4 ? 28 : 32) / Q) s
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
   // the tile's pixels are all 4 or more inside the square [0, 2 nh - 1]
   const bool edge = blockIdx.x * 32 < 4 || by * 16 < 4 || blockIdx.x * 32 + 36 > 2 * nh || by * 16 + 20 > 2 * nh;
+  const float near = 1.0f - (float)n * 0x1p-22f;
   bool marked = false;  // rows of this warp's share
   if (Q > 1) {
     for (int u = q + Q * lane; u < na; u += Q * 32) marked |= __ldg(raw + z * na + u) != 0;
     marked = __any_sync(0xffffffffu, marked);
   }
   if (a0 < n && b0 < n) {
-    const float near = 1.0f - (float)n * 0x1p-22f;
     const float2 *row = pairs + (z * na + q) * (size_t)w2 + pads + nh - kSsMagicBits;
     const int2 *lrow = lim + (size_t)q * 2 * nh;
 #pragma unroll 1
@@ -276,14 +299,14 @@ __global__ void __launch_bounds__(32 * Q, (Q == 1 ? 0 : Q == 4 ? 28 : 32) / Q) s
       const bool nr = fabsf(g.rb) * near < 1.0f;
       if (marked && __ldg(raw + z * na + u)) continue;
       if (nr) {
-        if (g.steep) ss_adj_angle<true, true, true, Q == 1>(g, row, lrow, a0, b0, nh, acc);
-        else ss_adj_angle<false, true, true, Q == 1>(g, row, lrow, a0, b0, nh, acc);
+        if (g.steep) ss_adj_angle<true, true, true, Q == 1, BOTH>(g, row, lrow, a0, b0, nh, acc);
+        else ss_adj_angle<false, true, true, Q == 1, BOTH>(g, row, lrow, a0, b0, nh, acc);
       } else if (edge) {
-        if (g.steep) ss_adj_angle<true, true, false, Q == 1>(g, row, lrow, a0, b0, nh, acc);
-        else ss_adj_angle<false, true, false, Q == 1>(g, row, lrow, a0, b0, nh, acc);
+        if (g.steep) ss_adj_angle<true, true, false, Q == 1, BOTH>(g, row, lrow, a0, b0, nh, acc);
+        else ss_adj_angle<false, true, false, Q == 1, BOTH>(g, row, lrow, a0, b0, nh, acc);
       } else {
-        if (g.steep) ss_adj_angle<true, false, false, Q == 1>(g, row, lrow, a0, b0, nh, acc);
-        else ss_adj_angle<false, false, false, Q == 1>(g, row, lrow, a0, b0, nh, acc);
+        if (g.steep) ss_adj_angle<true, false, false, Q == 1, BOTH>(g, row, lrow, a0, b0, nh, acc);
+        else ss_adj_angle<false, false, false, Q == 1, BOTH>(g, row, lrow, a0, b0, nh, acc);
       }
     }
     if (marked)
@@ -296,6 +319,40 @@ __global__ void __launch_bounds__(32 * Q, (Q == 1 ? 0 : Q == 4 ? 28 : 32) / Q) s
             for (int j = 0; j < 4; ++j)
               acc[i][j] = ss_adj_raw(acc[i][j], tab + u, pairs + (z * na + u) * (size_t)w2 + pads, lim + (size_t)u * 2 * nh,
                                      a0 + i, b0 + j, nh);
+  }
+  // the columns nh - 1 and nh + 1 of the tile for steep angles, a pixel a lane; the
+  // rows for the others
+  const int X0 = blockIdx.x * 32, Y0 = by * 16;
+  const bool midx = X0 <= nh + 1 && X0 + 31 >= nh - 1, midy = Y0 <= nh + 1 && Y0 + 15 >= nh - 1;
+  if (Q > 1 && !BOTH && (midx || midy)) {
+    float cc = 0.0f, r0 = 0.0f, r1 = 0.0f;
+    const int R = Y0 + (lane & 15), side = lane < 16 ? -1 : 1, C = X0 + lane;
+#pragma unroll 2
+    for (int u = q; u < na; u += Q) {
+      if (marked && __ldg(raw + z * na + u)) continue;
+      const SsAngle g = tab[u];
+      const float2 *row = pairs + (z * na + u) * (size_t)w2 + pads;
+      const int2 *lrow = lim + (size_t)u * 2 * nh;
+      const bool nr = fabsf(g.rb) * near < 1.0f, limits = edge || nr;
+      if (g.steep) {
+        if (midx) cc += ss_centre(g, row, lrow, R - nh, side, nh, limits, nr);
+      } else if (midy) {
+        r0 += ss_centre(g, row, lrow, C - nh, -1, nh, limits, nr);
+        r1 += ss_centre(g, row, lrow, C - nh, 1, nh, limits, nr);
+      }
+    }
+    centre[q][0][lane] = cc;
+    centre[q][1][lane] = r0;
+    centre[q][2][lane] = r1;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int x = b0 + j - nh, y = a0 + i - nh;
+        if (x == -1 || x == 1) acc[i][j] += centre[q][0][(a0 + i - Y0) + (x > 0 ? 16 : 0)];
+        if (y == -1 || y == 1) acc[i][j] += centre[q][y > 0 ? 2 : 1][b0 + j - X0];
+      }
   }
   if (q > 0)
 #pragma unroll
@@ -320,11 +377,17 @@ __global__ void __launch_bounds__(32 * Q, (Q == 1 ? 0 : Q == 4 ? 28 : 32) / Q) s
     }
 }
 
-// Warps of an adjoint tile.  ms with 4, 8, 16: 256^2 x 300 0.118, 0.077, 0.058; 512^2 x 500
+// Warps of an adjoint tile.  ms (without the centre's part) with 4, 8, 16: 256^2 x 300 0.118, 0.077, 0.058; 512^2 x 500
 // 0.271, 0.255, 0.222; 768^2 x 720 0.558, 0.536, 0.486; 1280^2 x 1024 1.69, 1.66, 1.62; 1600^2 x
 // 1400 3.32, 3.33, 3.30; 2048^2 x 1800 6.72, 6.78, 6.75; also for several slices (4 x 641^2 x
 // 600: 1.23, 1.21, 1.16).
 int ss_adj_warps(int n) { return n > 1800 ? 4 : 16; }
+
+// Both forms of the weight in the main loop (BOTH) or the centre's columns and rows
+// afterwards, whose few pixels in a row of angles make long chains in small images: ms
+// 128^2 x 120 0.034, 0.036; 256^2 x 300 0.060, 0.069; 384^2 x 400 0.134, 0.142; 448^2 x 450 0.183,
+// 0.173; 768^2 x 720 0.527, 0.499; 1280^2 x 1024 1.74, 1.61.
+bool ss_adj_both(int n) { return n <= 384; }
 
 struct SsState {
   float2 *pairs = nullptr;                 // [chunk][na][w2]
@@ -429,7 +492,8 @@ int ss_adjoint(Plan &p, const float *d_sino, float *d_img, cudaStream_t s, const
   const int n = p.g.n, na = p.g.na, nz = p.g.nz;
   SsState &st = *(SsState *)p.ext;
   const int Q = ep.ordered ? 1 : ss_adj_warps(n);
-  auto fn = Q == 1 ? ss_adjoint_kernel<1> : Q == 4 ? ss_adjoint_kernel<4> : ss_adjoint_kernel<16>;
+  auto fn = Q == 1 ? ss_adjoint_kernel<1, false> : Q == 4 ? ss_adjoint_kernel<4, false>
+            : ss_adj_both(n) ? ss_adjoint_kernel<16, true> : ss_adjoint_kernel<16, false>;
   const size_t per = (size_t)n * n, per_sino = (size_t)na * n;
   for (int z0 = 0; z0 < nz; z0 += st.chunk) {
     const int zc = std::min(st.chunk, nz - z0);

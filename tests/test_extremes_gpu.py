@@ -67,6 +67,20 @@ def test_infinite_values_at_zero_weights(cuda, oracle, oper, n):
         _compare(cuda, tp.At, ref, y)
 
 
+@pytest.mark.parametrize("n", [32, 33, 384, 385, 1900])
+def test_ss_small_weights_at_the_centre(cuda, oracle, n):
+    """Next to the centre a crossing has bits below those of the pixel's coordinate: a single bin
+    of 1 gives every pixel its weight, each right to 9 x 2^-24 of itself however small."""
+    deg = np.concatenate([np.linspace(3.1, 87.3, 9), np.linspace(92.2, 148.7, 6)])
+    tp, orc = _pair("ss", n, deg, oracle)
+    for b in (n // 2 - 1, n // 2, n // 2 + 1):
+        y = np.zeros((len(deg), n), np.float32)
+        for v in range(0, len(deg), 1 if n < 100 else 4):
+            y[:] = 0.0
+            y[v, b] = 1.0
+            assert _compare(cuda, tp.At, orc(1, y), y).all()
+
+
 def _bspline(n, oracle):
     from iterative_tomographic_reconstruction_algorithms_b200 import class_projectors_bspline as cpb
     tp = cpb.projectors(n, np.arange(24))  # 0, 45, 90 and 135 degrees among them
