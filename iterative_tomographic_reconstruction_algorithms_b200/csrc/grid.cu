@@ -139,8 +139,10 @@ __device__ __forceinline__ void fft_pass(const float2 *a, float2 *b, int N, int 
       float2 e[4], d[4];
       dft4<2>(v, e);
       dft4<2>(v + 1, d);
-      const float2 w[4] = {d[0], make_float2(c8 * (d[1].x + d[1].y), c8 * (d[1].y - d[1].x)),
-                           make_float2(d[2].y, -d[2].x), make_float2(c8 * (d[3].y - d[3].x), -c8 * (d[3].x + d[3].y))};
+      // multiplied before they are added: the sums may pass the largest float where the results do not
+      const float2 s1 = make_float2(c8 * d[1].x, c8 * d[1].y), s3 = make_float2(c8 * d[3].x, c8 * d[3].y);
+      const float2 w[4] = {d[0], make_float2(fmaf(c8, d[1].x, s1.y), fmaf(c8, d[1].y, -s1.x)),
+                           make_float2(d[2].y, -d[2].x), make_float2(fmaf(c8, d[3].y, -s3.x), -fmaf(c8, d[3].x, s3.y))};
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         o[k] = make_float2(e[k].x + w[k].x, e[k].y + w[k].y);

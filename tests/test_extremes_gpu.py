@@ -136,3 +136,24 @@ def test_bspline_table_that_is_not_finite(cuda, oracle):
     plan = _lib.Plan(_lib.KIND_BSPLINE, n, tp.angles, lut=lut, lut_size=lut.shape[1], support=float(tp.param_spline[1]))
     got = plan.forward(cuda.from_numpy(x[None]).cuda()).cpu().numpy()[0]
     assert np.array_equal(np.isnan(got), np.isnan(ref))
+
+
+@pytest.mark.parametrize("n", [41, 251, 600])
+def test_grid_adjoint_next_to_the_largest_float(cuda, n):
+    """A sum of the 1-D transform that passes the largest float makes NaN of the whole slice in the 2-D
+    one: its butterflies add no more than the results do.  (The unnormalised 2-D transform may
+    still pass it at single pixels, as the reference's does.)  Elsewhere the pixels are those of
+    2^-60 of the value, times 2^60: powers of two round nothing, and the FFTs' log2(pdim) = 11 rounds
+    and windows of 25 products stay within 1e-5 of the largest entry."""
+    torch = cuda
+    from iterative_tomographic_reconstruction_algorithms_b200 import class_projectors_grid as cpg
+    tp = cpg.projectors(n, np.array([3.0, 31.0, 77.0, 118.0, 162.0]), verbose=False)
+    lim = float(np.finfo(np.float32).max)
+    for v, b in ((0, n // 2), (2, n // 3), (3, n - 7)):
+        y = np.zeros((5, n), np.float32)
+        y[v, b] = BIG
+        small = tp.At(torch.from_numpy(y * np.float32(2.0 ** -60)).cuda()).cpu().numpy().astype(np.float64) * 2.0 ** 60
+        got = tp.At(torch.from_numpy(y).cuda()).cpu().numpy().astype(np.float64)
+        inside = np.isfinite(got) & (np.abs(small) < lim)
+        assert inside.sum() > 0.9 * n * n
+        assert np.abs(got[inside] - small[inside]).max() <= 1e-5 * np.abs(small[inside]).max()
